@@ -397,175 +397,6 @@ moe_down_stream_kernel(const T* __restrict__ hidden, const T* __restrict__ down,
     }
 }
 
-// ---------------------------------------------------------------- many tokens: pairs grouped by expert, tensor cores
-// Pairs sorted by expert: offsets[e] .. offsets[e + 1] are the places of expert e's pairs in `sorted` (pairs whose
-// expert is no expert are left out).  One block; the order of an expert's pairs among themselves is whatever the
-// shared-memory counters give, which changes no result: every pair's row is computed by itself.
-__global__ void moe_sort_kernel(const int* __restrict__ chosen, int pairs, int experts, int* __restrict__ offsets, int* __restrict__ sorted) {
-    extern __shared__ int counters[];   // experts counts, then experts cursors
-    int* cursors = counters + experts;
-    for (int e = threadIdx.x; e < experts; e += blockDim.x) counters[e] = 0;
-    __syncthreads();
-    for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
-        const int e = chosen[p];
-        if (e >= 0 && e < experts) atomicAdd(&counters[e], 1);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int total = 0;
-        for (int e = 0; e < experts; ++e) {
-            offsets[e] = total;
-            cursors[e] = total;
-            total += counters[e];
-        }
-        offsets[experts] = total;
-    }
-    __syncthreads();
-    for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
-        const int e = chosen[p];
-        if (e >= 0 && e < experts) sorted[atomicAdd(&cursors[e], 1)] = p;
-    }
-}
-
-__device__ __forceinline__ void moe_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-
-__device__ __forceinline__ void moe_copy_16(void* shared_destination, const void* global_source, bool real) {
-    if (real) {
-        const uint32_t destination = static_cast<uint32_t>(__cvta_generic_to_shared(shared_destination));
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(destination), "l"(global_source) : "memory");
-    } else {
-        *reinterpret_cast<uint4*>(shared_destination) = make_uint4(0u, 0u, 0u, 0u);
-    }
-}
-
-constexpr int kGroupedM = 64, kGroupedN = 64, kGroupedK = 32, kGroupedPitch = kGroupedK + 8;   // bfloat16 elements; the pitch keeps fragment reads apart
-
-// One tile of 64 sorted pairs of one expert times 64 output columns, K in steps of 32 through two stages of
-// cp.async.  grid (tiles at most, column tiles); four warps of 16 rows each.
-//   MODE 1 (gated):  A = x rows gathered by the pairs' tokens [.., K = width], B = gate[e] and up[e] [N = ff][K];
-//           hidden[place, n] = T(act(A . gate[n]) * (A . up[n]))
-//   MODE 2 (no gate):  A as above, B = up[e];   hidden[place, n] = T(act(A . up[n]))
-//   MODE 0 (down):   A = hidden[place] [K = ff], B = down[e] [N = width][K];   out[pair, n] = A . down[n]  (32-bit)
-template <int MODE>
-__global__ void __launch_bounds__(128)
-moe_grouped_kernel(const __nv_bfloat16* __restrict__ a_base, const __nv_bfloat16* __restrict__ b_first, const __nv_bfloat16* __restrict__ b_second,
-                   const int* __restrict__ offsets, const int* __restrict__ sorted, __nv_bfloat16* __restrict__ hidden_out, float* __restrict__ pair_out,
-                   int experts, int top, int n_total, int k_total, int activation, float limit, const float* __restrict__ pair_weight) {
-    constexpr bool GATED = MODE == 1, UP = MODE != 0;   // UP: rows gathered by token, hidden values out
-    __shared__ __align__(16) __nv_bfloat16 a_s[2][kGroupedM][kGroupedPitch];
-    __shared__ __align__(16) __nv_bfloat16 b_s[GATED ? 2 : 1][2][kGroupedN][kGroupedPitch];
-    __shared__ int row_source[kGroupedM];   // GATED: the token of the row's pair; else: the pair itself; -1 past the expert's pairs
-    __shared__ int tile_info[3];            // expert, first place, rows
-    if (threadIdx.x == 0) {
-        int expert = -1, first = 0, rows = 0, seen = 0;
-        for (int e = 0; e < experts; ++e) {
-            const int begin = offsets[e], count = offsets[e + 1] - begin;
-            const int tiles = (count + kGroupedM - 1) / kGroupedM;
-            if (static_cast<int>(blockIdx.x) < seen + tiles) {
-                expert = e;
-                first = begin + (static_cast<int>(blockIdx.x) - seen) * kGroupedM;
-                rows = min(kGroupedM, begin + count - first);
-                break;
-            }
-            seen += tiles;
-        }
-        tile_info[0] = expert, tile_info[1] = first, tile_info[2] = rows;
-    }
-    __syncthreads();
-    const int expert = tile_info[0], first = tile_info[1], rows = tile_info[2];
-    if (expert < 0) return;
-    if (threadIdx.x < kGroupedM) {
-        const int pair = static_cast<int>(threadIdx.x) < rows ? sorted[first + threadIdx.x] : -1;
-        row_source[threadIdx.x] = pair < 0 ? -1 : (UP ? pair / top : pair);
-    }
-    __syncthreads();
-    const int n0 = blockIdx.y * kGroupedN;
-    const size_t b_expert = static_cast<size_t>(expert) * n_total * k_total;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-
-    auto load_stage = [&](int stage, int k0) {
-        // 64 rows x 4 chunks of 16 bytes per operand: two chunks a thread
-        for (int index = threadIdx.x; index < kGroupedM * 4; index += 128) {
-            const int row = index >> 2, chunk = index & 3, k = k0 + 8 * chunk;
-            const bool in_k = k < k_total;
-            const int source = row_source[row];
-            const size_t a_row = UP ? static_cast<size_t>(source < 0 ? 0 : source) : static_cast<size_t>(first + row);
-            moe_copy_16(&a_s[stage][row][8 * chunk], a_base + a_row * k_total + k, in_k && source >= 0);
-            const bool in_n = n0 + row < n_total;
-            const size_t b_row = b_expert + static_cast<size_t>(in_n ? n0 + row : 0) * k_total + k;
-            moe_copy_16(&b_s[0][stage][row][8 * chunk], b_first + b_row, in_k && in_n);
-            if constexpr (GATED) moe_copy_16(&b_s[1][stage][row][8 * chunk], b_second + b_row, in_k && in_n);
-        }
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-    };
-
-    float acc[GATED ? 2 : 1][kGroupedN / 8][4];
-#pragma unroll
-    for (int which = 0; which < (GATED ? 2 : 1); ++which)
-#pragma unroll
-        for (int j = 0; j < kGroupedN / 8; ++j) acc[which][j][0] = acc[which][j][1] = acc[which][j][2] = acc[which][j][3] = 0.0f;
-
-    const int k_steps = (k_total + kGroupedK - 1) / kGroupedK;
-    load_stage(0, 0);
-    for (int step = 0; step < k_steps; ++step) {
-        const int stage = step & 1;
-        if (step + 1 < k_steps) {
-            load_stage(stage ^ 1, (step + 1) * kGroupedK);
-            asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < kGroupedK; kk += 16) {
-            uint32_t a[4];
-            a[0] = *reinterpret_cast<const uint32_t*>(&a_s[stage][16 * warp + g][kk + 2 * t]);
-            a[1] = *reinterpret_cast<const uint32_t*>(&a_s[stage][16 * warp + g + 8][kk + 2 * t]);
-            a[2] = *reinterpret_cast<const uint32_t*>(&a_s[stage][16 * warp + g][kk + 2 * t + 8]);
-            a[3] = *reinterpret_cast<const uint32_t*>(&a_s[stage][16 * warp + g + 8][kk + 2 * t + 8]);
-#pragma unroll
-            for (int which = 0; which < (GATED ? 2 : 1); ++which) {
-#pragma unroll
-                for (int j = 0; j < kGroupedN / 8; ++j) {
-                    const uint32_t b0 = *reinterpret_cast<const uint32_t*>(&b_s[which][stage][8 * j + g][kk + 2 * t]);
-                    const uint32_t b1 = *reinterpret_cast<const uint32_t*>(&b_s[which][stage][8 * j + g][kk + 2 * t + 8]);
-                    moe_mma(acc[which][j], a, b0, b1);
-                }
-            }
-        }
-        __syncthreads();   // the stage is refilled in the turn after the next
-    }
-    // c[0], c[1]: row g, columns 2t and 2t + 1 of the 8-column tile; c[2], c[3]: row g + 8
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
-        const int row = 16 * warp + g + 8 * half;
-        if (row >= rows) continue;
-        const float factor = UP && pair_weight != nullptr ? pair_weight[sorted[first + row]] : 1.0f;
-#pragma unroll
-        for (int j = 0; j < kGroupedN / 8; ++j) {
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int n = n0 + 8 * j + 2 * t + e;
-                if (n >= n_total) continue;
-                if constexpr (GATED) {
-                    using T = __nv_bfloat16;
-                    const float gate_value = acc[0][j][2 * half + e] * factor, up_value = acc[1][j][2 * half + e] * factor;
-                    hidden_out[static_cast<size_t>(first + row) * n_total + n] = from_float<T>(moe_hidden<T>(gate_value, up_value, activation, limit));
-                } else if constexpr (UP) {
-                    using T = __nv_bfloat16;
-                    hidden_out[static_cast<size_t>(first + row) * n_total + n] = from_float<T>(moe_plain_hidden<T>(acc[0][j][2 * half + e] * factor, activation));
-                } else {
-                    pair_out[static_cast<size_t>(row_source[row]) * n_total + n] = acc[0][j][2 * half + e];
-                }
-            }
-        }
-    }
-}
-
 }  // namespace lb
 
 extern "C" {
@@ -647,29 +478,6 @@ int lb_moe_expert_stream_wide(const void* x, const void* gate, const void* up, c
                                                                                 pair_weight);
         second<<<down_grid, 32 * lb::kStreamWarps, ff * sizeof(float), stream>>>(static_cast<const T*>(hidden), static_cast<const T*>(down), chosen, out, width, ff, experts);
     })
-    return LB_LAUNCH_RESULT();
-}
-
-// The grouped path (bfloat16; width and ff multiples of 8; at most 1024 experts): sorts the pairs by expert into
-// `offsets` [experts + 1] and `sorted` [pairs], then the two grouped products.  `hidden` is [pairs, ff] (rows in sorted
-// order), `out` [pairs, width] in 32-bit (rows in pair order; rows of pairs without an expert are not written).
-int lb_moe_experts_grouped(const void* x, const void* gate, const void* up, const void* down, const int* chosen, int* offsets, int* sorted, void* hidden,
-                           float* out, int pairs, int top, int width, int ff, int experts, int activation, cudaStream_t stream, float limit, const float* pair_weight) {
-    if (pairs == 0) return 0;
-    if (width % 8 != 0 || ff % 8 != 0 || experts < 1 || experts > 1024) return -2;
-    lb::moe_sort_kernel<<<1, 1024, 2 * experts * sizeof(int), stream>>>(chosen, pairs, experts, offsets, sorted);
-    const int tiles = (pairs + lb::kGroupedM - 1) / lb::kGroupedM + experts;   // no fewer than the experts' tiles together
-    const auto* x16 = static_cast<const __nv_bfloat16*>(x);
-    if (gate != nullptr)
-        lb::moe_grouped_kernel<1><<<dim3(tiles, (ff + lb::kGroupedN - 1) / lb::kGroupedN), 128, 0, stream>>>(
-            x16, static_cast<const __nv_bfloat16*>(gate), static_cast<const __nv_bfloat16*>(up), offsets, sorted, static_cast<__nv_bfloat16*>(hidden), nullptr, experts,
-            top, ff, width, activation, limit, pair_weight);
-    else
-        lb::moe_grouped_kernel<2><<<dim3(tiles, (ff + lb::kGroupedN - 1) / lb::kGroupedN), 128, 0, stream>>>(
-            x16, static_cast<const __nv_bfloat16*>(up), nullptr, offsets, sorted, static_cast<__nv_bfloat16*>(hidden), nullptr, experts, top, ff, width, activation,
-            limit, pair_weight);
-    lb::moe_grouped_kernel<0><<<dim3(tiles, (width + lb::kGroupedN - 1) / lb::kGroupedN), 128, 0, stream>>>(
-        static_cast<const __nv_bfloat16*>(hidden), static_cast<const __nv_bfloat16*>(down), nullptr, offsets, sorted, nullptr, out, experts, top, width, ff, activation, limit, nullptr);
     return LB_LAUNCH_RESULT();
 }
 

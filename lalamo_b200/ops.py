@@ -1603,20 +1603,25 @@ def moe_route(x: torch.Tensor, router: torch.Tensor, *, top: int, group_count: i
     return chosen, weights
 
 
-MOE_STREAM_MAX_PAIRS = 32  # up to this many (token, expert) pairs each pair streams its expert's weights; more are grouped by expert (measured: 24 pairs 30 % faster streamed, 48 pairs as fast either way)
+# Up to this many (token, expert) pairs each pair streams its expert's weights; more are grouped by expert.  Measured over both products, cold caches: 16 pairs of
+# 2048 x 2048 experts 85 us streamed, 92 grouped, 32 pairs 132 and 97; of 1024 x 1152 experts 16 pairs 48 and 51, 32 pairs 52 and 50.
+MOE_STREAM_MAX_PAIRS = 16
 
 
 def moe_experts(x: torch.Tensor, gate: "torch.Tensor | None", up: torch.Tensor, down: torch.Tensor, chosen: torch.Tensor, weights: torch.Tensor,
                 activation: str = "silu", path: str | None = None, limit: float = 0.0, combine: bool = True,
-                weigh_input: bool = False) -> "torch.Tensor | ExpertSum":
+                weigh_input: bool = False, status: torch.Tensor | None = None) -> "torch.Tensor | ExpertSum":
     """``out[t] = sum_k weights[t, k] * down[e] (act(gate[e] x[t]) * (up[e] x[t]))`` with ``e = chosen[t, k]``;
     ``gate`` and ``up`` are ``[experts, ff, width]``, ``down`` ``[experts, width, ff]``.  The weighted sum is
     32-bit, in the order of ``k``; a pair whose expert is no expert counts nothing.  ``path`` forces one of the
     three ways the pairs' products are computed (``"grouped"``, ``"stream"``, ``"plain"``); left out, the sizes
     choose.  ``combine=False`` leaves the weighted sum to the consumer (an :class:`ExpertSum`).  ``gate=None``: experts
     without a gate, ``down[e] act(up[e] x[t])`` (the activation in 32-bit on the 32-bit sums, rounded once).  ``weigh_input``: a weight
-    multiplies its expert's input, not its output, ``sum_k expert_e(weights[t, k] x[t])`` (the 32-bit sums ``gate[e] x`` and ``up[e] x`` are multiplied)."""
+    multiplies its expert's input, not its output, ``sum_k expert_e(weights[t, k] x[t])`` (the 32-bit sums ``gate[e] x`` and ``up[e] x`` are multiplied).
+    ``status``: the int32 word in which the grouped products report a wait that gave up."""
     _check(x, "x")
+    if status is not None:
+        _check(status, "status", torch.int32)
     input_weight = weights if weigh_input else None
     for name, tensor in (("gate", gate), ("up", up), ("down", down)):
         if tensor is not None:
@@ -1640,15 +1645,19 @@ def moe_experts(x: torch.Tensor, gate: "torch.Tensor | None", up: torch.Tensor, 
     if path is None:
         path = "grouped" if x.dtype == torch.bfloat16 and wide_rows and experts <= 1024 and pairs > MOE_STREAM_MAX_PAIRS else "stream" if wide_rows else "plain"
     if path == "grouped":
-        # many pairs: sorted by expert, 64 at a time on the tensor cores, every expert's weights read once per 64 pairs
+        # many pairs: sorted by expert, 128 at a time on the tensor cores
         if not (x.dtype == torch.bfloat16 and wide_rows and experts <= 1024):
             raise KernelError("moe_experts: the grouped kernels take bfloat16, rows of 16-byte multiples and at most 1024 experts")
         offsets = torch.empty(experts + 1, dtype=torch.int32, device=x.device)
         order = torch.empty(pairs, dtype=torch.int32, device=x.device)
+        gathered = torch.empty(pairs, width, dtype=x.dtype, device=x.device)
         hidden = torch.empty(pairs, ff, dtype=x.dtype, device=x.device)
-        code = lib.lb_moe_experts_grouped(_ptr(x), _ptr(gate), _ptr(up), _ptr(down), _ptr(chosen), _ptr(offsets), _ptr(order), _ptr(hidden), _ptr(pair_out),
-                                          c_int(pairs), c_int(top), c_int(width), c_int(ff), c_int(experts), c_int(_ACTIVATIONS[activation]), _stream(), c_float(limit), _ptr(input_weight))
-        _done(code, "moe_experts_grouped", 3)
+        code = lib.lb_moe_experts_grouped(_ptr(x), _ptr(gate), _ptr(up), _ptr(down), _ptr(chosen), _ptr(offsets), _ptr(order), _ptr(gathered), _ptr(hidden), _ptr(pair_out),
+                                          c_int(pairs), c_int(top), c_int(width), c_int(ff), c_int(experts), c_int(_ACTIVATIONS[activation]), _stream(), c_float(limit), _ptr(input_weight),
+                                          _ptr(status))
+        if code == -5:
+            raise KernelError("moe_experts: the driver gave no tensor map (cuTensorMapEncodeTiled)")
+        _done(code, "moe_experts_grouped", 4)
     elif path == "stream":
         # few pairs: each streams its expert's rows, 16 bytes a lane, the rows shared out over many blocks
         if not wide_rows:

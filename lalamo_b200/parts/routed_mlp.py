@@ -79,7 +79,7 @@ class RoutedMLP(FeedForward):
         shared_gate = routing[2] if spec.shared_gate else None
         # with a shared feed-forward the consumer adds two terms anyway: the experts' weighted sum is left to it as well
         routed = ops.moe_experts(x, self.gate, self.up, self.down, chosen, weights, spec.activation, limit=spec.limit,
-                                 combine=self.shared is None and residual is None and not defer, weigh_input=spec.weigh_input)
+                                 combine=self.shared is None and residual is None and not defer, weigh_input=spec.weigh_input, status=self.runtime.status)
         everyone = None
         if self.shared is not None:
             if defer and residual is None and shared_gate is not None and self.shared.can_defer:

@@ -1,0 +1,44 @@
+"""The grouped experts' products where tiles end: experts without a pair, with one, with a row more or less than a box of 32 or a
+tile of 128; matrices whose rows and columns end inside a tile; pairs whose expert is no expert."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("gated,weigh", [(True, False), (True, True), (False, False)])
+@pytest.mark.parametrize("counts,width,ff", [((0, 1, 31, 33, 0, 127), 72, 40), ((129, 128, 0, 257), 256, 264), ((5, 0, 3), 1032, 136), ((700, 9), 64, 520)])
+def test_ragged_experts(counts, width, ff, gated, weigh):
+    from lalamo_b200 import ops
+
+    generator = torch.Generator().manual_seed(sum(counts))
+    experts, missing = len(counts), 4   # four pairs more whose expert is none
+    chosen = torch.cat([torch.full((n,), e) for e, n in enumerate(counts)] + [torch.tensor([-1, experts, -1, experts + 7])])
+    chosen = chosen[torch.randperm(chosen.numel(), generator=generator)]
+    if chosen.numel() % 2:
+        chosen = torch.cat([chosen, torch.tensor([-1])])
+    chosen = chosen.view(-1, 2).to(torch.int32)
+    tokens = chosen.shape[0]
+    assert tokens * 2 >= sum(counts) + missing
+    random = lambda *shape: torch.randn(*shape, generator=generator)  # noqa: E731
+    x = random(tokens, width).bfloat16()
+    gate, up, down = (random(experts, *shape).mul(shape[1] ** -0.5).bfloat16() for shape in ((ff, width), (ff, width), (width, ff)))
+    weights = torch.rand(tokens, 2, generator=generator) + 0.5
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    got = ops.moe_experts(x.cuda(), gate.cuda() if gated else None, up.cuda(), down.cuda(), chosen.cuda(), weights.cuda(), "silu" if gated else "gelu", path="grouped",
+                          weigh_input=weigh, status=status).double().cpu()
+    want = torch.zeros(tokens, width, dtype=torch.float64)
+    for t in range(tokens):
+        for k in range(2):
+            e = int(chosen[t, k])
+            if not 0 <= e < experts:
+                continue
+            before, after = (weights[t, k].double(), 1.0) if weigh else (1.0, weights[t, k].double())
+            u = up[e].double() @ x[t].double() * before
+            hidden = torch.nn.functional.silu(gate[e].double() @ x[t].double() * before) * u if gated else torch.nn.functional.gelu(u)
+            want[t] += after * (down[e].double() @ hidden)
+    # Rounded to bfloat16 on the way: both sides, the activated gate, the hidden value, the result, each by at most 2**-9 of itself
+    # and in no common direction: sqrt(5) * 2**-9 of the norm at the most.
+    assert float((got - want).norm() / want.norm()) < 5 ** 0.5 * 2 ** -9
+    assert int(status.item()) == 0
