@@ -19,8 +19,9 @@ __device__ __forceinline__ void warp_argmax(float& value, int& index) {
     }
 }
 
-// One warp per token or, with `block_per_token`, one block per token whose warps share out the experts' logits (few
-// tokens: more loads on their way at once), the first warp choosing afterwards.  A logit's sum is the same either way.
+// A block takes TT tokens: its warps share out the experts' logits (EPW experts at a time, for all of the block's tokens, so that a
+// router row is loaded once for TT tokens), then the tokens.  Every lane adds the same products in the same order whatever TT
+// and EPW are, so a token's logits do not depend on the step it is in.
 //   z[e] = x . router[e] (+ bias[e])  (32-bit);   s[e] = sigmoid(z[e])   (score_kind 0),  softmax(z)[e]   (score_kind 1)  or  z[e]  (score_kind 2)
 //   experts form `group_count` equal groups of neighbours; a group's score is the sum of its two largest s (of its
 //   only one, in groups of one), or with `group_top` 1 its largest s; experts outside the best `group_keep` groups cannot be chosen;
@@ -29,155 +30,176 @@ __device__ __forceinline__ void warp_argmax(float& value, int& index) {
 //   `choice_bias` (may be null): experts (and groups) are ranked by s[e] + choice_bias[e]; the weights stay the s themselves.
 //   `extra` further rows of `router` after the experts' are gates of something every token runs: extra_out[t, x] =
 //   sigmoid(x_t . router[experts + x]), 32-bit like the scores.
-// Shared memory per warp: s[experts], candidates[experts], group score[group_count], and the token's row in 32-bit where it is staged.
-template <typename T>
-__global__ void moe_route_kernel(const T* __restrict__ x, const float* __restrict__ router, int* __restrict__ chosen, float* __restrict__ weights,
-                                 int tokens, int width, int experts, int top, int group_count, int group_keep, int score_kind, int renormalize,
-                                 float weight_scale, int row_floats, int group_floats, const float* __restrict__ bias, int block_per_token,
-                                 const float* __restrict__ choice_bias, int extra, float* __restrict__ extra_out, int group_top) {
+// Shared memory per token: s[experts], candidates[experts], group score[group_count], and the token's row in 32-bit where it is staged.
+// Few tokens are bound by the latency of the router's loads (hence 16 warps of one expert each, all of a row's loads on their way at
+// once), many by the loads themselves (hence 8 tokens a load).  Measured, 16 experts and rows of
+// 2,048: 8 tokens 9.6 us (20.6 with four warps a token, four experts each), 2,048 tokens 20.7 us (48.5 with one token a warp).
+template <typename T, int TT, int EPW>
+__global__ void __launch_bounds__(TT == 1 ? 512 : 256)
+moe_route_kernel(const T* __restrict__ x, const float* __restrict__ router, int* __restrict__ chosen, float* __restrict__ weights,
+                 int tokens, int width, int experts, int top, int group_count, int group_keep, int score_kind, int renormalize,
+                 float weight_scale, int row_floats, int group_floats, const float* __restrict__ bias,
+                 const float* __restrict__ choice_bias, int extra, float* __restrict__ extra_out, int group_top) {
     extern __shared__ __align__(16) float shared[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-    const int token = block_per_token ? blockIdx.x : blockIdx.x * warps + warp;
-    if (token >= tokens) return;
-    const int sharers = block_per_token ? warps : 1, share = block_per_token ? warp : 0;   // the logits of experts 4 (share + i sharers) .. + 3 are this warp's
+    const int token0 = blockIdx.x * TT, tokens_here = min(TT, tokens - token0);
     const int logits = experts + extra;   // rows of the router
-    float* scores = shared + static_cast<size_t>(block_per_token ? 0 : warp) * (experts + logits + group_floats + row_floats);   // a multiple of 4 floats per warp
-    float* candidates = scores + logits;
-    float* group_score = candidates + experts;   // group_floats >= group_count of them
-    float* x_s = group_score + group_floats;   // row_floats = width (rounded up to a multiple of 4) if the row is staged, else 0
-    const T* row = x + static_cast<size_t>(token) * width;
+    const int pitch = experts + logits + group_floats;   // floats of a token's scratch, a multiple of 4
+    float* rows_s = shared + TT * pitch;   // row_floats = width (a multiple of 4) a token if the rows are staged, else 0
     if (row_floats > 0) {
-        // the token's row once into shared memory (32-bit), then four experts' rows at a time, 16 bytes a lane and turn
-        if (block_per_token) {
-            for (int d = threadIdx.x; d < width; d += blockDim.x) x_s[d] = to_float(row[d]);
-            __syncthreads();
-        } else {
+        // the tokens' rows once into shared memory (32-bit, four elements a thread and turn), then EPW experts' rows at a time, 16
+        // bytes a lane and turn
+        const T* rows = x + static_cast<size_t>(token0) * width;
 #pragma unroll 8
-            for (int d = lane; d < width; d += 32) x_s[d] = to_float(row[d]);
-            __syncwarp();
+        for (int d = 4 * threadIdx.x; d < tokens_here * width; d += 4 * blockDim.x) {
+            if constexpr (sizeof(T) == 4) {
+                *reinterpret_cast<float4*>(rows_s + d) = *reinterpret_cast<const float4*>(rows + d);
+            } else {
+                const uint2 raw = *reinterpret_cast<const uint2*>(rows + d);
+                const float2 low = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162&>(raw.x)), high = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162&>(raw.y));
+                *reinterpret_cast<float4*>(rows_s + d) = make_float4(low.x, low.y, high.x, high.y);
+            }
         }
-        for (int e0 = 4 * share; e0 < logits; e0 += 4 * sharers) {
-            float dots[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll 4
-            for (int c = 4 * lane; c < width; c += 128) {   // sixteen loads of the router's rows on their way at a time
-                const float4 xv = *reinterpret_cast<const float4*>(x_s + c);
+        __syncthreads();
+        for (int e0 = EPW * warp; e0 < logits; e0 += EPW * warps) {
+            float dots[TT][EPW];
 #pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    const float4 w = *reinterpret_cast<const float4*>(router + static_cast<size_t>(e0 + r < logits ? e0 + r : e0) * width + c);
-                    dots[r] += xv.x * w.x;
-                    dots[r] += xv.y * w.y;
-                    dots[r] += xv.z * w.z;
-                    dots[r] += xv.w * w.w;
+            for (int t = 0; t < TT; ++t)
+#pragma unroll
+                for (int r = 0; r < EPW; ++r) dots[t][r] = 0.0f;
+#pragma unroll (16 / EPW)
+            for (int c = 4 * lane; c < width; c += 128) {   // sixteen loads of the router's rows on their way at a time
+                float4 w[EPW];
+#pragma unroll
+                for (int r = 0; r < EPW; ++r) w[r] = *reinterpret_cast<const float4*>(router + static_cast<size_t>(e0 + r < logits ? e0 + r : e0) * width + c);
+#pragma unroll
+                for (int t = 0; t < TT; ++t) {
+                    const float4 xv = *reinterpret_cast<const float4*>(rows_s + (t < tokens_here ? t : 0) * row_floats + c);
+#pragma unroll
+                    for (int r = 0; r < EPW; ++r) {
+                        dots[t][r] += xv.x * w[r].x;
+                        dots[t][r] += xv.y * w[r].y;
+                        dots[t][r] += xv.z * w[r].z;
+                        dots[t][r] += xv.w * w[r].w;
+                    }
                 }
             }
 #pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const float dot = warp_sum(dots[r]);
-                if (lane == 0 && e0 + r < logits) scores[e0 + r] = dot;
+            for (int t = 0; t < TT; ++t) {
+#pragma unroll
+                for (int r = 0; r < EPW; ++r) {
+                    const float dot = warp_sum(dots[t][r]);
+                    if (lane == 0 && e0 + r < logits) shared[t * pitch + e0 + r] = dot;
+                }
             }
         }
     } else {
-        for (int e = share; e < logits; e += sharers) {
-            const float* w = router + static_cast<size_t>(e) * width;
-            float dot = 0.0f;
-            for (int d = lane; d < width; d += 32) dot += to_float(row[d]) * w[d];
-            dot = warp_sum(dot);
-            if (lane == 0) scores[e] = dot;
+        for (int t = 0; t < tokens_here; ++t) {
+            const T* row = x + static_cast<size_t>(token0 + t) * width;
+            for (int e = warp; e < logits; e += warps) {
+                const float* w = router + static_cast<size_t>(e) * width;
+                float dot = 0.0f;
+                for (int d = lane; d < width; d += 32) dot += to_float(row[d]) * w[d];
+                dot = warp_sum(dot);
+                if (lane == 0) shared[t * pitch + e] = dot;
+            }
         }
     }
-    if (block_per_token) {
-        __syncthreads();
-        if (warp != 0) return;
-    }
-    __syncwarp();
-    for (int x = lane; x < extra; x += 32) extra_out[static_cast<size_t>(token) * extra + x] = 1.0f / (1.0f + expf(-scores[experts + x]));
-    if (bias != nullptr) {
-        for (int e = lane; e < experts; e += 32) scores[e] += bias[e];
+    __syncthreads();
+    for (int t = warp; t < tokens_here; t += warps) {
+        const int token = token0 + t;
+        float* scores = shared + t * pitch;
+        float* candidates = scores + logits;
+        float* group_score = candidates + experts;   // group_floats >= group_count of them
+        for (int x = lane; x < extra; x += 32) extra_out[static_cast<size_t>(token) * extra + x] = 1.0f / (1.0f + expf(-scores[experts + x]));
+        if (bias != nullptr) {
+            for (int e = lane; e < experts; e += 32) scores[e] += bias[e];
+            __syncwarp();
+        }
+        if (score_kind == 2) {
+            // the logits themselves rank the experts
+        } else if (score_kind == 1) {
+            float largest = -INFINITY;
+            for (int e = lane; e < experts; e += 32) largest = fmaxf(largest, scores[e]);
+            largest = warp_max(largest);
+            float total = 0.0f;
+            for (int e = lane; e < experts; e += 32) total += expf(scores[e] - largest);
+            total = warp_sum(total);
+            for (int e = lane; e < experts; e += 32) scores[e] = expf(scores[e] - largest) / total;
+        } else {
+            for (int e = lane; e < experts; e += 32) scores[e] = 1.0f / (1.0f + expf(-scores[e]));
+        }
         __syncwarp();
-    }
-    if (score_kind == 2) {
-        // the logits themselves rank the experts
-    } else if (score_kind == 1) {
-        float largest = -INFINITY;
-        for (int e = lane; e < experts; e += 32) largest = fmaxf(largest, scores[e]);
-        largest = warp_max(largest);
-        float total = 0.0f;
-        for (int e = lane; e < experts; e += 32) total += expf(scores[e] - largest);
-        total = warp_sum(total);
-        for (int e = lane; e < experts; e += 32) scores[e] = expf(scores[e] - largest) / total;
-    } else {
-        for (int e = lane; e < experts; e += 32) scores[e] = 1.0f / (1.0f + expf(-scores[e]));
-    }
-    __syncwarp();
-    const int members = experts / group_count;
-    for (int group = lane; group < group_count; group += 32) {
-        float first = -INFINITY, second = -INFINITY;
-        for (int m = 0; m < members; ++m) {
-            const float s = scores[group * members + m] + (choice_bias != nullptr ? choice_bias[group * members + m] : 0.0f);
-            if (s > first) {
-                second = first;
-                first = s;
-            } else if (s > second) {
-                second = s;
-            }
-        }
-        group_score[group] = members >= 2 && group_top != 1 ? first + second : first;
-    }
-    for (int e = lane; e < experts; e += 32) candidates[e] = -INFINITY;
-    __syncwarp();
-    for (int round = 0; round < group_keep; ++round) {
-        float best = -INFINITY;
-        int best_group = 0x7fffffff;
+        const int members = experts / group_count;
         for (int group = lane; group < group_count; group += 32) {
-            const float s = group_score[group];
-            if (s > best) {   // ascending scan: the lowest index among equals stays
-                best = s;
-                best_group = group;
+            float first = -INFINITY, second = -INFINITY;
+            for (int m = 0; m < members; ++m) {
+                const float s = scores[group * members + m] + (choice_bias != nullptr ? choice_bias[group * members + m] : 0.0f);
+                if (s > first) {
+                    second = first;
+                    first = s;
+                } else if (s > second) {
+                    second = s;
+                }
             }
+            group_score[group] = members >= 2 && group_top != 1 ? first + second : first;
         }
-        warp_argmax(best, best_group);
-        if (best_group == 0x7fffffff) break;
-        for (int m = lane; m < members; m += 32)
-            candidates[best_group * members + m] = scores[best_group * members + m] + (choice_bias != nullptr ? choice_bias[best_group * members + m] : 0.0f);
-        if (lane == 0) group_score[best_group] = -INFINITY;
+        for (int e = lane; e < experts; e += 32) candidates[e] = -INFINITY;
         __syncwarp();
-    }
-    float total = 0.0f;
-    for (int round = 0; round < top; ++round) {
-        float best = -INFINITY;
-        int best_expert = 0x7fffffff;
-        for (int e = lane; e < experts; e += 32) {
-            const float s = candidates[e];
-            if (s > best) {
-                best = s;
-                best_expert = e;
+        for (int round = 0; round < group_keep; ++round) {
+            float best = -INFINITY;
+            int best_group = 0x7fffffff;
+            for (int group = lane; group < group_count; group += 32) {
+                const float s = group_score[group];
+                if (s > best) {   // ascending scan: the lowest index among equals stays
+                    best = s;
+                    best_group = group;
+                }
             }
+            warp_argmax(best, best_group);
+            if (best_group == 0x7fffffff) break;
+            for (int m = lane; m < members; m += 32)
+                candidates[best_group * members + m] = scores[best_group * members + m] + (choice_bias != nullptr ? choice_bias[best_group * members + m] : 0.0f);
+            if (lane == 0) group_score[best_group] = -INFINITY;
+            __syncwarp();
         }
-        warp_argmax(best, best_expert);
-        if (best_expert == 0x7fffffff) best_expert = 0, best = 0.0f;   // fewer eligible experts than `top`: a weight of zero
-        else if (choice_bias != nullptr) best = scores[best_expert];   // ranked with the bias, weighed without it
-        total += best;
-        if (lane == 0) {
-            chosen[static_cast<size_t>(token) * top + round] = best_expert;
-            weights[static_cast<size_t>(token) * top + round] = best;
-            if (best_expert < experts) candidates[best_expert] = -INFINITY;
-        }
-        __syncwarp();
-    }
-    if (lane == 0 && renormalize == 2) {
-        // the softmax over the chosen scores only (the first chosen is the largest)
-        float* mine = weights + static_cast<size_t>(token) * top;
-        const float largest = mine[0];
-        float sum = 0.0f;
+        float total = 0.0f;
         for (int round = 0; round < top; ++round) {
-            mine[round] = expf(mine[round] - largest);
-            sum += mine[round];
+            float best = -INFINITY;
+            int best_expert = 0x7fffffff;
+            for (int e = lane; e < experts; e += 32) {
+                const float s = candidates[e];
+                if (s > best) {
+                    best = s;
+                    best_expert = e;
+                }
+            }
+            warp_argmax(best, best_expert);
+            if (best_expert == 0x7fffffff) best_expert = 0, best = 0.0f;   // fewer eligible experts than `top`: a weight of zero
+            else if (choice_bias != nullptr) best = scores[best_expert];   // ranked with the bias, weighed without it
+            total += best;
+            if (lane == 0) {
+                chosen[static_cast<size_t>(token) * top + round] = best_expert;
+                weights[static_cast<size_t>(token) * top + round] = best;
+                if (best_expert < experts) candidates[best_expert] = -INFINITY;
+            }
+            __syncwarp();
         }
-        for (int round = 0; round < top; ++round) mine[round] = mine[round] / sum * weight_scale;
-    } else if (lane == 0) {
-        const float factor = (renormalize && total > 0.0f ? 1.0f / total : 1.0f) * weight_scale;
-        if (factor != 1.0f)
-            for (int round = 0; round < top; ++round) weights[static_cast<size_t>(token) * top + round] *= factor;
+        if (lane == 0 && renormalize == 2) {
+            // the softmax over the chosen scores only (the first chosen is the largest)
+            float* mine = weights + static_cast<size_t>(token) * top;
+            const float largest = mine[0];
+            float sum = 0.0f;
+            for (int round = 0; round < top; ++round) {
+                mine[round] = expf(mine[round] - largest);
+                sum += mine[round];
+            }
+            for (int round = 0; round < top; ++round) mine[round] = mine[round] / sum * weight_scale;
+        } else if (lane == 0) {
+            const float factor = (renormalize && total > 0.0f ? 1.0f / total : 1.0f) * weight_scale;
+            if (factor != 1.0f)
+                for (int round = 0; round < top; ++round) weights[static_cast<size_t>(token) * top + round] *= factor;
+        }
     }
 }
 
@@ -408,21 +430,23 @@ int lb_moe_route(const void* x, const float* router, int* chosen, float* weights
     if (tokens == 0) return 0;
     if (experts < 1 || top < 1 || top > experts || group_count < 1 || experts % group_count != 0 || group_keep < 1 || group_keep > group_count) return -2;
     if (extra < 0 || (extra > 0 && extra_out == nullptr) || group_top < 1 || group_top > 2) return -2;
-    constexpr int kWarps = 4;
-    // A warp's scratch: scores, candidates, group scores (padded so that the staged row starts on 16 bytes), and the row.
+    // A token's scratch: scores, candidates, group scores (padded so that the staged row starts on 16 bytes), and the row.
     const int scratch = (2 * experts + extra + group_count + 3) / 4 * 4;
-    if (static_cast<size_t>(kWarps) * scratch * sizeof(float) > 48 * 1024) return -2;
-    int row_floats = width % 4 == 0 ? width : 0;   // rows of 16-byte multiples are staged and read 16 bytes a lane
-    if (static_cast<size_t>(kWarps) * (scratch + row_floats) * sizeof(float) > 160 * 1024) row_floats = 0;
-    const size_t shared = static_cast<size_t>(kWarps) * (scratch + row_floats) * sizeof(float);
-    const int block_per_token = tokens <= 512 ? 1 : 0;   // few tokens: a block's warps share out a token's experts
+    if (4 * static_cast<size_t>(scratch) * sizeof(float) > 48 * 1024) return -2;
+    int row_floats = width % 4 == 0 && reinterpret_cast<uintptr_t>(x) % (dtype == lb::kBFloat16 ? 8 : 16) == 0 ? width : 0;   // rows that start on 16 bytes (8, in bfloat16) are staged and read 16 bytes a lane
+    if (4 * static_cast<size_t>(scratch + row_floats) * sizeof(float) > 160 * 1024) row_floats = 0;   // by the sizes alone, not by the tokens (see the kernel)
     const int padded_groups = scratch - 2 * experts - extra;   // the kernel lays the three arrays out by these counts
+    // Tokens a block: one while that leaves the multiprocessors no more than two blocks each, then 2, 4, 8 (four times as many fit).
+    const int sms = lb::multiprocessor_count();
+    int per_block = tokens <= 2 * sms ? 1 : tokens <= 4 * sms ? 2 : tokens <= 8 * sms ? 4 : 8;
+    if (per_block == 8 && 8 * static_cast<size_t>(scratch + row_floats) * sizeof(float) > 160 * 1024) per_block = 4;
+    const size_t shared = per_block * static_cast<size_t>(scratch + row_floats) * sizeof(float);
     LB_DISPATCH_DTYPE(dtype, {
-        auto kernel = lb::moe_route_kernel<T>;
+        auto kernel = per_block == 1 ? lb::moe_route_kernel<T, 1, 1> : per_block == 2 ? lb::moe_route_kernel<T, 2, 2> : per_block == 4 ? lb::moe_route_kernel<T, 4, 2> : lb::moe_route_kernel<T, 8, 2>;
         if (shared > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(shared));
-        kernel<<<block_per_token ? tokens : (tokens + kWarps - 1) / kWarps, 32 * kWarps, shared, stream>>>(
+        kernel<<<(tokens + per_block - 1) / per_block, per_block == 1 ? 512 : 256, shared, stream>>>(
             static_cast<const T*>(x), router, chosen, weights, tokens, width, experts, top, group_count, group_keep, score_kind, renormalize, weight_scale,
-            row_floats, padded_groups, bias, block_per_token, choice_bias, extra, extra_out, group_top);
+            row_floats, padded_groups, bias, choice_bias, extra, extra_out, group_top);
     })
     return LB_LAUNCH_RESULT();
 }

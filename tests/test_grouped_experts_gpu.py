@@ -42,3 +42,22 @@ def test_ragged_experts(counts, width, ff, gated, weigh):
     # and in no common direction: sqrt(5) * 2**-9 of the norm at the most.
     assert float((got - want).norm() / want.norm()) < 5 ** 0.5 * 2 ** -9
     assert int(status.item()) == 0
+
+
+@pytest.mark.parametrize("tokens", [1, 297, 593, 1187])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_router_at_every_number_of_tokens_a_block(tokens, dtype):
+    """One, two, four and eight tokens a block (the last block partly filled), an odd number of router rows."""
+    from lalamo_b200 import ops
+
+    generator = torch.Generator().manual_seed(tokens)
+    x, router = torch.randn(tokens, 516, generator=generator).to(dtype), torch.randn(11, 516, generator=generator) * 0.05
+    chosen, weights, gates = ops.moe_route(x.cuda(), router.cuda(), top=3, extra=1)
+    logits = x.double() @ router.double().T
+    scores = torch.sigmoid(logits[:, :10])
+    want = torch.gather(scores, 1, chosen.long().cpu())
+    # a lane adds 20 products at the most, then five sums are added: 25 roundings of the products' sizes (together below 20), the
+    # sigmoid's slope a quarter; and the sigmoid's own roundings
+    bound = 25 * 2 ** -24 * 20 / 4 + 4 * 2 ** -24
+    assert float((weights.double().cpu() - want).abs().max()) < bound and float((gates.double().cpu() - torch.sigmoid(logits[:, 10:])).abs().max()) < bound
+    assert float((scores.topk(3).values - want).abs().max()) < 2 * bound   # the best ones, but for ties within the rounding
