@@ -5,8 +5,8 @@
 // with S a [key_dim, value_dim] matrix per request and head, kept in 32-bit in the request's state
 // slot.  Four kernels: `prepare` (short causal convolutions with silu over q, k and v, unit q and k,
 // beta and the decays, all in 32-bit), `conv_state` (the convolutions' last inputs into the slot),
-// `scan` (the recurrence, token by token) and `output` (per-head RMS norm times a sigmoid gate).
-// The order of every sum depends on the token's place in its request only, never on how the
+// `scan` (the recurrence, token by token; long portions go through recurrent_blocks.cu instead) and `output` (per-head RMS norm
+// times a sigmoid gate).  The order of every sum depends on the token's place in its request only, never on how the
 // request was cut into steps or on what else is in the batch.
 #include "common.cuh"
 
@@ -184,9 +184,8 @@ __global__ void __launch_bounds__((kScanCols / kScanThreadCols) * SPLIT)
 gdr_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ g, const float* __restrict__ v,
                 const float* __restrict__ beta, float* __restrict__ state, float* __restrict__ out, const int* __restrict__ segment_start,
                 const int* __restrict__ segment_length, const int* __restrict__ segment_slot, int heads, int groups, int dk, int dv,
-                int num_slots, int* status, const int* __restrict__ segment_list, int v_columns, int from_zero) {
-    // from_zero: the state starts at zero (the slot is only written).  segment_list (may be null): the portions this launch runs.  v_columns <= dv: the columns `v` really has (rows of
-    // heads x v_columns); the columns past them get zeros as values (they carry a transition matrix, see the chunked path).
+                int num_slots, int* status, const int* __restrict__ segment_list) {
+    // segment_list (may be null): the portions this launch runs.
     constexpr int R = kScanThreadRows, C = kScanThreadCols;
     static_assert(DKP == R * SPLIT && SPLIT <= 32, "a column's rows lie in one warp");
     using Shared = ScanShared<DKP>;
@@ -219,7 +218,7 @@ gdr_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, const 
     }
     for (int index = tid; index < 2 * kBatch * kScanCols; index += blockDim.x) {
         const int stage = index / (kBatch * kScanCols), rest = index - stage * kBatch * kScanCols;
-        if (col0 + rest % kScanCols >= v_columns) v_of(stage)[rest] = 0.0f;
+        if (col0 + rest % kScanCols >= dv) v_of(stage)[rest] = 0.0f;
     }
     const bool wide = dk % 4 == 0;   // rows of 16-byte multiples (the buffers are 16-byte aligned)
     auto fetch = [&](int stage, int t0) {
@@ -242,10 +241,10 @@ gdr_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, const 
                 scan_copy_4(g_of(stage) + tt * DKP + c, g + (token * heads + head) * dk + c);
             }
         }
-        const int columns = min(kScanCols, v_columns - col0);
+        const int columns = min(kScanCols, dv - col0);
         for (int index = tid; index < n * columns; index += blockDim.x) {
             const int tt = index / columns, c = index - tt * columns;
-            scan_copy_4(v_of(stage) + tt * kScanCols + c, v + (static_cast<size_t>(start + t0 + tt) * heads + head) * v_columns + col0 + c);
+            scan_copy_4(v_of(stage) + tt * kScanCols + c, v + (static_cast<size_t>(start + t0 + tt) * heads + head) * dv + col0 + c);
         }
         if constexpr (DELTA)
             for (int tt = tid; tt < n; tt += blockDim.x) scan_copy_4(beta_of(stage) + tt, beta + static_cast<size_t>(start + t0 + tt) * heads + head);
@@ -258,7 +257,7 @@ gdr_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, const 
     for (int i = 0; i < R; ++i) {
         const int row = ((i >> 2) * SPLIT + part) * 4 + (i & 3);
 #pragma unroll
-        for (int c = 0; c < C; ++c) S[c][i] = (row < dk && column + c < dv && !from_zero) ? S_base[static_cast<size_t>(row) * dv + column + c] : 0.0f;
+        for (int c = 0; c < C; ++c) S[c][i] = (row < dk && column + c < dv) ? S_base[static_cast<size_t>(row) * dv + column + c] : 0.0f;
     }
     int stage = 0;
     for (int t0 = 0; t0 < length; t0 += kBatch, stage ^= 1) {
@@ -368,181 +367,20 @@ __global__ void gdr_output_kernel(const float* __restrict__ o, const T* __restri
     }
 }
 
-// ------------------------------------------------------------------------------------ long portions in chunks
-// The recurrence is linear in the state: S_t = M_t S_{t-1} + k_t (beta_t v_t)^T with M_t = (I - beta_t k_t k_t^T) diag(g_t).
-// A long portion is cut into chunks that the scan above runs side by side, each from a zero state and, in dk further
-// columns that start as the identity and take zeros as values, the chunk's transition P_t = M_t ... M_1; the scan's
-// read-out of those columns is P_t^T q_t.  With S_in the state at a chunk's start,
-//   S_t = S0_t + P_t S_in    and    o_t = o0_t + (P_t^T q_t)^T S_in,
-// so one short pass over a portion's chunks in order gives every chunk's S_in (and the portion's last state), and one
-// pass over the tokens adds the second term to the read-outs.  All in 32-bit.
-
-// state[chunk, head] (dk x (dv + dk)) = [0 | I].  One block per (chunk, head).
-__global__ void gdr_chunk_init_kernel(float* __restrict__ chunk_state, int dk, int dv) {
-    const int width = dv + dk;
-    float* S = chunk_state + static_cast<size_t>(blockIdx.x) * dk * width;
-    for (int index = threadIdx.x; index < dk * width; index += blockDim.x) {
-        const int row = index / width, col = index - row * width;
-        S[index] = col == dv + row ? 1.0f : 0.0f;
-    }
-}
-
-// grid (long portions, heads, ceil(dv / 32)), block (32, 32): thread (j, y) holds the rows y, y + 32, ... of column j of
-// S_in.  long_table rows: (portion, first chunk, chunks).  For each chunk in order: S_in is written to chunk_in[chunk]
-// (dk x dv per head), then S_in <- S0_L + P_L S_in, with P_L staged in shared memory where it fits (p_in_shared).  The
-// last S_in goes to the portion's state slot, from which the first was read.
-constexpr int kPropagateRows = 8;   // dk <= 256
-__global__ void __launch_bounds__(1024)
-gdr_chunk_propagate_kernel(const float* __restrict__ chunk_state, float* __restrict__ chunk_in, float* __restrict__ state,
-                           const int* __restrict__ long_table, const int* __restrict__ segment_slot, int heads, int dk, int dv, int num_slots,
-                           int p_in_shared) {
-    extern __shared__ float propagate_memory[];
-    float* s_in = propagate_memory;          // dk x 32
-    float* p_s = propagate_memory + dk * 32;   // dk x (dk + 1) if p_in_shared
-    const int portion = long_table[3 * blockIdx.x], first_chunk = long_table[3 * blockIdx.x + 1], chunks = long_table[3 * blockIdx.x + 2];
-    const int head = blockIdx.y, j = threadIdx.x, column = blockIdx.z * 32 + j, y = threadIdx.y;
-    const int slot = segment_slot[portion];
-    if (slot < 0 || slot >= num_slots) return;   // reported by the kernels before
-    const bool live = column < dv;
-    const int width = dv + dk, pitch = dk + 1;
-    float* S_slot = state + (static_cast<size_t>(slot) * heads + head) * dk * dv;
-    float mine[kPropagateRows];
-#pragma unroll
-    for (int r = 0; r < kPropagateRows; ++r) {
-        const int row = y + 32 * r;
-        mine[r] = (live && row < dk) ? S_slot[static_cast<size_t>(row) * dv + column] : 0.0f;
-    }
-    for (int c = 0; c < chunks; ++c) {
-        const size_t chunk_head = static_cast<size_t>(first_chunk + c) * heads + head;
-        float* in_tile = chunk_in + chunk_head * dk * dv;
-        const float* S_end = chunk_state + chunk_head * dk * width;   // [S0_L | P_L]
-        __syncthreads();   // the turn before has read s_in and p_s
-#pragma unroll
-        for (int r = 0; r < kPropagateRows; ++r) {
-            const int row = y + 32 * r;
-            if (row < dk) {
-                s_in[row * 32 + j] = mine[r];
-                if (live) in_tile[static_cast<size_t>(row) * dv + column] = mine[r];
-            }
-        }
-        if (p_in_shared) {
-            for (int index = y * 32 + j; index < dk * dk; index += 1024) {
-                const int row = index / dk, m = index - row * dk;
-                p_s[row * pitch + m] = S_end[static_cast<size_t>(row) * width + dv + m];
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int r = 0; r < kPropagateRows; ++r) {
-            const int row = y + 32 * r;
-            if (row < dk) {
-                const float* p_row = p_in_shared ? p_s + row * pitch : S_end + static_cast<size_t>(row) * width + dv;
-                float sums[4] = {live ? S_end[static_cast<size_t>(row) * width + column] : 0.0f, 0.0f, 0.0f, 0.0f};
-                int m = 0;
-                for (; m + 4 <= dk; m += 4) {
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) sums[e] += p_row[m + e] * s_in[(m + e) * 32 + j];
-                }
-                for (; m < dk; ++m) sums[0] += p_row[m] * s_in[m * 32 + j];
-                mine[r] = (sums[0] + sums[1]) + (sums[2] + sums[3]);
-            }
-        }
-    }
-#pragma unroll
-    for (int r = 0; r < kPropagateRows; ++r) {
-        const int row = y + 32 * r;
-        if (live && row < dk) S_slot[static_cast<size_t>(row) * dv + column] = mine[r];
-    }
-}
-
-// grid (chunks x tiles of 16 tokens, heads): out[t, h, j] = base[t, h, j] + sum_m turned[t, h, m] * chunk_in[chunk, h, m, j]
-// for the tile's tokens, which share what is read of chunk_in.  `base` (which may be `out`) and `turned` have rows of their own pitch per
-// token and head.  decay (may be null): one number per head; `turned` then counts decay^(i + 1) times at the chunk's token i.
-constexpr int kReadoutTokens = 16;
-__global__ void gdr_chunk_readout_kernel(const float* base, int base_pitch, const float* __restrict__ turned, int turned_pitch, const float* __restrict__ decay,
-                                         const float* __restrict__ chunk_in, const int* __restrict__ chunk_start, const int* __restrict__ chunk_length,
-                                         int tiles_per_chunk, float* out, int heads, int dk, int dv) {
-    extern __shared__ __align__(16) float r_s[];   // dk x 16: the tokens' values of one m side by side (zeros past the tile's end)
-    const int chunk = blockIdx.x / tiles_per_chunk, tile = blockIdx.x - chunk * tiles_per_chunk, head = blockIdx.y;
-    const int first = kReadoutTokens * tile, count = min(kReadoutTokens, chunk_length[chunk] - first);
-    if (count <= 0) return;
-    const int token0 = chunk_start[chunk] + first;
-    const float log_decay = decay != nullptr ? log2f(decay[head]) : 0.0f;
-    for (int index = threadIdx.x; index < kReadoutTokens * dk; index += blockDim.x) {
-        const int tt = index / dk, m = index - tt * dk;
-        float r = 0.0f;
-        if (tt < count) {
-            r = turned[(static_cast<size_t>(token0 + tt) * heads + head) * turned_pitch + m];
-            if (decay != nullptr) r *= exp2f(log_decay * static_cast<float>(first + tt + 1));
-        }
-        r_s[m * kReadoutTokens + tt] = r;
-    }
-    __syncthreads();
-    const float* S_in = chunk_in + (static_cast<size_t>(chunk) * heads + head) * dk * dv;
-    for (int j = threadIdx.x; j < dv; j += blockDim.x) {
-        float sums[kReadoutTokens];
-#pragma unroll
-        for (int tt = 0; tt < kReadoutTokens; ++tt) sums[tt] = tt < count ? base[(static_cast<size_t>(token0 + tt) * heads + head) * base_pitch + j] : 0.0f;
-#pragma unroll 4
-        for (int m = 0; m < dk; ++m) {   // four loads of S_in on their way at a time
-            const float s = S_in[static_cast<size_t>(m) * dv + j];
-            const float4* r4 = reinterpret_cast<const float4*>(r_s + m * kReadoutTokens);
-#pragma unroll
-            for (int quad = 0; quad < kReadoutTokens / 4; ++quad) {
-                const float4 r = r4[quad];
-                sums[4 * quad] += r.x * s;
-                sums[4 * quad + 1] += r.y * s;
-                sums[4 * quad + 2] += r.z * s;
-                sums[4 * quad + 3] += r.w * s;
-            }
-        }
-#pragma unroll
-        for (int tt = 0; tt < kReadoutTokens; ++tt)
-            if (tt < count) out[(static_cast<size_t>(token0 + tt) * heads + head) * dv + j] = sums[tt];
-    }
-}
-
-// One fixed decay a per head, no correction: a chunk of L tokens turns S_in into a^L S_in + S0_L, element by element, so chunks need no
-// further columns.  grid (long portions, heads, pieces of dk * dv), threads over the elements; tables as above, chunk_state [chunks, heads, dk, dv].
-__global__ void retention_chunk_propagate_kernel(const float* __restrict__ chunk_state, float* __restrict__ chunk_in, float* __restrict__ state,
-                                                 const int* __restrict__ long_table, const int* __restrict__ segment_slot, const int* __restrict__ chunk_length,
-                                                 const float* __restrict__ decay, int heads, int elements, int num_slots) {
-    const int portion = long_table[3 * blockIdx.x], first_chunk = long_table[3 * blockIdx.x + 1], chunks = long_table[3 * blockIdx.x + 2];
-    const int head = blockIdx.y, element = blockIdx.z * blockDim.x + threadIdx.x, slot = segment_slot[portion];
-    if (slot < 0 || slot >= num_slots || element >= elements) return;   // (a bad slot is reported by the host's checks and the scan)
-    const float log_decay = log2f(decay[head]);
-    float* mine = state + (static_cast<size_t>(slot) * heads + head) * elements + element;
-    float s = *mine;
-    for (int c0 = 0; c0 < chunks; c0 += 8) {   // eight chunks' loads on their way at a time
-        float end[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u)
-            if (c0 + u < chunks) end[u] = chunk_state[(static_cast<size_t>(first_chunk + c0 + u) * heads + head) * elements + element];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            if (c0 + u < chunks) {
-                chunk_in[(static_cast<size_t>(first_chunk + c0 + u) * heads + head) * elements + element] = s;
-                s = exp2f(log_decay * static_cast<float>(chunk_length[first_chunk + c0 + u])) * s + end[u];
-            }
-        }
-    }
-    *mine = s;
-}
-
 template <int DKP, int SPLIT>
 inline void launch_scan(dim3 grid, cudaStream_t stream, const float* q, const float* k, const float* g, const float* v, const float* beta,
                         float* state, float* out, const int* segment_start, const int* segment_length, const int* segment_slot, int heads,
-                        int groups, int dk, int dv, int num_slots, int* status, const int* segment_list, int v_columns, int from_zero) {
+                        int groups, int dk, int dv, int num_slots, int* status, const int* segment_list) {
     if (beta != nullptr) {
         static OncePerDevice once;
         allow_shared_memory(once, gdr_scan_kernel<DKP, SPLIT, true>, static_cast<int>(ScanShared<DKP>::kBytes));
         gdr_scan_kernel<DKP, SPLIT, true><<<grid, (kScanCols / kScanThreadCols) * SPLIT, ScanShared<DKP>::kBytes, stream>>>(
-            q, k, g, v, beta, state, out, segment_start, segment_length, segment_slot, heads, groups, dk, dv, num_slots, status, segment_list, v_columns, from_zero);
+            q, k, g, v, beta, state, out, segment_start, segment_length, segment_slot, heads, groups, dk, dv, num_slots, status, segment_list);
     } else {
         static OncePerDevice once;
         allow_shared_memory(once, gdr_scan_kernel<DKP, SPLIT, false>, static_cast<int>(ScanShared<DKP>::kBytes));
         gdr_scan_kernel<DKP, SPLIT, false><<<grid, (kScanCols / kScanThreadCols) * SPLIT, ScanShared<DKP>::kBytes, stream>>>(
-            q, k, g, v, beta, state, out, segment_start, segment_length, segment_slot, heads, groups, dk, dv, num_slots, status, segment_list, v_columns, from_zero);
+            q, k, g, v, beta, state, out, segment_start, segment_length, segment_slot, heads, groups, dk, dv, num_slots, status, segment_list);
     }
 }
 
@@ -584,69 +422,22 @@ int lb_gdr_conv_state(const void* proj, int proj_width, void* conv_state, const 
     return LB_LAUNCH_RESULT();
 }
 
-// segment_list (may be null): the portions to run, `segments` of them.  v_columns: the columns `v` has (0: dv).  from_zero: states start at
-// zero and are only written.
+// segment_list (may be null): the portions to run, `segments` of them.
 // beta null: the plain linear recurrence (no delta rule).
 int lb_gdr_scan(const float* q, const float* k, const float* g, const float* v, const float* beta, float* state, float* out,
                 const int* segment_start, const int* segment_length, const int* segment_slot, int segments, int heads, int groups, int dk, int dv,
-                int num_slots, int* status, cudaStream_t stream, const int* segment_list, int v_columns, int from_zero) {
+                int num_slots, int* status, cudaStream_t stream, const int* segment_list) {
     if (segments == 0) return 0;
-    if (v_columns <= 0) v_columns = dv;
-    if (dk < 1 || dk > 256 || dv < 1 || heads % groups != 0 || v_columns > dv) return -2;
+    if (dk < 1 || dk > 256 || dv < 1 || heads % groups != 0) return -2;
     const dim3 grid(segments, heads, (dv + lb::kScanCols - 1) / lb::kScanCols);
     if (dk <= 32)
-        lb::launch_scan<32, 4>(grid, stream, q, k, g, v, beta, state, out, segment_start, segment_length, segment_slot, heads, groups, dk, dv, num_slots, status, segment_list, v_columns, from_zero);
+        lb::launch_scan<32, 4>(grid, stream, q, k, g, v, beta, state, out, segment_start, segment_length, segment_slot, heads, groups, dk, dv, num_slots, status, segment_list);
     else if (dk <= 64)
-        lb::launch_scan<64, 8>(grid, stream, q, k, g, v, beta, state, out, segment_start, segment_length, segment_slot, heads, groups, dk, dv, num_slots, status, segment_list, v_columns, from_zero);
+        lb::launch_scan<64, 8>(grid, stream, q, k, g, v, beta, state, out, segment_start, segment_length, segment_slot, heads, groups, dk, dv, num_slots, status, segment_list);
     else if (dk <= 128)
-        lb::launch_scan<128, 16>(grid, stream, q, k, g, v, beta, state, out, segment_start, segment_length, segment_slot, heads, groups, dk, dv, num_slots, status, segment_list, v_columns, from_zero);
+        lb::launch_scan<128, 16>(grid, stream, q, k, g, v, beta, state, out, segment_start, segment_length, segment_slot, heads, groups, dk, dv, num_slots, status, segment_list);
     else
-        lb::launch_scan<256, 32>(grid, stream, q, k, g, v, beta, state, out, segment_start, segment_length, segment_slot, heads, groups, dk, dv, num_slots, status, segment_list, v_columns, from_zero);
-    return LB_LAUNCH_RESULT();
-}
-
-// The passes around the chunks' scan (which is lb_gdr_scan over the chunk tables with dv + dk columns): `chunk_state`
-// [chunks, heads, dk, dv + dk] is set to [0 | I] by lb_gdr_chunk_init before the scan; after it lb_gdr_chunk_finish gives every
-// chunk its incoming state (`chunk_in` [chunks, heads, dk, dv]), the portions' slots their last state, and the tokens
-// of chunks their read-out (`wide` [tokens, heads, dv + dk] is what the scan wrote; `out` [tokens, heads, dv]).
-int lb_gdr_chunk_init(float* chunk_state, int chunks, int heads, int dk, int dv, cudaStream_t stream) {
-    if (chunks == 0) return 0;
-    lb::gdr_chunk_init_kernel<<<chunks * heads, 256, 0, stream>>>(chunk_state, dk, dv);
-    return LB_LAUNCH_RESULT();
-}
-
-int lb_gdr_chunk_finish(const float* chunk_state, float* chunk_in, float* state, const float* wide, float* out, const int* long_table, int long_portions,
-                        const int* segment_slot, const int* chunk_start, const int* chunk_length, int chunks, int chunk_tokens, int heads, int dk, int dv,
-                        int num_slots, cudaStream_t stream) {
-    if (long_portions == 0 || chunks == 0) return 0;
-    if (dk > 32 * lb::kPropagateRows || chunk_tokens < 1) return -2;
-    size_t shared = static_cast<size_t>(dk) * 32 * sizeof(float);
-    const size_t with_p = shared + static_cast<size_t>(dk) * (dk + 1) * sizeof(float);
-    const int p_in_shared = with_p <= 160 * 1024 ? 1 : 0;
-    if (p_in_shared) shared = with_p;
-    static lb::OncePerDevice once;
-    lb::allow_shared_memory(once, lb::gdr_chunk_propagate_kernel, 160 * 1024);
-    lb::gdr_chunk_propagate_kernel<<<dim3(long_portions, heads, (dv + 31) / 32), dim3(32, 32), shared, stream>>>(
-        chunk_state, chunk_in, state, long_table, segment_slot, heads, dk, dv, num_slots, p_in_shared);
-    const int tiles_per_chunk = (chunk_tokens + lb::kReadoutTokens - 1) / lb::kReadoutTokens;
-    lb::gdr_chunk_readout_kernel<<<dim3(chunks * tiles_per_chunk, heads), 128, static_cast<size_t>(lb::kReadoutTokens) * dk * sizeof(float), stream>>>(
-        wide, dv + dk, wide + dv, dv + dk, nullptr, chunk_in, chunk_start, chunk_length, tiles_per_chunk, out, heads, dk, dv);
-    return LB_LAUNCH_RESULT();
-}
-
-// The same for one fixed decay per head (see retention_chunk_propagate_kernel): `chunk_state` [chunks, heads, dk, dv] is what the scan over the
-// chunk tables left from zero states; `out` [tokens, heads, dv] holds the chunks' own read-outs and gets what came in; q [tokens, heads, dk].
-int lb_retention_chunk_finish(const float* chunk_state, float* chunk_in, float* state, const float* q, const float* decay, float* out, const int* long_table,
-                              int long_portions, const int* segment_slot, const int* chunk_start, const int* chunk_length, int chunks, int chunk_tokens, int heads,
-                              int dk, int dv, int num_slots, cudaStream_t stream) {
-    if (long_portions == 0 || chunks == 0) return 0;
-    if (dk < 1 || dk > 256 || dv < 1 || chunk_tokens < 1) return -2;
-    const int elements = dk * dv;
-    lb::retention_chunk_propagate_kernel<<<dim3(long_portions, heads, (elements + 255) / 256), 256, 0, stream>>>(chunk_state, chunk_in, state, long_table, segment_slot,
-                                                                                                             chunk_length, decay, heads, elements, num_slots);
-    const int tiles_per_chunk = (chunk_tokens + lb::kReadoutTokens - 1) / lb::kReadoutTokens;
-    lb::gdr_chunk_readout_kernel<<<dim3(chunks * tiles_per_chunk, heads), 128, static_cast<size_t>(lb::kReadoutTokens) * dk * sizeof(float), stream>>>(
-        out, dv, q, dk, decay, chunk_in, chunk_start, chunk_length, tiles_per_chunk, out, heads, dk, dv);
+        lb::launch_scan<256, 32>(grid, stream, q, k, g, v, beta, state, out, segment_start, segment_length, segment_slot, heads, groups, dk, dv, num_slots, status, segment_list);
     return LB_LAUNCH_RESULT();
 }
 

@@ -1175,24 +1175,17 @@ def short_conv(
 
 
 # ---------------------------------------------------------------------- gated delta rule
-GDR_CHUNK_TOKENS = 256  # long portions are scanned in chunks of this many tokens, side by side
-GDR_LONG_PORTION = 768  # portions of at least this many tokens count as long
-RETENTION_CHUNK_TOKENS = 128  # the same where the decay is one fixed number per head: chunks cost less there
-RETENTION_LONG_PORTION = 384
-
-
-def gated_delta_chunks_pay(key_dim: int, value_dim: int) -> bool:
-    """Whether long portions should run as chunks: a chunk's scan carries ``key_dim`` further columns beside the
-    ``value_dim`` of the state, and the chunks' states are put together in order afterwards.  Measured on 2,048-token
-    portions: 64 x 128 heads 0.36 against 0.56 ms a layer, 128 x 128 heads 0.93 against 0.69 ms."""
-    return 2 * key_dim <= value_dim
+RECURRENT_BLOCK = 32  # tokens that the kernels for long portions of a recurrence take at a time
+GDR_CHUNK_TOKENS = RECURRENT_BLOCK  # long portions are cut into chunks of this many tokens
+# Portions of at least this many tokens count as long; shorter ones are scanned token by token.  One portion of 8 heads, scan against blocks: delta rule, 128 x 128,
+# 64 tokens 28.7 and 33.8 us, 128 tokens 49 and 38, 2,048 tokens 672 and 157; linear, 64 x 128, 64 tokens 20.5 and 33.8, 128 tokens 35 and 35, 2,048 tokens 428 and 75.
+GDR_LONG_PORTION = 112
 
 
 def gated_delta_chunk_plan(starts, lengths, chunk_tokens: int = GDR_CHUNK_TOKENS, long_portion: int = GDR_LONG_PORTION) -> dict:
-    """The host's part of the chunked gated delta rule, from the portions' first rows and lengths alone: ``direct``
-    (the portions scanned whole), ``chunk_start`` / ``chunk_length`` / ``chunk_slot`` (the chunks of the long portions,
-    each with a temporary state of its own) and ``long_table`` (per long portion: its index, its first chunk, its number of
-    chunks).  NumPy int32 arrays."""
+    """The host's part of the recurrences over long portions, from the portions' first rows and lengths alone: ``direct``
+    (the portions scanned token by token), ``chunk_start`` / ``chunk_length`` / ``chunk_slot`` (the chunks of the long portions, numbered
+    through) and ``long_table`` (per long portion: its index, its first chunk, its number of chunks).  NumPy int32 arrays."""
     import numpy as np
 
     direct, chunk_start, chunk_length, long_table = [], [], [], []
@@ -1209,6 +1202,38 @@ def gated_delta_chunk_plan(starts, lengths, chunk_tokens: int = GDR_CHUNK_TOKENS
     as_array = lambda values: np.asarray(values, dtype=np.int32).reshape(-1)
     return {"direct": as_array(direct), "chunk_start": as_array(chunk_start), "chunk_length": as_array(chunk_length),
             "chunk_slot": np.arange(len(chunk_start), dtype=np.int32), "long_table": as_array(long_table)}
+
+
+def _recurrence(q: torch.Tensor, k: torch.Tensor, decay: torch.Tensor, v: torch.Tensor, beta: torch.Tensor | None, matrix_state: torch.Tensor, *,
+                num_groups: int, segment_start: torch.Tensor, segment_length: torch.Tensor, segment_slot: torch.Tensor, segments: int,
+                status: torch.Tensor, chunk_plan: dict | None) -> torch.Tensor:
+    """The recurrence's read-outs, 32-bit ``[tokens, heads, value_dim]``, and its state in ``matrix_state``: long portions in blocks of tokens,
+    the others token by token.  ``beta=None``: without the delta rule's correction."""
+    tokens, num_heads, key_dim = decay.shape
+    value_dim = v.shape[2]
+    num_slots = matrix_state.shape[0]
+    lib = _lib()
+    read_out = torch.empty(tokens, num_heads, value_dim, dtype=torch.float32, device=q.device)
+    direct_list, num_direct = None, segments
+    if chunk_plan is not None and chunk_plan["num_chunks"] > 0:
+        chunk_tokens = chunk_plan.get("chunk_tokens", GDR_CHUNK_TOKENS)
+        if chunk_tokens >= RECURRENT_BLOCK and chunk_tokens % RECURRENT_BLOCK == 0:   # chunks of whole blocks (any other plan: every portion token by token)
+            num_chunks, num_long, blocks = chunk_plan["num_chunks"], chunk_plan["num_long"], chunk_tokens // RECURRENT_BLOCK
+            block_heads, delta = num_chunks * blocks * num_heads, 0 if beta is None else 1
+            pack = torch.empty(block_heads * lib.lb_recurrent_pack_floats(c_int(key_dim), c_int(value_dim), c_int(delta)), dtype=torch.float32, device=q.device)
+            values = torch.empty(block_heads * lib.lb_recurrent_value_floats(c_int(value_dim), c_int(delta)), dtype=torch.float32, device=q.device)
+            code = lib.lb_recurrent_blocks(_ptr(q), _ptr(k), _ptr(decay), _ptr(v), _ptr(beta), _ptr(pack), _ptr(values), _ptr(matrix_state), _ptr(read_out),
+                                           _ptr(chunk_plan["chunk_start"]), _ptr(chunk_plan["chunk_length"]), c_int(num_chunks), c_int(blocks),
+                                           _ptr(chunk_plan["long_table"]), c_int(num_long), _ptr(segment_start), _ptr(segment_length), _ptr(segment_slot),
+                                           c_int(num_heads), c_int(num_groups), c_int(key_dim), c_int(value_dim), c_int(num_slots), _ptr(status), _stream())
+            _done(code, "recurrent_blocks", 2 if delta else 3)
+            direct_list, num_direct = chunk_plan["direct"], chunk_plan["num_direct"]
+    if num_direct > 0:
+        code = lib.lb_gdr_scan(_ptr(q), _ptr(k), _ptr(decay), _ptr(v), _ptr(beta), _ptr(matrix_state), _ptr(read_out), _ptr(segment_start), _ptr(segment_length),
+                               _ptr(segment_slot), c_int(num_direct), c_int(num_heads), c_int(num_groups), c_int(key_dim), c_int(value_dim), c_int(num_slots),
+                               _ptr(status), _stream(), _ptr(direct_list))
+        _done(code, "gdr_scan")
+    return read_out
 
 
 def gated_delta_rule(
@@ -1303,34 +1328,8 @@ def gated_delta_rule(
         code = lib.lb_gdr_conv_state(_ptr(proj), c_int(proj.shape[1]), _ptr(conv_state), _ptr(segment_start), _ptr(segment_length), _ptr(segment_slot),
                                      c_int(segments), c_int(channels), c_int(taps), c_int(num_slots), c_int(dtype_code(proj.dtype)), _stream())
         _done(code, "gdr_conv_state")
-    read_out = torch.empty(tokens, num_heads, value_dim, dtype=torch.float32, device=device)
-    direct_list, num_direct = None, segments
-    if chunk_plan is not None and chunk_plan["num_chunks"] > 0 and not gated_delta_chunks_pay(key_dim, value_dim):
-        chunk_plan = None
-    if chunk_plan is not None and chunk_plan["num_chunks"] > 0:
-        # Long portions: their chunks are scanned side by side from zero states, with key_dim further columns that carry
-        # each chunk's transition; then the chunks' incoming states in order, and the read-outs' second term.
-        num_chunks, num_long = chunk_plan["num_chunks"], chunk_plan["num_long"]
-        wide_dim = value_dim + key_dim
-        wide = torch.empty(tokens, num_heads, wide_dim, dtype=torch.float32, device=device)
-        chunk_state = torch.empty(num_chunks, num_heads, key_dim, wide_dim, dtype=torch.float32, device=device)
-        chunk_in = torch.empty(num_chunks, num_heads, key_dim, value_dim, dtype=torch.float32, device=device)
-        _done(lib.lb_gdr_chunk_init(_ptr(chunk_state), c_int(num_chunks), c_int(num_heads), c_int(key_dim), c_int(value_dim), _stream()), "gdr_chunk_init")
-        code = lib.lb_gdr_scan(_ptr(q), _ptr(k), _ptr(decay), _ptr(v), _ptr(beta), _ptr(chunk_state), _ptr(wide), _ptr(chunk_plan["chunk_start"]),
-                               _ptr(chunk_plan["chunk_length"]), _ptr(chunk_plan["chunk_slot"]), c_int(num_chunks), c_int(num_heads), c_int(num_groups),
-                               c_int(key_dim), c_int(wide_dim), c_int(num_chunks), _ptr(status), _stream(), _ptr(None), c_int(value_dim), c_int(0))
-        _done(code, "gdr_scan (chunks)")
-        code = lib.lb_gdr_chunk_finish(_ptr(chunk_state), _ptr(chunk_in), _ptr(matrix_state), _ptr(wide), _ptr(read_out), _ptr(chunk_plan["long_table"]),
-                                       c_int(num_long), _ptr(segment_slot), _ptr(chunk_plan["chunk_start"]), _ptr(chunk_plan["chunk_length"]), c_int(num_chunks),
-                                       c_int(chunk_plan.get("chunk_tokens", GDR_CHUNK_TOKENS)), c_int(num_heads), c_int(key_dim), c_int(value_dim), c_int(num_slots),
-                                       _stream())
-        _done(code, "gdr_chunk_finish", 2)
-        direct_list, num_direct = chunk_plan["direct"], chunk_plan["num_direct"]
-    if num_direct > 0:
-        code = lib.lb_gdr_scan(_ptr(q), _ptr(k), _ptr(decay), _ptr(v), _ptr(beta), _ptr(matrix_state), _ptr(read_out), _ptr(segment_start), _ptr(segment_length),
-                               _ptr(segment_slot), c_int(num_direct), c_int(num_heads), c_int(num_groups), c_int(key_dim), c_int(value_dim), c_int(num_slots),
-                               _ptr(status), _stream(), _ptr(direct_list), c_int(value_dim), c_int(0))
-        _done(code, "gdr_scan")
+    read_out = _recurrence(q, k, decay, v, beta, matrix_state, num_groups=num_groups, segment_start=segment_start, segment_length=segment_length,
+                           segment_slot=segment_slot, segments=segments, status=status, chunk_plan=chunk_plan)
     out = torch.empty(tokens, num_heads * value_dim, dtype=proj.dtype, device=device)
     code = lib.lb_gdr_output(_ptr(read_out), _ptr(low_rank), c_int(low_rank.stride(0)), c_int(gate_offset), _ptr(norm_weight), _ptr(out), c_int(tokens),
                              c_int(num_heads), c_int(value_dim), c_float(norm_eps), c_int(dtype_code(proj.dtype)), _stream(), c_int(1 if gate_activation == "silu" else 0))
@@ -1801,46 +1800,8 @@ def linear_attention(proj: torch.Tensor, matrix_state: torch.Tensor, *, num_head
                                            _ptr(lower), c_int(1 if query_silu else 0), _ptr(inv_freq), _ptr(positions if inv_freq is not None else None),
                                            c_int(2 * inv_freq.numel() if inv_freq is not None else 0), c_float(turn_scale))
     _done(code, "linear_attention_prepare")
-    read_out = torch.empty(tokens, num_heads, value_dim, dtype=torch.float32, device=device)
-    # the scan of the gated delta rule without its correction (no beta), long portions in chunks where that pays
-    direct_list, num_direct = None, segments
-    if chunk_plan is not None and chunk_plan["num_chunks"] > 0 and fixed_decay is not None:
-        # one number per head: what a chunk does to the state it is given needs no further columns
-        num_chunks, num_long = chunk_plan["num_chunks"], chunk_plan["num_long"]
-        chunk_state = torch.empty(num_chunks, num_heads, key_dim, value_dim, dtype=torch.float32, device=device)
-        chunk_in = torch.empty_like(chunk_state)
-        code = lib.lb_gdr_scan(_ptr(q), _ptr(k), _ptr(decay), _ptr(v), _ptr(None), _ptr(chunk_state), _ptr(read_out), _ptr(chunk_plan["chunk_start"]),
-                               _ptr(chunk_plan["chunk_length"]), _ptr(chunk_plan["chunk_slot"]), c_int(num_chunks), c_int(num_heads), c_int(num_heads),
-                               c_int(key_dim), c_int(value_dim), c_int(num_chunks), _ptr(status), _stream(), _ptr(None), c_int(value_dim), c_int(1))
-        _done(code, "linear_attention_scan (chunks)")
-        code = lib.lb_retention_chunk_finish(_ptr(chunk_state), _ptr(chunk_in), _ptr(matrix_state), _ptr(q), _ptr(fixed_decay), _ptr(read_out), _ptr(chunk_plan["long_table"]),
-                                             c_int(num_long), _ptr(segment_slot), _ptr(chunk_plan["chunk_start"]), _ptr(chunk_plan["chunk_length"]), c_int(num_chunks),
-                                             c_int(chunk_plan.get("chunk_tokens", GDR_CHUNK_TOKENS)), c_int(num_heads), c_int(key_dim), c_int(value_dim), c_int(num_slots),
-                                             _stream())
-        _done(code, "retention_chunk_finish", 2)
-        direct_list, num_direct = chunk_plan["direct"], chunk_plan["num_direct"]
-    elif chunk_plan is not None and chunk_plan["num_chunks"] > 0 and gated_delta_chunks_pay(key_dim, value_dim):
-        num_chunks, num_long = chunk_plan["num_chunks"], chunk_plan["num_long"]
-        wide_dim = value_dim + key_dim
-        wide = torch.empty(tokens, num_heads, wide_dim, dtype=torch.float32, device=device)
-        chunk_state = torch.empty(num_chunks, num_heads, key_dim, wide_dim, dtype=torch.float32, device=device)
-        chunk_in = torch.empty(num_chunks, num_heads, key_dim, value_dim, dtype=torch.float32, device=device)
-        _done(lib.lb_gdr_chunk_init(_ptr(chunk_state), c_int(num_chunks), c_int(num_heads), c_int(key_dim), c_int(value_dim), _stream()), "gdr_chunk_init")
-        code = lib.lb_gdr_scan(_ptr(q), _ptr(k), _ptr(decay), _ptr(v), _ptr(None), _ptr(chunk_state), _ptr(wide), _ptr(chunk_plan["chunk_start"]),
-                               _ptr(chunk_plan["chunk_length"]), _ptr(chunk_plan["chunk_slot"]), c_int(num_chunks), c_int(num_heads), c_int(num_heads),
-                               c_int(key_dim), c_int(wide_dim), c_int(num_chunks), _ptr(status), _stream(), _ptr(None), c_int(value_dim), c_int(0))
-        _done(code, "linear_attention_scan (chunks)")
-        code = lib.lb_gdr_chunk_finish(_ptr(chunk_state), _ptr(chunk_in), _ptr(matrix_state), _ptr(wide), _ptr(read_out), _ptr(chunk_plan["long_table"]),
-                                       c_int(num_long), _ptr(segment_slot), _ptr(chunk_plan["chunk_start"]), _ptr(chunk_plan["chunk_length"]), c_int(num_chunks),
-                                       c_int(chunk_plan.get("chunk_tokens", GDR_CHUNK_TOKENS)), c_int(num_heads), c_int(key_dim), c_int(value_dim), c_int(num_slots),
-                                       _stream())
-        _done(code, "gdr_chunk_finish", 2)
-        direct_list, num_direct = chunk_plan["direct"], chunk_plan["num_direct"]
-    if num_direct > 0:
-        code = lib.lb_gdr_scan(_ptr(q), _ptr(k), _ptr(decay), _ptr(v), _ptr(None), _ptr(matrix_state), _ptr(read_out), _ptr(segment_start), _ptr(segment_length),
-                               _ptr(segment_slot), c_int(num_direct), c_int(num_heads), c_int(num_heads), c_int(key_dim), c_int(value_dim), c_int(num_slots),
-                               _ptr(status), _stream(), _ptr(direct_list), c_int(value_dim), c_int(0))
-        _done(code, "linear_attention_scan")
+    read_out = _recurrence(q, k, decay, v, None, matrix_state, num_groups=num_heads, segment_start=segment_start, segment_length=segment_length,
+                           segment_slot=segment_slot, segments=segments, status=status, chunk_plan=chunk_plan)
     out = torch.empty(tokens, num_heads * value_dim, dtype=proj.dtype, device=device)
     gated = gate_offset is not None
     code = lib.lb_gdr_output(_ptr(read_out), _ptr(proj if gated else None), c_int(proj.shape[1]), c_int(gate_offset if gated else 0), _ptr(norm_weight), _ptr(out), c_int(tokens),
