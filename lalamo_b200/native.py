@@ -1,7 +1,9 @@
 """Builds and loads the CUDA extension (the ``.cu`` files under ``csrc/``).
 
 The extension is one shared library of ``extern "C"`` launchers, compiled with ``nvcc`` for
-sm_100a and loaded with ``ctypes``; launchers take raw device pointers and a stream.  It is built
+sm_100a; launchers take raw device pointers and a stream.  Python calls them through wrappers that are
+made from their prototypes and compiled into the same library (:func:`launchers`): a call of twenty arguments
+through ``ctypes`` costs as much as the launch it makes.  The library is built
 in-tree (``lalamo_b200/_native/``) when that folder can be written, otherwise under the
 temporary directory, and rebuilt when a source file changes.  There is no fallback: if the
 library cannot be built or loaded, :func:`library` raises.
@@ -11,16 +13,20 @@ from __future__ import annotations
 
 import ctypes
 import hashlib
+import importlib.machinery
+import importlib.util
 import os
+import re
 import shutil
 import subprocess
 import sys
+import sysconfig
 import tempfile
 import threading
 import time
 from pathlib import Path
 
-__all__ = ["NativeBuildError", "build", "library", "library_path", "source_files"]
+__all__ = ["NativeBuildError", "build", "launchers", "library", "library_path", "source_files"]
 
 _SOURCE_DIR = Path(__file__).resolve().parent / "csrc"
 _LIBRARY_NAME = "liblalamo_b200_kernels.so"
@@ -38,6 +44,7 @@ _NVCC_FLAGS = [
 
 _lock = threading.Lock()
 _library: ctypes.CDLL | None = None
+_launchers: object | None = None
 
 
 class NativeBuildError(RuntimeError):
@@ -54,7 +61,109 @@ def _source_digest() -> str:
         digest.update(path.name.encode())
         digest.update(path.read_bytes())
     digest.update(" ".join(_NVCC_FLAGS).encode())
+    digest.update(_wrappers_source().encode())
     return digest.hexdigest()[:16]
+
+
+def _prototypes() -> dict[str, tuple[str, list[str]]]:
+    """The launchers' prototypes as the sources define them: name -> (result type, type of every parameter), all pointers being ``void*``."""
+    found: dict[str, tuple[str, list[str]]] = {}
+    for path in source_files():
+        text = re.sub(r"//[^\n]*", "", path.read_text())
+        for result, name, parameters in re.findall(r"^(int|long long) (lb_\w+)\(([^)]*)\)\s*\{", text, re.MULTILINE):
+            declared = filter(None, (" ".join(part.split()) for part in parameters.split(",")))
+            found[name] = (result, ["void*" if "*" in part or "cudaStream_t" in part else part.rsplit(" ", 1)[0] for part in declared])
+    return found
+
+
+_WRAPPERS_HEAD = """// Made from the launchers' prototypes: a function of the same name and arguments for each, callable from Python.  A pointer is
+// None, an address, or anything with a data_ptr() (a tensor); numbers may also be ctypes objects.
+#define Py_LIMITED_API 0x030A0000
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+
+static bool take_integer(PyObject* object, long long* value) {
+    if (PyLong_Check(object)) {
+        *value = PyLong_AsLongLong(object);
+    } else if (object == Py_None) {
+        *value = 0;
+    } else {
+        PyObject* number = PyIndex_Check(object) ? PyNumber_Index(object) : PyObject_GetAttrString(object, "value");
+        if (number == nullptr) return false;
+        const bool taken = PyLong_Check(number) || number == Py_None ? take_integer(number, value) : (PyErr_SetString(PyExc_TypeError, "a launcher wants a number here"), false);
+        Py_DECREF(number);
+        return taken;
+    }
+    return !(*value == -1 && PyErr_Occurred());
+}
+
+static bool take_pointer(PyObject* object, void** value) {
+    static PyObject* method = PyUnicode_InternFromString("data_ptr");
+    long long address = 0;
+    if (PyLong_Check(object) || object == Py_None || !PyObject_HasAttr(object, method)) {
+        if (!take_integer(object, &address)) return false;
+    } else {
+        PyObject* result = PyObject_CallMethodObjArgs(object, method, nullptr);
+        if (result == nullptr) return false;
+        const bool taken = take_integer(result, &address);
+        Py_DECREF(result);
+        if (!taken) return false;
+    }
+    *value = reinterpret_cast<void*>(address);
+    return true;
+}
+
+static bool take_float(PyObject* object, double* value) {
+    if (PyFloat_Check(object) || PyLong_Check(object)) {
+        *value = PyFloat_AsDouble(object);
+        return !(*value == -1.0 && PyErr_Occurred());
+    }
+    PyObject* number = PyObject_GetAttrString(object, "value");
+    if (number == nullptr) return false;
+    *value = PyFloat_AsDouble(number);
+    Py_DECREF(number);
+    return !(*value == -1.0 && PyErr_Occurred());
+}
+"""
+
+
+def _wrappers_source() -> str:
+    """C++ source of the wrappers through which Python calls the launchers (a module named ``lalamo_b200_launchers``)."""
+    taken_as = {"void*": ("pointer", "void*"), "float": ("float", "double")}
+    parts, table = [_WRAPPERS_HEAD], []
+    for name, (result, types) in _prototypes().items():
+        lines = [f"extern \"C\" {result} {name}({', '.join(types)});",
+                 f"static PyObject* wrap_{name}(PyObject*, PyObject* const* arguments, Py_ssize_t count) {{",
+                 f"    if (count != {len(types)}) return PyErr_Format(PyExc_TypeError, \"{name} takes {len(types)} arguments, got %zd\", count);"]
+        for index, declared in enumerate(types):
+            kind, variable = taken_as.get(declared, ("integer", "long long"))
+            lines.append(f"    {variable} a{index};\n    if (!take_{kind}(arguments[{index}], &a{index})) return nullptr;")
+        call = ", ".join(f"static_cast<{declared}>(a{index})" for index, declared in enumerate(types))
+        lines += [f"    {result} code;", "    Py_BEGIN_ALLOW_THREADS", f"    code = {name}({call});", "    Py_END_ALLOW_THREADS", "    return PyLong_FromLongLong(code);", "}"]
+        parts.append("\n".join(lines))
+        table.append(f"    {{\"{name}\", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(wrap_{name})), METH_FASTCALL, nullptr}},")
+    parts.append("static PyMethodDef methods[] = {\n" + "\n".join(table) + "\n    {nullptr, nullptr, 0, nullptr}};\n"
+                 'static PyModuleDef module = {PyModuleDef_HEAD_INIT, "lalamo_b200_launchers", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};\n'
+                 "PyMODINIT_FUNC PyInit_lalamo_b200_launchers() { return PyModule_Create(&module); }\n")
+    return "\n\n".join(parts)
+
+
+class _CtypesLaunchers:
+    """The same through ``ctypes``, for a library built where Python's headers were missing."""
+
+    def __init__(self, loaded: ctypes.CDLL) -> None:
+        c_types = {"void*": ctypes.c_void_p, "float": ctypes.c_float, "int": ctypes.c_int, "unsigned": ctypes.c_uint, "long long": ctypes.c_longlong}
+        for name, (result, types) in _prototypes().items():
+            function = getattr(loaded, name)
+            function.restype, function.argtypes = c_types[result], [c_types[declared] for declared in types]
+            setattr(self, name, self._taking_tensors(function))
+
+    @staticmethod
+    def _taking_tensors(function):
+        def call(*arguments):
+            return function(*(argument.data_ptr() if hasattr(argument, "data_ptr") else argument for argument in arguments))
+
+        return call
 
 
 def _find_nvcc() -> str:
@@ -113,6 +222,13 @@ def build(verbose: bool = True, force: bool = False) -> Path:
     started = time.time()
     processes: list[tuple[Path, subprocess.Popen]] = []
     compile_flags = [flag for flag in _NVCC_FLAGS if flag != "--shared"]
+    wrappers = None
+    headers = sysconfig.get_paths()["include"]
+    if os.path.isfile(os.path.join(headers, "Python.h")):
+        wrappers = directory / f"launchers.{os.getpid()}.cpp"
+        wrappers.write_text(_wrappers_source())
+        sources = [*sources, wrappers]
+        compile_flags += ["-I", headers]
     for source in sources:
         target = directory / (source.stem + f".{os.getpid()}.o")
         objects.append(target)
@@ -140,7 +256,7 @@ def build(verbose: bool = True, force: bool = False) -> Path:
         stderr=subprocess.STDOUT,
         text=True,
     )
-    for target in objects:
+    for target in objects + ([wrappers] if wrappers is not None else []):
         target.unlink(missing_ok=True)
     if link.returncode != 0:
         raise NativeBuildError(f"linking the kernel library failed:\n{link.stdout}")
@@ -162,3 +278,18 @@ def library() -> ctypes.CDLL:
             except OSError as error:
                 raise NativeBuildError(f"cannot load {path}: {error}") from error
         return _library
+
+
+def launchers() -> object:
+    """The library's launchers as functions: a pointer may be given as a tensor, ``None`` or an address, numbers as they are."""
+    global _launchers
+    loaded = library()
+    with _lock:
+        if _launchers is None:
+            if hasattr(loaded, "PyInit_lalamo_b200_launchers"):
+                loader = importlib.machinery.ExtensionFileLoader("lalamo_b200_launchers", loaded._name)
+                _launchers = importlib.util.module_from_spec(importlib.util.spec_from_loader("lalamo_b200_launchers", loader))
+                loader.exec_module(_launchers)
+            else:
+                _launchers = _CtypesLaunchers(loaded)
+        return _launchers

@@ -12,8 +12,9 @@ from __future__ import annotations
 from dataclasses import dataclass
 
 import ctypes
+import functools
 import os
-from ctypes import c_float, c_int, c_longlong, c_void_p
+from ctypes import c_int, c_longlong, c_void_p
 
 import torch
 
@@ -109,8 +110,7 @@ class ExpertSum:
     def sum(self) -> torch.Tensor:
         tokens, top = self.chosen.shape
         out = torch.empty(tokens, self.pair_out.shape[1], dtype=self.dtype, device=self.pair_out.device)
-        code = _lib().lb_moe_combine(_ptr(self.pair_out), _ptr(self.weights), _ptr(self.chosen), c_int(self.experts), _ptr(out), c_int(tokens), c_int(top),
-                                     c_int(self.pair_out.shape[1]), c_int(dtype_code(self.dtype)), _stream())
+        code = _lib().lb_moe_combine(self.pair_out, self.weights, self.chosen, self.experts, out, tokens, top, self.pair_out.shape[1], dtype_code(self.dtype), _stream())
         _done(code, "moe_combine")
         return out
 
@@ -208,19 +208,24 @@ _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 _raw_device = getattr(torch._C, "_cuda_getDevice", None)
 
 
-def _stream() -> c_void_p:
+def _current_device() -> int:
+    return _raw_device() if _raw_device is not None else torch.cuda.current_device()
+
+
+def _stream() -> int:
     if _raw_stream is not None and _raw_device is not None:
-        return c_void_p(_raw_stream(_raw_device()))
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+        return _raw_stream(_raw_device())
+    return torch.cuda.current_stream().cuda_stream
 
 
-def _ptr(tensor: torch.Tensor | None) -> c_void_p:
-    if tensor is None:
-        return c_void_p(0)
-    return c_void_p(tensor.data_ptr())
+def _ptr(tensor: torch.Tensor | None) -> int:
+    """A tensor's address, or 0.  (The launchers take tensors and ``None`` as they are.)"""
+    return 0 if tensor is None else tensor.data_ptr()
 
 
 def _check(tensor: torch.Tensor, name: str, dtype: torch.dtype | None = None) -> None:
+    if tensor.is_cuda and tensor.is_contiguous() and (dtype is None or tensor.dtype is dtype):
+        return
     if not tensor.is_cuda:
         raise KernelError(f"{name} must live on a CUDA device (there is no CPU path)")
     if not tensor.is_contiguous():
@@ -240,8 +245,14 @@ def _done(code: int, what: str, launches: int = 1) -> None:
     _launches += launches
 
 
-def _lib() -> ctypes.CDLL:
-    return native.library()
+_launchers = None
+
+
+def _lib():
+    global _launchers
+    if _launchers is None:
+        _launchers = native.launchers()
+    return _launchers
 
 
 # --------------------------------------------------------------------------- elementwise
@@ -254,8 +265,8 @@ def embed(table: torch.Tensor, ids: torch.Tensor, out: torch.Tensor, scale: floa
     vocab = table.shape[0]
     if table.shape[1] != dim or ids.numel() < tokens:
         raise KernelError("embed: shapes of table, ids and out do not agree")
-    code = _lib().lb_embed(_ptr(table), _ptr(ids), _ptr(out), c_int(tokens), c_int(dim), c_int(vocab), c_float(scale),
-                           c_int(dtype_code(table.dtype)), _ptr(status), _stream(), c_int(1 if accumulate else 0))
+    code = _lib().lb_embed(table, ids, out, tokens, dim, vocab, scale,
+                           dtype_code(table.dtype), status, _stream(), 1 if accumulate else 0)
     _done(code, "embed")
 
 
@@ -322,10 +333,10 @@ def rmsnorm(
         raise KernelError("rmsnorm: x and out differ in rows")
     if dim > 50000:
         raise KernelError(f"rmsnorm: rows of {dim} elements exceed the supported 50000")
-    code = _lib().lb_rmsnorm(_ptr(x), c_int(1 if x.dtype == torch.float32 else 0),
-                             _ptr(delta), _ptr(partials), c_int(slices), c_longlong(slice_stride), _ptr(weight), _ptr(rows), _ptr(out), c_int(out_rows), c_int(dim), c_float(eps),
-                             c_float(scale_offset), c_int(1 if write_back else 0), c_int(dtype_code(out.dtype)), _stream(), c_int(1 if exact else 0),
-                             _ptr(bias), c_int(1 if centred else 0), _ptr(delta_bias))
+    code = _lib().lb_rmsnorm(x, 1 if x.dtype == torch.float32 else 0,
+                             delta, partials, slices, slice_stride, weight, rows, out, out_rows, dim, eps,
+                             scale_offset, 1 if write_back else 0, dtype_code(out.dtype), _stream(), 1 if exact else 0,
+                             bias, 1 if centred else 0, delta_bias)
     _done(code, "rmsnorm")
 
 
@@ -334,7 +345,7 @@ def _sum_slices(partials: torch.Tensor, out: torch.Tensor, epilogue: str) -> Non
     slices, tokens, rows = partials.shape
     if out.shape != (tokens, rows):
         raise KernelError("sum_slices: out must be [tokens, rows]")
-    code = _lib().lb_sum_slices(_ptr(partials), _ptr(out), c_int(tokens), c_int(rows), c_int(slices), c_int(_TC_EPILOGUES[epilogue]), _stream())
+    code = _lib().lb_sum_slices(partials, out, tokens, rows, slices, _TC_EPILOGUES[epilogue], _stream())
     _done(code, "sum_slices")
 
 
@@ -354,7 +365,7 @@ def residual_add(x: torch.Tensor, delta: torch.Tensor | SlicedSum) -> None:
     _check(delta, "delta")
     if x.shape != delta.shape:
         raise KernelError("residual_add: shapes differ")
-    code = _lib().lb_residual_add(_ptr(x), _ptr(delta), c_longlong(x.numel()), c_int(dtype_code(delta.dtype)), _stream())
+    code = _lib().lb_residual_add(x, delta, x.numel(), dtype_code(delta.dtype), _stream())
     _done(code, "residual_add")
 
 
@@ -364,7 +375,7 @@ def cast_rows(x: torch.Tensor, out: torch.Tensor) -> None:
     _check(out, "out")
     if x.shape != out.shape:
         raise KernelError("cast_rows: shapes differ")
-    code = _lib().lb_cast_rows(_ptr(x), _ptr(out), c_longlong(x.numel()), c_int(dtype_code(out.dtype)), _stream())
+    code = _lib().lb_cast_rows(x, out, x.numel(), dtype_code(out.dtype), _stream())
     _done(code, "cast_rows")
 
 
@@ -374,7 +385,7 @@ def add_bias(x: torch.Tensor, bias: torch.Tensor) -> None:
     _check(bias, "bias", torch.float32)
     if x.dim() != 2 or bias.numel() != x.shape[1]:
         raise KernelError("add_bias: bias must have one element per column of x")
-    code = _lib().lb_add_bias(_ptr(x), _ptr(bias), c_int(x.shape[0]), c_int(x.shape[1]), c_int(dtype_code(x.dtype)), _stream())
+    code = _lib().lb_add_bias(x, bias, x.shape[0], x.shape[1], dtype_code(x.dtype), _stream())
     _done(code, "add_bias")
 
 
@@ -420,12 +431,12 @@ def norm_accumulate(residual: torch.Tensor, delta: "torch.Tensor | ScaledSum", w
         _check(next_weight, "next_norm weight", torch.float32)
         if rounded is None or next_weight.numel() != residual.shape[1]:
             raise KernelError("norm_accumulate: the next norm needs `rounded` and a weight of one element per column")
-    code = _lib().lb_norm_accumulate(_ptr(residual), _ptr(first), _ptr(terms[0][2]), c_float(terms[0][1]), _ptr(second[0]), _ptr(second[2]), c_float(second[1]),
-                                     _ptr(weight), _ptr(rounded), c_int(residual.shape[0]), c_int(residual.shape[1]), c_float(eps), c_float(scale_offset),
-                                     c_int(dtype_code(first.dtype)), _stream(), _ptr(next_weight), c_float(next_eps), c_float(next_offset),
-                                     _ptr(routed.pair_out if routed is not None else None), _ptr(routed.weights if routed is not None else None),
-                                     _ptr(routed.chosen if routed is not None else None), c_int(routed.chosen.shape[1] if routed is not None else 0),
-                                     c_int(routed.experts if routed is not None else 0))
+    code = _lib().lb_norm_accumulate(residual, first, terms[0][2], terms[0][1], second[0], second[2], second[1],
+                                     weight, rounded, residual.shape[0], residual.shape[1], eps, scale_offset,
+                                     dtype_code(first.dtype), _stream(), next_weight, next_eps, next_offset,
+                                     routed.pair_out if routed is not None else None, routed.weights if routed is not None else None,
+                                     routed.chosen if routed is not None else None, routed.chosen.shape[1] if routed is not None else 0,
+                                     routed.experts if routed is not None else 0)
     _done(code, "norm_accumulate")
 
 
@@ -498,8 +509,8 @@ def residual_terms(x: torch.Tensor, terms: TermSum, weight: torch.Tensor | None 
         _check(weight, "weight", torch.float32)
         if out.shape != (out_rows, dim) or weight.numel() != dim:
             raise KernelError("residual_terms: out must be [rows, dim] and weight [dim]")
-    code = _lib().lb_residual_terms(_ptr(x), records, c_int(len(terms.terms)), _ptr(weight), _ptr(rows), _ptr(out), c_int(out_rows), c_int(dim), c_float(eps),
-                                    c_int(1 if write_back else 0), c_int(dtype_code(dtype)), _stream(), c_int(0 if terms.joined else 1))
+    code = _lib().lb_residual_terms(x, ctypes.addressof(records), len(terms.terms), weight, rows, out, out_rows, dim, eps,
+                                    1 if write_back else 0, dtype_code(dtype), _stream(), 0 if terms.joined else 1)
     _done(code, "residual_terms")
 
 
@@ -508,7 +519,7 @@ def scale_(x: torch.Tensor, factor: float, softcap: float = 0.0) -> None:
     _check(x, "x", torch.float32)
     if softcap < 0.0:
         raise KernelError("scale_: the cap must not be negative")
-    _done(_lib().lb_scale(_ptr(x), c_float(factor), c_longlong(x.numel()), _stream(), c_float(softcap)), "scale")
+    _done(_lib().lb_scale(x, factor, x.numel(), _stream(), softcap), "scale")
 
 
 def bias_activation(x: torch.Tensor, bias: torch.Tensor | None, activation: str) -> torch.Tensor:
@@ -521,8 +532,8 @@ def bias_activation(x: torch.Tensor, bias: torch.Tensor | None, activation: str)
         if x.dim() != 2 or bias.numel() != x.shape[1]:
             raise KernelError("bias_activation: bias must have one element per column of x")
     out = torch.empty_like(x)
-    code = _lib().lb_bias_activation(_ptr(x), _ptr(bias), _ptr(out), c_int(x.shape[0]), c_int(x.shape[1]), c_int(_ACTIVATIONS[activation]),
-                                     c_int(dtype_code(x.dtype)), _stream())
+    code = _lib().lb_bias_activation(x, bias, out, x.shape[0], x.shape[1], _ACTIVATIONS[activation],
+                                     dtype_code(x.dtype), _stream())
     _done(code, "bias_activation")
     return out
 
@@ -535,7 +546,7 @@ def poly_norm(z: torch.Tensor, coefficients: torch.Tensor, eps: float) -> torch.
     if z.dim() != 2 or coefficients.numel() != 4:
         raise KernelError("poly_norm: z must be [rows, dim] with four coefficients")
     out = torch.empty_like(z)
-    _done(_lib().lb_poly_norm(_ptr(z), _ptr(coefficients), _ptr(out), c_int(z.shape[0]), c_int(z.shape[1]), c_float(eps), c_int(dtype_code(z.dtype)), _stream()), "poly_norm")
+    _done(_lib().lb_poly_norm(z, coefficients, out, z.shape[0], z.shape[1], eps, dtype_code(z.dtype), _stream()), "poly_norm")
     return out
 
 
@@ -617,13 +628,13 @@ def stream_step(streams: ResidualStreams, update: StreamWrite | None, read: torc
             if state.shape != (num_slots, taps - 1, dim):
                 raise KernelError("stream_step: the convolution's state must be [slots, taps - 1, dim]")
     h = torch.empty(out_rows, dim, dtype=dtype, device=x.device)
-    code = _lib().lb_stream_step(_ptr(x), _ptr(x_out), c_int(1 if streams.equal else 0), c_int(count), _ptr(update.mix if update is not None else None),
-                                 _ptr(update.write if update is not None else None), _ptr(read), _ptr(y), _ptr(partials), c_int(slices), c_longlong(stride), _ptr(bias),
-                                 _ptr(routed.pair_out if routed is not None else None), _ptr(routed.weights if routed is not None else None),
-                                 _ptr(routed.chosen if routed is not None else None), c_int(routed.chosen.shape[1] if routed is not None else 0),
-                                 c_int(routed.experts if routed is not None else 0), _ptr(norm_weight), c_float(eps), _ptr(h), _ptr(rows), c_int(out_rows), c_int(dim),
-                                 _ptr(weight), _ptr(state if taps > 1 else None), _ptr(conv.get("token_segment")), _ptr(conv.get("segment_slot")), c_int(taps),
-                                 c_int(num_slots), c_int(dtype_code(dtype)), _ptr(conv.get("status")), _stream())
+    code = _lib().lb_stream_step(x, x_out, 1 if streams.equal else 0, count, update.mix if update is not None else None,
+                                 update.write if update is not None else None, read, y, partials, slices, stride, bias,
+                                 routed.pair_out if routed is not None else None, routed.weights if routed is not None else None,
+                                 routed.chosen if routed is not None else None, routed.chosen.shape[1] if routed is not None else 0,
+                                 routed.experts if routed is not None else 0, norm_weight, eps, h, rows, out_rows, dim,
+                                 weight, state if taps > 1 else None, conv.get("token_segment"), conv.get("segment_slot"), taps,
+                                 num_slots, dtype_code(dtype), conv.get("status"), _stream())
     _done(code, "stream_step")
     if x_out is not None:
         streams.tensor = x_out
@@ -658,9 +669,9 @@ def causal_conv(x: torch.Tensor, state: torch.Tensor | None, weight: torch.Tenso
     for name, tensor in (("segment_start", segment_start), ("segment_length", segment_length), ("segment_slot", segment_slot)):
         _check(tensor, name, torch.int32)
     out = torch.empty(x.shape[0], channels, dtype=x.dtype, device=x.device)
-    code = _lib().lb_causal_conv(_ptr(x), c_int(x.stride(0)), _ptr(state if taps > 1 else None), _ptr(weight), _ptr(out), c_int(channels), c_int(channels), c_int(taps),
-                                 c_int(1 if add_input else 0), _ptr(segment_start), _ptr(segment_length), _ptr(segment_slot), c_int(segments), c_int(max_length),
-                                 c_int(num_slots), c_int(dtype_code(x.dtype)), _ptr(status), _stream())
+    code = _lib().lb_causal_conv(x, x.stride(0), state if taps > 1 else None, weight, out, channels, channels, taps,
+                                 1 if add_input else 0, segment_start, segment_length, segment_slot, segments, max_length,
+                                 num_slots, dtype_code(x.dtype), status, _stream())
     _done(code, "causal_conv")
     return out
 
@@ -675,8 +686,8 @@ def stream_concat(stream: torch.Tensor, table: torch.Tensor, ids: torch.Tensor, 
     if table.shape[1] != dim or ids.numel() < tokens:
         raise KernelError("stream_concat: shapes of stream, table and ids do not agree")
     out = torch.empty(tokens, 2 * dim, dtype=table.dtype, device=stream.device)
-    code = _lib().lb_stream_concat(_ptr(stream), _ptr(table), _ptr(ids), _ptr(out), c_int(tokens), c_int(dim), c_int(table.shape[0]), c_float(scale),
-                                   c_int(dtype_code(table.dtype)), _ptr(status), _stream())
+    code = _lib().lb_stream_concat(stream, table, ids, out, tokens, dim, table.shape[0], scale,
+                                   dtype_code(table.dtype), status, _stream())
     _done(code, "stream_concat")
     return out
 
@@ -688,7 +699,7 @@ def gather_rows(src: torch.Tensor, rows: torch.Tensor, out: torch.Tensor) -> Non
     dim = src.shape[-1]
     if out.shape[-1] != dim or rows.numel() < out.shape[0]:
         raise KernelError("gather_rows: shapes do not agree")
-    code = _lib().lb_gather_rows(_ptr(src), _ptr(rows), _ptr(out), c_int(out.shape[0]), c_int(dim), c_int(src.element_size()), _stream())
+    code = _lib().lb_gather_rows(src, rows, out, out.shape[0], dim, src.element_size(), _stream())
     _done(code, "gather_rows")
 
 
@@ -700,7 +711,7 @@ def fill_slots(table: torch.Tensor, largest_bytes: int, slot: int, pattern: int 
         raise KernelError("fill_slots: table must be [states, 2]")
     if slot < 0:
         raise KernelError("fill_slots: negative slot")
-    code = _lib().lb_fill_slots(_ptr(table), c_int(table.shape[0]), c_longlong(largest_bytes), c_int(slot), ctypes.c_uint(pattern & 0xFFFFFFFF), _stream())
+    code = _lib().lb_fill_slots(table, table.shape[0], largest_bytes, slot, pattern & 0xFFFFFFFF, _stream())
     _done(code, "fill_slots")
 
 
@@ -715,8 +726,8 @@ def feed_tokens(token_ids: torch.Tensor, segment_start: torch.Tensor, segment_le
         raise KernelError("feed_tokens: one start, length and source per segment")
     if status is not None:
         _check(status, "status", torch.int32)
-    code = _lib().lb_feed_tokens(_ptr(token_ids), _ptr(segment_start), _ptr(segment_length), _ptr(source), _ptr(sampled), c_int(sampled.numel()),
-                                 c_int(segments), _ptr(status), _stream())
+    code = _lib().lb_feed_tokens(token_ids, segment_start, segment_length, source, sampled, sampled.numel(),
+                                 segments, status, _stream())
     _done(code, "feed_tokens")
 
 
@@ -730,8 +741,8 @@ def gated_activation(fused: torch.Tensor, out: torch.Tensor, activation: str, li
     tokens, hidden = out.shape
     if fused.shape != (tokens, 2 * hidden):
         raise KernelError("gated_activation: fused must be [tokens, 2 * hidden]")
-    code = _lib().lb_gated_activation(_ptr(fused), _ptr(out), c_int(tokens), c_int(hidden), c_int(_ACTIVATIONS[activation]),
-                                      c_int(dtype_code(out.dtype)), _stream(), c_float(limit))
+    code = _lib().lb_gated_activation(fused, out, tokens, hidden, _ACTIVATIONS[activation],
+                                      dtype_code(out.dtype), _stream(), limit)
     _done(code, "gated_activation")
 
 
@@ -823,11 +834,11 @@ def qk_norm_rope_write(
     _check(positions, "positions", torch.int32)
     _check(token_segment, "token_segment", torch.int32)
     code = _lib().lb_qk_norm_rope_write(
-        _ptr(qkv), _ptr(q_out), _ptr(k_pages), _ptr(v_pages), _ptr(q_weight), _ptr(k_weight), c_float(eps), c_float(scale_offset),
-        _ptr(inv_freq), c_int(rotary_dim), _ptr(positions), _ptr(token_segment), _ptr(block_table), c_int(tokens), c_int(num_heads),
-        c_int(num_groups), c_int(head_dim), c_int(page_size), c_int(num_pages), c_int(max_blocks), c_int(1 if write_kv else 0),
-        c_int(dtype_code(qkv.dtype)), _ptr(status), _stream(), c_int(value_dim), _ptr(bias), _ptr(row_inv), c_float(turn_scale), c_int(qkv.stride(0)),
-        c_int(value_groups or 0), c_float(temperature), c_int(temperature_every))
+        qkv, q_out, k_pages, v_pages, q_weight, k_weight, eps, scale_offset,
+        inv_freq, rotary_dim, positions, token_segment, block_table, tokens, num_heads,
+        num_groups, head_dim, page_size, num_pages, max_blocks, 1 if write_kv else 0,
+        dtype_code(qkv.dtype), status, _stream(), value_dim, bias, row_inv, turn_scale, qkv.stride(0),
+        value_groups or 0, temperature, temperature_every)
     _done(code, "qk_norm_rope_write", 2 if whole_norm and tokens > 64 else 1)   # few tokens: the statistic is computed in the rewrite itself
 
 
@@ -870,10 +881,10 @@ def paged_attention_plain(
     if num_heads % num_groups:
         raise KernelError("paged_attention: num_heads must be a multiple of num_groups")
     code = _lib().lb_paged_attention_plain(
-        _ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(out), _ptr(positions), _ptr(token_segment), _ptr(block_table), c_int(tokens),
-        c_int(num_heads), c_int(num_groups), c_int(head_dim), c_int(page_size), c_int(num_pages), c_int(max_blocks), c_float(scale),
-        c_int(window if window else 0), c_int(dtype_code(q.dtype)), _ptr(status), _stream(), c_int(value_dim), c_int(keep_first),
-        c_int(value_groups or 0), c_int(1 if out.dtype == torch.float32 and q.dtype != torch.float32 else 0))
+        q, k_pages, v_pages, out, positions, token_segment, block_table, tokens,
+        num_heads, num_groups, head_dim, page_size, num_pages, max_blocks, scale,
+        window if window else 0, dtype_code(q.dtype), status, _stream(), value_dim, keep_first,
+        value_groups or 0, 1 if out.dtype == torch.float32 and q.dtype != torch.float32 else 0)
     _done(code, "paged_attention_plain")
 
 
@@ -889,8 +900,8 @@ def combine_maps(maps: torch.Tensor, gate: torch.Tensor | None, out: torch.Tenso
         raise KernelError("combine_maps: maps must be [tokens, groups, 2, heads / groups, value_dim] and out [tokens, heads * value_dim]")
     if gate is not None and (not gate.is_cuda or gate.dtype != out.dtype or gate.shape != (tokens, num_heads) or gate.stride(1) != 1):
         raise KernelError("combine_maps: gate must be [tokens, heads] of out's type with unit column stride")
-    code = _lib().lb_combine_maps(_ptr(maps), _ptr(gate), c_int(gate.stride(0) if gate is not None else 0), _ptr(out), c_int(tokens), c_int(num_heads), c_int(num_groups),
-                                  c_int(value_dim), c_float(lam), c_float(eps), c_float(factor), c_int(dtype_code(out.dtype)), _stream())
+    code = _lib().lb_combine_maps(maps, gate, gate.stride(0) if gate is not None else 0, out, tokens, num_heads, num_groups,
+                                  value_dim, lam, eps, factor, dtype_code(out.dtype), _stream())
     _done(code, "combine_maps")
 
 
@@ -901,7 +912,7 @@ _decode_ctas_per_sm: dict[tuple[int, int], int] = {}
 
 def sm_count() -> int:
     """Multiprocessors of the current device (asked once per device)."""
-    device = torch.cuda.current_device()
+    device = _current_device()
     if device not in _sm_counts:
         _sm_counts[device] = torch.cuda.get_device_properties(device).multi_processor_count
     return _sm_counts[device]
@@ -910,9 +921,9 @@ def sm_count() -> int:
 def decode_ctas_per_sm(head_dim: int) -> int:
     """CTAs of the split-key attention kernel an SM of the current device holds at this head size
     (the library asks the runtime; registers and the ring's shared memory decide)."""
-    key = (torch.cuda.current_device(), head_dim)
+    key = (_current_device(), head_dim)
     if key not in _decode_ctas_per_sm:
-        _decode_ctas_per_sm[key] = max(1, int(_lib().lb_attention_decode_ctas_per_sm(c_int(head_dim))))
+        _decode_ctas_per_sm[key] = max(1, int(_lib().lb_attention_decode_ctas_per_sm(head_dim)))
     return _decode_ctas_per_sm[key]
 
 
@@ -937,6 +948,12 @@ def decode_attention_plan(tokens: int, num_heads: int, num_groups: int, max_cont
         blocks_total = min(max_context // 16 + 1, blocks_total + -(-keep_first // 16))  # the blocks of the kept first keys come before the window's
     pairs = max(1, tokens * num_groups * -(-(num_heads // num_groups) // 16))
     slots = resident_ctas if resident_ctas is not None else sm_count() * ((3 * decode_ctas_per_sm(head_dim) + 2) // 4)
+    return _fewest_rounds(blocks_total, pairs, slots)
+
+
+@functools.lru_cache(maxsize=4096)
+def _fewest_rounds(blocks_total: int, pairs: int, slots: int) -> tuple[int, int]:
+    """The search of :func:`decode_attention_plan`, remembered by its sizes: every layer of a step asks the same."""
     best, best_cost = 1, None
     for splits in range(1, max(1, blocks_total // 8) + 1):
         per_warp = -(-(-(-blocks_total // splits)) // 4)
@@ -1010,11 +1027,11 @@ def attention_decode(
         if scratch.numel() < needed:
             raise KernelError(f"attention_decode: scratch holds {scratch.numel()} floats, {needed} are needed")
     code = _lib().lb_attention_decode(
-        _ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(out), _ptr(scratch), _ptr(positions), _ptr(token_segment), _ptr(block_table),
-        _ptr(token_list), c_int(tokens), c_int(num_heads), c_int(num_groups), c_int(head_dim), c_int(page_size), c_int(num_pages), c_int(max_blocks),
-        c_float(scale), c_int(window if window else 0), c_int(splits), c_int(blocks_per_split), c_int(-1 if fresh_keys is None else fresh_keys),
-        _ptr(status), _stream(), c_int(keep_first), c_int(value_dim), c_int(value_groups or 0), c_int(1 if two_maps else 0),
-        c_int(1 if out.dtype == torch.float32 else 0))
+        q, k_pages, v_pages, out, scratch, positions, token_segment, block_table,
+        token_list, tokens, num_heads, num_groups, head_dim, page_size, num_pages, max_blocks,
+        scale, window if window else 0, splits, blocks_per_split, -1 if fresh_keys is None else fresh_keys,
+        status, _stream(), keep_first, value_dim, value_groups or 0, 1 if two_maps else 0,
+        1 if out.dtype == torch.float32 else 0)
     _done(code, "attention_decode", 2 if splits > 1 else 1)   # the kernel and the merge of its splits
 
 
@@ -1099,19 +1116,19 @@ def attention_prefill(
         raise KernelError(f"attention_prefill: the tcgen05 kernel takes head size 64 (or key heads of up to 64 channels with value heads of 64 or 128) and up to 128 query heads per K/V head, not {head_dim} and {num_heads // num_groups}")
     if kernel == "tcgen05" or (kernel is None and takes_tcgen05 and USE_TCGEN05_ATTENTION):
         code = _lib().lb_attention_prefill_tcgen05(
-            _ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(out), _ptr(tiles), c_int(num_tiles), c_int(q.shape[0]), _ptr(positions), _ptr(token_segment),
-            _ptr(block_table), c_int(num_heads), c_int(num_groups), c_int(head_dim), c_int(page_size), c_int(num_pages), c_int(max_blocks),
-            c_float(scale), c_int(window if window else 0), c_int(split_tiles), _ptr(status), _stream(), c_int(keep_first if window else 0),
-            c_int(value_dim), c_int(value_groups or 0), c_int(1 if out.dtype == torch.float32 else 0))
+            q, k_pages, v_pages, out, tiles, num_tiles, q.shape[0], positions, token_segment,
+            block_table, num_heads, num_groups, head_dim, page_size, num_pages, max_blocks,
+            scale, window if window else 0, split_tiles, status, _stream(), keep_first if window else 0,
+            value_dim, value_groups or 0, 1 if out.dtype == torch.float32 else 0)
         if code == -5:
             raise KernelError("attention_prefill: the driver made no tensor map for these tensors")
         _done(code, "attention_prefill (tcgen05)")
         return
     code = _lib().lb_attention_prefill(
-        _ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(out), _ptr(tiles), c_int(num_tiles), _ptr(positions), _ptr(token_segment), _ptr(block_table),
-        c_int(num_heads), c_int(num_groups), c_int(head_dim), c_int(page_size), c_int(num_pages), c_int(max_blocks), c_float(scale),
-        c_int(window if window else 0), _ptr(status), _stream(), c_int(keep_first if window else 0), c_int(value_dim), c_int(value_groups or 0),
-        c_int(1 if out.dtype == torch.float32 else 0))
+        q, k_pages, v_pages, out, tiles, num_tiles, positions, token_segment, block_table,
+        num_heads, num_groups, head_dim, page_size, num_pages, max_blocks, scale,
+        window if window else 0, status, _stream(), keep_first if window else 0, value_dim, value_groups or 0,
+        1 if out.dtype == torch.float32 else 0)
     _done(code, "attention_prefill")
 
 
@@ -1162,15 +1179,15 @@ def short_conv(
     if single_tokens:
         # every portion is one token: one kernel for the slices' sum, the convolution and the state
         code = _lib().lb_short_conv_single(
-            _ptr(proj.partials if sliced else None), c_int(proj.partials.shape[0] if sliced else 0), _ptr(None if sliced else proj), _ptr(state), _ptr(weight),
-            _ptr(bias), _ptr(out), _ptr(token_segment), _ptr(segment_slot), c_int(tokens), c_int(dim), c_int(kernel_size), c_int(state.shape[0]), _ptr(status),
+            proj.partials if sliced else None, proj.partials.shape[0] if sliced else 0, None if sliced else proj, state, weight,
+            bias, out, token_segment, segment_slot, tokens, dim, kernel_size, state.shape[0], status,
             _stream())
         _done(code, "short_conv_single")
         return
     code = _lib().lb_short_conv(
-        _ptr(proj), _ptr(state), _ptr(weight), _ptr(bias), _ptr(out), _ptr(token_segment), _ptr(segment_start), _ptr(segment_length),
-        _ptr(segment_slot), c_int(tokens), c_int(segments), c_int(dim), c_int(kernel_size), c_int(state.shape[0]),
-        c_int(dtype_code(proj.dtype)), _ptr(status), _stream())
+        proj, state, weight, bias, out, token_segment, segment_start, segment_length,
+        segment_slot, tokens, segments, dim, kernel_size, state.shape[0],
+        dtype_code(proj.dtype), status, _stream())
     _done(code, "short_conv", 2 if kernel_size > 1 else 1)
 
 
@@ -1220,18 +1237,18 @@ def _recurrence(q: torch.Tensor, k: torch.Tensor, decay: torch.Tensor, v: torch.
         if chunk_tokens >= RECURRENT_BLOCK and chunk_tokens % RECURRENT_BLOCK == 0:   # chunks of whole blocks (any other plan: every portion token by token)
             num_chunks, num_long, blocks = chunk_plan["num_chunks"], chunk_plan["num_long"], chunk_tokens // RECURRENT_BLOCK
             block_heads, delta = num_chunks * blocks * num_heads, 0 if beta is None else 1
-            pack = torch.empty(block_heads * lib.lb_recurrent_pack_floats(c_int(key_dim), c_int(value_dim), c_int(delta)), dtype=torch.float32, device=q.device)
-            values = torch.empty(block_heads * lib.lb_recurrent_value_floats(c_int(value_dim), c_int(delta)), dtype=torch.float32, device=q.device)
-            code = lib.lb_recurrent_blocks(_ptr(q), _ptr(k), _ptr(decay), _ptr(v), _ptr(beta), _ptr(pack), _ptr(values), _ptr(matrix_state), _ptr(read_out),
-                                           _ptr(chunk_plan["chunk_start"]), _ptr(chunk_plan["chunk_length"]), c_int(num_chunks), c_int(blocks),
-                                           _ptr(chunk_plan["long_table"]), c_int(num_long), _ptr(segment_start), _ptr(segment_length), _ptr(segment_slot),
-                                           c_int(num_heads), c_int(num_groups), c_int(key_dim), c_int(value_dim), c_int(num_slots), _ptr(status), _stream())
+            pack = torch.empty(block_heads * lib.lb_recurrent_pack_floats(key_dim, value_dim, delta), dtype=torch.float32, device=q.device)
+            values = torch.empty(block_heads * lib.lb_recurrent_value_floats(value_dim, delta), dtype=torch.float32, device=q.device)
+            code = lib.lb_recurrent_blocks(q, k, decay, v, beta, pack, values, matrix_state, read_out,
+                                           chunk_plan["chunk_start"], chunk_plan["chunk_length"], num_chunks, blocks,
+                                           chunk_plan["long_table"], num_long, segment_start, segment_length, segment_slot,
+                                           num_heads, num_groups, key_dim, value_dim, num_slots, status, _stream())
             _done(code, "recurrent_blocks", 2 if delta else 3)
             direct_list, num_direct = chunk_plan["direct"], chunk_plan["num_direct"]
     if num_direct > 0:
-        code = lib.lb_gdr_scan(_ptr(q), _ptr(k), _ptr(decay), _ptr(v), _ptr(beta), _ptr(matrix_state), _ptr(read_out), _ptr(segment_start), _ptr(segment_length),
-                               _ptr(segment_slot), c_int(num_direct), c_int(num_heads), c_int(num_groups), c_int(key_dim), c_int(value_dim), c_int(num_slots),
-                               _ptr(status), _stream(), _ptr(direct_list))
+        code = lib.lb_gdr_scan(q, k, decay, v, beta, matrix_state, read_out, segment_start, segment_length,
+                               segment_slot, num_direct, num_heads, num_groups, key_dim, value_dim, num_slots,
+                               status, _stream(), direct_list)
         _done(code, "gdr_scan")
     return read_out
 
@@ -1318,21 +1335,21 @@ def gated_delta_rule(
     decay = torch.empty(tokens, num_heads, key_dim, dtype=torch.float32, device=device)
     lib = _lib()
     single_tokens = segments == tokens   # every portion is one token: the convolutions' kernel also writes their new state
-    code = lib.lb_gdr_prepare(_ptr(proj), c_int(proj.shape[1]), _ptr(low_rank), c_int(low_rank.stride(0)), _ptr(conv_state), _ptr(conv_weight), _ptr(a_log),
-                              _ptr(dt_bias), _ptr(q), _ptr(k), _ptr(v), _ptr(beta), _ptr(decay), _ptr(token_segment), _ptr(segment_start), _ptr(segment_slot),
-                              c_int(tokens), c_int(num_heads), c_int(num_groups), c_int(key_dim), c_int(value_dim), c_int(taps), c_int(num_slots),
-                              c_float(unit_eps), c_float(key_dim ** -0.5), c_int(dtype_code(proj.dtype)), _ptr(status), _stream(), c_int(1 if single_tokens else 0),
-                              c_int(1 if decay_per_head else 0))
+    code = lib.lb_gdr_prepare(proj, proj.shape[1], low_rank, low_rank.stride(0), conv_state, conv_weight, a_log,
+                              dt_bias, q, k, v, beta, decay, token_segment, segment_start, segment_slot,
+                              tokens, num_heads, num_groups, key_dim, value_dim, taps, num_slots,
+                              unit_eps, key_dim ** -0.5, dtype_code(proj.dtype), status, _stream(), 1 if single_tokens else 0,
+                              1 if decay_per_head else 0)
     _done(code, "gdr_prepare")
     if taps > 1 and not single_tokens:
-        code = lib.lb_gdr_conv_state(_ptr(proj), c_int(proj.shape[1]), _ptr(conv_state), _ptr(segment_start), _ptr(segment_length), _ptr(segment_slot),
-                                     c_int(segments), c_int(channels), c_int(taps), c_int(num_slots), c_int(dtype_code(proj.dtype)), _stream())
+        code = lib.lb_gdr_conv_state(proj, proj.shape[1], conv_state, segment_start, segment_length, segment_slot,
+                                     segments, channels, taps, num_slots, dtype_code(proj.dtype), _stream())
         _done(code, "gdr_conv_state")
     read_out = _recurrence(q, k, decay, v, beta, matrix_state, num_groups=num_groups, segment_start=segment_start, segment_length=segment_length,
                            segment_slot=segment_slot, segments=segments, status=status, chunk_plan=chunk_plan)
     out = torch.empty(tokens, num_heads * value_dim, dtype=proj.dtype, device=device)
-    code = lib.lb_gdr_output(_ptr(read_out), _ptr(low_rank), c_int(low_rank.stride(0)), c_int(gate_offset), _ptr(norm_weight), _ptr(out), c_int(tokens),
-                             c_int(num_heads), c_int(value_dim), c_float(norm_eps), c_int(dtype_code(proj.dtype)), _stream(), c_int(1 if gate_activation == "silu" else 0))
+    code = lib.lb_gdr_output(read_out, low_rank, low_rank.stride(0), gate_offset, norm_weight, out, tokens,
+                             num_heads, value_dim, norm_eps, dtype_code(proj.dtype), _stream(), 1 if gate_activation == "silu" else 0)
     _done(code, "gdr_output")
     return out
 
@@ -1364,9 +1381,9 @@ def heads_product(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, *, w
     for name, tensor in (("x", x), ("out", out), ("gate", gate)):
         if tensor is not None and (not tensor.is_cuda or tensor.dtype != torch.bfloat16 or tensor.stride(2) != 1 or (name == "gate" and tensor.shape != out.shape)):
             raise KernelError(f"heads_product: {name} must be a bfloat16 CUDA tensor [tokens, heads, .] with unit stride along the last dimension")
-    code = _lib().lb_heads_product(_ptr(x), c_longlong(x.stride(0)), c_int(x.stride(1)), _ptr(weight), c_int(1 if weight_is_kn else 0), _ptr(out),
-                                   c_longlong(out.stride(0)), c_int(out.stride(1)), _ptr(gate), c_longlong(gate.stride(0) if gate is not None else 0),
-                                   c_int(gate.stride(1) if gate is not None else 0), c_int(tokens), c_int(heads), c_int(k), c_int(n), _stream())
+    code = _lib().lb_heads_product(x, x.stride(0), x.stride(1), weight, 1 if weight_is_kn else 0, out,
+                                   out.stride(0), out.stride(1), gate, gate.stride(0) if gate is not None else 0,
+                                   gate.stride(1) if gate is not None else 0, tokens, heads, k, n, _stream())
     _done(code, "heads_product")
 
 
@@ -1409,10 +1426,10 @@ def latent_prepare(q: torch.Tensor, q_latent: torch.Tensor | None, down: torch.T
     page_size, num_pages, max_blocks = _check_latent_pages(pages, block_table, latent, rope)
     if pages.dtype != q_out.dtype:
         raise KernelError("latent_prepare: cache and activations differ in type")
-    code = _lib().lb_latent_prepare(_ptr(q), c_int(q.stride(0)), _ptr(q_latent), _ptr(down if write_kv else None), c_int(down.stride(0) if write_kv else 0), _ptr(q_out), _ptr(pages), _ptr(norm_weight),
-                                    c_float(eps), c_float(scale_offset), _ptr(inv_freq), _ptr(positions), _ptr(token_segment), _ptr(block_table), c_int(tokens),
-                                    c_int(num_heads), c_int(head_dim), c_int(latent), c_int(rope), c_int(page_size), c_int(num_pages), c_int(max_blocks),
-                                    c_int(1 if write_kv else 0), c_int(dtype_code(q_out.dtype)), _ptr(status), _stream(), c_float(turn_scale))
+    code = _lib().lb_latent_prepare(q, q.stride(0), q_latent, down if write_kv else None, down.stride(0) if write_kv else 0, q_out, pages, norm_weight,
+                                    eps, scale_offset, inv_freq, positions, token_segment, block_table, tokens,
+                                    num_heads, head_dim, latent, rope, page_size, num_pages, max_blocks,
+                                    1 if write_kv else 0, dtype_code(q_out.dtype), status, _stream(), turn_scale)
     _done(code, "latent_prepare")
 
 
@@ -1442,10 +1459,10 @@ def latent_down(q_down: torch.Tensor, down: torch.Tensor | None, q_latent: torch
         _check(norm_weight, "norm_weight", torch.float32)
         if down.shape[1] != latent + rope or norm_weight.numel() != latent:
             raise KernelError("latent_down: down must be [tokens, latent + rope] with a norm weight of latent elements")
-    code = _lib().lb_latent_down(_ptr(q_down), _ptr(down), c_int(q_down.stride(0)), _ptr(q_latent), c_int(q_latent.shape[1]), c_int(q_rank), _ptr(q_norm_weight),
-                                 c_float(q_eps), _ptr(pages), _ptr(norm_weight), c_float(eps), c_float(scale_offset), _ptr(inv_freq), c_float(turn_scale), _ptr(positions),
-                                 _ptr(token_segment), _ptr(block_table), c_int(tokens), c_int(latent), c_int(rope), c_int(page_size), c_int(num_pages), c_int(max_blocks),
-                                 c_int(dtype_code(q_latent.dtype)), _ptr(status), _stream())
+    code = _lib().lb_latent_down(q_down, down, q_down.stride(0), q_latent, q_latent.shape[1], q_rank, q_norm_weight,
+                                 q_eps, pages, norm_weight, eps, scale_offset, inv_freq, turn_scale, positions,
+                                 token_segment, block_table, tokens, latent, rope, page_size, num_pages, max_blocks,
+                                 dtype_code(q_latent.dtype), status, _stream())
     _done(code, "latent_down")
 
 
@@ -1473,9 +1490,9 @@ def latent_attention_plain(q: torch.Tensor, pages: torch.Tensor, out: torch.Tens
         raise KernelError("latent_attention: cache and queries differ in type")
     if latent > 1024 or (latent + rope) * 4 > 40 * 1024:
         raise KernelError(f"latent_attention: latent {latent} + rope {rope} exceed what the kernel supports")
-    code = _lib().lb_latent_attention_plain(_ptr(q), _ptr(pages), _ptr(out), _ptr(positions), _ptr(token_segment), _ptr(block_table), c_int(tokens),
-                                            c_int(num_heads), c_int(latent), c_int(rope), c_int(page_size), c_int(num_pages), c_int(max_blocks),
-                                            c_float(scale), c_int(window if window else 0), c_int(dtype_code(q.dtype)), _ptr(status), _stream(), _ptr(sink))
+    code = _lib().lb_latent_attention_plain(q, pages, out, positions, token_segment, block_table, tokens,
+                                            num_heads, latent, rope, page_size, num_pages, max_blocks,
+                                            scale, window if window else 0, dtype_code(q.dtype), status, _stream(), sink)
     _done(code, "latent_attention_plain")
 
 
@@ -1524,10 +1541,10 @@ def latent_attention(q: torch.Tensor, pages: torch.Tensor, out: torch.Tensor, *,
         raise KernelError(f"latent_attention: latent {latent}, rope {rope}, pages of {page_size} are not sizes the tensor-core kernel takes")
     heads_per_cta, tokens_per_cta = latent_attention_tiling(num_heads)
     partial = torch.empty(tokens, num_heads, splits, latent + 2, dtype=torch.float32, device=q.device) if splits > 1 else None
-    code = _lib().lb_latent_attention_mma(_ptr(q), _ptr(pages), _ptr(out), _ptr(partial), _ptr(items), c_int(num_items), _ptr(positions), _ptr(token_segment),
-                                          _ptr(block_table), c_int(tokens), c_int(num_heads), c_int(latent), c_int(rope), c_int(page_size), c_int(num_pages),
-                                          c_int(max_blocks), c_float(scale), c_int(window if window else 0), c_int(heads_per_cta), c_int(tokens_per_cta),
-                                          c_int(splits), _ptr(status), _stream(), _ptr(sink))
+    code = _lib().lb_latent_attention_mma(q, pages, out, partial, items, num_items, positions, token_segment,
+                                          block_table, tokens, num_heads, latent, rope, page_size, num_pages,
+                                          max_blocks, scale, window if window else 0, heads_per_cta, tokens_per_cta,
+                                          splits, status, _stream(), sink)
     _done(code, "latent_attention_mma", 2 if splits > 1 else 1)
 
 
@@ -1544,8 +1561,8 @@ def gate_heads(values: torch.Tensor, gate: torch.Tensor | None, out: torch.Tenso
         if not gate.is_cuda or gate.dtype != values.dtype or gate.shape != out.shape or gate.stride(1) != 1:
             raise KernelError("gate_heads: gate must be [tokens, heads * vdim] of the values' type with unit column stride")
         stride = gate.stride(0)
-    code = _lib().lb_gate_heads(_ptr(values), _ptr(gate), c_int(stride), _ptr(out), c_int(tokens), c_int(heads), c_int(value_dim),
-                                c_int(dtype_code(values.dtype)), _stream())
+    code = _lib().lb_gate_heads(values, gate, stride, out, tokens, heads, value_dim,
+                                dtype_code(values.dtype), _stream())
     _done(code, "gate_heads")
 
 
@@ -1592,10 +1609,10 @@ def moe_route(x: torch.Tensor, router: torch.Tensor, *, top: int, group_count: i
     chosen = torch.empty(tokens, top, dtype=torch.int32, device=x.device)
     weights = torch.empty(tokens, top, dtype=torch.float32, device=x.device)
     extra_out = torch.empty(tokens, extra, dtype=torch.float32, device=x.device) if extra else None
-    code = _lib().lb_moe_route(_ptr(x), _ptr(router), _ptr(chosen), _ptr(weights), c_int(tokens), c_int(width), c_int(experts), c_int(top), c_int(group_count),
-                               c_int(group_keep), c_int(_ROUTER_SCORES[score]), c_int(2 if chosen_softmax else 1 if renormalize else 0), c_float(weight_scale),
-                               c_int(dtype_code(x.dtype)), _stream(), _ptr(bias), _ptr(choice_bias), c_int(extra), _ptr(extra_out),
-                               c_int(1 if group_score == "largest" else 2))
+    code = _lib().lb_moe_route(x, router, chosen, weights, tokens, width, experts, top, group_count,
+                               group_keep, _ROUTER_SCORES[score], 2 if chosen_softmax else 1 if renormalize else 0, weight_scale,
+                               dtype_code(x.dtype), _stream(), bias, choice_bias, extra, extra_out,
+                               1 if group_score == "largest" else 2)
     _done(code, "moe_route")
     if extra:
         return chosen, weights, extra_out
@@ -1651,9 +1668,9 @@ def moe_experts(x: torch.Tensor, gate: "torch.Tensor | None", up: torch.Tensor, 
         order = torch.empty(pairs, dtype=torch.int32, device=x.device)
         gathered = torch.empty(pairs, width, dtype=x.dtype, device=x.device)
         hidden = torch.empty(pairs, ff, dtype=x.dtype, device=x.device)
-        code = lib.lb_moe_experts_grouped(_ptr(x), _ptr(gate), _ptr(up), _ptr(down), _ptr(chosen), _ptr(offsets), _ptr(order), _ptr(gathered), _ptr(hidden), _ptr(pair_out),
-                                          c_int(pairs), c_int(top), c_int(width), c_int(ff), c_int(experts), c_int(_ACTIVATIONS[activation]), _stream(), c_float(limit), _ptr(input_weight),
-                                          _ptr(status))
+        code = lib.lb_moe_experts_grouped(x, gate, up, down, chosen, offsets, order, gathered, hidden, pair_out,
+                                          pairs, top, width, ff, experts, _ACTIVATIONS[activation], _stream(), limit, input_weight,
+                                          status)
         if code == -5:
             raise KernelError("moe_experts: the driver gave no tensor map (cuTensorMapEncodeTiled)")
         _done(code, "moe_experts_grouped", 4)
@@ -1662,12 +1679,12 @@ def moe_experts(x: torch.Tensor, gate: "torch.Tensor | None", up: torch.Tensor, 
         if not wide_rows:
             raise KernelError("moe_experts: the streaming kernels take rows of 16-byte multiples")
         hidden = torch.empty(pairs, ff, dtype=x.dtype, device=x.device)
-        code = lib.lb_moe_expert_stream_wide(_ptr(x), _ptr(gate), _ptr(up), _ptr(down), _ptr(chosen), _ptr(hidden), _ptr(pair_out), c_int(pairs), c_int(top),
-                                             c_int(width), c_int(ff), c_int(experts), c_int(_ACTIVATIONS[activation]), c_int(dtype_code(x.dtype)), _stream(), c_float(limit), _ptr(input_weight))
+        code = lib.lb_moe_expert_stream_wide(x, gate, up, down, chosen, hidden, pair_out, pairs, top,
+                                             width, ff, experts, _ACTIVATIONS[activation], dtype_code(x.dtype), _stream(), limit, input_weight)
         _done(code, "moe_expert_stream_wide", 2)
     elif path == "plain":
-        code = lib.lb_moe_expert_stream(_ptr(x), _ptr(gate), _ptr(up), _ptr(down), _ptr(chosen), _ptr(pair_out), c_int(pairs), c_int(top), c_int(width),
-                                        c_int(ff), c_int(experts), c_int(_ACTIVATIONS[activation]), c_int(dtype_code(x.dtype)), _stream(), c_float(limit), _ptr(input_weight))
+        code = lib.lb_moe_expert_stream(x, gate, up, down, chosen, pair_out, pairs, top, width,
+                                        ff, experts, _ACTIVATIONS[activation], dtype_code(x.dtype), _stream(), limit, input_weight)
         _done(code, "moe_expert_stream")
     else:
         raise KernelError(f"moe_experts: unknown path {path!r}")
@@ -1675,8 +1692,8 @@ def moe_experts(x: torch.Tensor, gate: "torch.Tensor | None", up: torch.Tensor, 
     if not combine:
         return ExpertSum(pair_out, output_weight, chosen, experts, x.dtype)   # the consumer adds the pairs' outputs
     out = torch.empty(tokens, width, dtype=x.dtype, device=x.device)
-    code = lib.lb_moe_combine(_ptr(pair_out), _ptr(output_weight), _ptr(chosen), c_int(experts), _ptr(out), c_int(tokens), c_int(top), c_int(width),
-                              c_int(dtype_code(x.dtype)), _stream())
+    code = lib.lb_moe_combine(pair_out, output_weight, chosen, experts, out, tokens, top, width,
+                              dtype_code(x.dtype), _stream())
     _done(code, "moe_combine")
     return out
 
@@ -1701,8 +1718,8 @@ def moe_combine_add(routed: ExpertSum, residual: torch.Tensor, every: torch.Tens
         _check(every_gate, "every_gate", torch.float32)
         if every is None or every_gate.numel() != tokens:
             raise KernelError("moe_combine_add: the gate needs `every` and one element per token")
-    code = _lib().lb_moe_combine_add(_ptr(routed.pair_out), _ptr(routed.weights), _ptr(routed.chosen), c_int(routed.experts), _ptr(every), _ptr(every_gate), c_int(1),
-                                     _ptr(residual), c_int(tokens), c_int(top), c_int(width), c_int(dtype_code(routed.dtype)), _stream())
+    code = _lib().lb_moe_combine_add(routed.pair_out, routed.weights, routed.chosen, routed.experts, every, every_gate, 1,
+                                     residual, tokens, top, width, dtype_code(routed.dtype), _stream())
     _done(code, "moe_combine_add")
 
 
@@ -1720,8 +1737,8 @@ def branch_norms_accumulate(residual: torch.Tensor, terms: list, eps: float) -> 
         if tensor.shape != residual.shape or weight.numel() != residual.shape[1]:
             raise KernelError("branch_norms_accumulate: a branch's output or weight does not fit the residual stream")
     second = terms[1] if len(terms) == 2 else (None, None, 0.0)
-    code = _lib().lb_branch_norms_accumulate(_ptr(residual), _ptr(first), _ptr(terms[0][1]), c_float(terms[0][2]), _ptr(second[0]), _ptr(second[1]), c_float(second[2]),
-                                             c_int(residual.shape[0]), c_int(residual.shape[1]), c_float(eps), c_int(dtype_code(first.dtype)), _stream())
+    code = _lib().lb_branch_norms_accumulate(residual, first, terms[0][1], terms[0][2], second[0], second[1], second[2],
+                                             residual.shape[0], residual.shape[1], eps, dtype_code(first.dtype), _stream())
     _done(code, "branch_norms_accumulate")
 
 
@@ -1794,18 +1811,18 @@ def linear_attention(proj: torch.Tensor, matrix_state: torch.Tensor, *, num_head
     decay = torch.empty_like(q)
     v = torch.empty(tokens, num_heads, value_dim, dtype=torch.float32, device=device)
     lib = _lib()
-    code = lib.lb_linear_attention_prepare(_ptr(proj), c_int(proj.shape[1]), _ptr(decay_logits), c_int(decay_logits.stride(0) if decay_logits is not None else 0),
-                                           _ptr(decay_bias), _ptr(fixed_decay), c_float(1.0 / tau), c_float(query_scale), c_float(key_scale), _ptr(q), _ptr(k), _ptr(v),
-                                           _ptr(decay), c_int(tokens), c_int(num_heads), c_int(key_dim), c_int(value_dim), c_int(dtype_code(proj.dtype)), _stream(),
-                                           _ptr(lower), c_int(1 if query_silu else 0), _ptr(inv_freq), _ptr(positions if inv_freq is not None else None),
-                                           c_int(2 * inv_freq.numel() if inv_freq is not None else 0), c_float(turn_scale))
+    code = lib.lb_linear_attention_prepare(proj, proj.shape[1], decay_logits, decay_logits.stride(0) if decay_logits is not None else 0,
+                                           decay_bias, fixed_decay, 1.0 / tau, query_scale, key_scale, q, k, v,
+                                           decay, tokens, num_heads, key_dim, value_dim, dtype_code(proj.dtype), _stream(),
+                                           lower, 1 if query_silu else 0, inv_freq, positions if inv_freq is not None else None,
+                                           2 * inv_freq.numel() if inv_freq is not None else 0, turn_scale)
     _done(code, "linear_attention_prepare")
     read_out = _recurrence(q, k, decay, v, None, matrix_state, num_groups=num_heads, segment_start=segment_start, segment_length=segment_length,
                            segment_slot=segment_slot, segments=segments, status=status, chunk_plan=chunk_plan)
     out = torch.empty(tokens, num_heads * value_dim, dtype=proj.dtype, device=device)
     gated = gate_offset is not None
-    code = lib.lb_gdr_output(_ptr(read_out), _ptr(proj if gated else None), c_int(proj.shape[1]), c_int(gate_offset if gated else 0), _ptr(norm_weight), _ptr(out), c_int(tokens),
-                             c_int(num_heads), c_int(value_dim), c_float(norm_eps), c_int(dtype_code(proj.dtype)), _stream(), c_int(1 if gate_activation == "silu" else 0))
+    code = lib.lb_gdr_output(read_out, proj if gated else None, proj.shape[1], gate_offset if gated else 0, norm_weight, out, tokens,
+                             num_heads, value_dim, norm_eps, dtype_code(proj.dtype), _stream(), 1 if gate_activation == "silu" else 0)
     _done(code, "linear_attention_output")
     return out
 
@@ -1847,10 +1864,10 @@ def pooled_rewrite(qkv: torch.Tensor, q_out: torch.Tensor, pages: torch.Tensor, 
             raise KernelError("pooled_rewrite: rotated values need an even value_dim and one frequency per pair")
     for name, tensor in (("positions", positions), ("token_segment", token_segment)):
         _check(tensor, name, torch.int32)
-    code = _lib().lb_pooled_rewrite(_ptr(qkv), c_int(qkv.stride(0)), _ptr(q_out), _ptr(pages), _ptr(qk_freq if rotary_dim else None), c_int(rotary_dim),
-                                    c_int(1 if interleaved else 0), _ptr(value_freq), c_int(1 if interleaved else 0), _ptr(positions), _ptr(token_segment),
-                                    _ptr(block_table), c_int(tokens), c_int(num_heads), c_int(num_groups), c_int(head_dim), c_int(value_dim), c_int(page_size),
-                                    c_int(count), c_int(max_blocks), c_int(1 if write_kv else 0), c_int(dtype_code(qkv.dtype)), _ptr(status), _stream())
+    code = _lib().lb_pooled_rewrite(qkv, qkv.stride(0), q_out, pages, qk_freq if rotary_dim else None, rotary_dim,
+                                    1 if interleaved else 0, value_freq, 1 if interleaved else 0, positions, token_segment,
+                                    block_table, tokens, num_heads, num_groups, head_dim, value_dim, page_size,
+                                    count, max_blocks, 1 if write_kv else 0, dtype_code(qkv.dtype), status, _stream())
     _done(code, "pooled_rewrite")
 
 
@@ -1865,10 +1882,10 @@ def pooled_means(pages: torch.Tensor, pool_pages: torch.Tensor, *, segment_lengt
         raise KernelError("pooled_means: pages of one type and a positive block size")
     for name, tensor in (("segment_length", segment_length), ("segment_context", segment_context)):
         _check(tensor, name, torch.int32)
-    code = _lib().lb_pooled_means(_ptr(pages), _ptr(pool_pages), _ptr(segment_length), _ptr(segment_context), _ptr(block_table),
-                                  _ptr(pool_table), c_int(segments), c_int(max_length), c_int(num_groups), c_int(head_dim), c_int(value_dim), c_int(page_size),
-                                  c_int(count), c_int(max_blocks), c_int(pool_rows), c_int(pool_count), c_int(pool_blocks), c_int(pool), c_int(dtype_code(pages.dtype)),
-                                  _ptr(status), _stream())
+    code = _lib().lb_pooled_means(pages, pool_pages, segment_length, segment_context, block_table,
+                                  pool_table, segments, max_length, num_groups, head_dim, value_dim, page_size,
+                                  count, max_blocks, pool_rows, pool_count, pool_blocks, pool, dtype_code(pages.dtype),
+                                  status, _stream())
     _done(code, "pooled_means")
 
 
@@ -1942,11 +1959,11 @@ def pooled_attention_plain(q: torch.Tensor, pages: torch.Tensor, pool_pages: tor
     tokens, (count, page_size, max_blocks), (pool_count, pool_rows, pool_blocks) = _pooled_arguments(
         q, pages, pool_pages, out, positions, token_segment, block_table, pool_table, num_heads, num_groups, head_dim, value_dim, head_bias, window, pool,
         value_freq, "pooled_attention_plain")
-    code = _lib().lb_pooled_attention_plain(_ptr(q), _ptr(pages), _ptr(pool_pages if pool else None), _ptr(out),
-                                            _ptr(positions), _ptr(token_segment), _ptr(block_table), _ptr(pool_table if pool else None), c_int(tokens), c_int(num_heads),
-                                            c_int(num_groups), c_int(head_dim), c_int(value_dim), c_int(page_size), c_int(count), c_int(max_blocks), c_int(pool_rows),
-                                            c_int(pool_count), c_int(pool_blocks), c_float(scale), c_float(softcap), _ptr(head_bias), c_int(window), c_int(pool),
-                                            _ptr(value_freq), c_int(1 if interleaved else 0), c_int(dtype_code(q.dtype)), _ptr(status), _stream())
+    code = _lib().lb_pooled_attention_plain(q, pages, pool_pages if pool else None, out,
+                                            positions, token_segment, block_table, pool_table if pool else None, tokens, num_heads,
+                                            num_groups, head_dim, value_dim, page_size, count, max_blocks, pool_rows,
+                                            pool_count, pool_blocks, scale, softcap, head_bias, window, pool,
+                                            value_freq, 1 if interleaved else 0, dtype_code(q.dtype), status, _stream())
     _done(code, "pooled_attention_plain")
 
 
@@ -1973,11 +1990,11 @@ def pooled_attention(q: torch.Tensor, pages: torch.Tensor, pool_pages: torch.Ten
     if not 1 <= shares <= 64:
         raise KernelError("pooled_attention: 1 to 64 shares")
     partial = torch.empty(shares, tokens, num_heads * value_dim, dtype=torch.float32, device=q.device) if shares > 1 else None
-    code = _lib().lb_pooled_attention_mma(_ptr(q), _ptr(pages), _ptr(pool_pages if pool else None), _ptr(out), _ptr(tiles), c_int(num_tiles), _ptr(positions),
-                                          _ptr(token_segment), _ptr(block_table), _ptr(pool_table if pool else None), c_int(num_heads), c_int(num_groups),
-                                          c_int(head_dim), c_int(value_dim), c_int(page_size), c_int(count), c_int(max_blocks), c_int(pool_rows), c_int(pool_count),
-                                          c_int(pool_blocks), c_int(head_block), c_float(scale), c_float(softcap), _ptr(head_bias), c_int(window), c_int(pool),
-                                          _ptr(value_freq), c_int(1 if interleaved else 0), _ptr(status), _stream(), c_int(shares), _ptr(partial), c_int(tokens))
+    code = _lib().lb_pooled_attention_mma(q, pages, pool_pages if pool else None, out, tiles, num_tiles, positions,
+                                          token_segment, block_table, pool_table if pool else None, num_heads, num_groups,
+                                          head_dim, value_dim, page_size, count, max_blocks, pool_rows, pool_count,
+                                          pool_blocks, head_block, scale, softcap, head_bias, window, pool,
+                                          value_freq, 1 if interleaved else 0, status, _stream(), shares, partial, tokens)
     _done(code, "pooled_attention", 2 if shares > 1 else 1)
 
 
@@ -2002,11 +2019,11 @@ def pooled_attention_single(q: torch.Tensor, pages: torch.Tensor, pool_pages: to
     if not 1 <= shares <= 64:
         raise KernelError("pooled_attention_single: 1 to 64 shares")
     partial = torch.empty(shares, tokens, num_heads * value_dim, dtype=torch.float32, device=q.device) if shares > 1 else None
-    code = _lib().lb_pooled_attention_single(_ptr(q), _ptr(pages), _ptr(pool_pages if pool else None), _ptr(out), _ptr(singles), c_int(num_singles), _ptr(positions),
-                                             _ptr(token_segment), _ptr(block_table), _ptr(pool_table if pool else None), c_int(num_heads), c_int(num_groups),
-                                             c_int(head_dim), c_int(value_dim), c_int(page_size), c_int(count), c_int(max_blocks), c_int(pool_rows), c_int(pool_count),
-                                             c_int(pool_blocks), c_float(scale), c_float(softcap), _ptr(head_bias), c_int(window), c_int(pool),
-                                             _ptr(value_freq), c_int(1 if interleaved else 0), _ptr(status), _stream(), c_int(shares), _ptr(partial), c_int(tokens))
+    code = _lib().lb_pooled_attention_single(q, pages, pool_pages if pool else None, out, singles, num_singles, positions,
+                                             token_segment, block_table, pool_table if pool else None, num_heads, num_groups,
+                                             head_dim, value_dim, page_size, count, max_blocks, pool_rows, pool_count,
+                                             pool_blocks, scale, softcap, head_bias, window, pool,
+                                             value_freq, 1 if interleaved else 0, status, _stream(), shares, partial, tokens)
     _done(code, "pooled_attention_single", 2 if shares > 1 else 1)
 
 
@@ -2029,7 +2046,7 @@ def sample(logits: torch.Tensor, work: torch.Tensor, counts: torch.Tensor | None
     lib = _lib()
     if lib.lb_sample_params_size() != 4 * SAMPLE_PARAM_WORDS:
         raise KernelError("sample: parameter record sizes of the library and the bindings differ")
-    code = lib.lb_sample(_ptr(logits), _ptr(work), _ptr(counts), _ptr(params), _ptr(out_tokens), c_int(rows), c_int(vocab), _stream())
+    code = lib.lb_sample(logits, work, counts, params, out_tokens, rows, vocab, _stream())
     _done(code, "sample")
 
 
@@ -2043,10 +2060,10 @@ def argmax(logits: torch.Tensor, out_tokens: torch.Tensor) -> None:
         # Few long rows: spread each over many blocks.
         chunks = max(2, min(64, vocab // 2048))
         scratch = torch.empty(2 * rows * chunks, dtype=torch.float32, device=logits.device)
-        code = _lib().lb_argmax_chunked(_ptr(logits), _ptr(scratch), _ptr(out_tokens), c_int(rows), c_int(vocab), c_int(chunks), _stream())
+        code = _lib().lb_argmax_chunked(logits, scratch, out_tokens, rows, vocab, chunks, _stream())
         _done(code, "argmax", 2)
         return
-    code = _lib().lb_argmax(_ptr(logits), _ptr(out_tokens), c_int(rows), c_int(vocab), _stream())
+    code = _lib().lb_argmax(logits, out_tokens, rows, vocab, _stream())
     _done(code, "argmax")
 
 
@@ -2057,7 +2074,7 @@ def update_counts(counts: torch.Tensor, slots: torch.Tensor, add: torch.Tensor, 
     rows = slots.numel()
     if add.numel() != rows or remove.numel() != rows:
         raise KernelError("update_counts: slots, add and remove differ in length")
-    code = _lib().lb_update_counts(_ptr(counts), _ptr(slots), _ptr(add), _ptr(remove), c_int(rows), c_int(counts.shape[1]), _stream())
+    code = _lib().lb_update_counts(counts, slots, add, remove, rows, counts.shape[1], _stream())
     _done(code, "update_counts")
 
 
@@ -2077,29 +2094,25 @@ SKINNY_MAX_TOKENS = 16
 def skinny_supported(x: torch.Tensor, rows: int) -> bool:
     """Whether the weight-streaming kernel takes this product: bfloat16, 1..16 tokens, an input width
     that is a multiple of 32 and a multiple of 8 output rows."""
-    return (
-        x.dtype == torch.bfloat16
-        and x.dim() == 2
-        and 1 <= x.shape[0] <= SKINNY_MAX_TOKENS
-        and x.shape[1] % 32 == 0
-        and x.shape[1] >= 32
-        and rows % 8 == 0
-        and rows > 0
-    )
+    if x.dtype is not torch.bfloat16 or x.dim() != 2:
+        return False
+    tokens, width = x.shape
+    return 1 <= tokens <= SKINNY_MAX_TOKENS and width % 32 == 0 and width >= 32 and rows % 8 == 0 and rows > 0
 
 
 def _skinny(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, n: int, epilogue: str, activation: str = "identity", conv: dict | None = None,
             prefetch: bool = True, limit: float = 0.0, bias: torch.Tensor | None = None) -> None:
     """``prefetch``: the kernel asks for its weights towards L2 before it waits for the kernel before it; off where
     that kernel does not let it start early (see :func:`successor_starts_early`)."""
-    conv = conv or {}
-    code = _lib().lb_gemm_skinny(
-        _ptr(x), _ptr(weight), _ptr(out), c_int(x.shape[0]), c_int(x.shape[1]), c_int(n), c_int(_SKINNY_EPILOGUES[epilogue]),
-        c_int(_ACTIVATIONS[activation]), _ptr(conv.get("state")), _ptr(conv.get("weight")), _ptr(conv.get("bias")), _ptr(conv.get("token_segment")),
-        _ptr(conv.get("segment_start")), _ptr(conv.get("segment_length")), _ptr(conv.get("segment_slot")), c_int(conv.get("segments", 0)),
-        c_int(conv.get("taps", 0)), c_int(conv.get("num_slots", 0)), c_int(1 if prefetch else 0), _ptr(conv.get("status")), _stream(), c_float(limit),
-        _ptr(bias))
-    _done(code, f"gemm_skinny[{epilogue}]")
+    tokens, width = x.shape
+    if conv is None:
+        code = _lib().lb_gemm_skinny(x, weight, out, tokens, width, n, _SKINNY_EPILOGUES[epilogue], _ACTIVATIONS[activation], None, None, None, None, None, None, None, 0,
+                                     0, 0, 1 if prefetch else 0, None, _stream(), limit, bias)
+    else:
+        code = _lib().lb_gemm_skinny(x, weight, out, tokens, width, n, _SKINNY_EPILOGUES[epilogue], _ACTIVATIONS[activation], conv["state"], conv["weight"], conv["bias"],
+                                     conv["token_segment"], conv["segment_start"], conv["segment_length"], conv["segment_slot"], conv["segments"], conv["taps"],
+                                     conv["num_slots"], 1 if prefetch else 0, conv["status"], _stream(), limit, bias)
+    _done(code, "gemm_skinny")
 
 
 # Products of more than 16 tokens run on the tcgen05 kernel when this is on (LALAMO_B200_TCGEN05=0
@@ -2191,15 +2204,15 @@ def linear_tcgen05(x: torch.Tensor, weight: torch.Tensor, epilogue: str = "store
         scratch = torch.empty(slices, tokens, rows, dtype=torch.float32, device=x.device)
     elif slices > 1:
         needed = slices * tokens * rows
-        index = (x.device.index if x.device.index is not None else torch.cuda.current_device(), _stream().value or 0)
+        index = (x.device.index if x.device.index is not None else torch.cuda.current_device(), _stream())
         if index not in _tc_scratch or _tc_scratch[index].numel() < needed:
             if index in _tc_scratch:
                 _tc_retired.append(_tc_scratch[index])  # recorded graphs may still write there
             _tc_scratch[index] = torch.empty(max(needed, 1 << 22), dtype=torch.float32, device=x.device)
         scratch = _tc_scratch[index]
-    code = _lib().lb_gemm_tcgen05(_ptr(x), _ptr(weight), _ptr(out), _ptr(scratch), c_longlong(scratch.numel() if scratch is not None else 0),
-                                  c_int(tokens), c_int(width), c_int(rows), c_int(_TC_EPILOGUES[epilogue]), c_int(_ACTIVATIONS[activation]), c_int(slices),
-                                  c_int(1 if deferred else 0), _ptr(status), _stream(), c_float(limit))
+    code = _lib().lb_gemm_tcgen05(x, weight, out, scratch, scratch.numel() if scratch is not None else 0,
+                                  tokens, width, rows, _TC_EPILOGUES[epilogue], _ACTIVATIONS[activation], slices,
+                                  1 if deferred else 0, status, _stream(), limit)
     if code == -5:
         raise KernelError("linear_tcgen05: the driver gave no tensor map (cuTensorMapEncodeTiled)")
     _done(code, "gemm_tcgen05", 2 if slices > 1 and not deferred else 1)
@@ -2213,7 +2226,7 @@ def tcgen05_wait_probe(status: torch.Tensor, nanoseconds: int = 1_000_000) -> No
     (after ``nanoseconds``, at most 0.1 s) and report it in ``status``, as a product would whose
     copy or arrival got lost."""
     _check(status, "status", torch.int32)
-    _done(_lib().lb_tcgen05_wait_probe(_ptr(status), c_longlong(nanoseconds), _stream()), "tcgen05_wait_probe")
+    _done(_lib().lb_tcgen05_wait_probe(status, nanoseconds, _stream()), "tcgen05_wait_probe")
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype | None = None, status: torch.Tensor | None = None) -> torch.Tensor:
@@ -2222,14 +2235,15 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype | None 
     kernel, everything else to the library."""
     _check(x, "x")
     _check(weight, "weight", x.dtype)
-    if x.shape[-1] != weight.shape[1]:
-        raise KernelError(f"linear: input width {x.shape[-1]} does not match the weight's {weight.shape[1]}")
+    rows, width = weight.shape
+    if x.shape[-1] != width:
+        raise KernelError(f"linear: input width {x.shape[-1]} does not match the weight's {width}")
     wants_float = out_dtype is not None and out_dtype != x.dtype
-    if USE_TCGEN05 and x.shape[0] <= SKINNY_MAX_TOKENS and weight.shape[0] >= TCGEN05_MIN_ROWS_FEW_TOKENS and tcgen05_supported(x, weight.shape[0]):
+    if USE_TCGEN05 and x.shape[0] <= SKINNY_MAX_TOKENS and rows >= TCGEN05_MIN_ROWS_FEW_TOKENS and tcgen05_supported(x, rows):
         return linear_tcgen05(x, weight, "store_float" if wants_float else "store", slices=1, status=status)
-    if skinny_supported(x, weight.shape[0]):
-        out = torch.empty(x.shape[0], weight.shape[0], dtype=torch.float32 if wants_float else x.dtype, device=x.device)
-        _skinny(x, weight, out, weight.shape[0], "store_float" if wants_float else "store")
+    if skinny_supported(x, rows):
+        out = torch.empty(x.shape[0], rows, dtype=torch.float32 if wants_float else x.dtype, device=x.device)
+        _skinny(x, weight, out, rows, "store_float" if wants_float else "store")
         return out
     if USE_TCGEN05 and tcgen05_supported(x, weight.shape[0]):
         return linear_tcgen05(x, weight, "store_float" if wants_float else "store", status=status)
@@ -2273,8 +2287,8 @@ def linear_bias_activation(x: torch.Tensor, weight: torch.Tensor, bias: torch.Te
         return out
     if USE_TCGEN05 and tcgen05_supported(x, weight.shape[0]):
         out = torch.empty(x.shape[0], weight.shape[0], dtype=x.dtype, device=x.device)
-        code = _lib().lb_gemm_tcgen05_bias_activation(_ptr(x), _ptr(weight), _ptr(bias), _ptr(out), c_int(x.shape[0]), c_int(x.shape[1]), c_int(weight.shape[0]),
-                                                      c_int(_ACTIVATIONS[activation]), _ptr(status), _stream())
+        code = _lib().lb_gemm_tcgen05_bias_activation(x, weight, bias, out, x.shape[0], x.shape[1], weight.shape[0],
+                                                      _ACTIVATIONS[activation], status, _stream())
         if code == -5:
             raise KernelError("linear_bias_activation: the driver gave no tensor map (cuTensorMapEncodeTiled)")
         _done(code, "gemm_tcgen05_bias_activation")
