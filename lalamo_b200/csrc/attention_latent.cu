@@ -265,7 +265,7 @@ __global__ void gate_heads_kernel(const T* __restrict__ values, const T* __restr
 // (ldmatrix.trans).  Rows that no query of the item sees are zero-filled, never read.  grid.z shares out the latent's
 // channels in chunks of CHUNK (128, or 256 for latents wider than 128; every chunk computes the scores again); grid.y = head blocks x key splits: with splits > 1
 // every CTA takes a share of the item's blocks and leaves (maximum, sum, unnormalised O) for latent_merge_kernel.
-constexpr int kLatentMmaRows = 64, kLatentMmaKeys = 64, kLatentMmaThreads = 128;
+constexpr int kLatentMmaKeys = 64;
 
 struct LatentMmaParams {
     const __nv_bfloat16* q;       // [tokens][heads][latent + rope]
@@ -318,14 +318,19 @@ __device__ __forceinline__ uint32_t latent_pack(float low, float high) {
     return *reinterpret_cast<const uint32_t*>(&pair);
 }
 
-template <int CHUNK>
-__global__ void __launch_bounds__(kLatentMmaThreads)
+// WARPS of 16 query rows each: four, or eight for runs of more than 64 rows.  A multiprocessor's shared memory holds one CTA of either
+// (115 and 152 KB at 256 + 32 channels), so that with four warps every scheduler has one, which waits for its own loads; eight also share what
+// is loaded of the cached rows.  Measured, 16 heads over 256 + 32 channels, 1,023 tokens behind 1,500 cached ones under a window of 2,048: 251 us,
+// 331 us with four warps (and two CTAs an item, merged); bound by each warp's chain of loads, products and softmax, at a quarter of
+// what mma.sync reaches.
+template <int CHUNK, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS)
 latent_attention_mma_kernel(LatentMmaParams p) {
-    constexpr int kLatentMmaChunk = CHUNK;
+    constexpr int kLatentMmaChunk = CHUNK, kLatentMmaRows = 16 * WARPS, kLatentMmaThreads = 32 * WARPS;
     extern __shared__ __align__(16) unsigned char latent_shared[];
     const int latent = p.layout.latent, full = p.layout.latent + p.layout.rope;
     const int pitch = full + 8;   // elements: rows 16 bytes apart modulo 128, so that ldmatrix meets no bank twice
-    __nv_bfloat16* q_s = reinterpret_cast<__nv_bfloat16*>(latent_shared);          // [64][pitch]
+    __nv_bfloat16* q_s = reinterpret_cast<__nv_bfloat16*>(latent_shared);          // [16 WARPS][pitch]
     __nv_bfloat16* k_s = q_s + kLatentMmaRows * pitch;                             // [2][64][pitch]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int item = gridDim.x - 1 - blockIdx.x;   // a prompt's last items see the most rows: they start first
@@ -391,7 +396,7 @@ latent_attention_mma_kernel(LatentMmaParams p) {
     asm volatile("cp.async.commit_group;\n" ::: "memory");
 
     const int g = lane >> 2, t = lane & 3;
-    const int row_a = warp * 16 + g, row_b = row_a + 8;   // this thread's two rows of the CTA's 64
+    const int row_a = warp * 16 + g, row_b = row_a + 8;   // this thread's two rows of the CTA's
     const bool warp_active = warp * 16 < rows_used;
     const int position_a = position0 + (row_a < rows_used ? row_a / heads_here : 0);
     const int position_b = position0 + (row_b < rows_used ? row_b / heads_here : 0);
@@ -749,7 +754,7 @@ int lb_latent_attention_plain(const void* q, const void* pages, void* out, const
 }
 
 // bfloat16; latent and rope multiples of 16, page sizes that are multiples of 16.  items: [num_items][2] (first token row, count),
-// each at most tokens_per_cta consecutive tokens of one request; heads_per_cta * tokens_per_cta <= 64.  partial: splits > 1 only,
+// each at most tokens_per_cta consecutive tokens of one request; heads_per_cta * tokens_per_cta <= 128 (more than 64 take eight warps).  partial: splits > 1 only,
 // [tokens][heads][splits][latent + 2] floats.  Returns -2 for sizes it does not take.
 int lb_latent_attention_mma(const void* q, const void* pages, void* out, float* partial, const int* items, int num_items, const int* positions,
                             const int* token_segment, const int* block_table, int tokens, int num_heads, int latent, int rope, int page_size,
@@ -757,15 +762,17 @@ int lb_latent_attention_mma(const void* q, const void* pages, void* out, float* 
                             cudaStream_t stream, const float* sink) {
     if (num_items == 0 || tokens == 0) return 0;
     if (latent < 16 || latent % 16 != 0 || rope % 16 != 0 || page_size % 16 != 0 || heads_per_cta < 1 || tokens_per_cta < 1 ||
-        heads_per_cta * tokens_per_cta > lb::kLatentMmaRows || splits < 1 || (splits > 1 && partial == nullptr))
+        heads_per_cta * tokens_per_cta > 128 || splits < 1 || (splits > 1 && partial == nullptr))
         return -2;
     const int full = latent + rope;
-    const size_t shared = static_cast<size_t>(3) * lb::kLatentMmaRows * (full + 8) * sizeof(__nv_bfloat16);
+    const int warps = heads_per_cta * tokens_per_cta > 64 ? 8 : 4;
+    const size_t shared = static_cast<size_t>(16 * warps + 2 * lb::kLatentMmaKeys) * (full + 8) * sizeof(__nv_bfloat16);
     if (shared > 227 * 1024) return -2;
-    static lb::OncePerDevice once_narrow, once_wide;
+    static lb::OncePerDevice once[4];
     const bool wide = latent > 128;   // 256 channels of the sums per CTA: twice the accumulators, the scores computed half as often
-    const cudaError_t allowed = wide ? lb::allow_shared_memory(once_wide, lb::latent_attention_mma_kernel<256>, 227 * 1024)
-                                     : lb::allow_shared_memory(once_narrow, lb::latent_attention_mma_kernel<128>, 227 * 1024);
+    auto kernel = wide ? (warps == 8 ? lb::latent_attention_mma_kernel<256, 8> : lb::latent_attention_mma_kernel<256, 4>)
+                       : (warps == 8 ? lb::latent_attention_mma_kernel<128, 8> : lb::latent_attention_mma_kernel<128, 4>);
+    const cudaError_t allowed = lb::allow_shared_memory(once[(wide ? 2 : 0) + (warps == 8 ? 1 : 0)], kernel, 227 * 1024);
     if (allowed != cudaSuccess) return static_cast<int>(allowed);
     lb::LatentMmaParams p;
     p.q = static_cast<const __nv_bfloat16*>(q);
@@ -788,11 +795,7 @@ int lb_latent_attention_mma(const void* q, const void* pages, void* out, float* 
     p.sink = sink;
     const int chunk = wide ? 256 : 128;
     const dim3 grid(num_items, p.head_blocks * splits, (latent + chunk - 1) / chunk);
-    if (wide) {
-        lb::latent_attention_mma_kernel<256><<<grid, lb::kLatentMmaThreads, shared, stream>>>(p);
-    } else {
-        lb::latent_attention_mma_kernel<128><<<grid, lb::kLatentMmaThreads, shared, stream>>>(p);
-    }
+    kernel<<<grid, 32 * warps, shared, stream>>>(p);
     if (splits > 1) lb::latent_merge_kernel<<<tokens * num_heads, 128, splits * sizeof(float), stream>>>(partial, static_cast<__nv_bfloat16*>(out), splits, latent, sink, num_heads);
     return LB_LAUNCH_RESULT();
 }

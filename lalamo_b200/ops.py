@@ -1510,8 +1510,15 @@ def latent_attention_tiling(num_heads: int) -> tuple[int, int]:
     return heads, max(1, LATENT_MMA_ROWS // heads)
 
 
-def latent_attention_splits(num_items: int, num_heads: int, latent: int, window: int | None, max_context: int, sms: int | None = None) -> int:
-    """Over how many CTAs an item's cached rows are shared out: 1 where the items fill the GPU by themselves."""
+def latent_attention_takes_double(latent: int, rope: int) -> bool:
+    """Whether :func:`latent_attention` takes runs of twice as many tokens (``double``): eight warps' rows beside two blocks of cached ones
+    have to fit the shared memory."""
+    return (128 + 2 * 64) * (latent + rope + 8) * 2 <= 227 * 1024
+
+
+def latent_attention_splits(num_items: int, num_heads: int, latent: int, window: int | None, max_context: int, sms: int | None = None, double: bool = False) -> int:
+    """Over how many CTAs an item's cached rows are shared out: 1 where the items fill the GPU by themselves.  CTAs of eight warps (``double``)
+    hold a multiprocessor each, so that two thirds of a round of them are left as they are: merging costs 22 us for 1,023 tokens of 16 heads."""
     heads, tokens = latent_attention_tiling(num_heads)
     ctas = num_items * -(-num_heads // heads) * -(-latent // (256 if latent > 128 else 128))
     sms = sms or sm_count()
@@ -1519,15 +1526,17 @@ def latent_attention_splits(num_items: int, num_heads: int, latent: int, window:
     blocks = -(-(rows + tokens) // 64) + 1
     if ctas >= 2 * sms or blocks <= 2:
         return 1
+    if double:
+        return max(1, min(blocks // 2, 3 * sms // 2 // ctas, 32))
     return max(1, min(blocks // 2, -(-2 * sms // ctas), 32))   # two blocks a CTA: one block each was measured 1 % slower
 
 
 def latent_attention(q: torch.Tensor, pages: torch.Tensor, out: torch.Tensor, *, items: torch.Tensor, num_items: int, positions: torch.Tensor,
                      token_segment: torch.Tensor, block_table: torch.Tensor, num_heads: int, latent: int, rope: int, scale: float, window: int | None,
-                     status: torch.Tensor, splits: int = 1, sink: torch.Tensor | None = None) -> None:
+                     status: torch.Tensor, splits: int = 1, sink: torch.Tensor | None = None, double: bool = False) -> None:
     """:func:`latent_attention_plain` on the tensor cores (bfloat16).  ``items``: int32 ``[num_items, 2]`` (first token row,
-    count), each at most ``latent_attention_tiling(num_heads)[1]`` consecutive tokens of one request, together all tokens.
-    ``splits`` > 1 shares an item's cached rows out over that many CTAs, merged in split order.  ``sink``: as for
+    count), each at most ``latent_attention_tiling(num_heads)[1]`` consecutive tokens of one request (twice as many with
+    ``double``, where :func:`latent_attention_takes_double`), together all tokens.  ``splits`` > 1 shares an item's cached rows out over that many CTAs, merged in split order.  ``sink``: as for
     :func:`latent_attention_plain`."""
     _check_sink(sink, num_heads)
     _check(q, "q", torch.bfloat16)
@@ -1540,6 +1549,10 @@ def latent_attention(q: torch.Tensor, pages: torch.Tensor, out: torch.Tensor, *,
     if pages.dtype != q.dtype or not latent_attention_supported(q.dtype, latent, rope, page_size):
         raise KernelError(f"latent_attention: latent {latent}, rope {rope}, pages of {page_size} are not sizes the tensor-core kernel takes")
     heads_per_cta, tokens_per_cta = latent_attention_tiling(num_heads)
+    if double:
+        if not latent_attention_takes_double(latent, rope):
+            raise KernelError(f"latent_attention: rows of {latent} + {rope} channels leave no room for runs of twice as many tokens")
+        tokens_per_cta *= 2
     partial = torch.empty(tokens, num_heads, splits, latent + 2, dtype=torch.float32, device=q.device) if splits > 1 else None
     code = _lib().lb_latent_attention_mma(q, pages, out, partial, items, num_items, positions, token_segment,
                                           block_table, tokens, num_heads, latent, rope, page_size, num_pages,

@@ -76,6 +76,7 @@ class LatentAttention(Mixer):
         self.sink = runtime.vector(tensors["sink"]) if spec.sink else None
         self.position = build_part(spec.position, {}, runtime)
         self.scale = spec.scale if spec.scale is not None else (dim + rope) ** -0.5
+        self.takes_double = ops.latent_attention_takes_double(spec.latent_dim, rope)
 
     @classmethod
     def tensor_decls(cls, spec: LatentAttentionSpec) -> dict[str, TensorDecl]:
@@ -111,11 +112,14 @@ class LatentAttention(Mixer):
     step_plan_uses_context = False
 
     def step_plan_key(self) -> object:
-        return ("latent_attention", ops.latent_attention_tiling(self.spec.num_heads))
+        return ("latent_attention", ops.latent_attention_tiling(self.spec.num_heads), self.takes_double)
 
     def plan_step(self, segments: HostSegments) -> dict[str, np.ndarray]:
-        """``items``: ``(first row, count)`` of every run of consecutive tokens that one CTA takes."""
+        """``items``: ``(first row, count)`` of every run of consecutive tokens that one CTA takes (twice as many a run where some portion
+        fills such runs)."""
         _, run = ops.latent_attention_tiling(self.spec.num_heads)
+        if self.takes_double and max(segments.length, default=0) > run:
+            run *= 2
         items = [(first, min(run, start + length - first)) for start, length in zip(segments.start, segments.length) for first in range(start, start + length, run)]
         return {"items": np.asarray(items, dtype=np.int32).reshape(-1)}
 
@@ -164,8 +168,9 @@ class LatentAttention(Mixer):
         if ops.latent_attention_supported(runtime.dtype, latent, rope, cache.k_pages.shape[1]):
             lists, host_lists = step.plan_of(self)
             num_items = host_lists["items"].size // 2
-            splits = ops.latent_attention_splits(num_items, heads, latent, spec.window, step.max_context)
-            ops.latent_attention(queries, cache.k_pages, summed, items=lists["items"], num_items=num_items, splits=splits, **common)
+            double = num_items > 0 and int(host_lists["items"][1::2].max()) > ops.latent_attention_tiling(heads)[1]
+            splits = ops.latent_attention_splits(num_items, heads, latent, spec.window, step.max_context, double=double)
+            ops.latent_attention(queries, cache.k_pages, summed, items=lists["items"], num_items=num_items, splits=splits, double=double, **common)
         else:
             ops.latent_attention_plain(queries, cache.k_pages, summed, **common)
         mixed = runtime.empty(tokens, heads * spec.value_dim)
