@@ -34,6 +34,7 @@ struct TcParams {
     int hidden;         // kTcGated: W is [2 * hidden, k], rows [up ; gate]; out is [tokens, hidden]
     int activation;
     float limit;        // of activation 3 (the limited sigmoid gate, see common.cuh)
+    int tile_tokens;    // the walking kernel: tokens a tile, a multiple of 32, at most BN
     int bulk_store;     // the walking kernel writes its output by bulk tensor stores (rows of the output 16-byte aligned)
     int early_successor;   // the one-tile kernel lets the kernel after it start before it has finished
     int* status;
@@ -299,7 +300,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 }
 
 // ---------------------------------------------------------------------------------------------
-// The same product for many tokens (prefill): tiles of 128 rows of W x 256 tokens, one CTA per SM that
+// The same product for many tokens (prefill): tiles of 128 rows of W x up to 256 tokens, one CTA per SM that
 // walks tiles m + n * m_tiles in steps of the grid, and two accumulators in tensor memory, so that the
 // epilogue of a tile (tensor memory -> registers -> the output, by eight warps) runs while the
 // products of the next tile are issued.  All of K per tile; epilogues as above except the partial one.
@@ -319,6 +320,9 @@ struct PersistShape {
     static constexpr int kStages = 4 * 48 * 1024 / kStageBytes;
     static_assert(kStages * kStageBytes == 4 * 48 * 1024 && kStages <= 8, "the stages fill 192 KB");
 };
+// What a tile costs beside its tokens, in tokens: a round of tiles of 256 takes 15.5 us and one of 128 takes 12.4 us at 2,048 columns (the
+// tiles of W come through L2 whatever the tokens).
+constexpr int kTileCost = 384;
 constexpr int kPersistExchangePitch = 80;   // bytes a thread's 32 activated gates take (64) and 16 to spread the banks
 constexpr int kPersistRegionBytes = 16 * 1024;   // per half of the epilogue: two output buffers of 8 KB, or (gated) two of 4 KB and the exchange
 constexpr int kPersistExchangeBytes = 2 * kPersistRegionBytes;
@@ -332,7 +336,7 @@ __global__ void __launch_bounds__(kPersistThreads)
 gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                                const __grid_constant__ CUtensorMap map_out, const TcParams p, int m_tiles, int n_tiles, int slices) {
     constexpr int STAGES = PersistShape<BN, PAIR>::kStages, kPersistStageBytes = PersistShape<BN, PAIR>::kStageBytes;
-    constexpr int kXTokens = PersistShape<BN, PAIR>::kXTokens;
+    const int tile_tokens = p.tile_tokens, x_tokens = PAIR ? tile_tokens / 2 : tile_tokens;   // of a tile, and what of it a CTA loads
     // With PAIR the walkers are the pairs: `walker` of `walkers`, and `rank` within the pair; m_tiles
     // counts tiles of both CTAs' rows.
     const int rank = PAIR ? static_cast<int>(cluster_rank()) : 0;
@@ -400,7 +404,7 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const 
         bool ok = true;
         const int early = walker < num_items ? min(STAGES, block_count(walker)) : 0;
         auto arm = [&](int s) {
-            if (rank == 0) barrier_expect(&full[s], (PAIR ? 2 : 1) * kPersistStageBytes);
+            if (rank == 0) barrier_expect(&full[s], (PAIR ? 2 : 1) * (kWBytes + x_tokens * kTcBlockK * 2));
         };
         auto load = [&](unsigned char* destination, const CUtensorMap* map, int x, int y, int s) {
             if constexpr (PAIR) tma_load_2d_pair(destination, map, x, y, cluster_address(&full[s], 0));
@@ -415,11 +419,11 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const 
         }
         wait_for_previous_kernel();
         for (int block = 0; block < early; ++block)
-            load(tiles + block * kPersistStageBytes + kWBytes, &map_x, (first_block(walker) + block) * kTcBlockK, ((walker % num_tiles) / m_tiles) * BN + rank * kXTokens, block);
+            load(tiles + block * kPersistStageBytes + kWBytes, &map_x, (first_block(walker) + block) * kTcBlockK, ((walker % num_tiles) / m_tiles) * tile_tokens + rank * x_tokens, block);
         issued = early;
         for (int item = walker; item < num_items && ok; item += walkers) {
             const int tile = item % num_tiles;
-            const int row0 = (tile % m_tiles) * rows_per_tile + rank * rows_per_cta, token0 = (tile / m_tiles) * BN + rank * kXTokens;
+            const int row0 = (tile % m_tiles) * rows_per_tile + rank * rows_per_cta, token0 = (tile / m_tiles) * tile_tokens + rank * x_tokens;
             const int first = first_block(item), count = block_count(item);
             for (int block = item == walker ? early : 0; block < count; ++block, ++issued) {
                 const int s = issued % STAGES, round = issued / STAGES;
@@ -437,7 +441,8 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const 
             }
         }
     } else if (warp == 1 && lane == 0 && rank == 0) {
-        constexpr uint32_t idesc = PAIR ? instruction_descriptor_pair<BN>() : instruction_descriptor<BN>();
+        // as instruction_descriptor and instruction_descriptor_pair, for the tile's tokens
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(tile_tokens >> 3) << 17) | (static_cast<uint32_t>((PAIR ? 256 : 128) >> 4) << 24);
         int consumed = 0, local = 0;
         bool ok = true;
         for (int item = walker; item < num_items && ok; item += walkers, ++local) {
@@ -479,6 +484,8 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const 
         // 64 (bfloat16) bytes in the output, so that nothing has to be turned in shared memory.
         wait_for_previous_kernel();   // before anything of the output is read or written
         const int quarter = warp & 3, half = (warp - 2) >> 2;
+        // the tile's tokens in two parts of whole 32
+        const int lower_part = (tile_tokens / 2 + 31) / 32 * 32, part_begin = half ? lower_part : 0, part_tokens = half ? tile_tokens - lower_part : lower_part;
         const int half_barrier = 5 + half;   // 1..4 belong to the pairs of warps of the gated epilogue
         const bool issuer = quarter == 0 && lane == 0;
         unsigned char* region = exchange + half * kPersistRegionBytes;
@@ -486,7 +493,7 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const 
         for (int item = walker; item < num_items; item += walkers, ++local) {
             const int accumulator = local & 1, use = local >> 1;
             const int tile = item % num_tiles, slice = item / num_tiles;
-            const int row0 = (tile % m_tiles) * rows_per_tile + rank * rows_per_cta, token0 = (tile / m_tiles) * BN + half * (BN / 2);
+            const int row0 = (tile % m_tiles) * rows_per_tile + rank * rows_per_cta, token0 = (tile / m_tiles) * tile_tokens + part_begin;
             uint32_t arrived = barrier_wait(&tmem_full[accumulator], use & 1) ? 1u : 0u;
             {
                 // Warps that meet at named barriers below go on together or not at all.
@@ -508,7 +515,7 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const 
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(accumulator * BN + half * (BN / 2)) + (static_cast<uint32_t>(quarter * 32) << 16);
+            const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(accumulator * BN + part_begin) + (static_cast<uint32_t>(quarter * 32) << 16);
             // Where the output's rows are 16-byte aligned it leaves by bulk tensor stores: the four
             // warps of a half set 32 tokens (16 of float32) x 128 rows down in shared memory, token by
             // token as the output has them, and one thread sends the box off.  Stores issued by the
@@ -520,7 +527,7 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const 
             const bool transformed = p.epilogue == kTcStore && p.store_activation >= 0;
             const float bias_here = transformed && p.bias != nullptr && row0 + quarter * 32 + lane < p.n ? p.bias[row0 + quarter * 32 + lane] : 0.0f;
 #pragma unroll 1
-            for (int column = 0; p.bulk_store && column < BN / 2; column += step, ++groups) {
+            for (int column = 0; p.bulk_store && column < part_tokens; column += step, ++groups) {
                 if (token0 + column >= p.tokens) break;   // the same for the whole half
                 unsigned char* out_buffer = region + (groups & 1) * (gated ? 4096 : 8192);
                 // the store before last, which read this buffer, has read it
@@ -593,7 +600,7 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const 
                 }
             }
 #pragma unroll 1
-            for (int column = 0; !p.bulk_store && column < BN / 2; column += 32) {
+            for (int column = 0; !p.bulk_store && column < part_tokens; column += 32) {
                 if (token0 + column >= p.tokens) break;   // the same for the whole warp
                 uint32_t v[32];
                 tmem_load_32(tmem_d + static_cast<uint32_t>(column), v);
@@ -829,9 +836,10 @@ static bool make_partial_map(CUtensorMap* map, void* base, int slices, int token
 }
 
 template <int BN, bool PAIR>
-int launch_persistent(const CUtensorMap& map_w, const void* x, TcParams p, int m_tiles, int sms, int slices, cudaStream_t stream) {
+int launch_persistent(const CUtensorMap& map_w, const void* x, TcParams p, int m_tiles, int sms, int slices, cudaStream_t stream, int tile_tokens = BN) {
     CUtensorMap map_x;
-    if (!make_map(&map_x, x, p.tokens, p.k, PersistShape<BN, PAIR>::kXTokens)) return -5;
+    p.tile_tokens = tile_tokens;
+    if (!make_map(&map_x, x, p.tokens, p.k, PAIR ? tile_tokens / 2 : tile_tokens)) return -5;
     const bool is_partial = p.epilogue == kTcPartial;
     const bool is_float = p.epilogue == kTcStoreFloat || p.epilogue == kTcResidualAdd || is_partial, is_gated = p.epilogue == kTcGated;
     const int width = is_gated ? p.hidden : p.n;
@@ -842,7 +850,7 @@ int launch_persistent(const CUtensorMap& map_w, const void* x, TcParams p, int m
     auto kernel = gemm_tcgen05_persistent_kernel<BN, PAIR>;
     static OncePerDevice configured;
     if (allow_shared_memory(configured, kernel, kPersistSharedBytes) != cudaSuccess) return static_cast<int>(cudaGetLastError());
-    const int n_tiles = (p.tokens + BN - 1) / BN;
+    const int n_tiles = (p.tokens + tile_tokens - 1) / tile_tokens;
     const int items = m_tiles * n_tiles * slices;
     if constexpr (!PAIR) {
         const int grid = items < sms ? items : sms;
@@ -866,6 +874,21 @@ int launch_persistent(const CUtensorMap& map_w, const void* x, TcParams p, int m
         config.numAttrs = 2;
         return static_cast<int>(cudaLaunchKernelEx(&config, kernel, map_w, map_x, map_out, p, m_tiles, n_tiles, slices));
     }
+}
+
+// Tokens of a tile of the walking kernel with tiles of up to 256: instructions take any number of columns, so tiles are made equal (and whole
+// 32s) instead of leaving the last one partly empty, and narrower where that fills the walkers' rounds better.  Measured against tiles of
+// 256: 777 tokens x [13824, 1536] gated 48.1 and 51.2 us, 2,048 tokens x [3072, 2048] (tiles of 192) 33.8 and 35.8, 600 tokens x
+// [9216, 1024] gated 28.7 and 31.6.
+inline int even_tile_tokens(int tokens, int row_tiles, int walkers, int slices) {
+    int best = 256;
+    long long best_cost = -1;
+    for (int n_tiles = (tokens + 255) / 256; n_tiles <= (tokens + 127) / 128; ++n_tiles) {
+        const int tile = ((tokens + n_tiles - 1) / n_tiles + 31) / 32 * 32;
+        const long long rounds = (static_cast<long long>(row_tiles) * n_tiles * slices + walkers - 1) / walkers, cost = rounds * (tile + kTileCost);
+        if (best_cost < 0 || cost < best_cost) best = tile, best_cost = cost;
+    }
+    return best;
 }
 
 }  // namespace lb
@@ -950,10 +973,10 @@ static int gemm_tcgen05_launch(const void* x, const void* w, void* out, float* s
         int tile = tiles_64 <= sms ? 64 : tiles_128 <= sms ? 128 : narrow_cost * 18 < wide_cost * 25 / 2 ? 128 : 256;
         if (tile == 256 && (epilogue == lb::kTcGated || work >= 12000)) tile = 512;   // the pair
         if (const char* forced = getenv("LALAMO_B200_TCGEN05_TILE")) tile = atoi(forced);
-        if (tile == 512) return lb::launch_persistent<256, true>(map_w, x, p, (m_tiles + 1) / 2, sms, 1, stream);
+        if (tile == 512) return lb::launch_persistent<256, true>(map_w, x, p, (m_tiles + 1) / 2, sms, 1, stream, lb::even_tile_tokens(tokens, (m_tiles + 1) / 2, sms / 2, 1));
         if (tile == 64) return lb::launch_persistent<64, false>(map_w, x, p, m_tiles, sms, 1, stream);
         if (tile == 128) return lb::launch_persistent<128, false>(map_w, x, p, m_tiles, sms, 1, stream);
-        return lb::launch_persistent<256, false>(map_w, x, p, m_tiles, sms, 1, stream);
+        return lb::launch_persistent<256, false>(map_w, x, p, m_tiles, sms, 1, stream, lb::even_tile_tokens(tokens, m_tiles, sms, 1));
     }
     static const bool walk_slices = []() {
         const char* setting = getenv("LALAMO_B200_TCGEN05_WALK_SLICES");
@@ -967,9 +990,10 @@ static int gemm_tcgen05_launch(const void* x, const void* w, void* out, float* s
         const int m_tiles = (n + lb::kTcRows - 1) / lb::kTcRows;
         int tile = 256;
         if (const char* forced = getenv("LALAMO_B200_TCGEN05_TILE")) tile = atoi(forced);
-        if (tile == 512) code = lb::launch_persistent<256, true>(map_w, x, p, (m_tiles + 1) / 2, sms, slices, stream);
+        const int even = ((tokens + (tokens + 255) / 256 - 1) / ((tokens + 255) / 256) + 31) / 32 * 32;   // the slices are counted for tiles of 256
+        if (tile == 512) code = lb::launch_persistent<256, true>(map_w, x, p, (m_tiles + 1) / 2, sms, slices, stream, even);
         else if (tile == 128) code = lb::launch_persistent<128, false>(map_w, x, p, m_tiles, sms, slices, stream);
-        else code = lb::launch_persistent<256, false>(map_w, x, p, m_tiles, sms, slices, stream);
+        else code = lb::launch_persistent<256, false>(map_w, x, p, m_tiles, sms, slices, stream, even);
         if (code != 0 || defer_sum) return code;
         return lb_sum_slices(scratch, out, tokens, n, slices, epilogue, stream);
     }
