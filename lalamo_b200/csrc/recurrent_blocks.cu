@@ -206,14 +206,33 @@ __device__ __forceinline__ void between_halves(float* a_s, float* bt_s, const fl
     bt_s[j * TP + i] = b;
 }
 
-// grid (blocks, heads).  Block `b` of `chunk_*`'s chunks of `subs` blocks each: tokens chunk_start[b / subs] + 32 (b % subs) and so on.
+// The blocks of all long portions are numbered through: portion 0's, portion 1's, and so on.
+struct PortionBlock {
+    int portion, block;   // block < 0: there is no such block
+};
+__device__ __forceinline__ int blocks_before(const int* __restrict__ long_table, const int* __restrict__ segment_length, int entry) {
+    int blocks = 0;
+    for (int i = 0; i < entry; ++i) blocks += (segment_length[long_table[3 * i]] + kBlockTokens - 1) / kBlockTokens;
+    return blocks;
+}
+__device__ __forceinline__ PortionBlock find_block(const int* __restrict__ long_table, const int* __restrict__ segment_length, int long_portions, int index) {
+    for (int i = 0; i < long_portions; ++i) {
+        const int portion = long_table[3 * i], blocks = (segment_length[portion] + kBlockTokens - 1) / kBlockTokens;
+        if (index < blocks) return PortionBlock{portion, index};
+        index -= blocks;
+    }
+    return PortionBlock{0, -1};
+}
+
+// grid (blocks, heads).  blockIdx.x is a block's number among those of the long portions that `long_table` lists (rows of three numbers, the
+// first of which is the portion).
 //   q, k [tokens, groups, dk], g [tokens, heads, dk], v [tokens, heads, dv], beta [tokens, heads]
 //   pack [block][head][BlockPack::kFloats], vpack [block][head][ceil(dv / 8)][BlockPack::kValues]
 template <int DKP>
 __global__ void __launch_bounds__(kBlockThreads, DKP <= 128 ? 3 : 1)
 recurrent_prepare_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ g, const float* __restrict__ v,
-                         const float* __restrict__ beta, float* __restrict__ pack, float* __restrict__ vpack, const int* __restrict__ chunk_start,
-                         const int* __restrict__ chunk_length, int subs, int heads, int groups, int dk, int dv) {
+                         const float* __restrict__ beta, float* __restrict__ pack, float* __restrict__ vpack, const int* __restrict__ long_table, int long_portions, const int* __restrict__ segment_start,
+                const int* __restrict__ segment_length, int heads, int groups, int dk, int dv) {
     using Pack = BlockPack<DKP>;
     using Shared = PrepareShared<DKP>;
     constexpr int P = Shared::kPitch, VP = Shared::kValuePitch, TP = kTrianglePitch;
@@ -227,10 +246,10 @@ recurrent_prepare_kernel(const float* __restrict__ q, const float* __restrict__ 
     float* tt_s = bt_s + 32 * TP;           // T[i][j] at [j][i]
     float* d_half = tt_s + 32 * TP;         // the decays' product over the lower half
     float* beta_s = d_half + DKP;
-    const int chunk = blockIdx.x / subs, first = kBlockTokens * (blockIdx.x % subs);
-    const int n = min(kBlockTokens, chunk_length[chunk] - first);
-    if (n <= 0) return;
-    const int start = chunk_start[chunk] + first, head = blockIdx.y, group = head / (heads / groups);
+    const PortionBlock here = find_block(long_table, segment_length, long_portions, blockIdx.x);
+    if (here.block < 0) return;
+    const int first = kBlockTokens * here.block, n = min(kBlockTokens, segment_length[here.portion] - first);
+    const int start = segment_start[here.portion] + first, head = blockIdx.y, group = head / (heads / groups);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     float* out = pack + (static_cast<size_t>(blockIdx.x) * heads + head) * Pack::kFloats;
     const int slices = (dv + kWalkCols - 1) / kWalkCols;
@@ -401,12 +420,11 @@ struct WalkShared {
     static constexpr int kBytes = kFloats * 4;
 };
 
-// grid (long portions, heads, ceil(dv / 8)).  long_table rows: (portion, first chunk, chunks); a portion's blocks follow one another from
-// block `first chunk * subs` on.
+// grid (long portions, heads, ceil(dv / 8)).
 template <int DKP>
 __global__ void __launch_bounds__(kBlockThreads, DKP <= 64 ? 2 : 1)
 recurrent_walk_kernel(const float* __restrict__ pack, const float* __restrict__ vpack, float* __restrict__ state, float* __restrict__ out,
-                      const int* __restrict__ long_table, int subs, const int* __restrict__ segment_start, const int* __restrict__ segment_length,
+                      const int* __restrict__ long_table, const int* __restrict__ segment_start, const int* __restrict__ segment_length,
                       const int* __restrict__ segment_slot, int heads, int dk, int dv, int num_slots, int* status) {
     using Pack = BlockPack<DKP>;
     using Shared = WalkShared<DKP>;
@@ -419,7 +437,7 @@ recurrent_walk_kernel(const float* __restrict__ pack, const float* __restrict__ 
     float* part_s = walk_memory + kStages * Shared::kStage;
     float* state_s = part_s + 16 * 256;                 // [DKP][8]
     float* u_s = state_s + DKP * kWalkCols;             // [32][8]
-    const int portion = long_table[3 * blockIdx.x], first_block = long_table[3 * blockIdx.x + 1] * subs;
+    const int portion = long_table[3 * blockIdx.x], first_block = blocks_before(long_table, segment_length, blockIdx.x);
     const int head = blockIdx.y, slice = blockIdx.z, column0 = slice * kWalkCols, slices = gridDim.z;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int slot = segment_slot[portion];
@@ -554,7 +572,8 @@ recurrent_walk_kernel(const float* __restrict__ pack, const float* __restrict__ 
 template <int DKP>
 __global__ void __launch_bounds__(kBlockThreads, DKP <= 128 ? 3 : 1)
 linear_prepare_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ g, const float* __restrict__ v, float* __restrict__ sums,
-                      float* __restrict__ decays, float* __restrict__ out, const int* __restrict__ chunk_start, const int* __restrict__ chunk_length, int subs, int heads,
+                      float* __restrict__ decays, float* __restrict__ out, const int* __restrict__ long_table, int long_portions, const int* __restrict__ segment_start,
+                const int* __restrict__ segment_length, int heads,
                       int groups, int dk, int dv) {
     constexpr int P = DKP + 4, VP = 132;
     extern __shared__ __align__(16) float prepare_memory[];
@@ -563,10 +582,10 @@ linear_prepare_kernel(const float* __restrict__ q, const float* __restrict__ k, 
     float* g_s = q_s + 32 * P;     // decays; then K^
     float* v_s = g_s + 32 * P;     // values, 128 columns at a time
     float* bt_s = v_s + 32 * VP;
-    const int chunk = blockIdx.x / subs, first = kBlockTokens * (blockIdx.x % subs);
-    const int n = min(kBlockTokens, chunk_length[chunk] - first);
-    if (n <= 0) return;
-    const int start = chunk_start[chunk] + first, head = blockIdx.y, group = head / (heads / groups);
+    const PortionBlock here = find_block(long_table, segment_length, long_portions, blockIdx.x);
+    if (here.block < 0) return;
+    const int first = kBlockTokens * here.block, n = min(kBlockTokens, segment_length[here.portion] - first);
+    const int start = segment_start[here.portion] + first, head = blockIdx.y, group = head / (heads / groups);
     const int tid = threadIdx.x;
     const size_t block_head = static_cast<size_t>(blockIdx.x) * heads + head;
     load_block<DKP>(k_s, q_s, g_s, q, k, g, start, n, head, group, heads, groups, dk);
@@ -654,9 +673,9 @@ linear_prepare_kernel(const float* __restrict__ q, const float* __restrict__ k, 
 // grid (long portions, heads, pieces of dk * dv): every block's sum becomes the state that the block starts from, the portion's slot the
 // state after the last.  One thread an element, eight blocks' loads on their way at a time.
 __global__ void __launch_bounds__(kBlockThreads)
-linear_states_kernel(float* __restrict__ sums, const float* __restrict__ decays, float* __restrict__ state, const int* __restrict__ long_table, int subs,
+linear_states_kernel(float* __restrict__ sums, const float* __restrict__ decays, float* __restrict__ state, const int* __restrict__ long_table,
                      const int* __restrict__ segment_length, const int* __restrict__ segment_slot, int heads, int dk, int dv, int num_slots, int* status) {
-    const int portion = long_table[3 * blockIdx.x], first_block = long_table[3 * blockIdx.x + 1] * subs;
+    const int portion = long_table[3 * blockIdx.x], first_block = blocks_before(long_table, segment_length, blockIdx.x);
     const int blocks = (segment_length[portion] + kBlockTokens - 1) / kBlockTokens;
     const int head = blockIdx.y, element = blockIdx.z * kBlockThreads + threadIdx.x, elements = dk * dv, slot = segment_slot[portion];
     if (slot < 0 || slot >= num_slots) {
@@ -697,18 +716,18 @@ struct ReadShared {
 // by themselves, as the split sums of the token-by-token kernel are.  VECTOR: dv is a multiple of 4.
 template <int DKP, bool VECTOR>
 __global__ void __launch_bounds__(kBlockThreads)
-linear_read_kernel(const float* __restrict__ q, const float* __restrict__ g, const float* __restrict__ states, float* __restrict__ out, const int* __restrict__ chunk_start,
-                   const int* __restrict__ chunk_length, int subs, int heads, int groups, int dk, int dv) {
+linear_read_kernel(const float* __restrict__ q, const float* __restrict__ g, const float* __restrict__ states, float* __restrict__ out, const int* __restrict__ long_table, int long_portions, const int* __restrict__ segment_start,
+                const int* __restrict__ segment_length, int heads, int groups, int dk, int dv) {
     constexpr int P = DKP + 4;
     extern __shared__ __align__(16) float prepare_memory[];
     float* q_s = prepare_memory;
     float* g_s = q_s + 32 * P;
     float* piece_s = prepare_memory;
     float* qt_s = prepare_memory + ReadShared<DKP>::kPiece;   // Q~ at [channel][token], rows of kTrianglePitch
-    const int chunk = blockIdx.x / subs, first = kBlockTokens * (blockIdx.x % subs);
-    const int n = min(kBlockTokens, chunk_length[chunk] - first);
-    if (n <= 0) return;
-    const int start = chunk_start[chunk] + first, head = blockIdx.y, group = head / (heads / groups), tid = threadIdx.x;
+    const PortionBlock here = find_block(long_table, segment_length, long_portions, blockIdx.x);
+    if (here.block < 0) return;
+    const int first = kBlockTokens * here.block, n = min(kBlockTokens, segment_length[here.portion] - first);
+    const int start = segment_start[here.portion] + first, head = blockIdx.y, group = head / (heads / groups), tid = threadIdx.x;
 #pragma unroll 8
     for (int index = tid; index < 32 * DKP; index += kBlockThreads) {
         const int t = index / DKP, c = index % DKP;
@@ -791,18 +810,18 @@ linear_read_kernel(const float* __restrict__ q, const float* __restrict__ g, con
 // beta null: `pack` holds the blocks' sums, then their decays; `vpack` is not used.
 template <int DKP>
 int launch_recurrent_blocks(const float* q, const float* k, const float* g, const float* v, const float* beta, float* pack, float* vpack, float* state, float* out,
-                            const int* chunk_start, const int* chunk_length, int chunks, int subs, const int* long_table, int long_portions, const int* segment_start,
+                            int most_blocks, const int* long_table, int long_portions, const int* segment_start,
                             const int* segment_length, const int* segment_slot, int heads, int groups, int dk, int dv, int num_slots, int* status, cudaStream_t stream) {
-    const dim3 blocks(chunks * subs, heads);
+    const dim3 blocks(most_blocks, heads);
     if (beta != nullptr) {
         static OncePerDevice prepared, walked;
         auto prepare = recurrent_prepare_kernel<DKP>;
         auto walk = recurrent_walk_kernel<DKP>;
         if (allow_shared_memory(prepared, prepare, PrepareShared<DKP>::kBytes) != cudaSuccess) return static_cast<int>(cudaGetLastError());
         if (allow_shared_memory(walked, walk, WalkShared<DKP>::kBytes) != cudaSuccess) return static_cast<int>(cudaGetLastError());
-        prepare<<<blocks, kBlockThreads, PrepareShared<DKP>::kBytes, stream>>>(q, k, g, v, beta, pack, vpack, chunk_start, chunk_length, subs, heads, groups, dk, dv);
+        prepare<<<blocks, kBlockThreads, PrepareShared<DKP>::kBytes, stream>>>(q, k, g, v, beta, pack, vpack, long_table, long_portions, segment_start, segment_length, heads, groups, dk, dv);
         walk<<<dim3(long_portions, heads, (dv + kWalkCols - 1) / kWalkCols), kBlockThreads, WalkShared<DKP>::kBytes, stream>>>(
-            pack, vpack, state, out, long_table, subs, segment_start, segment_length, segment_slot, heads, dk, dv, num_slots, status);
+            pack, vpack, state, out, long_table, segment_start, segment_length, segment_slot, heads, dk, dv, num_slots, status);
         return static_cast<int>(cudaGetLastError());
     }
     static OncePerDevice prepared, read, read_any;
@@ -811,11 +830,11 @@ int launch_recurrent_blocks(const float* q, const float* k, const float* g, cons
     constexpr int prepare_bytes = (3 * 32 * (DKP + 4) + 32 * 132 + 32 * kTrianglePitch) * 4, read_bytes = ReadShared<DKP>::kBytes;
     if (allow_shared_memory(prepared, prepare, prepare_bytes) != cudaSuccess) return static_cast<int>(cudaGetLastError());
     if (allow_shared_memory(dv % 4 == 0 ? read : read_any, read_out, read_bytes) != cudaSuccess) return static_cast<int>(cudaGetLastError());
-    float* decays = pack + static_cast<size_t>(chunks) * subs * heads * dk * dv;
-    prepare<<<blocks, kBlockThreads, prepare_bytes, stream>>>(q, k, g, v, pack, decays, out, chunk_start, chunk_length, subs, heads, groups, dk, dv);
+    float* decays = pack + static_cast<size_t>(most_blocks) * heads * dk * dv;
+    prepare<<<blocks, kBlockThreads, prepare_bytes, stream>>>(q, k, g, v, pack, decays, out, long_table, long_portions, segment_start, segment_length, heads, groups, dk, dv);
     linear_states_kernel<<<dim3(long_portions, heads, (dk * dv + kBlockThreads - 1) / kBlockThreads), kBlockThreads, 0, stream>>>(
-        pack, decays, state, long_table, subs, segment_length, segment_slot, heads, dk, dv, num_slots, status);
-    read_out<<<blocks, kBlockThreads, read_bytes, stream>>>(q, g, pack, out, chunk_start, chunk_length, subs, heads, groups, dk, dv);
+        pack, decays, state, long_table, segment_length, segment_slot, heads, dk, dv, num_slots, status);
+    read_out<<<blocks, kBlockThreads, read_bytes, stream>>>(q, g, pack, out, long_table, long_portions, segment_start, segment_length, heads, groups, dk, dv);
     return static_cast<int>(cudaGetLastError());
 }
 
@@ -831,15 +850,15 @@ int lb_recurrent_pack_floats(int dk, int dv, int delta) {
 }
 int lb_recurrent_value_floats(int dv, int delta) { return delta ? (dv + lb::kWalkCols - 1) / lb::kWalkCols * 64 * lb::kWalkCols : 0; }
 
-// The long portions of `long_table`, block by block, from and into their state slots.  The chunks of `chunk_start` / `chunk_length` are of
-// 32 * subs tokens, but for each portion's last; `pack` and `vpack` have room for chunks * subs blocks of every head.  beta null: no delta rule.
+// The long portions of `long_table`, block by block, from and into their state slots.  `most_blocks`: no fewer than their
+// blocks of 32 tokens together; `pack` and `vpack` have room for so many of every head.  beta null: no delta rule.
 int lb_recurrent_blocks(const float* q, const float* k, const float* g, const float* v, const float* beta, float* pack, float* vpack, float* state, float* out,
-                        const int* chunk_start, const int* chunk_length, int chunks, int subs, const int* long_table, int long_portions, const int* segment_start,
+                        int most_blocks, const int* long_table, int long_portions, const int* segment_start,
                         const int* segment_length, const int* segment_slot, int heads, int groups, int dk, int dv, int num_slots, int* status, cudaStream_t stream) {
-    if (long_portions == 0 || chunks == 0) return 0;
-    if (dk < 1 || dk > 256 || dv < 1 || heads % groups != 0 || subs < 1) return -2;
+    if (long_portions == 0 || most_blocks == 0) return 0;
+    if (dk < 1 || dk > 256 || dv < 1 || heads % groups != 0) return -2;
     auto launch = dk <= 32 ? lb::launch_recurrent_blocks<32> : dk <= 64 ? lb::launch_recurrent_blocks<64> : dk <= 128 ? lb::launch_recurrent_blocks<128> : lb::launch_recurrent_blocks<256>;
-    return launch(q, k, g, v, beta, pack, vpack, state, out, chunk_start, chunk_length, chunks, subs, long_table, long_portions, segment_start, segment_length, segment_slot,
+    return launch(q, k, g, v, beta, pack, vpack, state, out, most_blocks, long_table, long_portions, segment_start, segment_length, segment_slot,
                   heads, groups, dk, dv, num_slots, status, stream);
 }
 

@@ -1233,18 +1233,15 @@ def _recurrence(q: torch.Tensor, k: torch.Tensor, decay: torch.Tensor, v: torch.
     read_out = torch.empty(tokens, num_heads, value_dim, dtype=torch.float32, device=q.device)
     direct_list, num_direct = None, segments
     if chunk_plan is not None and chunk_plan["num_chunks"] > 0:
-        chunk_tokens = chunk_plan.get("chunk_tokens", GDR_CHUNK_TOKENS)
-        if chunk_tokens >= RECURRENT_BLOCK and chunk_tokens % RECURRENT_BLOCK == 0:   # chunks of whole blocks (any other plan: every portion token by token)
-            num_chunks, num_long, blocks = chunk_plan["num_chunks"], chunk_plan["num_long"], chunk_tokens // RECURRENT_BLOCK
-            block_heads, delta = num_chunks * blocks * num_heads, 0 if beta is None else 1
-            pack = torch.empty(block_heads * lib.lb_recurrent_pack_floats(key_dim, value_dim, delta), dtype=torch.float32, device=q.device)
-            values = torch.empty(block_heads * lib.lb_recurrent_value_floats(value_dim, delta), dtype=torch.float32, device=q.device)
-            code = lib.lb_recurrent_blocks(q, k, decay, v, beta, pack, values, matrix_state, read_out,
-                                           chunk_plan["chunk_start"], chunk_plan["chunk_length"], num_chunks, blocks,
-                                           chunk_plan["long_table"], num_long, segment_start, segment_length, segment_slot,
-                                           num_heads, num_groups, key_dim, value_dim, num_slots, status, _stream())
-            _done(code, "recurrent_blocks", 2 if delta else 3)
-            direct_list, num_direct = chunk_plan["direct"], chunk_plan["num_direct"]
+        # (which chunks the plan makes of a long portion does not matter: the kernels take its tokens 32 at a time)
+        num_long, delta = chunk_plan["num_long"], 0 if beta is None else 1
+        most_blocks = tokens // RECURRENT_BLOCK + num_long
+        pack = torch.empty(most_blocks * num_heads * lib.lb_recurrent_pack_floats(key_dim, value_dim, delta), dtype=torch.float32, device=q.device)
+        values = torch.empty(most_blocks * num_heads * lib.lb_recurrent_value_floats(value_dim, delta), dtype=torch.float32, device=q.device)
+        code = lib.lb_recurrent_blocks(q, k, decay, v, beta, pack, values, matrix_state, read_out, most_blocks, chunk_plan["long_table"], num_long, segment_start,
+                                       segment_length, segment_slot, num_heads, num_groups, key_dim, value_dim, num_slots, status, _stream())
+        _done(code, "recurrent_blocks", 2 if delta else 3)
+        direct_list, num_direct = chunk_plan["direct"], chunk_plan["num_direct"]
     if num_direct > 0:
         code = lib.lb_gdr_scan(q, k, decay, v, beta, matrix_state, read_out, segment_start, segment_length,
                                segment_slot, num_direct, num_heads, num_groups, key_dim, value_dim, num_slots,

@@ -1,5 +1,5 @@
 """Long portions in blocks of 32 tokens against the recurrence itself in 64 bits: portions that end at, before and behind a block's end,
-key and value sizes with padding, decays of exactly zero, chunks of two blocks; and a token without a number reaches none before it."""
+key and value sizes with padding, decays of exactly zero, plans of other chunks; and a token without a number reaches none before it."""
 
 import numpy as np
 import pytest
@@ -19,14 +19,14 @@ def make(lengths, heads, groups, dk, dv, delta):
     return q, k, v, decay, beta, random(len(lengths) + 1, heads, dk, dv)
 
 
-def run(q, k, v, decay, beta, state, lengths, blocks):
+def run(q, k, v, decay, beta, state, lengths, chunk):
     from lalamo_b200 import ops
 
     starts, slots = np.cumsum([0] + list(lengths[:-1])), list(range(len(lengths)))[::-1]
     ints = lambda values: torch.tensor(np.asarray(values), dtype=torch.int32, device="cuda")  # noqa: E731
-    plan = ops.gated_delta_chunk_plan(starts.tolist(), lengths, chunk_tokens=32 * blocks, long_portion=16)
+    plan = ops.gated_delta_chunk_plan(starts.tolist(), lengths, chunk_tokens=chunk, long_portion=16)
     chunk_plan = {**{name: ints(values) for name, values in plan.items()}, "num_chunks": plan["chunk_start"].size, "num_long": plan["long_table"].size // 3,
-                  "num_direct": plan["direct"].size, "chunk_tokens": 32 * blocks}
+                  "num_direct": plan["direct"].size}
     status, on_device = torch.zeros(1, dtype=torch.int32, device="cuda"), state.cuda()
     out = ops._recurrence(q.cuda(), k.cuda(), decay.cuda(), v.cuda(), None if beta is None else beta.cuda(), on_device, num_groups=q.shape[1], segment_start=ints(starts),
                           segment_length=ints(lengths), segment_slot=ints(slots), segments=len(lengths), status=status, chunk_plan=chunk_plan)
@@ -35,11 +35,11 @@ def run(q, k, v, decay, beta, state, lengths, blocks):
 
 
 @pytest.mark.parametrize("delta", [True, False])
-@pytest.mark.parametrize("dk,dv,blocks", [(20, 8, 1), (32, 130, 2), (66, 7, 1), (64, 128, 1), (128, 72, 2), (256, 40, 1)])
-def test_blocks(dk, dv, blocks, delta):
+@pytest.mark.parametrize("dk,dv,chunk", [(20, 8, 32), (32, 130, 64), (66, 7, 40), (64, 128, 32), (128, 72, 256), (256, 40, 32)])
+def test_blocks(dk, dv, chunk, delta):
     lengths, heads, groups = [33, 5, 96, 31, 130], 4, 2
     q, k, v, decay, beta, state = make(lengths, heads, groups, dk, dv, delta)
-    got, new_state, slots = run(q, k, v, decay, beta, state, lengths, blocks)
+    got, new_state, slots = run(q, k, v, decay, beta, state, lengths, chunk)
     want, want_state, at = torch.zeros_like(got, dtype=torch.float64), state.double(), 0
     for length, slot in zip(lengths, slots):
         S = want_state[slot].clone()
@@ -60,7 +60,7 @@ def test_blocks(dk, dv, blocks, delta):
 def test_a_token_without_a_number_reaches_none_before_it(delta):
     lengths = [70]
     q, k, v, decay, beta, state = make(lengths, 2, 2, 64, 24, delta)
-    clean, _, _ = run(q, k, v, decay, beta, state, lengths, 1)
+    clean, _, _ = run(q, k, v, decay, beta, state, lengths, 32)
     v[41], k[45] = float("nan"), float("inf")
-    got, _, _ = run(q, k, v, decay, beta, state, lengths, 1)
+    got, _, _ = run(q, k, v, decay, beta, state, lengths, 32)
     assert torch.equal(got[:41], clean[:41]) and bool(torch.isnan(got[41:]).any())
