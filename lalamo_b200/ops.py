@@ -1194,9 +1194,11 @@ def short_conv(
 # ---------------------------------------------------------------------- gated delta rule
 RECURRENT_BLOCK = 32  # tokens that the kernels for long portions of a recurrence take at a time
 GDR_CHUNK_TOKENS = RECURRENT_BLOCK  # long portions are cut into chunks of this many tokens
-# Portions of at least this many tokens count as long; shorter ones are scanned token by token.  One portion of 8 heads, scan against blocks: delta rule, 128 x 128,
-# 64 tokens 28.7 and 33.8 us, 128 tokens 49 and 38, 2,048 tokens 672 and 157; linear, 64 x 128, 64 tokens 20.5 and 33.8, 128 tokens 35 and 35, 2,048 tokens 428 and 75.
-GDR_LONG_PORTION = 112
+# Portions of at least this many tokens count as long; shorter ones are scanned token by token, several side by side in the time of one.  Scan against blocks, 8
+# heads: one portion, delta rule, 128 x 128, 64 tokens 28.7 and 33.8 us, 128 tokens 49 and 38, 2,048 tokens 672 and 157; linear, 64 x 128, 128 tokens 35 and 35,
+# 2,048 tokens 428 and 75; four portions of 512, linear 145 and 73.  Eight portions of 130 tokens gain nothing (delta rule, a layer 188 and 194), five of 120 lose (linear, a layer
+# 90 and 115), hence a line beyond where one portion alone would break even.
+GDR_LONG_PORTION = 192
 
 
 def gated_delta_chunk_plan(starts, lengths, chunk_tokens: int = GDR_CHUNK_TOKENS, long_portion: int = GDR_LONG_PORTION) -> dict:
@@ -1629,9 +1631,11 @@ def moe_route(x: torch.Tensor, router: torch.Tensor, *, top: int, group_count: i
     return chosen, weights
 
 
-# Up to this many (token, expert) pairs each pair streams its expert's weights; more are grouped by expert.  Measured over both products, cold caches: 16 pairs of
-# 2048 x 2048 experts 85 us streamed, 92 grouped, 32 pairs 132 and 97; of 1024 x 1152 experts 16 pairs 48 and 51, 32 pairs 52 and 50.
-MOE_STREAM_MAX_PAIRS = 16
+# Up to this many (token, expert) pairs, and this many of their experts' elements a matrix, each pair streams its expert's weights; more are grouped by expert.  Measured
+# over both products, cold caches: of 2048 x 2048 experts 16 pairs 85 us streamed and 92 grouped, 32 pairs 132 and 97; of 1024 x 1152 experts a layer of 20 pairs 66.5 and
+# 72.7, of 32 pairs 72.7 and 74.8, 48 pairs' products 75 and 52.
+MOE_STREAM_MAX_PAIRS = 32
+MOE_STREAM_MAX_ELEMENTS = 16 * 2048 * 2048
 
 
 def moe_experts(x: torch.Tensor, gate: "torch.Tensor | None", up: torch.Tensor, down: torch.Tensor, chosen: torch.Tensor, weights: torch.Tensor,
@@ -1669,7 +1673,7 @@ def moe_experts(x: torch.Tensor, gate: "torch.Tensor | None", up: torch.Tensor, 
     wide_rows = width % vector == 0 and ff % vector == 0 and max(width, ff) * 4 <= 160 * 1024
     lib = _lib()
     if path is None:
-        path = "grouped" if x.dtype == torch.bfloat16 and wide_rows and experts <= 1024 and pairs > MOE_STREAM_MAX_PAIRS else "stream" if wide_rows else "plain"
+        path = "grouped" if x.dtype == torch.bfloat16 and wide_rows and experts <= 1024 and (pairs > MOE_STREAM_MAX_PAIRS or pairs * width * ff > MOE_STREAM_MAX_ELEMENTS) else "stream" if wide_rows else "plain"
     if path == "grouped":
         # many pairs: sorted by expert, 128 at a time on the tensor cores
         if not (x.dtype == torch.bfloat16 and wide_rows and experts <= 1024):
