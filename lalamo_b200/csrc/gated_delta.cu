@@ -6,8 +6,8 @@
 // slot.  Four kernels: `prepare` (short causal convolutions with silu over q, k and v, unit q and k,
 // beta and the decays, all in 32-bit), `conv_state` (the convolutions' last inputs into the slot),
 // `scan` (the recurrence, token by token; long portions go through recurrent_blocks.cu instead) and `output` (per-head RMS norm
-// times a sigmoid gate).  The order of every sum depends on the token's place in its request only, never on how the
-// request was cut into steps or on what else is in the batch.
+// times a sigmoid gate).  The order of every sum in these kernels is the same however the request was cut into steps and whatever else is in
+// the batch.  Long portions' blocks add up in an order of their own: there a result depends on the cutting, to rounding.
 #include "common.cuh"
 
 #include <type_traits>
@@ -131,9 +131,11 @@ __global__ void gdr_prepare_kernel(const T* __restrict__ proj, int proj_width, c
 
 // The same for portions of several tokens, four taps and heads of up to 128 channels that come in fours: a piece of L lanes (L a power of two,
 // four neighbouring channels a lane) walks over kPrepareRun neighbouring rows of one unit with the convolution's last inputs and the taps' weights
-// in registers, so that an input is read once and not once a tap.  grid (groups of tokens, units), four warps.
+// in registers, so that an input is read once and not once a tap.  The squares of a unit norm are added up as the kernel above adds them (channels
+// 32 apart, then over the warp), by way of shared memory, so that a token's numbers are the same bits whatever else is in its step.
+// grid (groups of tokens, units), four warps.
 // What bounds it: the 32-bit rows it writes (16 KB a token at 8 heads of 128 x 128).  Measured at
-// those sizes and 2,048 tokens: 24.7 us, 67 us with a lane per channel that reads its taps' inputs each for itself.
+// those sizes and 2,048 tokens: 25.4 us, 67 us with a lane per channel that reads its taps' inputs each for itself.
 constexpr int kPrepareRun = 8, kPrepareTaps = 4;
 
 template <typename T>
@@ -156,6 +158,7 @@ gdr_prepare_run_kernel(const T* __restrict__ proj, int proj_width, const T* __re
                        const int* __restrict__ token_segment, const int* __restrict__ segment_start, const int* __restrict__ segment_slot, int tokens, int heads, int groups,
                        int dk, int dv, int num_slots, float unit_eps, float q_scale, int* status, int decay_per_head) {
     constexpr int TAPS = kPrepareTaps;
+    __shared__ __align__(16) float rows_s[4][128];   // a warp's rows of queries or keys, its pieces' side by side
     const int unit = blockIdx.y, warp = threadIdx.x >> 5;
     const bool is_value = unit >= 2 * groups && unit < 2 * groups + heads, is_decay = unit >= 2 * groups + heads;
     const int width = is_value ? dv : dk;
@@ -217,17 +220,16 @@ gdr_prepare_run_kernel(const T* __restrict__ proj, int proj_width, const T* __re
                 }
             }
         }
-        float values[4] = {}, sum = 0.0f;
+        float values[4] = {};
         if (good && live) {
             float input[4];
             load_four(proj + static_cast<size_t>(token) * proj_width + ch0 + c, input);
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                float acc = weight[e][TAPS - 1] * input[e];
+                float acc = weight[e][TAPS - 1] * input[e];   // as conv_silu: left to itself the compiler fuses the first product, not the second
 #pragma unroll
-                for (int j = 1; j < TAPS; ++j) acc += weight[e][TAPS - 1 - j] * before[j - 1][e];
+                for (int j = 1; j < TAPS; ++j) acc = fmaf(weight[e][TAPS - 1 - j], before[j - 1][e], acc);
                 values[e] = acc * sigmoidf_(acc);
-                sum += values[e] * values[e];
             }
 #pragma unroll
             for (int j = TAPS - 2; j > 0; --j)
@@ -240,7 +242,20 @@ gdr_prepare_run_kernel(const T* __restrict__ proj, int proj_width, const T* __re
             if (good && live) *reinterpret_cast<float4*>(v_out + (static_cast<size_t>(token) * heads + unit - 2 * groups) * dv + c) = make_float4(values[0], values[1], values[2], values[3]);
         } else {
             // unit length (and the query's scale)
-            for (int offset = lanes >> 1; offset > 0; offset >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, offset);
+            const int warp_lane = threadIdx.x & 31;
+            float sum = 0.0f;
+            __syncwarp();   // the token before's rows have been read
+            *reinterpret_cast<float4*>(&rows_s[warp][4 * warp_lane]) = make_float4(values[0], values[1], values[2], values[3]);
+            __syncwarp();
+            for (int other = 0; other < pieces; ++other) {
+                float squares = 0.0f;
+                for (int channel = warp_lane; channel < width; channel += 32) {
+                    const float value = rows_s[warp][4 * lanes * other + channel];
+                    squares += value * value;
+                }
+                squares = warp_sum(squares);
+                if (other == piece) sum = squares;
+            }
             const bool is_query = unit < groups;
             const float inv = rsqrtf(sum + unit_eps) * (is_query ? q_scale : 1.0f);
             float* destination = (is_query ? q_out : k_out) + (static_cast<size_t>(token) * groups + (is_query ? unit : unit - groups)) * dk + c;
