@@ -224,15 +224,17 @@ __device__ __forceinline__ PortionBlock find_block(const int* __restrict__ long_
     return PortionBlock{0, -1};
 }
 
-// grid (blocks, heads).  blockIdx.x is a block's number among those of the long portions that `long_table` lists (rows of three numbers, the
-// first of which is the portion).
+// A launch takes the blocks of the numbers window .. window + gridDim.x - 1: scratch is for so many, whatever the step's size.
+
+// grid (blocks, heads).  window + blockIdx.x is a block's number among those of the long portions that `long_table` lists (rows of three
+// numbers, the first of which is the portion).
 //   q, k [tokens, groups, dk], g [tokens, heads, dk], v [tokens, heads, dv], beta [tokens, heads]
 //   pack [block][head][BlockPack::kFloats], vpack [block][head][ceil(dv / 8)][BlockPack::kValues]
 template <int DKP>
 __global__ void __launch_bounds__(kBlockThreads, DKP <= 128 ? 3 : 1)
 recurrent_prepare_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ g, const float* __restrict__ v,
                          const float* __restrict__ beta, float* __restrict__ pack, float* __restrict__ vpack, const int* __restrict__ long_table, int long_portions, const int* __restrict__ segment_start,
-                const int* __restrict__ segment_length, int heads, int groups, int dk, int dv) {
+                const int* __restrict__ segment_length, int heads, int groups, int dk, int dv, int window) {
     using Pack = BlockPack<DKP>;
     using Shared = PrepareShared<DKP>;
     constexpr int P = Shared::kPitch, VP = Shared::kValuePitch, TP = kTrianglePitch;
@@ -246,7 +248,7 @@ recurrent_prepare_kernel(const float* __restrict__ q, const float* __restrict__ 
     float* tt_s = bt_s + 32 * TP;           // T[i][j] at [j][i]
     float* d_half = tt_s + 32 * TP;         // the decays' product over the lower half
     float* beta_s = d_half + DKP;
-    const PortionBlock here = find_block(long_table, segment_length, long_portions, blockIdx.x);
+    const PortionBlock here = find_block(long_table, segment_length, long_portions, window + static_cast<int>(blockIdx.x));
     if (here.block < 0) return;
     const int first = kBlockTokens * here.block, n = min(kBlockTokens, segment_length[here.portion] - first);
     const int start = segment_start[here.portion] + first, head = blockIdx.y, group = head / (heads / groups);
@@ -420,12 +422,12 @@ struct WalkShared {
     static constexpr int kBytes = kFloats * 4;
 };
 
-// grid (long portions, heads, ceil(dv / 8)).
+// grid (long portions, heads, ceil(dv / 8)); of each portion the blocks within the window, from the slot's state and back into it.
 template <int DKP>
 __global__ void __launch_bounds__(kBlockThreads, DKP <= 64 ? 2 : 1)
 recurrent_walk_kernel(const float* __restrict__ pack, const float* __restrict__ vpack, float* __restrict__ state, float* __restrict__ out,
                       const int* __restrict__ long_table, const int* __restrict__ segment_start, const int* __restrict__ segment_length,
-                      const int* __restrict__ segment_slot, int heads, int dk, int dv, int num_slots, int* status) {
+                      const int* __restrict__ segment_slot, int heads, int dk, int dv, int num_slots, int* status, int window, int window_blocks) {
     using Pack = BlockPack<DKP>;
     using Shared = WalkShared<DKP>;
     constexpr int kStages = Shared::kStages;
@@ -437,7 +439,7 @@ recurrent_walk_kernel(const float* __restrict__ pack, const float* __restrict__ 
     float* part_s = walk_memory + kStages * Shared::kStage;
     float* state_s = part_s + 16 * 256;                 // [DKP][8]
     float* u_s = state_s + DKP * kWalkCols;             // [32][8]
-    const int portion = long_table[3 * blockIdx.x], first_block = blocks_before(long_table, segment_length, blockIdx.x);
+    const int portion = long_table[3 * blockIdx.x], offset = blocks_before(long_table, segment_length, blockIdx.x) - window;   // of its blocks' numbers
     const int head = blockIdx.y, slice = blockIdx.z, column0 = slice * kWalkCols, slices = gridDim.z;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int slot = segment_slot[portion];
@@ -446,11 +448,12 @@ recurrent_walk_kernel(const float* __restrict__ pack, const float* __restrict__ 
         return;
     }
     const int start = segment_start[portion], length = segment_length[portion];
-    const int blocks = (length + kBlockTokens - 1) / kBlockTokens;
-    auto load = [&](int block) {   // one thread
+    const int first = max(0, -offset), blocks = min((length + kBlockTokens - 1) / kBlockTokens, window_blocks - offset) - first;
+    if (blocks <= 0) return;
+    auto load = [&](int block) {   // one thread; block counts from the portion's first within the window
         float* stage = walk_memory + (block % kStages) * Shared::kStage;
         uint64_t* barrier = &full[block % kStages];
-        const size_t index = static_cast<size_t>(first_block + block) * heads + head;
+        const size_t index = static_cast<size_t>(offset + first + block) * heads + head;
         barrier_expect(barrier, Shared::kStage * 4);
         bulk_load(stage, pack + index * Pack::kFloats, Pack::kFloats * 4, barrier);
         bulk_load(stage + Pack::kFloats, vpack + (index * slices + slice) * Pack::kValues, Pack::kValues * 4, barrier);
@@ -505,7 +508,7 @@ recurrent_walk_kernel(const float* __restrict__ pack, const float* __restrict__ 
         }
         __syncthreads();
         const float* values = stage + Pack::kFloats;
-        const int t0 = kBlockTokens * block, n = min(kBlockTokens, length - t0);
+        const int t0 = kBlockTokens * (first + block), n = min(kBlockTokens, length - t0);
         {
             // two sums a thread
             float2 sum = *reinterpret_cast<const float2*>(part_s + 2 * tid);
@@ -574,7 +577,7 @@ __global__ void __launch_bounds__(kBlockThreads, DKP <= 128 ? 3 : 1)
 linear_prepare_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ g, const float* __restrict__ v, float* __restrict__ sums,
                       float* __restrict__ decays, float* __restrict__ out, const int* __restrict__ long_table, int long_portions, const int* __restrict__ segment_start,
                 const int* __restrict__ segment_length, int heads,
-                      int groups, int dk, int dv) {
+                      int groups, int dk, int dv, int window) {
     constexpr int P = DKP + 4, VP = 132;
     extern __shared__ __align__(16) float prepare_memory[];
     float* k_s = prepare_memory;   // keys; then as between_halves wants them
@@ -582,7 +585,7 @@ linear_prepare_kernel(const float* __restrict__ q, const float* __restrict__ k, 
     float* g_s = q_s + 32 * P;     // decays; then K^
     float* v_s = g_s + 32 * P;     // values, 128 columns at a time
     float* bt_s = v_s + 32 * VP;
-    const PortionBlock here = find_block(long_table, segment_length, long_portions, blockIdx.x);
+    const PortionBlock here = find_block(long_table, segment_length, long_portions, window + static_cast<int>(blockIdx.x));
     if (here.block < 0) return;
     const int first = kBlockTokens * here.block, n = min(kBlockTokens, segment_length[here.portion] - first);
     const int start = segment_start[here.portion] + first, head = blockIdx.y, group = head / (heads / groups);
@@ -670,23 +673,24 @@ linear_prepare_kernel(const float* __restrict__ q, const float* __restrict__ k, 
     }
 }
 
-// grid (long portions, heads, pieces of dk * dv): every block's sum becomes the state that the block starts from, the portion's slot the
+// grid (long portions, heads, pieces of dk * dv): within the window every block's sum becomes the state that the block starts from, the portion's slot the
 // state after the last.  One thread an element, eight blocks' loads on their way at a time.
 __global__ void __launch_bounds__(kBlockThreads)
 linear_states_kernel(float* __restrict__ sums, const float* __restrict__ decays, float* __restrict__ state, const int* __restrict__ long_table,
-                     const int* __restrict__ segment_length, const int* __restrict__ segment_slot, int heads, int dk, int dv, int num_slots, int* status) {
-    const int portion = long_table[3 * blockIdx.x], first_block = blocks_before(long_table, segment_length, blockIdx.x);
-    const int blocks = (segment_length[portion] + kBlockTokens - 1) / kBlockTokens;
+                     const int* __restrict__ segment_length, const int* __restrict__ segment_slot, int heads, int dk, int dv, int num_slots, int* status,
+                     int window, int window_blocks) {
+    const int portion = long_table[3 * blockIdx.x], offset = blocks_before(long_table, segment_length, blockIdx.x) - window;   // of its blocks' numbers
+    const int first = max(0, -offset), blocks = min((segment_length[portion] + kBlockTokens - 1) / kBlockTokens, window_blocks - offset) - first;
     const int head = blockIdx.y, element = blockIdx.z * kBlockThreads + threadIdx.x, elements = dk * dv, slot = segment_slot[portion];
     if (slot < 0 || slot >= num_slots) {
         if (threadIdx.x == 0) report_error(status, kBadSlot);
         return;
     }
-    if (element >= elements) return;
+    if (element >= elements || blocks <= 0) return;
     float* mine = state + (static_cast<size_t>(slot) * heads + head) * elements + element;
     float s = *mine;
-    float* block_sums = sums + (static_cast<size_t>(first_block) * heads + head) * elements + element;
-    const float* block_decays = decays + (static_cast<size_t>(first_block) * heads + head) * dk + element / dv;
+    float* block_sums = sums + (static_cast<size_t>(offset + first) * heads + head) * elements + element;
+    const float* block_decays = decays + (static_cast<size_t>(offset + first) * heads + head) * dk + element / dv;
     const size_t sum_step = static_cast<size_t>(heads) * elements, decay_step = static_cast<size_t>(heads) * dk;
     for (int b0 = 0; b0 < blocks; b0 += 8) {
         float sum[8], decay[8];
@@ -717,14 +721,14 @@ struct ReadShared {
 template <int DKP, bool VECTOR>
 __global__ void __launch_bounds__(kBlockThreads)
 linear_read_kernel(const float* __restrict__ q, const float* __restrict__ g, const float* __restrict__ states, float* __restrict__ out, const int* __restrict__ long_table, int long_portions, const int* __restrict__ segment_start,
-                const int* __restrict__ segment_length, int heads, int groups, int dk, int dv) {
+                const int* __restrict__ segment_length, int heads, int groups, int dk, int dv, int window) {
     constexpr int P = DKP + 4;
     extern __shared__ __align__(16) float prepare_memory[];
     float* q_s = prepare_memory;
     float* g_s = q_s + 32 * P;
     float* piece_s = prepare_memory;
     float* qt_s = prepare_memory + ReadShared<DKP>::kPiece;   // Q~ at [channel][token], rows of kTrianglePitch
-    const PortionBlock here = find_block(long_table, segment_length, long_portions, blockIdx.x);
+    const PortionBlock here = find_block(long_table, segment_length, long_portions, window + static_cast<int>(blockIdx.x));
     if (here.block < 0) return;
     const int first = kBlockTokens * here.block, n = min(kBlockTokens, segment_length[here.portion] - first);
     const int start = segment_start[here.portion] + first, head = blockIdx.y, group = head / (heads / groups), tid = threadIdx.x;
@@ -810,18 +814,21 @@ linear_read_kernel(const float* __restrict__ q, const float* __restrict__ g, con
 // beta null: `pack` holds the blocks' sums, then their decays; `vpack` is not used.
 template <int DKP>
 int launch_recurrent_blocks(const float* q, const float* k, const float* g, const float* v, const float* beta, float* pack, float* vpack, float* state, float* out,
-                            int most_blocks, const int* long_table, int long_portions, const int* segment_start,
+                            int most_blocks, int window_blocks, const int* long_table, int long_portions, const int* segment_start,
                             const int* segment_length, const int* segment_slot, int heads, int groups, int dk, int dv, int num_slots, int* status, cudaStream_t stream) {
-    const dim3 blocks(most_blocks, heads);
+    const dim3 blocks(window_blocks, heads);
     if (beta != nullptr) {
         static OncePerDevice prepared, walked;
         auto prepare = recurrent_prepare_kernel<DKP>;
         auto walk = recurrent_walk_kernel<DKP>;
         if (allow_shared_memory(prepared, prepare, PrepareShared<DKP>::kBytes) != cudaSuccess) return static_cast<int>(cudaGetLastError());
         if (allow_shared_memory(walked, walk, WalkShared<DKP>::kBytes) != cudaSuccess) return static_cast<int>(cudaGetLastError());
-        prepare<<<blocks, kBlockThreads, PrepareShared<DKP>::kBytes, stream>>>(q, k, g, v, beta, pack, vpack, long_table, long_portions, segment_start, segment_length, heads, groups, dk, dv);
-        walk<<<dim3(long_portions, heads, (dv + kWalkCols - 1) / kWalkCols), kBlockThreads, WalkShared<DKP>::kBytes, stream>>>(
-            pack, vpack, state, out, long_table, segment_start, segment_length, segment_slot, heads, dk, dv, num_slots, status);
+        for (int window = 0; window < most_blocks; window += window_blocks) {
+            prepare<<<blocks, kBlockThreads, PrepareShared<DKP>::kBytes, stream>>>(q, k, g, v, beta, pack, vpack, long_table, long_portions, segment_start, segment_length, heads,
+                                                                                   groups, dk, dv, window);
+            walk<<<dim3(long_portions, heads, (dv + kWalkCols - 1) / kWalkCols), kBlockThreads, WalkShared<DKP>::kBytes, stream>>>(
+                pack, vpack, state, out, long_table, segment_start, segment_length, segment_slot, heads, dk, dv, num_slots, status, window, window_blocks);
+        }
         return static_cast<int>(cudaGetLastError());
     }
     static OncePerDevice prepared, read, read_any;
@@ -830,11 +837,13 @@ int launch_recurrent_blocks(const float* q, const float* k, const float* g, cons
     constexpr int prepare_bytes = (3 * 32 * (DKP + 4) + 32 * 132 + 32 * kTrianglePitch) * 4, read_bytes = ReadShared<DKP>::kBytes;
     if (allow_shared_memory(prepared, prepare, prepare_bytes) != cudaSuccess) return static_cast<int>(cudaGetLastError());
     if (allow_shared_memory(dv % 4 == 0 ? read : read_any, read_out, read_bytes) != cudaSuccess) return static_cast<int>(cudaGetLastError());
-    float* decays = pack + static_cast<size_t>(most_blocks) * heads * dk * dv;
-    prepare<<<blocks, kBlockThreads, prepare_bytes, stream>>>(q, k, g, v, pack, decays, out, long_table, long_portions, segment_start, segment_length, heads, groups, dk, dv);
-    linear_states_kernel<<<dim3(long_portions, heads, (dk * dv + kBlockThreads - 1) / kBlockThreads), kBlockThreads, 0, stream>>>(
-        pack, decays, state, long_table, segment_length, segment_slot, heads, dk, dv, num_slots, status);
-    read_out<<<blocks, kBlockThreads, read_bytes, stream>>>(q, g, pack, out, long_table, long_portions, segment_start, segment_length, heads, groups, dk, dv);
+    float* decays = pack + static_cast<size_t>(window_blocks) * heads * dk * dv;
+    for (int window = 0; window < most_blocks; window += window_blocks) {
+        prepare<<<blocks, kBlockThreads, prepare_bytes, stream>>>(q, k, g, v, pack, decays, out, long_table, long_portions, segment_start, segment_length, heads, groups, dk, dv, window);
+        linear_states_kernel<<<dim3(long_portions, heads, (dk * dv + kBlockThreads - 1) / kBlockThreads), kBlockThreads, 0, stream>>>(
+            pack, decays, state, long_table, segment_length, segment_slot, heads, dk, dv, num_slots, status, window, window_blocks);
+        read_out<<<blocks, kBlockThreads, read_bytes, stream>>>(q, g, pack, out, long_table, long_portions, segment_start, segment_length, heads, groups, dk, dv, window);
+    }
     return static_cast<int>(cudaGetLastError());
 }
 
@@ -851,14 +860,15 @@ int lb_recurrent_pack_floats(int dk, int dv, int delta) {
 int lb_recurrent_value_floats(int dv, int delta) { return delta ? (dv + lb::kWalkCols - 1) / lb::kWalkCols * 64 * lb::kWalkCols : 0; }
 
 // The long portions of `long_table`, block by block, from and into their state slots.  `most_blocks`: no fewer than their
-// blocks of 32 tokens together; `pack` and `vpack` have room for so many of every head.  beta null: no delta rule.
+// blocks of 32 tokens together; they are taken `window_blocks` at a time, for which `pack` and `vpack` have room in every head (the
+// states pass from one window to the next through their slots, in 32 bits as they are: the results are the same).  beta null: no delta rule.
 int lb_recurrent_blocks(const float* q, const float* k, const float* g, const float* v, const float* beta, float* pack, float* vpack, float* state, float* out,
-                        int most_blocks, const int* long_table, int long_portions, const int* segment_start,
+                        int most_blocks, int window_blocks, const int* long_table, int long_portions, const int* segment_start,
                         const int* segment_length, const int* segment_slot, int heads, int groups, int dk, int dv, int num_slots, int* status, cudaStream_t stream) {
     if (long_portions == 0 || most_blocks == 0) return 0;
-    if (dk < 1 || dk > 256 || dv < 1 || heads % groups != 0) return -2;
+    if (dk < 1 || dk > 256 || dv < 1 || heads % groups != 0 || window_blocks < 1) return -2;
     auto launch = dk <= 32 ? lb::launch_recurrent_blocks<32> : dk <= 64 ? lb::launch_recurrent_blocks<64> : dk <= 128 ? lb::launch_recurrent_blocks<128> : lb::launch_recurrent_blocks<256>;
-    return launch(q, k, g, v, beta, pack, vpack, state, out, most_blocks, long_table, long_portions, segment_start, segment_length, segment_slot,
+    return launch(q, k, g, v, beta, pack, vpack, state, out, most_blocks, window_blocks, long_table, long_portions, segment_start, segment_length, segment_slot,
                   heads, groups, dk, dv, num_slots, status, stream);
 }
 

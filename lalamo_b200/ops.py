@@ -1199,6 +1199,9 @@ GDR_CHUNK_TOKENS = RECURRENT_BLOCK  # long portions are cut into chunks of this 
 # 2,048 tokens 428 and 75; four portions of 512, linear 145 and 73.  Eight portions of 130 tokens gain nothing (delta rule, a layer 188 and 194), five of 120 lose (linear, a layer
 # 90 and 115), hence a line beyond where one portion alone would break even.
 GDR_LONG_PORTION = 192
+# What the blocks of long portions may take of memory at a time, beside the step's inputs; larger steps go through it in several turns.  Without a bound a layer's step
+# of 16,384 tokens and 16 heads of 128 x 128 took 677 MB.  13,000 tokens of 8 such heads fit one turn (a step is 2,048 tokens by default).
+RECURRENT_SCRATCH_BYTES = 256 << 20
 
 
 def gated_delta_chunk_plan(starts, lengths, chunk_tokens: int = GDR_CHUNK_TOKENS, long_portion: int = GDR_LONG_PORTION) -> dict:
@@ -1238,11 +1241,13 @@ def _recurrence(q: torch.Tensor, k: torch.Tensor, decay: torch.Tensor, v: torch.
         # (which chunks the plan makes of a long portion does not matter: the kernels take its tokens 32 at a time)
         num_long, delta = chunk_plan["num_long"], 0 if beta is None else 1
         most_blocks = tokens // RECURRENT_BLOCK + num_long
-        pack = torch.empty(most_blocks * num_heads * lib.lb_recurrent_pack_floats(key_dim, value_dim, delta), dtype=torch.float32, device=q.device)
-        values = torch.empty(most_blocks * num_heads * lib.lb_recurrent_value_floats(value_dim, delta), dtype=torch.float32, device=q.device)
-        code = lib.lb_recurrent_blocks(q, k, decay, v, beta, pack, values, matrix_state, read_out, most_blocks, chunk_plan["long_table"], num_long, segment_start,
+        pack_floats, value_floats = num_heads * lib.lb_recurrent_pack_floats(key_dim, value_dim, delta), num_heads * lib.lb_recurrent_value_floats(value_dim, delta)
+        window = max(1, min(most_blocks, RECURRENT_SCRATCH_BYTES // (4 * max(1, pack_floats + value_floats))))
+        pack = torch.empty(window * pack_floats, dtype=torch.float32, device=q.device)
+        values = torch.empty(window * value_floats, dtype=torch.float32, device=q.device)
+        code = lib.lb_recurrent_blocks(q, k, decay, v, beta, pack, values, matrix_state, read_out, most_blocks, window, chunk_plan["long_table"], num_long, segment_start,
                                        segment_length, segment_slot, num_heads, num_groups, key_dim, value_dim, num_slots, status, _stream())
-        _done(code, "recurrent_blocks", 2 if delta else 3)
+        _done(code, "recurrent_blocks", (2 if delta else 3) * -(-most_blocks // window))
         direct_list, num_direct = chunk_plan["direct"], chunk_plan["num_direct"]
     if num_direct > 0:
         code = lib.lb_gdr_scan(q, k, decay, v, beta, matrix_state, read_out, segment_start, segment_length,
