@@ -77,36 +77,37 @@ def _prototypes() -> dict[str, tuple[str, list[str]]]:
 
 
 _WRAPPERS_HEAD = """// Made from the launchers' prototypes: a function of the same name and arguments for each, callable from Python.  A pointer is
-// None, an address, or anything with a data_ptr() (a tensor); numbers may also be ctypes objects.
+// None, an address, or anything with a data_ptr() (a tensor); numbers are what ctypes takes for them (wider integers lose their upper
+// bits), or ctypes' own objects.
 #define Py_LIMITED_API 0x030A0000
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
 static bool take_integer(PyObject* object, long long* value) {
-    if (PyLong_Check(object)) {
-        *value = PyLong_AsLongLong(object);
-    } else if (object == Py_None) {
-        *value = 0;
-    } else {
-        PyObject* number = PyIndex_Check(object) ? PyNumber_Index(object) : PyObject_GetAttrString(object, "value");
+    PyObject* number = nullptr;
+    if (!PyLong_Check(object)) {
+        PyObject* held = PyIndex_Check(object) ? nullptr : PyObject_GetAttrString(object, "value");   // a ctypes object's
+        if (held == nullptr) PyErr_Clear();
+        number = PyNumber_Index(held != nullptr ? held : object);
+        Py_XDECREF(held);
         if (number == nullptr) return false;
-        const bool taken = PyLong_Check(number) || number == Py_None ? take_integer(number, value) : (PyErr_SetString(PyExc_TypeError, "a launcher wants a number here"), false);
-        Py_DECREF(number);
-        return taken;
     }
+    *value = static_cast<long long>(PyLong_AsUnsignedLongLongMask(number != nullptr ? number : object));
+    Py_XDECREF(number);
     return !(*value == -1 && PyErr_Occurred());
 }
 
 static bool take_pointer(PyObject* object, void** value) {
     static PyObject* method = PyUnicode_InternFromString("data_ptr");
     long long address = 0;
-    if (PyLong_Check(object) || object == Py_None || !PyObject_HasAttr(object, method)) {
-        if (!take_integer(object, &address)) return false;
-    } else {
-        PyObject* result = PyObject_CallMethodObjArgs(object, method, nullptr);
-        if (result == nullptr) return false;
-        const bool taken = take_integer(result, &address);
-        Py_DECREF(result);
+    if (object != Py_None) {
+        PyObject* held = nullptr;
+        if (!PyLong_Check(object)) {
+            held = PyObject_HasAttr(object, method) ? PyObject_CallMethodObjArgs(object, method, nullptr) : PyIndex_Check(object) ? PyNumber_Index(object) : PyObject_GetAttrString(object, "value");
+            if (held == nullptr) return false;
+        }
+        const bool taken = held == Py_None || take_integer(held != nullptr ? held : object, &address);   // (None: a null pointer of ctypes)
+        Py_XDECREF(held);
         if (!taken) return false;
     }
     *value = reinterpret_cast<void*>(address);
@@ -114,14 +115,21 @@ static bool take_pointer(PyObject* object, void** value) {
 }
 
 static bool take_float(PyObject* object, double* value) {
-    if (PyFloat_Check(object) || PyLong_Check(object)) {
-        *value = PyFloat_AsDouble(object);
-        return !(*value == -1.0 && PyErr_Occurred());
+    *value = PyFloat_AsDouble(object);
+    if (*value == -1.0 && PyErr_Occurred()) {
+        if (!PyErr_ExceptionMatches(PyExc_TypeError)) return false;
+        PyObject *type, *error, *trace;
+        PyErr_Fetch(&type, &error, &trace);
+        PyObject* held = PyObject_GetAttrString(object, "value");   // a ctypes object's
+        if (held == nullptr) {
+            PyErr_Clear();
+            PyErr_Restore(type, error, trace);
+            return false;
+        }
+        Py_XDECREF(type), Py_XDECREF(error), Py_XDECREF(trace);
+        *value = PyFloat_AsDouble(held);
+        Py_DECREF(held);
     }
-    PyObject* number = PyObject_GetAttrString(object, "value");
-    if (number == nullptr) return false;
-    *value = PyFloat_AsDouble(number);
-    Py_DECREF(number);
     return !(*value == -1.0 && PyErr_Occurred());
 }
 """
@@ -160,8 +168,17 @@ class _CtypesLaunchers:
 
     @staticmethod
     def _taking_tensors(function):
+        types = function.argtypes
+
+        def taken(argument, declared):
+            if declared is ctypes.c_void_p and hasattr(argument, "data_ptr"):
+                return argument.data_ptr()
+            return declared(argument.value if isinstance(argument, ctypes._SimpleCData) else argument)
+
         def call(*arguments):
-            return function(*(argument.data_ptr() if hasattr(argument, "data_ptr") else argument for argument in arguments))
+            if len(arguments) != len(types):
+                raise TypeError(f"{function.__name__} takes {len(types)} arguments, got {len(arguments)}")
+            return function(*map(taken, arguments, types))
 
         return call
 
