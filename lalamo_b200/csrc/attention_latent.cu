@@ -318,9 +318,9 @@ __device__ __forceinline__ uint32_t latent_pack(float low, float high) {
     return *reinterpret_cast<const uint32_t*>(&pair);
 }
 
-// WARPS of 16 query rows each: four, or eight for runs of more than 64 rows.  A multiprocessor's shared memory holds one CTA of either
-// (115 and 152 KB at 256 + 32 channels), so that with four warps every scheduler has one, which waits for its own loads; eight also share what
-// is loaded of the cached rows.  Measured, 16 heads over 256 + 32 channels, 1,023 tokens behind 1,500 cached ones under a window of 2,048: 251 us,
+// WARPS of 16 query rows each: four, or eight for runs of more than 64 rows.  A multiprocessor's shared memory holds two CTAs of four warps
+// or one of eight (111 and 148 KB at 256 + 32 channels); eight share what is loaded of the cached rows, and for their rows the next blocks' loads take
+// half as long.  Measured, 16 heads over 256 + 32 channels, 1,023 tokens behind 1,500 cached ones under a window of 2,048: 251 us,
 // 331 us with four warps (and two CTAs an item, merged); bound by each warp's chain of loads, products and softmax, at a quarter of
 // what mma.sync reaches.
 template <int CHUNK, int WARPS>

@@ -1520,9 +1520,25 @@ def latent_attention_takes_double(latent: int, rope: int) -> bool:
     return (128 + 2 * 64) * (latent + rope + 8) * 2 <= 227 * 1024
 
 
+def latent_attention_doubles(lengths: "tuple[int, ...] | list[int]", num_heads: int) -> bool:
+    """Whether a step of portions of these lengths should run in runs of twice as many tokens.  Of many items: where that leaves nine of sixteen or
+    fewer, since a multiprocessor holds two CTAs of four warps and one of eight.  Few have a multiprocessor each either way: then eight warps pay for tokens that
+    are alone in their run (its rows arrive sooner), not for long runs.  Attention alone, 16 heads over 256 + 32 channels, four warps and eight: 40
+    tokens behind 1,000 cached ones beside a portion of 9 (43 and 42 items) 43 and 66 us, 40 behind 2,000 beside 300 (115 and 78) 117 and 120; 8 behind 2,000
+    beside 300 (83 and 46) 89 and 68, 1,023 behind 1,500 (256 and 128) 336 and 257; few: 8 behind 2,000 beside 5 (10 and 9) 34 and 28, 33 behind none (9
+    and 5) 16 and 18, 9 behind 2,000 (3 and 2) 34 and 35."""
+    heads, run = latent_attention_tiling(num_heads)
+    if max(lengths, default=0) <= run:
+        return False
+    blocks = -(-num_heads // heads)
+    single, double = (blocks * sum(-(-length // tokens) for length in lengths) for tokens in (run, 2 * run))
+    return 16 * double <= 9 * single if single > 16 else 8 * double >= 7 * single
+
+
 def latent_attention_splits(num_items: int, num_heads: int, latent: int, window: int | None, max_context: int, sms: int | None = None, double: bool = False) -> int:
     """Over how many CTAs an item's cached rows are shared out: 1 where the items fill the GPU by themselves.  CTAs of eight warps (``double``)
-    hold a multiprocessor each, so that two thirds of a round of them are left as they are: merging costs 22 us for 1,023 tokens of 16 heads."""
+    hold a multiprocessor each, so that two thirds of a round of them are left as they are: merging costs 22 us for 1,023 tokens of 16 heads.  Many shares of
+    few such items just fill one round (25 items behind 1,500 rows: 61 us in 6 shares, 81 in 8; 13 behind 2,000: 45 in 12, 61 in 17)."""
     heads, tokens = latent_attention_tiling(num_heads)
     ctas = num_items * -(-num_heads // heads) * -(-latent // (256 if latent > 128 else 128))
     sms = sms or sm_count()
@@ -1531,7 +1547,8 @@ def latent_attention_splits(num_items: int, num_heads: int, latent: int, window:
     if ctas >= 2 * sms or blocks <= 2:
         return 1
     if double:
-        return max(1, min(blocks // 2, 3 * sms // 2 // ctas, 32))
+        shares = 3 * sms // 2 // ctas
+        return max(1, min(blocks // 2, shares if shares <= 5 else 9 * sms // 8 // ctas, 32))
     return max(1, min(blocks // 2, -(-2 * sms // ctas), 32))   # two blocks a CTA: one block each was measured 1 % slower
 
 

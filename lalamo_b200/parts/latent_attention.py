@@ -115,10 +115,10 @@ class LatentAttention(Mixer):
         return ("latent_attention", ops.latent_attention_tiling(self.spec.num_heads), self.takes_double)
 
     def plan_step(self, segments: HostSegments) -> dict[str, np.ndarray]:
-        """``items``: ``(first row, count)`` of every run of consecutive tokens that one CTA takes (twice as many a run where some portion
-        fills such runs)."""
+        """``items``: ``(first row, count)`` of every run of consecutive tokens that one CTA takes (twice as many a run where
+        :func:`ops.latent_attention_doubles` says so, and some portion is longer than a single run)."""
         _, run = ops.latent_attention_tiling(self.spec.num_heads)
-        if self.takes_double and max(segments.length, default=0) > run:
+        if self.takes_double and ops.latent_attention_doubles(segments.length, self.spec.num_heads):
             run *= 2
         items = [(first, min(run, start + length - first)) for start, length in zip(segments.start, segments.length) for first in range(start, start + length, run)]
         return {"items": np.asarray(items, dtype=np.int32).reshape(-1)}
