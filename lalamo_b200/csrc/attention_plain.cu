@@ -6,6 +6,8 @@
 // steps or on what else is in the batch.
 #include "common.cuh"
 
+#include <type_traits>
+
 namespace lb {
 
 struct PagedLayout {
@@ -750,8 +752,9 @@ __global__ void paged_attention_plain_kernel(const T* __restrict__ q, const T* _
 // lanes share two rows: every score, every element of a sum is one thread's, added up in the same order whatever shares the block.
 // Sizes of at most 128 that are multiples of 4, at most 16 query heads a K/V head; the kernel above takes the rest.
 // What bounds it: the latency of a chunk's loads and, with many rows, its shared-memory reads; the next chunk's copies (cp.async in 32-bit) are
-// on their way meanwhile.  Measured in 32-bit, 16 heads of 64 over 8: 300 tokens behind 100 cached ones 68 us (577 with a block per token
-// and head), a layer's step of 8 tokens behind 500 cached ones each, 32 heads, 131 us (250).
+// on their way meanwhile, or other blocks' work where there are more blocks than that leaves room for.  Measured in 32-bit: 16 heads of 64 over 8, 300 tokens behind
+// 100 cached ones 51 us (577 with a block per token and head); 8 tokens behind 500 and less each, 32 heads over 8, 48 us (169); 64 tokens behind 500
+// each, 16 heads over 16, 134 us (283; 309 with two stages whatever the blocks), behind 15 each 18 us (18; 47 with chunks of 64 keys copied whole).
 constexpr int kRowsPerBlock = 16, kRowsKeys = 64, kRowsThreads = 128, kRowsPad = 4;
 
 __device__ __forceinline__ void rows_copy_16(float* shared_destination, const float* source, bool real) {
@@ -762,14 +765,14 @@ template <typename T, typename TO>
 __global__ void __launch_bounds__(kRowsThreads)
 paged_attention_rows_kernel(const T* __restrict__ q, const T* __restrict__ k_pages, const T* __restrict__ v_pages, TO* __restrict__ out,
                             const int* __restrict__ positions, const int* __restrict__ token_segment, const int* __restrict__ block_table, PagedLayout layout,
-                            int tokens, int num_heads, int tokens_per_block, float scale, int window, int keep_first, int* status) {
+                            int tokens, int num_heads, int tokens_per_block, int rows_held, int two_stages, float scale, int window, int keep_first, int* status) {
     extern __shared__ __align__(16) float shared[];
     constexpr int kKeyPitch = kRowsKeys + kRowsPad;
     const int hd = layout.head_dim, vd = layout.value_dim, k_pitch = hd + kRowsPad;
     const int stage_floats = kRowsKeys * k_pitch + vd * kKeyPitch;
-    float* q_s = shared;                                  // [16][k_pitch]
-    float* p_s = q_s + kRowsPerBlock * k_pitch;           // [16][kKeyPitch]
-    float* stages = p_s + kRowsPerBlock * kKeyPitch;      // two of: keys [64][k_pitch], values [vd][kKeyPitch]
+    float* q_s = shared;                                  // [rows_held][k_pitch]: the block's rows in whole fours
+    float* p_s = q_s + rows_held * k_pitch;               // [rows_held][kKeyPitch]
+    float* stages = p_s + rows_held * kKeyPitch;          // two (or one) of: keys [64][k_pitch], values [vd][kKeyPitch]
     const int group = blockIdx.y, per_group = num_heads / layout.num_groups, value_group = group / (layout.num_groups / layout.value_groups);
     const int tid = threadIdx.x, pair = tid >> 4, lane = tid & 15;
     const int end = min(tokens, static_cast<int>(blockIdx.x + 1) * tokens_per_block);
@@ -785,7 +788,8 @@ paged_attention_rows_kernel(const T* __restrict__ q, const T* __restrict__ k_pag
         // the first chunk at or after `from` that holds a key someone sees
         auto chunk_from = [&](int from) { return from >= kept && from < window_chunk ? window_chunk : from; };
         // A thread copies half of one key's row, and the values of four neighbouring keys (a copy of 16 bytes where a page's rows come in
-        // fours) for every eighth channel.  Keys that nobody in the block sees are not looked up: their pages may be gone.
+        // fours) for every eighth channel.  Keys that nobody in the block sees are neither looked up (their pages may be gone) nor copied: what
+        // lies in their place meets no sum.
         auto fetch = [&](int chunk, int which) {
             float* k_s = stages + which * stage_floats;
             float* v_s = k_s + kRowsKeys * k_pitch;
@@ -795,7 +799,7 @@ paged_attention_rows_kernel(const T* __restrict__ q, const T* __restrict__ k_pag
                 const bool looked_up = seen(chunk + key);
                 const T* row = looked_up ? page_row(const_cast<T*>(k_pages), block_table, layout, segment, chunk + key, group) : nullptr;
                 if (looked_up && row == nullptr) report_error(status, kBadPage);
-                for (int d = from; d < to; d += 4) {
+                for (int d = from; looked_up && d < to; d += 4) {
                     float* destination = k_s + key * k_pitch + d;
                     if constexpr (sizeof(T) == 4) {
                         rows_copy_16(destination, row != nullptr ? row + d : k_pages, row != nullptr);
@@ -809,15 +813,15 @@ paged_attention_rows_kernel(const T* __restrict__ q, const T* __restrict__ k_pag
             if (sizeof(T) == 4 && layout.page_size % 4 == 0) {
                 const bool any = seen(chunk + quad) || seen(chunk + quad + 1) || seen(chunk + quad + 2) || seen(chunk + quad + 3);
                 const T* column = any ? value_column(const_cast<T*>(v_pages), block_table, layout, segment, chunk + quad, value_group) : nullptr;
-                for (int d = tid >> 4; d < vd; d += kRowsThreads / 16) {
+                for (int d = tid >> 4; any && d < vd; d += kRowsThreads / 16) {
                     const T* source = column != nullptr ? column + static_cast<size_t>(d) * layout.page_size : v_pages;
                     if constexpr (sizeof(T) == 4) rows_copy_16(v_s + d * kKeyPitch + quad, source, column != nullptr);
                 }
             } else {
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const int key = chunk + quad + i;
-                    const T* column = seen(key) ? value_column(const_cast<T*>(v_pages), block_table, layout, segment, key, value_group) : nullptr;
+                    if (!seen(chunk + quad + i)) continue;
+                    const T* column = value_column(const_cast<T*>(v_pages), block_table, layout, segment, chunk + quad + i, value_group);
                     for (int d = tid >> 4; d < vd; d += kRowsThreads / 16)
                         v_s[d * kKeyPitch + quad + i] = column != nullptr ? to_float(column[static_cast<size_t>(d) * layout.page_size]) : 0.0f;
                 }
@@ -826,6 +830,7 @@ paged_attention_rows_kernel(const T* __restrict__ q, const T* __restrict__ k_pag
         };
         int chunk = chunk_from(0), which = 0;
         fetch(chunk, 0);
+#pragma unroll 8
         for (int index = tid; index < rows * hd; index += kRowsThreads) {
             const int row = index / hd, d = index - row * hd;
             q_s[row * k_pitch + d] = to_float(q[(static_cast<size_t>(begin + row / per_group) * num_heads + group * per_group + row % per_group) * hd + d]);
@@ -838,9 +843,9 @@ paged_attention_rows_kernel(const T* __restrict__ q, const T* __restrict__ k_pag
             position[r] = row < rows ? positions[begin + row / per_group] : -1;   // a row that is none sees nothing
             first[r] = window > 0 ? max(0, position[r] - window + 1) : 0;
         }
-        for (; chunk <= highest; which ^= 1) {
+        for (; chunk <= highest; which ^= two_stages) {
             const int next = chunk_from(chunk + kRowsKeys);
-            if (next <= highest) {
+            if (two_stages && next <= highest) {
                 fetch(next, which ^ 1);
                 asm volatile("cp.async.wait_group 1;\n" ::: "memory");
             } else {
@@ -850,25 +855,30 @@ paged_attention_rows_kernel(const T* __restrict__ q, const T* __restrict__ k_pag
             const float* k_s = stages + which * stage_floats;
             const float* v_s = k_s + kRowsKeys * k_pitch;
             if (4 * (tid >> 5) < rows) {   // whole warps: their lanes exchange values
-                // scores of two rows with the keys lane, lane + 16, lane + 32, lane + 48
+                // scores of two rows with the keys lane, lane + 16, lane + 32, lane + 48, as far as there are any
                 float s[2][4] = {};
+                auto scores = [&](auto count) {
 #pragma unroll 4
-                for (int d = 0; d < hd; d += 4) {
-                    float4 query[2];
+                    for (int d = 0; d < hd; d += 4) {
+                        float4 query[2];
 #pragma unroll
-                    for (int r = 0; r < 2; ++r) query[r] = *reinterpret_cast<const float4*>(q_s + (2 * pair + r) * k_pitch + d);
+                        for (int r = 0; r < 2; ++r) query[r] = *reinterpret_cast<const float4*>(q_s + (2 * pair + r) * k_pitch + d);
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const float4 key = *reinterpret_cast<const float4*>(k_s + (lane + 16 * i) * k_pitch + d);
+                        for (int i = 0; i < count; ++i) {
+                            const float4 key = *reinterpret_cast<const float4*>(k_s + (lane + 16 * i) * k_pitch + d);
 #pragma unroll
-                        for (int r = 0; r < 2; ++r) {
-                            s[r][i] += query[r].x * key.x;
-                            s[r][i] += query[r].y * key.y;
-                            s[r][i] += query[r].z * key.z;
-                            s[r][i] += query[r].w * key.w;
+                            for (int r = 0; r < 2; ++r) {
+                                s[r][i] += query[r].x * key.x;
+                                s[r][i] += query[r].y * key.y;
+                                s[r][i] += query[r].z * key.z;
+                                s[r][i] += query[r].w * key.w;
+                            }
                         }
                     }
-                }
+                };
+                const int last = min(highest - chunk, kRowsKeys - 1);   // the last key that someone sees
+                if (last < 16) scores(std::integral_constant<int, 1>{});
+                else scores(std::integral_constant<int, 4>{});
                 float rescale[2];
 #pragma unroll
                 for (int r = 0; r < 2; ++r) {
@@ -901,8 +911,7 @@ paged_attention_rows_kernel(const T* __restrict__ q, const T* __restrict__ k_pag
 #pragma unroll
                     for (int e = 0; e < 8; ++e) acc[r][e] *= rescale[r];
                 // the values' channels lane + 16 e; a key that a row does not see (its value may be no number) is left out
-#pragma unroll 2
-                for (int key = 0; key < kRowsKeys; key += 4) {
+                auto values = [&](int key) {
                     float p[2][4];
 #pragma unroll
                     for (int r = 0; r < 2; ++r) {
@@ -920,9 +929,16 @@ paged_attention_rows_kernel(const T* __restrict__ q, const T* __restrict__ k_pag
                             for (int i = 0; i < 4; ++i)
                                 if (p[r][i] != 0.0f) acc[r][e] += p[r][i] * value[i];
                     }
+                };
+                if (last == kRowsKeys - 1) {
+#pragma unroll 2
+                    for (int key = 0; key < kRowsKeys; key += 4) values(key);
+                } else {
+                    for (int key = 0; key <= last; key += 4) values(key);
                 }
             }
             __syncthreads();   // this chunk's keys and values have been read
+            if (!two_stages && next <= highest) fetch(next, 0);
             chunk = next;
         }
 #pragma unroll
@@ -1083,7 +1099,8 @@ int lb_qk_norm_rope_write(const void* qkv, void* q_out, void* k_pages, void* v_p
 int lb_paged_attention_plain(const void* q, const void* k_pages, const void* v_pages, void* out, const int* positions,
                              const int* token_segment, const int* block_table, int tokens, int num_heads,
                              int num_groups, int head_dim, int page_size, int num_pages, int max_blocks, float scale,
-                             int window, int dtype, int* status, cudaStream_t stream, int value_dim, int keep_first, int value_groups, int out_float) {
+                             int window, int dtype, int* status, cudaStream_t stream, int value_dim, int keep_first, int value_groups, int out_float,
+                             int requests) {
     if (tokens == 0) return 0;
     if (value_dim <= 0) value_dim = head_dim;
     if (value_groups <= 0) value_groups = num_groups;
@@ -1095,15 +1112,21 @@ int lb_paged_attention_plain(const void* q, const void* k_pages, const void* v_p
     const int per_group = num_heads / num_groups;
     const bool aligned = reinterpret_cast<uintptr_t>(k_pages) % 16 == 0 && reinterpret_cast<uintptr_t>(v_pages) % 16 == 0;
     if (aligned && head_dim % 4 == 0 && value_dim % 4 == 0 && head_dim <= 128 && value_dim <= 128 && per_group <= lb::kRowsPerBlock) {
-        // Tokens a block: as many as have room, fewer where the multiprocessors would not get two blocks each.
+        // Tokens a block: as many as have room and a request has on average (only a request's tokens share keys), fewer where the multiprocessors
+        // would not get two blocks each.
         const int room = lb::kRowsPerBlock / per_group, filling = static_cast<int>(static_cast<long long>(tokens) * num_groups / (2 * lb::multiprocessor_count()));
-        const int per_block = filling < 1 ? 1 : filling < room ? filling : room;
+        const int shared_by = requests > 0 ? (tokens + requests - 1) / requests : room, most_tokens = shared_by < room ? shared_by : room;
+        const int per_block = filling < 1 ? 1 : filling < most_tokens ? filling : most_tokens;
         const dim3 blocks((tokens + per_block - 1) / per_block, num_groups);
-        auto shared_bytes = [](int key_dim, int values) {
+        const int rows_held = (per_block * per_group + 3) / 4 * 4;
+        auto shared_bytes = [](int key_dim, int values, int rows, int stages) {
             const int key_pitch = lb::kRowsKeys + lb::kRowsPad;
-            return 4 * (lb::kRowsPerBlock * (key_dim + lb::kRowsPad) + lb::kRowsPerBlock * key_pitch + 2 * (lb::kRowsKeys * (key_dim + lb::kRowsPad) + values * key_pitch));
+            return 4 * (rows * (key_dim + lb::kRowsPad + key_pitch) + stages * (lb::kRowsKeys * (key_dim + lb::kRowsPad) + values * key_pitch));
         };
-        const int bytes = shared_bytes(head_dim, value_dim), most = shared_bytes(128, 128);
+        // With more blocks than fit beside one another with two stages, one stage: the further blocks on a multiprocessor hide a chunk's loads.
+        const int resident = 228 * 1024 / (shared_bytes(head_dim, value_dim, rows_held, 2) + 1024);
+        const int two_stages = static_cast<long long>(blocks.x) * num_groups <= static_cast<long long>(resident) * lb::multiprocessor_count() ? 1 : 0;
+        const int bytes = shared_bytes(head_dim, value_dim, rows_held, 1 + two_stages), most = shared_bytes(128, 128, lb::kRowsPerBlock, 2);
         LB_DISPATCH_DTYPE(dtype, {
             static lb::OncePerDevice plain, wide;
             if (lb::allow_shared_memory(plain, lb::paged_attention_rows_kernel<T, T>, most) != cudaSuccess) return static_cast<int>(cudaGetLastError());
@@ -1111,11 +1134,11 @@ int lb_paged_attention_plain(const void* q, const void* k_pages, const void* v_p
             if (out_float)
                 lb::paged_attention_rows_kernel<T, float><<<blocks, lb::kRowsThreads, bytes, stream>>>(
                     static_cast<const T*>(q), static_cast<const T*>(k_pages), static_cast<const T*>(v_pages), static_cast<float*>(out), positions, token_segment,
-                    block_table, layout, tokens, num_heads, per_block, scale, window, window > 0 ? keep_first : 0, status);
+                    block_table, layout, tokens, num_heads, per_block, rows_held, two_stages, scale, window, window > 0 ? keep_first : 0, status);
             else
                 lb::paged_attention_rows_kernel<T, T><<<blocks, lb::kRowsThreads, bytes, stream>>>(
                     static_cast<const T*>(q), static_cast<const T*>(k_pages), static_cast<const T*>(v_pages), static_cast<T*>(out), positions, token_segment,
-                    block_table, layout, tokens, num_heads, per_block, scale, window, window > 0 ? keep_first : 0, status);
+                    block_table, layout, tokens, num_heads, per_block, rows_held, two_stages, scale, window, window > 0 ? keep_first : 0, status);
         })
         return LB_LAUNCH_RESULT();
     }

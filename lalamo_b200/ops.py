@@ -884,7 +884,7 @@ def paged_attention_plain(
         q, k_pages, v_pages, out, positions, token_segment, block_table, tokens,
         num_heads, num_groups, head_dim, page_size, num_pages, max_blocks, scale,
         window if window else 0, dtype_code(q.dtype), status, _stream(), value_dim, keep_first,
-        value_groups or 0, 1 if out.dtype == torch.float32 and q.dtype != torch.float32 else 0)
+        value_groups or 0, 1 if out.dtype == torch.float32 and q.dtype != torch.float32 else 0, block_table.shape[0])
     _done(code, "paged_attention_plain")
 
 

@@ -48,3 +48,49 @@ def test_rows(heads, groups, dim, vdim, value_groups, window, keep, page):
             want[t, h] = torch.softmax(scores, 0) @ values[i, j, g // (groups // value_groups)].double()
     # scores of size below 6 from sums of `dim` products in 32 bits: off by about sqrt(dim) roundings of 6, which is the weights' relative error
     assert float((out.cpu().view_as(want) - want).norm() / want.norm()) < 6 * dim ** 0.5 * 2 ** -24 + 2 ** -21
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads,groups,dim,window,page", [(16, 16, 64, 0, 16), (16, 16, 128, 0, 16), (16, 8, 64, 40, 16), (8, 8, 64, 0, 6)])
+def test_a_request_alone_and_beside_many(heads, groups, dim, window, page, dtype):
+    """The same bits whatever else is in the step, which decides a block's tokens and stages; few keys, and what nobody has written is no number."""
+    from lalamo_b200 import ops
+
+    generator = torch.Generator().manual_seed(dim + page)
+    random = lambda *shape: torch.randn(*shape, generator=generator)  # noqa: E731
+    lengths = [1, 2, 1, 5, 1, 1, 30] + [1] * 60
+    contexts = [0, 0, 15, 64, 127, 200, 3] + [(7 * i) % 140 for i in range(60)]
+    blocks = -(-max(n + c for n, c in zip(lengths, contexts)) // page)
+    table = torch.randperm(len(lengths) * blocks, generator=generator).view(len(lengths), blocks).to(torch.int32)
+    k_pages, v_pages = torch.empty(table.numel(), page, groups, dim), torch.empty(table.numel(), groups, dim, page)
+    for i, (n, c) in enumerate(zip(lengths, contexts)):
+        keys, values = random(blocks * page, groups, dim), random(blocks * page, groups, dim)
+        keys[n + c:] = values[n + c:] = float("nan")
+        k_pages[table[i].long()], v_pages[table[i].long()] = keys.view(blocks, page, groups, dim), values.view(blocks, page, groups, dim).permute(0, 2, 3, 1)
+    q = random(sum(lengths), heads * dim).to(dtype).cuda()
+    k_pages, v_pages = k_pages.to(dtype).cuda(), v_pages.to(dtype).cuda()
+
+    def attend(requests):
+        rows = [row for i in requests for row in range(sum(lengths[:i]), sum(lengths[:i]) + lengths[i])]
+        ints = lambda values: torch.tensor(values, dtype=torch.int32, device="cuda")  # noqa: E731
+        out, status = torch.empty(len(rows), heads * dim, dtype=dtype, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+        ops.paged_attention_plain(q[rows].contiguous(), k_pages, v_pages, out, positions=ints([c for i in requests for c in range(contexts[i], contexts[i] + lengths[i])]),
+                                  token_segment=ints([s for s, i in enumerate(requests) for _ in range(lengths[i])]), block_table=table[requests].contiguous().cuda(), num_heads=heads,
+                                  num_groups=groups, head_dim=dim, scale=dim ** -0.5, window=window or None, status=status)
+        assert int(status.item()) == 0
+        return out.cpu()
+
+    every, k_held, v_held = attend(list(range(len(lengths)))), k_pages.cpu(), v_pages.cpu()
+    assert bool(every.isfinite().all())
+    at = 0
+    for i in range(9):
+        assert torch.equal(attend([i]), every[at: at + lengths[i]]), i
+        at += lengths[i]
+    for t, (i, position) in enumerate((i, c) for i in range(9) for c in range(contexts[i], contexts[i] + lengths[i])):
+        keys = torch.arange(max(0, position - window + 1) if window else 0, position + 1)
+        k, v = k_held[table[i, keys // page].long(), keys % page].double(), v_held[table[i, keys // page].long(), :, :, keys % page].double()
+        query = q[t].cpu().double().view(groups, heads // groups, dim)
+        weights = torch.softmax(torch.einsum("gpd,kgd->gpk", query, k) * dim ** -0.5, -1)
+        want = torch.einsum("gpk,kgd->gpd", weights, v).reshape(-1)
+        # as above; in bfloat16 the result's rounding
+        assert float((every[t].double() - want).norm() / want.norm()) < 6 * dim ** 0.5 * 2 ** -24 + 2 ** -21 + (2 ** -8 if dtype == torch.bfloat16 else 0)
