@@ -1204,8 +1204,19 @@ GDR_LONG_PORTION = 192
 RECURRENT_SCRATCH_BYTES = 256 << 20
 
 
+def recurrent_plan(lengths, long_portion: int = GDR_LONG_PORTION) -> dict:
+    """What a recurrent layer plans for a step, from its portions' lengths alone: ``direct`` (the portions scanned token by token) and ``long_table`` (per long
+    portion: its index, its first block of 32 tokens among all of them, its number of blocks).  NumPy int32 arrays."""
+    import numpy as np
+
+    lengths = np.asarray(lengths, dtype=np.int32).reshape(-1)
+    direct, long = np.flatnonzero(lengths < long_portion), np.flatnonzero(lengths >= long_portion)
+    blocks = -(-lengths[long] // RECURRENT_BLOCK)
+    return {"direct": direct.astype(np.int32), "long_table": np.stack([long, np.cumsum(blocks) - blocks, blocks], axis=1).astype(np.int32).reshape(-1)}
+
+
 def gated_delta_chunk_plan(starts, lengths, chunk_tokens: int = GDR_CHUNK_TOKENS, long_portion: int = GDR_LONG_PORTION) -> dict:
-    """The host's part of the recurrences over long portions, from the portions' first rows and lengths alone: ``direct``
+    """:func:`recurrent_plan` for programs that number a portion's chunks themselves (the kernels take its tokens 32 at a time whatever the chunks): ``direct``
     (the portions scanned token by token), ``chunk_start`` / ``chunk_length`` / ``chunk_slot`` (the chunks of the long portions, numbered
     through) and ``long_table`` (per long portion: its index, its first chunk, its number of chunks).  NumPy int32 arrays."""
     import numpy as np
@@ -1237,8 +1248,8 @@ def _recurrence(q: torch.Tensor, k: torch.Tensor, decay: torch.Tensor, v: torch.
     lib = _lib()
     read_out = torch.empty(tokens, num_heads, value_dim, dtype=torch.float32, device=q.device)
     direct_list, num_direct = None, segments
-    if chunk_plan is not None and chunk_plan["num_chunks"] > 0:
-        # (which chunks the plan makes of a long portion does not matter: the kernels take its tokens 32 at a time)
+    if chunk_plan is not None and chunk_plan["num_long"] > 0:
+        # (the kernels read the first column of the table, the portions, and take their tokens 32 at a time)
         num_long, delta = chunk_plan["num_long"], 0 if beta is None else 1
         most_blocks = tokens // RECURRENT_BLOCK + num_long
         pack_floats, value_floats = num_heads * lib.lb_recurrent_pack_floats(key_dim, value_dim, delta), num_heads * lib.lb_recurrent_value_floats(value_dim, delta)
@@ -1285,9 +1296,8 @@ def gated_delta_rule(
     gate_offset: int | None = None,
 ) -> torch.Tensor:
     """The gated delta rule with a decay per head and key channel over the step's portions, from each
-    request's state slot and back into it.  ``chunk_plan`` (see :func:`gated_delta_chunk_plan`; int32 arrays on
-    the device with their sizes) lets long portions run as chunks side by side; without it every portion is
-    scanned from its first token to its last.
+    request's state slot and back into it.  ``chunk_plan`` (:func:`recurrent_plan`'s int32 arrays on the device, ``num_long`` and
+    ``num_direct``) lets long portions run in blocks of tokens; without it every portion is scanned from its first token to its last.
 
     ``proj`` ``[tokens, >= C + heads]`` holds, per token, the pre-convolution q (``groups x key_dim``), k
     (the same) and v (``heads x value_dim``), ``C`` channels in all, then one beta logit per head;
@@ -1792,9 +1802,8 @@ def linear_attention(proj: torch.Tensor, matrix_state: torch.Tensor, *, num_head
     (``heads x value_dim``) and, from column ``gate_offset`` on, the gate's logits.  The decay is ``fixed_decay`` (32-bit, one per
     head) or ``sigmoid(decay_logits + decay_bias) ** (1 / tau)`` (``decay_logits`` ``[tokens, heads * key_dim]`` in the
     activation type, the bias 32-bit).  ``matrix_state`` is ``[slots, heads, key_dim, value_dim]`` in 32-bit.  Returns
-    ``[tokens, heads * value_dim]`` in the activation type.  ``chunk_plan`` (see :func:`gated_delta_chunk_plan`) lets long portions run as
-    chunks side by side, as the gated delta rule's do: the recurrence is linear in the state, and the chunks' further columns carry
-    their decays' products.
+    ``[tokens, heads * value_dim]`` in the activation type.  ``chunk_plan`` (as :func:`gated_delta_rule`'s) lets long portions run in
+    blocks of tokens.
 
     ``lower`` (32-bit, ``heads * key_dim``): the decay is ``a = lower + (1 - lower) sigmoid(decay_logits + decay_bias)`` and the key
     ``1 - a``; ``proj`` then has no key columns (q, v).  ``query_silu``: q is silu of its columns.  ``gate_offset=None``: no gate.

@@ -110,15 +110,15 @@ class GatedDelta(Mixer):
         conv = SlotStateNeed(shape=(max(spec.conv_taps - 1, 1), self.channels))
         return CompositeNeed((matrix, conv))
 
-    # Long portions run in chunks side by side; which rows belong to which chunk depends on the portions' lengths
-    # only, and is the same for every layer of this kind.
+    # Long portions run in blocks of tokens; which portions are long depends on their lengths only, and is the same for every layer of
+    # this kind.
     step_plan_uses_context = False
 
     def step_plan_key(self) -> object:
-        return ("gated_delta", ops.GDR_CHUNK_TOKENS, ops.GDR_LONG_PORTION)
+        return ("gated_delta", ops.GDR_LONG_PORTION)
 
     def plan_step(self, segments: HostSegments) -> dict[str, np.ndarray]:
-        return ops.gated_delta_chunk_plan(segments.start, segments.length)
+        return ops.recurrent_plan(segments.length)
 
     def forward(self, x: torch.Tensor, step: StepInputs, cache: CompositeView) -> torch.Tensor:  # type: ignore[override]
         spec = self.spec
@@ -127,7 +127,7 @@ class GatedDelta(Mixer):
             raise ValueError("a gated-delta layer cannot read another layer's state")
         status = self.runtime.status
         lists, host_lists = step.plan_of(self)
-        chunk_plan = dict(lists, num_chunks=host_lists["chunk_start"].size, num_long=host_lists["long_table"].size // 3, num_direct=host_lists["direct"].size)
+        chunk_plan = dict(lists, num_long=host_lists["long_table"].size // 3, num_direct=host_lists["direct"].size)
         proj = ops.linear(x, self.in_proj, status=status)
         if self.direct:
             logits = proj[:, self.decay_offset :]

@@ -123,10 +123,10 @@ class LinearAttention(Mixer):
     step_plan_uses_context = False
 
     def step_plan_key(self) -> object:
-        return ("gated_delta", ops.GDR_CHUNK_TOKENS, ops.GDR_LONG_PORTION)
+        return ("gated_delta", ops.GDR_LONG_PORTION)
 
     def plan_step(self, segments: HostSegments) -> dict[str, np.ndarray]:
-        return ops.gated_delta_chunk_plan(segments.start, segments.length)
+        return ops.recurrent_plan(segments.length)
 
     can_accumulate = True
     can_defer = True
@@ -139,7 +139,7 @@ class LinearAttention(Mixer):
             raise ValueError("a linear-attention layer cannot read another layer's state")
         status = self.runtime.status
         lists, host_lists = step.plan_of(self)
-        chunk_plan = dict(lists, num_chunks=host_lists["chunk_start"].size, num_long=host_lists["long_table"].size // 3, num_direct=host_lists["direct"].size)
+        chunk_plan = dict(lists, num_long=host_lists["long_table"].size // 3, num_direct=host_lists["direct"].size)
         proj = ops.linear(x, self.in_proj, status=status)
         logits = proj[:, self.forget_offset :] if self.forget_offset is not None else None
         if self.decay_down is not None:
