@@ -441,7 +441,7 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const 
             }
         }
     } else if (warp == 1 && lane == 0 && rank == 0) {
-        // as instruction_descriptor and instruction_descriptor_pair, for the tile's tokens
+        // as instruction_descriptor, for the tile's tokens and (PAIR) 256 rows
         const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(tile_tokens >> 3) << 17) | (static_cast<uint32_t>((PAIR ? 256 : 128) >> 4) << 24);
         int consumed = 0, local = 0;
         bool ok = true;

@@ -10,7 +10,7 @@
 // What bounds it: with hundreds of rows an expert the way from L2 (an item reads 48 KB for 512 cycles of products; 12.5 TB/s
 // over all multiprocessors while it runs); with a few rows an expert the stream of the experts' matrices from HBM, each
 // read once.  Measured, 16 experts of 2048 x 2048, 4 a token: 2,048 tokens 144 us up and 81 us down (950 and 850 TFLOP/s; 632 and 379 us
-// on mma.sync tiles of 64 x 64), 8 tokens 97 us in all (113 us where every pair streams its expert's rows).
+// on mma.sync tiles of 64 x 64), 8 tokens, caches cold, 96 us in all (130 us where every pair streams its expert's rows).
 // Every wait on a barrier is bounded, as in gemm_tcgen05.cu.
 #include "tcgen05.cuh"
 

@@ -194,12 +194,8 @@ __device__ __forceinline__ void tma_load_2d_pair(void* destination, const CUtens
         ::"r"(smem_address(destination)), "l"(map), "r"(cluster_barrier), "r"(x), "r"(y)
         : "memory");
 }
-// D float32 [256, BN] over the pair (128 rows in each CTA's tensor memory), A [256, 16] and B [BN, 16]
-// bfloat16, K-major: each CTA holds its 128 rows of A and its BN / 2 rows of B at the same shared offsets.
-template <int BN>
-__device__ __forceinline__ constexpr uint32_t instruction_descriptor_pair() {
-    return (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(BN >> 3) << 17) | (static_cast<uint32_t>(256 >> 4) << 24);
-}
+// D float32 [256, N] over the pair (128 rows in each CTA's tensor memory), A [256, 16] and B [N, 16]
+// bfloat16, K-major: each CTA holds its 128 rows of A and its N / 2 rows of B at the same shared offsets.
 __device__ __forceinline__ void mma_f16_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, bool accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"

@@ -1664,7 +1664,7 @@ def moe_route(x: torch.Tensor, router: torch.Tensor, *, top: int, group_count: i
 
 
 # Up to this many (token, expert) pairs, and this many of their experts' elements a matrix, each pair streams its expert's weights; more are grouped by expert.  Measured
-# over both products, cold caches: of 2048 x 2048 experts 16 pairs 85 us streamed and 92 grouped, 32 pairs 132 and 97; of 1024 x 1152 experts a layer of 20 pairs 66.5 and
+# over both products, cold caches: of 2048 x 2048 experts 16 pairs 88 us streamed and 89 grouped, 24 pairs 130 and 94, 32 pairs 130 and 96; of 1024 x 1152 experts a layer of 20 pairs 66.5 and
 # 72.7, of 32 pairs 72.7 and 74.8, 48 pairs' products 75 and 52.
 MOE_STREAM_MAX_PAIRS = 32
 MOE_STREAM_MAX_ELEMENTS = 16 * 2048 * 2048

@@ -25,7 +25,7 @@ def test_products(tokens, rows, width, epilogue, slices):
         want = want + residual.double()
     got = ops.linear_tcgen05(x, w, epilogue, residual, slices=slices, activation="silu" if epilogue == "gated" else "identity", status=status)
     assert int(status.item()) == 0
-    # Rounded to bfloat16, each time by at most 2**-9 of the value: a stored sum once, a float one not at all (its sums are 32-bit); a gated
+    # Rounded to bfloat16, each time by at most 2**-8 of the value, over a row by less than 2**-9 in the root mean square: a stored sum once, a float one not at all (its sums are 32-bit); a gated
     # result four times, both sides, the activated gate and itself, of which the gate's own is passed on times g silu'(g) / silu(g), about one
     # where the result is not small: four times 2**-9 if all four went the same way.
     bound = {"gated": 4, "store": 1, "residual_add": 1, "store_float": 2 ** -10}[epilogue] * 2 ** -9

@@ -38,8 +38,8 @@ def test_ragged_experts(counts, width, ff, gated, weigh):
             u = up[e].double() @ x[t].double() * before
             hidden = torch.nn.functional.silu(gate[e].double() @ x[t].double() * before) * u if gated else torch.nn.functional.gelu(u)
             want[t] += after * (down[e].double() @ hidden)
-    # Rounded to bfloat16 on the way: both sides, the activated gate, the hidden value, the result, each by at most 2**-9 of itself
-    # and in no common direction: sqrt(5) * 2**-9 of the norm at the most.
+    # Rounded to bfloat16 on the way: both sides, the activated gate, the hidden value, the result, each by at most 2**-8 of itself, by less than
+    # 2**-9 in the root mean square, and in no common direction: sqrt(5) * 2**-9 of the norm at the most.
     assert float((got - want).norm() / want.norm()) < 5 ** 0.5 * 2 ** -9
     assert int(status.item()) == 0
 
