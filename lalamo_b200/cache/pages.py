@@ -78,7 +78,8 @@ class PagePool(_IdPool):
         return [self._take() for _ in range(count)]
 
     def release(self, pages: list[int]) -> None:
-        for page in pages:
+        """Gives the pages back, the first of them to be handed out first again: pages that follow one another stay neighbours."""
+        for page in reversed(pages):
             self._give_back(page)
 
 

@@ -255,7 +255,8 @@ __global__ void gate_heads_kernel(const T* __restrict__ values, const T* __restr
 
 
 // ------------------------------------------------------------------------------- tensor cores
-// The same attention on mma.sync (bfloat16, 32-bit accumulation) for latent + rope and latent multiples of 16.
+// The same attention on mma.sync (bfloat16, 32-bit accumulation) for latent + rope and latent multiples of 16, where attention_latent_tcgen05.cu does not
+// take the sizes (other latents than 64, 128, 192 and 256, more than 64 heads).
 //
 // A CTA of four warps takes one item: up to 64 query rows = consecutive tokens of one request x a block of heads,
 // 16 rows a warp.  All rows share the cached rows (there is one "key head"), which come through shared memory in blocks
@@ -599,6 +600,10 @@ __global__ void latent_merge_kernel(const float* __restrict__ partial, __nv_bflo
 }
 
 
+void launch_latent_merge(const float* partial, __nv_bfloat16* out, int rows, int splits, int latent, const float* sink, int num_heads, cudaStream_t stream) {
+    latent_merge_kernel<<<rows, 128, splits * sizeof(float), stream>>>(partial, out, splits, latent, sink, num_heads);
+}
+
 // ------------------------------------------------------------------ one small product per head
 // out[t][h][n] = sum_k a[t][h][k] * B_h[k][n] for every head h, with B_h stored [K][N] (B_KN: a head's key projection, which takes
 // the unrotated query channels into the latent's space) or [N][K] (a head's value projection applied to the summed rows), optionally
@@ -796,7 +801,7 @@ int lb_latent_attention_mma(const void* q, const void* pages, void* out, float* 
     const int chunk = wide ? 256 : 128;
     const dim3 grid(num_items, p.head_blocks * splits, (latent + chunk - 1) / chunk);
     kernel<<<grid, 32 * warps, shared, stream>>>(p);
-    if (splits > 1) lb::latent_merge_kernel<<<tokens * num_heads, 128, splits * sizeof(float), stream>>>(partial, static_cast<__nv_bfloat16*>(out), splits, latent, sink, num_heads);
+    if (splits > 1) lb::launch_latent_merge(partial, static_cast<__nv_bfloat16*>(out), tokens * num_heads, splits, latent, sink, num_heads, stream);
     return LB_LAUNCH_RESULT();
 }
 

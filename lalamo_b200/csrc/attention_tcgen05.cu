@@ -85,41 +85,9 @@ __device__ __forceinline__ uint64_t value_box_descriptor(const void* tile) {
     return ((address & 0x3FFFFull) >> 4) | (1ull << 16) | (static_cast<uint64_t>(256 >> 4) << 32) | (1ull << 46) | (6ull << 61);
 }
 
-__device__ __forceinline__ void tmem_store_32(uint32_t address, const uint32_t (&v)[32]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, "
-        "%23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-        ::"r"(address), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]),
-          "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]),
-          "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
-        : "memory");
-    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-}
-
 __device__ __forceinline__ float max3(float a, float b, float c) {
     float d;
     asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-    return d;
-}
-
-// Two float32 values in one 64-bit register, for the packed arithmetic of sm_100 (one instruction for two
-// fused multiply-adds or additions).
-__device__ __forceinline__ uint64_t pack2(float low, float high) {
-    uint64_t packed;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(packed) : "f"(low), "f"(high));
-    return packed;
-}
-__device__ __forceinline__ void unpack2(uint64_t packed, float& low, float& high) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(low), "=f"(high) : "l"(packed));
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
 

@@ -1562,12 +1562,32 @@ def latent_attention_splits(num_items: int, num_heads: int, latent: int, window:
     return max(1, min(blocks // 2, -(-2 * sms // ctas), 32))   # two blocks a CTA: one block each was measured 1 % slower
 
 
+def latent_attention_tcgen05_supported(dtype: torch.dtype, latent: int, rope: int, page_size: int, num_heads: int, scale: float) -> bool:
+    """Whether :func:`latent_attention` takes these sizes on the fifth-generation tensor cores (``tcgen05``): panels of 64 latent channels and one of
+    16, 32 or 64 rotated ones, of which 384 rows fit the shared memory, and every head of a token among an item's 128 rows."""
+    return (dtype == torch.bfloat16 and latent in (64, 128, 192, 256) and rope in (16, 32, 64) and page_size % 16 == 0 and 1 <= num_heads <= LATENT_MMA_ROWS and scale > 0.0
+            and 384 * 2 * (latent + rope) + 3328 <= 226 * 1024)
+
+
+def latent_attention_tcgen05_splits(num_items: int, tokens: int, num_heads: int, window: int | None, max_context: int, sms: int | None = None) -> int:
+    """Over how many CTAs an item's cached rows are shared out by the kernel on the fifth-generation tensor cores.  A CTA fills a multiprocessor, so that the
+    shares of all items are one round of them at most; a tile of 128 rows takes it 2.6 us, a merge 8 us, and 0.7 us and 1 us per 1,000 rows of queries more for
+    every share (16 heads over 256 + 32 channels, 1 share and the chosen: 8 tokens that decode behind 4,000 cached ones 54 and 24 us, 9 tokens behind
+    2,000 52 and 34, 300 behind 3,000 54 and 48; 512 behind 4,096 stay at 56, in 2 shares 60, 300 behind none at 24, in 2 shares 36)."""
+    rows = min(window, max_context) if window else max_context
+    tiles = -(-(rows + 2 * latent_attention_tiling(num_heads)[1]) // 128) + 1
+    most = min(tiles, (sms or sm_count()) // max(1, num_items), 32)
+    cost = lambda shares: 2.6 * -(-tiles // shares) + (8 + shares * (0.7 + tokens * num_heads / 1000) if shares > 1 else 0)  # noqa: E731
+    return min(range(1, max(1, most) + 1), key=cost)
+
+
 def latent_attention(q: torch.Tensor, pages: torch.Tensor, out: torch.Tensor, *, items: torch.Tensor, num_items: int, positions: torch.Tensor,
                      token_segment: torch.Tensor, block_table: torch.Tensor, num_heads: int, latent: int, rope: int, scale: float, window: int | None,
-                     status: torch.Tensor, splits: int = 1, sink: torch.Tensor | None = None, double: bool = False) -> None:
+                     status: torch.Tensor, splits: int = 1, sink: torch.Tensor | None = None, double: bool = False, tcgen05: bool = False) -> None:
     """:func:`latent_attention_plain` on the tensor cores (bfloat16).  ``items``: int32 ``[num_items, 2]`` (first token row,
     count), each at most ``latent_attention_tiling(num_heads)[1]`` consecutive tokens of one request (twice as many with
-    ``double``, where :func:`latent_attention_takes_double`), together all tokens.  ``splits`` > 1 shares an item's cached rows out over that many CTAs, merged in split order.  ``sink``: as for
+    ``double``, where :func:`latent_attention_takes_double`), together all tokens.  ``splits`` > 1 shares an item's cached rows out over that many CTAs, merged in split order.  ``tcgen05``: on
+    the fifth-generation ones, with runs of up to twice as many tokens, where :func:`latent_attention_tcgen05_supported`.  ``sink``: as for
     :func:`latent_attention_plain`."""
     _check_sink(sink, num_heads)
     _check(q, "q", torch.bfloat16)
@@ -1580,6 +1600,14 @@ def latent_attention(q: torch.Tensor, pages: torch.Tensor, out: torch.Tensor, *,
     if pages.dtype != q.dtype or not latent_attention_supported(q.dtype, latent, rope, page_size):
         raise KernelError(f"latent_attention: latent {latent}, rope {rope}, pages of {page_size} are not sizes the tensor-core kernel takes")
     heads_per_cta, tokens_per_cta = latent_attention_tiling(num_heads)
+    if tcgen05:
+        if not latent_attention_tcgen05_supported(q.dtype, latent, rope, page_size, num_heads, scale):
+            raise KernelError(f"latent_attention: latent {latent}, rope {rope}, {num_heads} heads, pages of {page_size} are not sizes the tcgen05 kernel takes")
+        partial = torch.empty(tokens, num_heads, splits, latent + 2, dtype=torch.float32, device=q.device) if splits > 1 else None
+        code = _lib().lb_latent_attention_tcgen05(q, pages, out, partial, items, num_items, positions, token_segment, block_table, tokens, num_heads, latent, rope,
+                                                  page_size, num_pages, max_blocks, scale, window if window else 0, splits, status, _stream(), sink)
+        _done(code, "latent_attention_tcgen05", 2 if splits > 1 else 1)
+        return
     if double:
         if not latent_attention_takes_double(latent, rope):
             raise KernelError(f"latent_attention: rows of {latent} + {rope} channels leave no room for runs of twice as many tokens")

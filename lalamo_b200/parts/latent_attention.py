@@ -76,7 +76,9 @@ class LatentAttention(Mixer):
         self.sink = runtime.vector(tensors["sink"]) if spec.sink else None
         self.position = build_part(spec.position, {}, runtime)
         self.scale = spec.scale if spec.scale is not None else (dim + rope) ** -0.5
-        self.takes_double = ops.latent_attention_takes_double(spec.latent_dim, rope)
+        # "always": sizes whose kernel has room for runs of twice as many tokens in every step
+        self.tcgen05 = ops.latent_attention_tcgen05_supported(runtime.dtype, spec.latent_dim, rope, 16, heads, self.scale)
+        self.takes_double = "always" if self.tcgen05 else ops.latent_attention_takes_double(spec.latent_dim, rope)
 
     @classmethod
     def tensor_decls(cls, spec: LatentAttentionSpec) -> dict[str, TensorDecl]:
@@ -115,10 +117,11 @@ class LatentAttention(Mixer):
         return ("latent_attention", ops.latent_attention_tiling(self.spec.num_heads), self.takes_double)
 
     def plan_step(self, segments: HostSegments) -> dict[str, np.ndarray]:
-        """``items``: ``(first row, count)`` of every run of consecutive tokens that one CTA takes (twice as many a run where
-        :func:`ops.latent_attention_doubles` says so, and some portion is longer than a single run)."""
+        """``items``: ``(first row, count)`` of every run of consecutive tokens that one CTA takes (twice as many a run for
+        the kernel on the fifth-generation tensor cores, and elsewhere where :func:`ops.latent_attention_doubles` says so and some portion is longer
+        than a single run)."""
         _, run = ops.latent_attention_tiling(self.spec.num_heads)
-        if self.takes_double and ops.latent_attention_doubles(segments.length, self.spec.num_heads):
+        if self.takes_double == "always" or self.takes_double and ops.latent_attention_doubles(segments.length, self.spec.num_heads):
             run *= 2
         items = [(first, min(run, start + length - first)) for start, length in zip(segments.start, segments.length) for first in range(start, start + length, run)]
         return {"items": np.asarray(items, dtype=np.int32).reshape(-1)}
@@ -168,9 +171,13 @@ class LatentAttention(Mixer):
         if ops.latent_attention_supported(runtime.dtype, latent, rope, cache.k_pages.shape[1]):
             lists, host_lists = step.plan_of(self)
             num_items = host_lists["items"].size // 2
-            double = num_items > 0 and int(host_lists["items"][1::2].max()) > ops.latent_attention_tiling(heads)[1]
-            splits = ops.latent_attention_splits(num_items, heads, latent, spec.window, step.max_context, double=double)
-            ops.latent_attention(queries, cache.k_pages, summed, items=lists["items"], num_items=num_items, splits=splits, double=double, **common)
+            double = False
+            if self.tcgen05:
+                splits = ops.latent_attention_tcgen05_splits(num_items, tokens, heads, spec.window, step.max_context)
+            else:
+                double = num_items > 0 and int(host_lists["items"][1::2].max()) > ops.latent_attention_tiling(heads)[1]
+                splits = ops.latent_attention_splits(num_items, heads, latent, spec.window, step.max_context, double=double)
+            ops.latent_attention(queries, cache.k_pages, summed, items=lists["items"], num_items=num_items, splits=splits, double=double, tcgen05=self.tcgen05, **common)
         else:
             ops.latent_attention_plain(queries, cache.k_pages, summed, **common)
         mixed = runtime.empty(tokens, heads * spec.value_dim)
