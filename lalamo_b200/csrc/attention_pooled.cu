@@ -12,7 +12,8 @@
 // Four kernels: `pooled_rewrite` (rotation of q, k and v in 32-bit, one rounding, pages written), `pooled_means` (the mean
 // of every block that the step completes, from the pages, into the pooled pages), `pooled_attention_plain` (a block per token
 // and head, everything 32-bit: the 32-bit path and the reference for the tensor-core kernel) and `pooled_attention_mma`
-// (bfloat16 on mma.sync m16n8k16: a CTA takes up to 64 consecutive tokens of a portion and up to four query heads of one K/V head).
+// (bfloat16 on mma.sync m16n8k16: a CTA takes up to 64 consecutive tokens of a portion and up to four query heads of one K/V head; heads of 64 + 64
+// channels run on attention_pooled_tcgen05.cu instead).
 // Keys are summed in the order blocks 0, 1, ... then positions upwards, whatever the step's cutting.
 //
 // Pages: a row holds all a position leaves behind, [page][row][group][key (dk) | value (dv)], `page_size` rows a page, found
@@ -792,6 +793,11 @@ __global__ void pooled_finish_kernel(const float* __restrict__ partial, int shar
     }
 }
 
+void launch_pooled_finish(const float* partial, int shares, __nv_bfloat16* out, const int* positions, int total_rows, int heads, int dv, const float* v_freq, int v_interleaved,
+                          const int* tiles, int num_tiles, int tile_tokens, cudaStream_t stream) {
+    pooled_finish_kernel<<<dim3(num_tiles, tile_tokens), 256, dv * sizeof(float), stream>>>(partial, shares, out, positions, total_rows, heads, dv, v_freq, v_interleaved, nullptr, tiles);
+}
+
 }  // namespace lb
 
 extern "C" {
@@ -874,9 +880,7 @@ int lb_pooled_attention_mma(const void* q, const void* pages, const void* pooled
             q16, pages16, pooled16, out16, tiles, positions, token_segment, block_table, pool_table, L, heads, head_block, scale, cap, head_bias, window, pool, v_freq,
             v_interleaved, status, partial, total_rows);
     }
-    if (shares > 1)
-        lb::pooled_finish_kernel<<<dim3(num_tiles, 16 * (lb::kPooledMmaWarps / head_block)), 256, dv * sizeof(float), stream>>>(partial, shares, out16, positions, total_rows, heads, dv, v_freq,
-                                                                                                            v_interleaved, nullptr, tiles);
+    if (shares > 1) lb::launch_pooled_finish(partial, shares, out16, positions, total_rows, heads, dv, v_freq, v_interleaved, tiles, num_tiles, 16 * (lb::kPooledMmaWarps / head_block), stream);
     return LB_LAUNCH_RESULT();
 }
 

@@ -1995,6 +1995,25 @@ def pooled_attention_supported(dtype: torch.dtype, head_dim: int, value_dim: int
     return dtype == torch.bfloat16 and head_dim % 16 == 0 and value_dim % 16 == 0 and 16 <= head_dim <= 128 and 16 <= value_dim <= 128
 
 
+def pooled_attention_tcgen05_supported(dtype: torch.dtype, head_dim: int, value_dim: int, page_size: int) -> bool:
+    """Whether :func:`pooled_attention` runs on the fifth-generation tensor cores: heads of 64 key and 64 value channels, pages of whole boxes of 16 rows."""
+    return dtype == torch.bfloat16 and head_dim == 64 and value_dim == 64 and page_size % 16 == 0
+
+
+def pooled_attention_tcgen05_shares(num_tiles: int, tokens: int, num_heads: int, num_groups: int, window: int, pool: int, max_context: int | None = None,
+                                    sms: int | None = None) -> int:
+    """Over how many CTAs a tile's rows of the cache are shared out by the kernel on the fifth-generation tensor cores.  A CTA takes 1.1 us for 64 rows, alone on its
+    multiprocessor or beside a second one; adding up takes 6 us, and 4 us a share for every 1,000 tokens of 16 heads.  Measured, 1 share and the chosen: 33 tokens
+    behind 3,000 39 and 22 us, 300 behind 3,000 41 and 28; 300 behind none stay at 16, in 3 shares 20; 2,048 behind none at 39, in 2 shares 56.
+    ``max_context``: positions of the longest request; left out, as many as a window has."""
+    head_block, tile_tokens = pooled_attention_tiling(num_heads, num_groups)
+    ctas, sms = num_tiles * num_groups * -(-(num_heads // num_groups) // head_block), sms or sm_count()
+    context = window if max_context is None else max_context
+    rows = -(-min(context, window + tile_tokens) // 64) + 1 + (-(-max(0, context - window) // (64 * pool)) if pool else 0)
+    cost = lambda shares: 1.1 * -(-rows // shares) * max(1.0, ctas * shares / sms) + (6 + shares * (0.1 + tokens * num_heads / 4000) if shares > 1 else 0)  # noqa: E731
+    return min(range(1, max(1, min(rows, 2 * sms // ctas, 16)) + 1), key=cost)
+
+
 def _pooled_arguments(q, pages, pool_pages, out, positions, token_segment, block_table, pool_table, num_heads, num_groups, head_dim, value_dim, head_bias,
                       window, pool, value_freq, what):
     _check(q, "q")
@@ -2040,15 +2059,15 @@ def pooled_attention_plain(q: torch.Tensor, pages: torch.Tensor, pool_pages: tor
     _done(code, "pooled_attention_plain")
 
 
-def pooled_attention(q: torch.Tensor, pages: torch.Tensor, pool_pages: torch.Tensor | None, out: torch.Tensor, *, tiles: torch.Tensor, num_tiles: int, shares: int | None = None,
+def pooled_attention(q: torch.Tensor, pages: torch.Tensor, pool_pages: torch.Tensor | None, out: torch.Tensor, *, tiles: torch.Tensor, num_tiles: int, shares: int | None = None, max_context: int | None = None,
                      positions: torch.Tensor, token_segment: torch.Tensor, block_table: torch.Tensor, pool_table: torch.Tensor | None, num_heads: int,
                      num_groups: int, head_dim: int, value_dim: int, scale: float, softcap: float, head_bias: torch.Tensor | None, window: int, pool: int,
                      value_freq: torch.Tensor | None, interleaved: bool = False, status: torch.Tensor) -> None:
     """The same attention on the tensor cores (bfloat16; see :func:`pooled_attention_supported`).  ``tiles``: int32 ``(first row, count)``
     per tile of consecutive tokens of one portion, at most :func:`pooled_attention_tiling`'s tokens each.  Weights in 32-bit (the cap's
     tanh and the sigmoid through the fast exponential and reciprocal), rounded to bfloat16 for the product with the values; sums in 32-bit.  Launches
-    of few CTAs share out every tile's rows of the cache over several CTAs (:func:`pooled_attention_shares`), whose 32-bit sums a second
-    kernel adds in order."""
+    of few CTAs share out every tile's rows of the cache over several CTAs (:func:`pooled_attention_shares`,
+    :func:`pooled_attention_tcgen05_shares`), whose 32-bit sums a second kernel adds in order."""
     tokens, (count, page_size, max_blocks), (pool_count, pool_rows, pool_blocks) = _pooled_arguments(
         q, pages, pool_pages, out, positions, token_segment, block_table, pool_table, num_heads, num_groups, head_dim, value_dim, head_bias, window, pool,
         value_freq, "pooled_attention")
@@ -2058,11 +2077,20 @@ def pooled_attention(q: torch.Tensor, pages: torch.Tensor, pool_pages: torch.Ten
     if tiles.numel() < 2 * num_tiles:
         raise KernelError("pooled_attention: fewer tile records than tiles")
     head_block, _ = pooled_attention_tiling(num_heads, num_groups)
+    tcgen05 = pooled_attention_tcgen05_supported(q.dtype, head_dim, value_dim, page_size)
     if shares is None:
-        shares = pooled_attention_shares(num_tiles, num_heads, num_groups)
+        shares = (pooled_attention_tcgen05_shares(num_tiles, tokens, num_heads, num_groups, window, pool, max_context) if tcgen05
+                  else pooled_attention_shares(num_tiles, num_heads, num_groups))
     if not 1 <= shares <= 64:
         raise KernelError("pooled_attention: 1 to 64 shares")
     partial = torch.empty(shares, tokens, num_heads * value_dim, dtype=torch.float32, device=q.device) if shares > 1 else None
+    if tcgen05:
+        code = _lib().lb_pooled_attention_tcgen05(q, pages, pool_pages if pool else None, out, tiles, num_tiles, positions, token_segment, block_table,
+                                                  pool_table if pool else None, num_heads, num_groups, page_size, count, max_blocks, pool_rows, pool_count, pool_blocks,
+                                                  head_block, scale, softcap, head_bias, window, pool, value_freq, 1 if interleaved else 0, status, _stream(), shares,
+                                                  partial, tokens)
+        _done(code, "pooled_attention_tcgen05", 2 if shares > 1 else 1)
+        return
     code = _lib().lb_pooled_attention_mma(q, pages, pool_pages if pool else None, out, tiles, num_tiles, positions,
                                           token_segment, block_table, pool_table if pool else None, num_heads, num_groups,
                                           head_dim, value_dim, page_size, count, max_blocks, pool_rows, pool_count,

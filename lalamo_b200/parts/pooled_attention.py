@@ -126,7 +126,8 @@ class PooledWindowAttention(Mixer):
             if host_lists["singles"].size:
                 ops.pooled_attention_single(queries, tokens_view.k_pages, pool_pages, mixed, singles=lists["singles"], num_singles=host_lists["singles"].size, **common)
             if host_lists["tiles"].size:
-                ops.pooled_attention(queries, tokens_view.k_pages, pool_pages, mixed, tiles=lists["tiles"], num_tiles=host_lists["tiles"].size // 2, **common)
+                ops.pooled_attention(queries, tokens_view.k_pages, pool_pages, mixed, tiles=lists["tiles"], num_tiles=host_lists["tiles"].size // 2,
+                                     max_context=step.max_context, **common)
         else:
             ops.pooled_attention_plain(queries, tokens_view.k_pages, pool_pages, mixed, **common)
         if residual is not None:
