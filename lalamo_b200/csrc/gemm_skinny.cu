@@ -25,9 +25,10 @@ constexpr int kSkinnyWarps = 8;
 enum SkinnyEpilogue : int { kStore = 0, kStoreFloat = 1, kResidualAdd = 2, kGated = 3, kShortConv = 4 };
 
 struct SkinnyParams {
-    const __nv_bfloat16* x;   // [tokens, k]
+    const __nv_bfloat16* x;   // [tokens, k], rows x_stride elements apart
     const __nv_bfloat16* w;   // [rows, k]
     void* out;                // see the epilogues
+    int x_stride;
     int tokens, k, n;         // n: output columns (rows of one row block of W)
     int row_block_stride;     // rows between the row blocks that the epilogue combines
     int activation;
@@ -102,8 +103,8 @@ gemm_skinny_kernel(const SkinnyParams p) {
     }
     wait_for_previous_kernel();
     const bool low_valid = g < p.tokens, high_valid = WIDE && g + 8 < p.tokens;
-    const __nv_bfloat16* x_low = p.x + static_cast<size_t>(low_valid ? g : 0) * p.k + 8 * t;
-    const __nv_bfloat16* x_high = p.x + static_cast<size_t>(high_valid ? g + 8 : 0) * p.k + 8 * t;
+    const __nv_bfloat16* x_low = p.x + static_cast<size_t>(low_valid ? g : 0) * p.x_stride + 8 * t;
+    const __nv_bfloat16* x_high = p.x + static_cast<size_t>(high_valid ? g + 8 : 0) * p.x_stride + 8 * t;
 
     // Chunks whose loads are issued together.  A small product is bound by latency unless (nearly) all
     // of the matrix is in flight at once, so the leanest variant loads eight chunks per lane at a time.
@@ -259,15 +260,18 @@ int launch_skinny(const SkinnyParams& p, cudaStream_t stream) {
 extern "C" {
 
 // Returns 0, a CUDA error, or -2 when the sizes are not the kernel's (1..16 tokens, k % 32 == 0,
-// n % 8 == 0, 16-byte aligned rows).
+// n % 8 == 0, 16-byte aligned rows).  The rows of x lie x_stride elements apart.
 int lb_gemm_skinny(const void* x, const void* w, void* out, int tokens, int k, int n, int epilogue, int activation,
                    void* state, const float* conv_weight, const float* conv_bias, const int* token_segment,
                    const int* segment_start, const int* segment_length, const int* segment_slot, int segments, int taps,
-                   int num_slots, int prefetch, int* status, cudaStream_t stream, float limit, const float* bias) {
+                   int num_slots, int prefetch, int* status, cudaStream_t stream, float limit, const float* bias, int x_stride) {
     if (tokens == 0) return 0;
-    if (tokens < 1 || tokens > 16 || k % 32 != 0 || n % 8 != 0 || k < 32) return -2;
+    if (tokens < 1 || tokens > 16 || k % 32 != 0 || n % 8 != 0 || k < 32 || x_stride < k || x_stride % 8 != 0 ||
+        ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15))
+        return -2;
     lb::SkinnyParams p;
     p.x = static_cast<const __nv_bfloat16*>(x);
+    p.x_stride = x_stride;
     p.w = static_cast<const __nv_bfloat16*>(w);
     p.out = out;
     p.tokens = tokens;
@@ -288,7 +292,7 @@ int lb_gemm_skinny(const void* x, const void* w, void* out, int tokens, int k, i
     p.num_slots = num_slots;
     p.status = status;
     p.bias = bias;
-    p.prefetch = prefetch && (reinterpret_cast<uintptr_t>(w) & 15) == 0 ? 1 : 0;
+    p.prefetch = prefetch ? 1 : 0;
     switch (epilogue) {
         case lb::kStore: return lb::launch_skinny<1, lb::kStore>(p, stream);
         case lb::kStoreFloat: return lb::launch_skinny<1, lb::kStoreFloat>(p, stream);

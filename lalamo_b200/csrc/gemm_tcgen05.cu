@@ -29,6 +29,7 @@ enum TcEpilogue : int { kTcStore = 0, kTcStoreFloat = 1, kTcResidualAdd = 2, kTc
 struct TcParams {
     void* out;          // [tokens, n] bfloat16 / float32 / residual, or partials [slices, tokens, n]
     int tokens, n, k;
+    int x_stride;       // elements between the rows of X
     int blocks_per_slice;   // 64-column blocks of K per slice
     int epilogue;
     int hidden;         // kTcGated: W is [2 * hidden, k], rows [up ; gate]; out is [tokens, hidden]
@@ -770,13 +771,13 @@ __global__ void gemm_tcgen05_reduce_kernel(const float* __restrict__ partials, v
     }
 }
 
-// A [rows, k] bfloat16 row-major matrix seen through boxes of [box_rows, 64] with 128-byte swizzle;
+// A [rows, k] bfloat16 matrix, rows `stride` elements apart, seen through boxes of [box_rows, 64] with 128-byte swizzle;
 // what lies outside the matrix reads as zero.
-static bool make_map(CUtensorMap* map, const void* base, int rows, int k, int box_rows) {
+static bool make_map(CUtensorMap* map, const void* base, int rows, int k, int box_rows, int stride) {
     EncodeTiled encode = encode_tiled();
     if (encode == nullptr) return false;
     const cuuint64_t dims[2] = {static_cast<cuuint64_t>(k), static_cast<cuuint64_t>(rows)};
-    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(k) * 2};
+    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(stride) * 2};
     const cuuint32_t box[2] = {kTcBlockK, static_cast<cuuint32_t>(box_rows)};
     const cuuint32_t element_strides[2] = {1, 1};
     return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, element_strides, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -799,7 +800,7 @@ int launch_tcgen05(const CUtensorMap& map_w, const void* x, TcParams p, int slic
     const int rows_per_cta = p.epilogue == kTcGated ? kTcRows / 2 : kTcRows;
     const int row_extent = p.epilogue == kTcGated ? p.hidden : p.n;
     CUtensorMap map_x;
-    if (!make_map(&map_x, x, p.tokens, p.k, BN)) return -5;
+    if (!make_map(&map_x, x, p.tokens, p.k, BN, p.x_stride)) return -5;
     const dim3 grid((row_extent + rows_per_cta - 1) / rows_per_cta, (p.tokens + BN - 1) / BN, slices);
     // About 100 KB of stages lets two CTAs share an SM, so that one's epilogue hides behind the other's
     // products.  A grid that does not even fill the SMs once gets all of an SM's shared memory instead:
@@ -839,7 +840,7 @@ template <int BN, bool PAIR>
 int launch_persistent(const CUtensorMap& map_w, const void* x, TcParams p, int m_tiles, int sms, int slices, cudaStream_t stream, int tile_tokens = BN) {
     CUtensorMap map_x;
     p.tile_tokens = tile_tokens;
-    if (!make_map(&map_x, x, p.tokens, p.k, PAIR ? tile_tokens / 2 : tile_tokens)) return -5;
+    if (!make_map(&map_x, x, p.tokens, p.k, PAIR ? tile_tokens / 2 : tile_tokens, p.x_stride)) return -5;
     const bool is_partial = p.epilogue == kTcPartial;
     const bool is_float = p.epilogue == kTcStoreFloat || p.epilogue == kTcResidualAdd || is_partial, is_gated = p.epilogue == kTcGated;
     const int width = is_gated ? p.hidden : p.n;
@@ -917,8 +918,8 @@ long long lb_gemm_tcgen05_scratch_floats(int tokens, int n, int slices) {
 // defer_sum: with more than one slice, leave the partial sums in `scratch` ([slices][tokens][n]) for the
 // caller (lb_sum_slices, or a consumer that adds them itself); `out` is not touched then.
 static int gemm_tcgen05_launch(const void* x, const void* w, void* out, float* scratch, long long scratch_floats, int tokens, int k, int n, int epilogue,
-                               int activation, int slices, int defer_sum, int* status, cudaStream_t stream, float limit, const float* bias, int store_activation) {
-    if (tokens < 1 || n < 1 || k < 8 || k % 8 != 0 || epilogue < 0 || epilogue == 3 || epilogue > 4) return -2;
+                               int activation, int slices, int defer_sum, int* status, cudaStream_t stream, float limit, const float* bias, int store_activation, int x_stride) {
+    if (tokens < 1 || n < 1 || k < 8 || k % 8 != 0 || epilogue < 0 || epilogue == 3 || epilogue > 4 || x_stride < k || x_stride % 8 != 0) return -2;
     if (store_activation >= 0) {
         if (epilogue != lb::kTcStore || store_activation > 2) return -2;
         slices = 1;   // the bias and the activation belong to the whole sum
@@ -934,6 +935,7 @@ static int gemm_tcgen05_launch(const void* x, const void* w, void* out, float* s
     p.tokens = tokens;
     p.n = n;
     p.k = k;
+    p.x_stride = x_stride;
     p.blocks_per_slice = (total_blocks + slices - 1) / slices;
     slices = (total_blocks + p.blocks_per_slice - 1) / p.blocks_per_slice;
     p.status = status;
@@ -953,7 +955,7 @@ static int gemm_tcgen05_launch(const void* x, const void* w, void* out, float* s
         p.epilogue = epilogue;
     }
     CUtensorMap map_w;
-    if (!lb::make_map(&map_w, w, n, k, epilogue == lb::kTcGated ? lb::kTcRows / 2 : lb::kTcRows)) return -5;
+    if (!lb::make_map(&map_w, w, n, k, epilogue == lb::kTcGated ? lb::kTcRows / 2 : lb::kTcRows, k)) return -5;
     int code;
     if (tokens > 128 && slices == 1) {
         // Many tokens: one CTA (or pair of CTAs) per SM walks the tiles.
@@ -1005,8 +1007,8 @@ static int gemm_tcgen05_launch(const void* x, const void* w, void* out, float* s
 }
 
 int lb_gemm_tcgen05(const void* x, const void* w, void* out, float* scratch, long long scratch_floats, int tokens, int k, int n, int epilogue,
-                    int activation, int slices, int defer_sum, int* status, cudaStream_t stream, float limit) {
-    return gemm_tcgen05_launch(x, w, out, scratch, scratch_floats, tokens, k, n, epilogue, activation, slices, defer_sum, status, stream, limit, nullptr, -1);
+                    int activation, int slices, int defer_sum, int* status, cudaStream_t stream, float limit, int x_stride) {
+    return gemm_tcgen05_launch(x, w, out, scratch, scratch_floats, tokens, k, n, epilogue, activation, slices, defer_sum, status, stream, limit, nullptr, -1, x_stride);
 }
 
 // out[t, r] = bfloat16(act(sum_k x[t, k] w[r, k] + bias[r])): the sum, the bias (32-bit, may be null) and the activation
@@ -1014,7 +1016,7 @@ int lb_gemm_tcgen05(const void* x, const void* w, void* out, float* scratch, lon
 int lb_gemm_tcgen05_bias_activation(const void* x, const void* w, const float* bias, void* out, int tokens, int k, int n, int activation, int* status,
                                     cudaStream_t stream) {
     if (activation < 0 || activation > 2) return -2;
-    return gemm_tcgen05_launch(x, w, out, nullptr, 0, tokens, k, n, lb::kTcStore, 2, 1, 0, status, stream, 0.0f, bias, activation);
+    return gemm_tcgen05_launch(x, w, out, nullptr, 0, tokens, k, n, lb::kTcStore, 2, 1, 0, status, stream, 0.0f, bias, activation, k);
 }
 
 // out = epilogue(partials[0] + partials[1] + ...), the slices added in order; partials is [slices][tokens][n].

@@ -2202,17 +2202,17 @@ def skinny_supported(x: torch.Tensor, rows: int) -> bool:
 
 
 def _skinny(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, n: int, epilogue: str, activation: str = "identity", conv: dict | None = None,
-            prefetch: bool = True, limit: float = 0.0, bias: torch.Tensor | None = None) -> None:
-    """``prefetch``: the kernel asks for its weights towards L2 before it waits for the kernel before it; off where
+            prefetch: bool = True, limit: float = 0.0, bias: torch.Tensor | None = None, x_stride: int = 0) -> None:
+    """``x_stride``: elements between the rows of ``x`` (0: as many as it has columns).  ``prefetch``: the kernel asks for its weights towards L2 before it waits for the kernel before it; off where
     that kernel does not let it start early (see :func:`successor_starts_early`)."""
     tokens, width = x.shape
     if conv is None:
         code = _lib().lb_gemm_skinny(x, weight, out, tokens, width, n, _SKINNY_EPILOGUES[epilogue], _ACTIVATIONS[activation], None, None, None, None, None, None, None, 0,
-                                     0, 0, 1 if prefetch else 0, None, _stream(), limit, bias)
+                                     0, 0, 1 if prefetch else 0, None, _stream(), limit, bias, x_stride or width)
     else:
         code = _lib().lb_gemm_skinny(x, weight, out, tokens, width, n, _SKINNY_EPILOGUES[epilogue], _ACTIVATIONS[activation], conv["state"], conv["weight"], conv["bias"],
                                      conv["token_segment"], conv["segment_start"], conv["segment_length"], conv["segment_slot"], conv["segments"], conv["taps"],
-                                     conv["num_slots"], 1 if prefetch else 0, conv["status"], _stream(), limit, bias)
+                                     conv["num_slots"], 1 if prefetch else 0, conv["status"], _stream(), limit, bias, width)
     _done(code, "gemm_skinny")
 
 
@@ -2268,16 +2268,18 @@ def _settled_slices(slices: int, width: int) -> int:
 
 def linear_tcgen05(x: torch.Tensor, weight: torch.Tensor, epilogue: str = "store", residual: torch.Tensor | None = None,
                    slices: int | None = None, activation: str = "identity", status: torch.Tensor | None = None,
-                   defer_sum: bool = False, limit: float = 0.0) -> torch.Tensor | SlicedSum:
+                   defer_sum: bool = False, limit: float = 0.0, x_stride: int = 0) -> torch.Tensor | SlicedSum:
     """``x @ weight.T`` on the tcgen05 tensor cores.  ``epilogue``: ``"store"`` (bfloat16),
     ``"store_float"``, ``"residual_add"`` (into ``residual``, float32, which is returned) or ``"gated"``
     (``weight`` is ``[up ; gate]``, the result ``up * activation(gate)`` of half as many columns).
     ``status``: the int32 word in which the kernel reports a wait that gave up.  ``defer_sum``: if the
     product is cut into K slices, return them as a :class:`SlicedSum` (nothing is stored or added) for a
-    consumer that adds them itself."""
+    consumer that adds them itself.  ``x_stride``: elements between the rows of ``x``, which then are columns of a wider matrix (the caller has
+    looked at them: :func:`linear_of_columns`)."""
     if status is not None:
         _check(status, "status", torch.int32)
-    _check(x, "x", torch.bfloat16)
+    if not x_stride:
+        _check(x, "x", torch.bfloat16)
     _check(weight, "weight", torch.bfloat16)
     tokens, width = x.shape
     rows = weight.shape[0]
@@ -2313,7 +2315,7 @@ def linear_tcgen05(x: torch.Tensor, weight: torch.Tensor, epilogue: str = "store
         scratch = _tc_scratch[index]
     code = _lib().lb_gemm_tcgen05(x, weight, out, scratch, scratch.numel() if scratch is not None else 0,
                                   tokens, width, rows, _TC_EPILOGUES[epilogue], _ACTIVATIONS[activation], slices,
-                                  1 if deferred else 0, status, _stream(), limit)
+                                  1 if deferred else 0, status, _stream(), limit, x_stride or width)
     if code == -5:
         raise KernelError("linear_tcgen05: the driver gave no tensor map (cuTensorMapEncodeTiled)")
     _done(code, "gemm_tcgen05", 2 if slices > 1 and not deferred else 1)
@@ -2351,6 +2353,28 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype | None 
     if wants_float:
         return torch.mm(x, weight.t(), out_dtype=out_dtype)
     return torch.mm(x, weight.t())
+
+
+def linear_of_columns(x: torch.Tensor, first: int, weight: torch.Tensor, status: torch.Tensor | None = None) -> torch.Tensor:
+    """``x[:, first : first + width] @ weight.T`` for a weight of ``width`` columns, on the kernels :func:`linear` takes for these sizes, without a
+    copy of the columns: what a product of several matrices over the same rows hands on to one that reads a part of it."""
+    _check(x, "x")
+    _check(weight, "weight", x.dtype)
+    rows, width = weight.shape
+    if x.dim() != 2 or first < 0 or first + width > x.shape[1]:
+        raise KernelError(f"linear_of_columns: columns {first} to {first + width} of a matrix of shape {tuple(x.shape)}")
+    columns = x[:, first : first + width]
+    if columns.data_ptr() % 16 or x.shape[1] % 8 or x.dtype != torch.bfloat16 or not x.shape[0]:   # rows that do not start on 16 bytes, and the 32-bit path
+        # (a copy also of a single row, whose columns count as contiguous where they lie)
+        return linear(columns.clone(memory_format=torch.contiguous_format), weight, status=status) if x.dtype == torch.bfloat16 else torch.mm(columns, weight.t())
+    if skinny_supported(columns, rows) and not (USE_TCGEN05 and rows >= TCGEN05_MIN_ROWS_FEW_TOKENS):
+        out = torch.empty(x.shape[0], rows, dtype=x.dtype, device=x.device)
+        _skinny(columns, weight, out, rows, "store", x_stride=x.shape[1])
+        return out
+    if USE_TCGEN05 and tcgen05_supported(columns, rows):
+        return linear_tcgen05(columns, weight, "store", slices=1 if x.shape[0] <= SKINNY_MAX_TOKENS and rows >= TCGEN05_MIN_ROWS_FEW_TOKENS else None, status=status,
+                              x_stride=x.shape[1])
+    return torch.mm(columns, weight.t())
 
 
 def linear_pending(x: torch.Tensor, weight: torch.Tensor, status: torch.Tensor | None = None, bias: torch.Tensor | None = None) -> "torch.Tensor | SlicedSum | BiasedSum":

@@ -57,15 +57,15 @@ class GatedDelta(Mixer):
             padded[self.decay_offset + self.gate_offset : self.decay_offset + self.gate_offset + heads * dv] = tensors["gate_proj"]
             self.in_proj = runtime.matrix(padded)
         else:
+            # [q ; k ; v ; beta | down-projection of the decays | of the gate]: one product for everything that reads the layer's input
             self.gate_offset = decay_columns
-            padded = torch.zeros(_round_up(rows.shape[0], 8), spec.model_dim, dtype=rows.dtype)
-            padded[: rows.shape[0]] = rows
-            self.in_proj = runtime.matrix(padded)
             decay_rank, gate_rank = _round_up(spec.decay_rank, 32), _round_up(spec.gate_rank, 32)
-            down = torch.zeros(decay_rank + gate_rank, spec.model_dim, dtype=rows.dtype)
-            down[: spec.decay_rank] = tensors["decay_down"]
-            down[decay_rank : decay_rank + spec.gate_rank] = tensors["gate_down"]
-            self.low_rank_down = runtime.matrix(down)
+            self.low_offset = _round_up(rows.shape[0], 8)
+            padded = torch.zeros(self.low_offset + decay_rank + gate_rank, spec.model_dim, dtype=rows.dtype)
+            padded[: rows.shape[0]] = rows
+            padded[self.low_offset : self.low_offset + spec.decay_rank] = tensors["decay_down"]
+            padded[self.low_offset + decay_rank : self.low_offset + decay_rank + spec.gate_rank] = tensors["gate_down"]
+            self.in_proj = runtime.matrix(padded)
             up = torch.zeros(decay_columns + heads * dv, decay_rank + gate_rank, dtype=rows.dtype)
             up[:decay_columns, : spec.decay_rank] = tensors["decay_up"]
             up[decay_columns:, decay_rank : decay_rank + spec.gate_rank] = tensors["gate_up"]
@@ -132,8 +132,7 @@ class GatedDelta(Mixer):
         if self.direct:
             logits = proj[:, self.decay_offset :]
         else:
-            low = ops.linear(x, self.low_rank_down, status=status)
-            logits = ops.linear(low, self.low_rank_up, status=status)
+            logits = ops.linear_of_columns(proj, self.low_offset, self.low_rank_up, status=status)
         read_out = ops.gated_delta_rule(
             proj,
             logits,

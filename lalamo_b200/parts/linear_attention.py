@@ -42,7 +42,7 @@ class LinearAttention(Mixer):
             raise ValueError(f"unknown gate activation {spec.gate_activation!r}; known: 'sigmoid', 'silu', 'none'")
         if spec.query_activation not in ("identity", "silu"):
             raise ValueError(f"unknown query activation {spec.query_activation!r}; known: 'identity', 'silu'")
-        # [q ; (k) ; v | gate | forget gate], each part of the product starting at a multiple of 8 rows
+        # [q ; (k) ; v | gate | forget gate or down-projection of the decays], each part of the product starting at a multiple of 8 rows
         names = ["q_proj", "v_proj"] if spec.decay == "forget" else ["q_proj", "k_proj", "v_proj"]
         parts = [torch.cat([tensors[name] for name in names], dim=0)]
         end = _round_up(parts[0].shape[0], 8)
@@ -53,13 +53,19 @@ class LinearAttention(Mixer):
         if spec.decay == "forget":
             self.forget_offset, end = end, _round_up(end + heads * dk, 8)
             parts.append(tensors["forget_proj"])
+        rank = _round_up(spec.decay_rank, 32)
+        if spec.decay == "channel":
+            if spec.decay_rank < 1 or spec.tau <= 0.0:
+                raise ValueError("a decay made from the token needs a bottleneck of positive rank and a positive tau")
+            self.low_offset, end = end, end + rank
+            parts.append(tensors["decay_down"])
         padded = torch.zeros(end, spec.model_dim, dtype=parts[0].dtype)
         offset = 0
         for part in parts:
             padded[offset : offset + part.shape[0]] = part
             offset = _round_up(offset + part.shape[0], 8)
         self.in_proj = runtime.matrix(padded)
-        self.fixed_decay = self.decay_down = self.decay_up = self.decay_bias = self.lower = None
+        self.fixed_decay = self.decay_up = self.decay_bias = self.lower = None
         if spec.decay == "forget":
             self.decay_bias = runtime.vector(tensors["forget_bias"])
             self.lower = runtime.vector(tensors["lower"])
@@ -68,14 +74,9 @@ class LinearAttention(Mixer):
                 raise ValueError(f"{len(spec.decay_values)} fixed decays for {heads} heads")
             self.fixed_decay = runtime.vector(torch.tensor(spec.decay_values, dtype=torch.float64))
         else:
-            if spec.decay_rank < 1 or spec.tau <= 0.0:
-                raise ValueError("a decay made from the token needs a bottleneck of positive rank and a positive tau")
-            rank = _round_up(spec.decay_rank, 32)
-            down = torch.zeros(rank, spec.model_dim, dtype=padded.dtype)
-            down[: spec.decay_rank] = tensors["decay_down"]
             up = torch.zeros(_round_up(heads * dk, 8), rank, dtype=padded.dtype)
             up[: heads * dk, : spec.decay_rank] = tensors["decay_up"]
-            self.decay_down, self.decay_up = runtime.matrix(down), runtime.matrix(up)
+            self.decay_up = runtime.matrix(up)
             self.decay_bias = runtime.vector(tensors["decay_bias"])
         self.norm_weight = runtime.vector(tensors["out_norm"] if spec.norm_weight else torch.ones(dv))
         self.out_proj = runtime.matrix(tensors["out_proj"])
@@ -142,8 +143,8 @@ class LinearAttention(Mixer):
         chunk_plan = dict(lists, num_long=host_lists["long_table"].size // 3, num_direct=host_lists["direct"].size)
         proj = ops.linear(x, self.in_proj, status=status)
         logits = proj[:, self.forget_offset :] if self.forget_offset is not None else None
-        if self.decay_down is not None:
-            logits = ops.linear(ops.linear(x, self.decay_down, status=status), self.decay_up, status=status)
+        if self.decay_up is not None:
+            logits = ops.linear_of_columns(proj, self.low_offset, self.decay_up, status=status)
         read_out = ops.linear_attention(
             proj,
             cache.state,
