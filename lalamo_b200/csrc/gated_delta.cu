@@ -54,6 +54,8 @@ __global__ void gdr_prepare_kernel(const T* __restrict__ proj, int proj_width, c
                                    const int* __restrict__ token_segment, const int* __restrict__ segment_start,
                                    const int* __restrict__ segment_slot, int heads, int groups, int dk, int dv, int taps,
                                    int num_slots, float unit_eps, float q_scale, int* status, int decay_per_head) {
+    wait_for_previous_kernel();
+    allow_next_kernel();
     // decay_per_head: `ag` holds one decay logit per head (heads columns) and dt_bias one element per head; the head's
     // decay is written to all of its key channels.
     // UPDATE: every portion of the step is one token, and the lane that convolves a channel (the only reader of that
@@ -157,6 +159,8 @@ gdr_prepare_run_kernel(const T* __restrict__ proj, int proj_width, const T* __re
                        float* __restrict__ k_out, float* __restrict__ v_out, float* __restrict__ beta_out, float* __restrict__ g_out,
                        const int* __restrict__ token_segment, const int* __restrict__ segment_start, const int* __restrict__ segment_slot, int tokens, int heads, int groups,
                        int dk, int dv, int num_slots, float unit_eps, float q_scale, int* status, int decay_per_head) {
+    wait_for_previous_kernel();
+    allow_next_kernel();
     constexpr int TAPS = kPrepareTaps;
     __shared__ __align__(16) float rows_s[4][128];   // a warp's rows of queries or keys, its pieces' side by side
     const int unit = blockIdx.y, warp = threadIdx.x >> 5;
@@ -270,6 +274,8 @@ template <typename T>
 __global__ void gdr_conv_state_kernel(const T* __restrict__ proj, int proj_width, T* __restrict__ conv_state, const int* __restrict__ segment_start,
                                       const int* __restrict__ segment_length, const int* __restrict__ segment_slot, int channels, int taps,
                                       int num_slots) {
+    wait_for_previous_kernel();
+    allow_next_kernel();
     const int segment = blockIdx.x;
     const int slot = segment_slot[segment];
     if (slot < 0 || slot >= num_slots) return;   // reported by the kernel before
@@ -320,6 +326,8 @@ gdr_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, const 
                 const float* __restrict__ beta, float* __restrict__ state, float* __restrict__ out, const int* __restrict__ segment_start,
                 const int* __restrict__ segment_length, const int* __restrict__ segment_slot, int heads, int groups, int dk, int dv,
                 int num_slots, int* status, const int* __restrict__ segment_list) {
+    wait_for_previous_kernel();
+    allow_next_kernel();
     // segment_list (may be null): the portions this launch runs.
     constexpr int R = kScanThreadRows, C = kScanThreadCols;
     static_assert(DKP == R * SPLIT && SPLIT <= 32, "a column's rows lie in one warp");
@@ -481,44 +489,60 @@ gdr_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, const 
 }
 
 // grid (tokens, slices of the heads), a warp per head: out[t, h, :] = T(o / sqrt(mean(o^2) + eps) * w * sigmoid(gate[t, h, :]));
-// without gates (ag null) the last factor is left out.
-template <typename T>
+// without gates (ag null) the last factor is left out.  FOURS: rows that come in fours, on addresses that do, of at most 128 channels: a lane has
+// four neighbours, and a row and its gates are on their way together (2,048 tokens of 8 heads of 128: see below 12 us without).
+template <typename T, bool FOURS>
 __global__ void gdr_output_kernel(const float* __restrict__ o, const T* __restrict__ ag, int ag_width, int gate_offset,
                                   const float* __restrict__ norm_weight, T* __restrict__ out, int heads, int dv, float eps, int gate_silu) {
+    wait_for_previous_kernel();
     allow_next_kernel();   // the out-projection, launched to start early, may ask for its weights meanwhile
     const int token = blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     for (int head = blockIdx.y * warps + warp; head < heads; head += gridDim.y * warps) {
         const float* row = o + (static_cast<size_t>(token) * heads + head) * dv;
         const T* gate = ag != nullptr ? ag + static_cast<size_t>(token) * ag_width + gate_offset + static_cast<size_t>(head) * dv : nullptr;
-        float sum = 0.0f;
-        for (int c = lane; c < dv; c += 32) sum += row[c] * row[c];
-        sum = warp_sum(sum);
-        const float inv = rsqrtf(sum / static_cast<float>(dv) + eps);
         T* dst = out + (static_cast<size_t>(token) * heads + head) * dv;
-        for (int c = lane; c < dv; c += 32) {
-            const float z = gate != nullptr ? to_float(gate[c]) : 0.0f;
-            const float factor = gate == nullptr ? 1.0f : (gate_silu ? z * sigmoidf_(z) : sigmoidf_(z));
-            dst[c] = from_float<T>(row[c] * inv * norm_weight[c] * factor);
+        auto factor_of = [&](float z) { return gate == nullptr ? 1.0f : (gate_silu ? z * sigmoidf_(z) : sigmoidf_(z)); };
+        if constexpr (FOURS) {
+            float x[4] = {}, z[4] = {}, w[4] = {};
+            const int c = 4 * lane;
+            if (c < dv) {
+                load_four(row + c, x);
+                if (gate != nullptr) load_four(gate + c, z);
+                load_four(norm_weight + c, w);
+            }
+            const float sum = warp_sum((x[0] * x[0] + x[1] * x[1]) + (x[2] * x[2] + x[3] * x[3]));
+            const float inv = rsqrtf(sum / static_cast<float>(dv) + eps);
+            if (c < dv) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) x[e] = x[e] * inv * w[e] * factor_of(z[e]);
+                if constexpr (sizeof(T) == 4) {
+                    *reinterpret_cast<float4*>(dst + c) = make_float4(x[0], x[1], x[2], x[3]);
+                } else {
+                    const __nv_bfloat162 low = __floats2bfloat162_rn(x[0], x[1]), high = __floats2bfloat162_rn(x[2], x[3]);
+                    *reinterpret_cast<uint2*>(dst + c) = make_uint2(*reinterpret_cast<const uint32_t*>(&low), *reinterpret_cast<const uint32_t*>(&high));
+                }
+            }
+        } else {
+            float sum = 0.0f;
+            for (int c = lane; c < dv; c += 32) sum += row[c] * row[c];
+            sum = warp_sum(sum);
+            const float inv = rsqrtf(sum / static_cast<float>(dv) + eps);
+            for (int c = lane; c < dv; c += 32) dst[c] = from_float<T>(row[c] * inv * norm_weight[c] * factor_of(gate != nullptr ? to_float(gate[c]) : 0.0f));
         }
     }
 }
 
 template <int DKP, int SPLIT>
-inline void launch_scan(dim3 grid, cudaStream_t stream, const float* q, const float* k, const float* g, const float* v, const float* beta,
-                        float* state, float* out, const int* segment_start, const int* segment_length, const int* segment_slot, int heads,
-                        int groups, int dk, int dv, int num_slots, int* status, const int* segment_list) {
-    if (beta != nullptr) {
-        static OncePerDevice once;
-        allow_shared_memory(once, gdr_scan_kernel<DKP, SPLIT, true>, static_cast<int>(ScanShared<DKP>::kBytes));
-        gdr_scan_kernel<DKP, SPLIT, true><<<grid, (kScanCols / kScanThreadCols) * SPLIT, ScanShared<DKP>::kBytes, stream>>>(
-            q, k, g, v, beta, state, out, segment_start, segment_length, segment_slot, heads, groups, dk, dv, num_slots, status, segment_list);
-    } else {
-        static OncePerDevice once;
-        allow_shared_memory(once, gdr_scan_kernel<DKP, SPLIT, false>, static_cast<int>(ScanShared<DKP>::kBytes));
-        gdr_scan_kernel<DKP, SPLIT, false><<<grid, (kScanCols / kScanThreadCols) * SPLIT, ScanShared<DKP>::kBytes, stream>>>(
-            q, k, g, v, beta, state, out, segment_start, segment_length, segment_slot, heads, groups, dk, dv, num_slots, status, segment_list);
-    }
+inline int launch_scan(dim3 grid, cudaStream_t stream, const float* q, const float* k, const float* g, const float* v, const float* beta,
+                       float* state, float* out, const int* segment_start, const int* segment_length, const int* segment_slot, int heads,
+                       int groups, int dk, int dv, int num_slots, int* status, const int* segment_list) {
+    static OncePerDevice once[2];
+    auto kernel = beta != nullptr ? gdr_scan_kernel<DKP, SPLIT, true> : gdr_scan_kernel<DKP, SPLIT, false>;
+    const cudaError_t allowed = allow_shared_memory(once[beta != nullptr ? 1 : 0], kernel, static_cast<int>(ScanShared<DKP>::kBytes));
+    if (allowed != cudaSuccess) return static_cast<int>(allowed);
+    return static_cast<int>(launch_overlapped(kernel, grid, dim3((kScanCols / kScanThreadCols) * SPLIT), ScanShared<DKP>::kBytes, stream, q, k, g, v, beta, state, out, segment_start,
+                                              segment_length, segment_slot, heads, groups, dk, dv, num_slots, status, segment_list));
 }
 
 }  // namespace lb
@@ -539,33 +563,27 @@ int lb_gdr_prepare(const void* proj, int proj_width, const void* ag, int ag_widt
         const auto in_fours = [](const void* address) { return reinterpret_cast<uintptr_t>(address) % (4 * sizeof(T)) == 0; };
         if (!update_state && taps == lb::kPrepareTaps && dk % 4 == 0 && dv % 4 == 0 && dk <= 128 && dv <= 128 && proj_width % 4 == 0 &&
             (decay_per_head || ag_width % 4 == 0) && in_fours(proj) && (decay_per_head || in_fours(ag)) && in_fours(conv_state) && reinterpret_cast<uintptr_t>(conv_weight) % 16 == 0) {
-            lb::gdr_prepare_run_kernel<T><<<dim3((tokens + 4 * lb::kPrepareRun - 1) / (4 * lb::kPrepareRun), units), 128, 0, stream>>>(
-                static_cast<const T*>(proj), proj_width, static_cast<const T*>(ag), ag_width, static_cast<const T*>(conv_state), conv_weight, a_log, dt_bias, q_out, k_out,
-                v_out, beta_out, g_out, token_segment, segment_start, segment_slot, tokens, heads, groups, dk, dv, num_slots, unit_eps, q_scale, status, decay_per_head);
-            return LB_LAUNCH_RESULT();
+            return static_cast<int>(lb::launch_overlapped(
+                lb::gdr_prepare_run_kernel<T>, dim3((tokens + 4 * lb::kPrepareRun - 1) / (4 * lb::kPrepareRun), units), dim3(128), 0, stream, static_cast<const T*>(proj),
+                proj_width, static_cast<const T*>(ag), ag_width, static_cast<const T*>(conv_state), conv_weight, a_log, dt_bias, q_out, k_out, v_out, beta_out, g_out, token_segment,
+                segment_start, segment_slot, tokens, heads, groups, dk, dv, num_slots, unit_eps, q_scale, status, decay_per_head));
         }
-        if (update_state)
-            lb::gdr_prepare_kernel<T, true><<<grid, 128, 0, stream>>>(static_cast<const T*>(proj), proj_width, static_cast<const T*>(ag), ag_width,
-                                                                       static_cast<T*>(conv_state), conv_weight, a_log, dt_bias, q_out, k_out, v_out, beta_out, g_out,
-                                                                       token_segment, segment_start, segment_slot, heads, groups, dk, dv, taps, num_slots, unit_eps,
-                                                                       q_scale, status, decay_per_head);
-        else
-            lb::gdr_prepare_kernel<T, false><<<grid, 128, 0, stream>>>(static_cast<const T*>(proj), proj_width, static_cast<const T*>(ag), ag_width,
-                                                                        static_cast<const T*>(conv_state), conv_weight, a_log, dt_bias, q_out, k_out, v_out, beta_out,
-                                                                        g_out, token_segment, segment_start, segment_slot, heads, groups, dk, dv, taps, num_slots,
-                                                                        unit_eps, q_scale, status, decay_per_head);
+        auto launch = [&](auto kernel, auto* slots) {
+            return static_cast<int>(lb::launch_overlapped(kernel, grid, dim3(128), 0, stream, static_cast<const T*>(proj), proj_width, static_cast<const T*>(ag), ag_width, slots,
+                                                          conv_weight, a_log, dt_bias, q_out, k_out, v_out, beta_out, g_out, token_segment, segment_start, segment_slot, heads, groups,
+                                                          dk, dv, taps, num_slots, unit_eps, q_scale, status, decay_per_head));
+        };
+        return update_state ? launch(lb::gdr_prepare_kernel<T, true>, static_cast<T*>(conv_state)) : launch(lb::gdr_prepare_kernel<T, false>, static_cast<const T*>(conv_state));
     })
-    return LB_LAUNCH_RESULT();
 }
 
 int lb_gdr_conv_state(const void* proj, int proj_width, void* conv_state, const int* segment_start, const int* segment_length,
                       const int* segment_slot, int segments, int channels, int taps, int num_slots, int dtype, cudaStream_t stream) {
     if (segments == 0 || taps <= 1) return 0;
     LB_DISPATCH_DTYPE(dtype, {
-        lb::gdr_conv_state_kernel<T><<<dim3(segments, (channels + 255) / 256), 256, 0, stream>>>(static_cast<const T*>(proj), proj_width, static_cast<T*>(conv_state), segment_start,
-                                                                   segment_length, segment_slot, channels, taps, num_slots);
+        return static_cast<int>(lb::launch_overlapped(lb::gdr_conv_state_kernel<T>, dim3(segments, (channels + 255) / 256), dim3(256), 0, stream, static_cast<const T*>(proj), proj_width,
+                                                      static_cast<T*>(conv_state), segment_start, segment_length, segment_slot, channels, taps, num_slots));
     })
-    return LB_LAUNCH_RESULT();
 }
 
 // segment_list (may be null): the portions to run, `segments` of them.
@@ -576,24 +594,21 @@ int lb_gdr_scan(const float* q, const float* k, const float* g, const float* v, 
     if (segments == 0) return 0;
     if (dk < 1 || dk > 256 || dv < 1 || heads % groups != 0) return -2;
     const dim3 grid(segments, heads, (dv + lb::kScanCols - 1) / lb::kScanCols);
-    if (dk <= 32)
-        lb::launch_scan<32, 4>(grid, stream, q, k, g, v, beta, state, out, segment_start, segment_length, segment_slot, heads, groups, dk, dv, num_slots, status, segment_list);
-    else if (dk <= 64)
-        lb::launch_scan<64, 8>(grid, stream, q, k, g, v, beta, state, out, segment_start, segment_length, segment_slot, heads, groups, dk, dv, num_slots, status, segment_list);
-    else if (dk <= 128)
-        lb::launch_scan<128, 16>(grid, stream, q, k, g, v, beta, state, out, segment_start, segment_length, segment_slot, heads, groups, dk, dv, num_slots, status, segment_list);
-    else
-        lb::launch_scan<256, 32>(grid, stream, q, k, g, v, beta, state, out, segment_start, segment_length, segment_slot, heads, groups, dk, dv, num_slots, status, segment_list);
-    return LB_LAUNCH_RESULT();
+    auto launch = dk <= 32 ? lb::launch_scan<32, 4> : dk <= 64 ? lb::launch_scan<64, 8> : dk <= 128 ? lb::launch_scan<128, 16> : lb::launch_scan<256, 32>;
+    return launch(grid, stream, q, k, g, v, beta, state, out, segment_start, segment_length, segment_slot, heads, groups, dk, dv, num_slots, status, segment_list);
 }
 
 int lb_gdr_output(const float* o, const void* ag, int ag_width, int gate_offset, const float* norm_weight, void* out, int tokens, int heads, int dv,
                   float eps, int dtype, cudaStream_t stream, int gate_silu) {
     if (tokens == 0) return 0;
     LB_DISPATCH_DTYPE(dtype, {
-        lb::gdr_output_kernel<T><<<dim3(tokens, (heads + 3) / 4), 128, 0, stream>>>(o, static_cast<const T*>(ag), ag_width, gate_offset, norm_weight, static_cast<T*>(out), heads, dv, eps, gate_silu);
+        const auto in_fours = [](const void* address) { return reinterpret_cast<uintptr_t>(address) % (4 * sizeof(T)) == 0; };
+        const bool fours = dv % 4 == 0 && dv <= 128 && (ag == nullptr || (ag_width % 4 == 0 && gate_offset % 4 == 0 && in_fours(ag))) && in_fours(out) &&
+                           ((reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(norm_weight)) & 15) == 0;
+        auto kernel = fours ? lb::gdr_output_kernel<T, true> : lb::gdr_output_kernel<T, false>;
+        return static_cast<int>(lb::launch_overlapped(kernel, dim3(tokens, (heads + 3) / 4), dim3(128), 0, stream, o, static_cast<const T*>(ag), ag_width, gate_offset, norm_weight,
+                                                      static_cast<T*>(out), heads, dv, eps, gate_silu));
     })
-    return LB_LAUNCH_RESULT();
 }
 
 }  // extern "C"

@@ -29,6 +29,8 @@ __global__ void linear_attention_prepare_kernel(const T* __restrict__ proj, int 
                                                 float* __restrict__ v_out, float* __restrict__ g_out, int heads, int dk, int dv, const float* __restrict__ lower,
                                                 int q_silu, const float* __restrict__ inv_freq, const int* __restrict__ positions, int half, float factor) {
     extern __shared__ float turns[];   // cosines, then sines: half of each
+    wait_for_previous_kernel();
+    allow_next_kernel();
     const int token = blockIdx.x;
     const T* row = proj + static_cast<size_t>(token) * stride;
     const int key_width = heads * dk, value_width = heads * dv;
@@ -93,11 +95,10 @@ int lb_linear_attention_prepare(const void* proj, int stride, const void* z, int
     if (inv_freq != nullptr && (positions == nullptr || rotary_dim < 2 || rotary_dim % 2 != 0 || rotary_dim > dk || lower != nullptr || q_silu)) return -2;
     const int half = inv_freq != nullptr ? rotary_dim / 2 : 0;
     LB_DISPATCH_DTYPE(dtype, {
-        lb::linear_attention_prepare_kernel<T><<<tokens, 256, 2 * half * sizeof(float), stream>>>(static_cast<const T*>(proj), stride, static_cast<const T*>(z), z_stride, z_bias,
-                                                                            fixed_decay, inverse_tau, q_scale, k_scale, q_out, k_out, v_out, g_out, heads, dk, dv, lower, q_silu,
-                                                                                                    inv_freq, positions, half, factor);
+        return static_cast<int>(lb::launch_overlapped(lb::linear_attention_prepare_kernel<T>, dim3(tokens), dim3(256), 2 * half * sizeof(float), stream, static_cast<const T*>(proj), stride,
+                                                      static_cast<const T*>(z), z_stride, z_bias, fixed_decay, inverse_tau, q_scale, k_scale, q_out, k_out, v_out, g_out, heads, dk, dv,
+                                                      lower, q_silu, inv_freq, positions, half, factor));
     })
-    return LB_LAUNCH_RESULT();
 }
 
 }  // extern "C"

@@ -235,6 +235,8 @@ __global__ void __launch_bounds__(kBlockThreads, DKP <= 128 ? 3 : 1)
 recurrent_prepare_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ g, const float* __restrict__ v,
                          const float* __restrict__ beta, float* __restrict__ pack, float* __restrict__ vpack, const int* __restrict__ long_table, int long_portions, const int* __restrict__ segment_start,
                 const int* __restrict__ segment_length, int heads, int groups, int dk, int dv, int window) {
+    wait_for_previous_kernel();
+    allow_next_kernel();
     using Pack = BlockPack<DKP>;
     using Shared = PrepareShared<DKP>;
     constexpr int P = Shared::kPitch, VP = Shared::kValuePitch, TP = kTrianglePitch;
@@ -418,27 +420,34 @@ struct WalkShared {
     static constexpr int kStage = Pack::kFloats + Pack::kValues;
     // Three or four blocks on their way at once (two at 256 key channels): a block's copies take longer to arrive than its work takes.
     static constexpr int kStages = DKP <= 32 ? 4 : DKP <= 128 ? 3 : 2;
-    static constexpr int kFloats = kStages * kStage + 16 * 256 /* partial sums */ + DKP * kWalkCols /* S */ + 32 * kWalkCols /* U */;
+    static constexpr int kFloats = kStages * kStage + 8 * 64 * kWalkCols /* partial sums */ + DKP * kWalkCols /* S */ + 32 * kWalkCols /* U */;
     static constexpr int kBytes = kFloats * 4;
 };
 
 // grid (long portions, heads, ceil(dv / 8)); of each portion the blocks within the window, from the slot's state and back into it.
+// A warp owns DKP / 8 key channels: their rows of S stay with it (in registers, and for its own reading in shared memory), it adds up their part of all 64
+// rows of the first product, a lane four rows by four columns, and it makes the second product's sums for them, four channels by four
+// columns a lane with the tokens shared out over the remaining lanes.  Only the first product's sums and U pass between warps.
 template <int DKP>
 __global__ void __launch_bounds__(kBlockThreads, DKP <= 64 ? 2 : 1)
 recurrent_walk_kernel(const float* __restrict__ pack, const float* __restrict__ vpack, float* __restrict__ state, float* __restrict__ out,
                       const int* __restrict__ long_table, const int* __restrict__ segment_start, const int* __restrict__ segment_length,
                       const int* __restrict__ segment_slot, int heads, int dk, int dv, int num_slots, int* status, int window, int window_blocks) {
+    wait_for_previous_kernel();
+    allow_next_kernel();
     using Pack = BlockPack<DKP>;
     using Shared = WalkShared<DKP>;
     constexpr int kStages = Shared::kStages;
-    constexpr int kSplits = 8;             // of the key channels in the first product
-    constexpr int kPerSplit = DKP / kSplits;
-    constexpr int kTiles = DKP * 2 <= kBlockThreads ? 1 : DKP * 2 / kBlockThreads;   // of 2 x 2 elements of S a thread
+    constexpr int kChannels = DKP / 8;                  // of a warp
+    constexpr int kTokenLanes = 64 / kChannels;         // lanes that share out a block's tokens in the second product
+    constexpr int kOwn = kWalkCols * kChannels / 32;    // elements of S a lane: after the sums over the lanes of a token, 16 / kTokenLanes of a tile of 4 x 4
+    static_assert(kTokenLanes * (kChannels / 4) == 16 && kOwn * kTokenLanes == 16, "a warp's lanes are its token lanes x groups of four channels x two halves of the columns");
     extern __shared__ __align__(128) float walk_memory[];
     __shared__ uint64_t full[kStages];
-    float* part_s = walk_memory + kStages * Shared::kStage;
-    float* state_s = part_s + 16 * 256;                 // [DKP][8]
-    float* u_s = state_s + DKP * kWalkCols;             // [32][8]
+    __shared__ int failed;
+    float* part_s = walk_memory + kStages * Shared::kStage;   // [warp][64 rows][8 columns]
+    float* state_s = part_s + 8 * 64 * kWalkCols;             // [DKP][8]
+    float* u_s = state_s + DKP * kWalkCols;                   // [32][8]
     const int portion = long_table[3 * blockIdx.x], offset = blocks_before(long_table, segment_length, blockIdx.x) - window;   // of its blocks' numbers
     const int head = blockIdx.y, slice = blockIdx.z, column0 = slice * kWalkCols, slices = gridDim.z;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -460,64 +469,72 @@ recurrent_walk_kernel(const float* __restrict__ pack, const float* __restrict__ 
     };
     if (tid == 0) {
         for (int s = 0; s < kStages; ++s) barrier_init(&full[s], 1);
+        failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         for (int block = 0; block < min(kStages, blocks); ++block) load(block);
     }
-    // A thread's elements of S: rows 2 pair, 2 pair + 1, columns 2 (item & 3), + 1.
+    // The lane's elements of S: of the tile of channels channel0 .. + 3 and columns 4 column_half .. + 3 those that the sums over the token lanes leave
+    // here, kOwn neighbours in the order of (channel, column).
+    const int token_lane = lane / (32 / kTokenLanes), group = (lane >> 1) % (kChannels / 4), column_half = lane & 1;
+    const int channel0 = warp * kChannels + 4 * group;
+    const int own_row = channel0 + token_lane * kOwn / 4, own_column = 4 * column_half + token_lane * kOwn % 4;   // kOwn > 4: two whole rows
     float* slot_state = state + (static_cast<size_t>(slot) * heads + head) * dk * dv;
-    float S[kTiles][2][2];
+    float S[kOwn];
 #pragma unroll
-    for (int tile = 0; tile < kTiles; ++tile) {
-        const int item = tid + tile * kBlockThreads, row = 2 * (item >> 2), column = 2 * (item & 3);
-#pragma unroll
-        for (int r = 0; r < 2; ++r)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                S[tile][r][e] = row + r < dk && column0 + column + e < dv ? slot_state[static_cast<size_t>(row + r) * dv + column0 + column + e] : 0.0f;
-                if (row + r < DKP) state_s[(row + r) * kWalkCols + column + e] = S[tile][r][e];
-            }
+    for (int i = 0; i < kOwn; ++i) {
+        const int row = own_row + (kOwn > 4 ? i / 4 : 0), column = own_column + (kOwn > 4 ? i % 4 : i);
+        S[i] = row < dk && column0 + column < dv ? slot_state[static_cast<size_t>(row) * dv + column0 + column] : 0.0f;
+        state_s[row * kWalkCols + column] = S[i];
     }
     __syncthreads();
     for (int block = 0; block < blocks; ++block) {
         const float* stage = walk_memory + (block % kStages) * Shared::kStage;
-        const bool arrived = barrier_wait_busy(&full[block % kStages], (block / kStages) & 1);
-        if (__syncthreads_or(arrived ? 0 : 1)) {
+        if (!barrier_wait_busy(&full[block % kStages], (block / kStages) & 1)) atomicExch(&failed, 1);
+        {
+            // the warp's channels' part of [U ; O]: rows 4 (lane & 15) .. + 3 by columns 4 (lane >> 4) .. + 3
+            const float* matrix = stage + warp * kChannels * Pack::kRows + 4 * (lane & 15);
+            const float* own = state_s + warp * kChannels * kWalkCols + 4 * (lane >> 4);
+            uint64_t acc[4][2] = {};
+#pragma unroll
+            for (int c = 0; c < kChannels; ++c) {
+                const float4 m = *reinterpret_cast<const float4*>(matrix + c * Pack::kRows);
+                const ulonglong2 columns = *reinterpret_cast<const ulonglong2*>(own + c * kWalkCols);
+                const float rows[4] = {m.x, m.y, m.z, m.w};
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const uint64_t row = pack2(rows[r], rows[r]);
+                    acc[r][0] = fma2(row, columns.x, acc[r][0]);
+                    acc[r][1] = fma2(row, columns.y, acc[r][1]);
+                }
+            }
+            // pieces of 16 bytes, two a row; the eight of four rows in an order of their own, so that eight lanes meet no bank twice
+            ulonglong2* part = reinterpret_cast<ulonglong2*>(part_s) + warp * 128 + 8 * (lane & 15);
+#pragma unroll
+            for (int r = 0; r < 4; ++r) part[(2 * r + (lane >> 4)) ^ (lane & 7)] = make_ulonglong2(acc[r][0], acc[r][1]);
+        }
+        __syncthreads();
+        if (failed) {
             if (tid == 0) report_error(status, kWaitTimeout);
             for (int spin = 0; spin < 2000; ++spin) __nanosleep(1000);   // copies in flight land
             return;
         }
-        {
-            // [U ; O] - their first terms: four rows by four columns a lane, key channels shared out over the warps
-            const int rows = lane & 15, columns = lane >> 4, split = warp;
-            const float* matrix = stage + split * kPerSplit * Pack::kRows + 4 * rows;
-            const float* s_row = state_s + split * kPerSplit * kWalkCols + 4 * columns;
-            float acc[4][4] = {};
-#pragma unroll
-            for (int c = 0; c < kPerSplit; ++c) {
-                const float4 m = *reinterpret_cast<const float4*>(matrix + c * Pack::kRows), s = *reinterpret_cast<const float4*>(s_row + c * kWalkCols);
-                const float mv[4] = {m.x, m.y, m.z, m.w}, sv[4] = {s.x, s.y, s.z, s.w};
-#pragma unroll
-                for (int r = 0; r < 4; ++r)
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) acc[r][e] += mv[r] * sv[e];
-            }
-            // [split][row of the four][lane's place][column of the four]
-            float4* part = reinterpret_cast<float4*>(part_s) + split * 4 * 32 + lane;
-#pragma unroll
-            for (int r = 0; r < 4; ++r) part[r * 32] = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+        // (every warp is past the block before: its stage may be filled again)
+        if (tid == 0 && block > 0 && block - 1 + kStages < blocks) {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            load(block - 1 + kStages);
         }
-        __syncthreads();
         const float* values = stage + Pack::kFloats;
         const int t0 = kBlockTokens * (first + block), n = min(kBlockTokens, length - t0);
         {
-            // two sums a thread
-            float2 sum = *reinterpret_cast<const float2*>(part_s + 2 * tid);
+            // two sums a thread, the warps' parts in their order
+            const int row = tid >> 2, column = 2 * (tid & 3), piece = 8 * (row >> 2) + ((2 * (row & 3) + (column >> 2)) ^ ((row >> 2) & 7));
+            const float* part = part_s + 4 * piece + (column & 3);
+            float2 sum = *reinterpret_cast<const float2*>(part);
 #pragma unroll
-            for (int split = 1; split < kSplits; ++split) {
-                const float2 other = *reinterpret_cast<const float2*>(part_s + split * 512 + 2 * tid);
+            for (int w = 1; w < 8; ++w) {
+                const float2 other = *reinterpret_cast<const float2*>(part + w * 64 * kWalkCols);
                 sum.x += other.x, sum.y += other.y;
             }
-            const int r = tid >> 6, place = (tid >> 1) & 31, row = 4 * (place & 15) + r, column = 4 * (place >> 4) + 2 * (tid & 1);
             const float2 own = *reinterpret_cast<const float2*>(values + row * kWalkCols + column);
             sum.x += own.x, sum.y += own.y;
             if (row < 32) {
@@ -529,40 +546,42 @@ recurrent_walk_kernel(const float* __restrict__ pack, const float* __restrict__ 
             }
         }
         __syncthreads();
-        // S <- diag(D_end) S + K^T U
-        const float* k_hat = stage + Pack::kMatrix;
+        {
+            // S <- diag(D_end) S + K^T U: a tile of 4 x 4 over the lane's tokens, then over the token lanes
+            const float* k_hat = stage + Pack::kMatrix;
+            float tile[16] = {};
 #pragma unroll
-        for (int tile = 0; tile < kTiles; ++tile) {
-            const int item = tid + tile * kBlockThreads, row = 2 * (item >> 2), column = 2 * (item & 3);
-            if (row < DKP) {
-                const float2 d = *reinterpret_cast<const float2*>(k_hat + 32 * DKP + row);
-                S[tile][0][0] *= d.x, S[tile][0][1] *= d.x, S[tile][1][0] *= d.y, S[tile][1][1] *= d.y;
+            for (int i = 0; i < 32 / kTokenLanes; ++i) {
+                const int t = i * kTokenLanes + token_lane;
+                const float4 key = *reinterpret_cast<const float4*>(k_hat + t * DKP + channel0), u = *reinterpret_cast<const float4*>(u_s + t * kWalkCols + 4 * column_half);
+                const float keys[4] = {key.x, key.y, key.z, key.w}, us[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
-                for (int t = 0; t < 32; ++t) {
-                    const float2 key = *reinterpret_cast<const float2*>(k_hat + t * DKP + row), w = *reinterpret_cast<const float2*>(u_s + t * kWalkCols + column);
-                    S[tile][0][0] += key.x * w.x;
-                    S[tile][0][1] += key.x * w.y;
-                    S[tile][1][0] += key.y * w.x;
-                    S[tile][1][1] += key.y * w.y;
-                }
+                for (int r = 0; r < 4; ++r)
 #pragma unroll
-                for (int r = 0; r < 2; ++r) *reinterpret_cast<float2*>(state_s + (row + r) * kWalkCols + column) = make_float2(S[tile][r][0], S[tile][r][1]);
+                    for (int e = 0; e < 4; ++e) tile[4 * r + e] += keys[r] * us[e];
             }
-        }
-        __syncthreads();   // S is whole, and this stage has been read
-        if (tid == 0 && block + kStages < blocks) {
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            load(block + kStages);
+#pragma unroll
+            for (int half = 8, bit = 16; half >= kOwn; half >>= 1, bit >>= 1) {   // (the token lanes are the upper bits of the lane)
+                const bool upper = (lane & bit) != 0;
+#pragma unroll
+                for (int i = 0; i < half; ++i) {
+                    const float keep = upper ? tile[i + half] : tile[i], give = upper ? tile[i] : tile[i + half];
+                    tile[i] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
+                }
+            }
+            const float* decays = k_hat + 32 * DKP + own_row;
+#pragma unroll
+            for (int i = 0; i < kOwn; ++i) {
+                S[i] = fmaf(decays[kOwn > 4 ? i / 4 : 0], S[i], tile[i]);
+                state_s[(own_row + (kOwn > 4 ? i / 4 : 0)) * kWalkCols + own_column + (kOwn > 4 ? i % 4 : i)] = S[i];
+            }
+            __syncwarp();   // S is this warp's alone
         }
     }
 #pragma unroll
-    for (int tile = 0; tile < kTiles; ++tile) {
-        const int item = tid + tile * kBlockThreads, row = 2 * (item >> 2), column = 2 * (item & 3);
-#pragma unroll
-        for (int r = 0; r < 2; ++r)
-#pragma unroll
-            for (int e = 0; e < 2; ++e)
-                if (row + r < dk && column0 + column + e < dv) slot_state[static_cast<size_t>(row + r) * dv + column0 + column + e] = S[tile][r][e];
+    for (int i = 0; i < kOwn; ++i) {
+        const int row = own_row + (kOwn > 4 ? i / 4 : 0), column = own_column + (kOwn > 4 ? i % 4 : i);
+        if (row < dk && column0 + column < dv) slot_state[static_cast<size_t>(row) * dv + column0 + column] = S[i];
     }
 }
 
@@ -578,6 +597,8 @@ linear_prepare_kernel(const float* __restrict__ q, const float* __restrict__ k, 
                       float* __restrict__ decays, float* __restrict__ out, const int* __restrict__ long_table, int long_portions, const int* __restrict__ segment_start,
                 const int* __restrict__ segment_length, int heads,
                       int groups, int dk, int dv, int window) {
+    wait_for_previous_kernel();
+    allow_next_kernel();
     constexpr int P = DKP + 4, VP = 132;
     extern __shared__ __align__(16) float prepare_memory[];
     float* k_s = prepare_memory;   // keys; then as between_halves wants them
@@ -679,6 +700,8 @@ __global__ void __launch_bounds__(kBlockThreads)
 linear_states_kernel(float* __restrict__ sums, const float* __restrict__ decays, float* __restrict__ state, const int* __restrict__ long_table,
                      const int* __restrict__ segment_length, const int* __restrict__ segment_slot, int heads, int dk, int dv, int num_slots, int* status,
                      int window, int window_blocks) {
+    wait_for_previous_kernel();
+    allow_next_kernel();
     const int portion = long_table[3 * blockIdx.x], offset = blocks_before(long_table, segment_length, blockIdx.x) - window;   // of its blocks' numbers
     const int first = max(0, -offset), blocks = min((segment_length[portion] + kBlockTokens - 1) / kBlockTokens, window_blocks - offset) - first;
     const int head = blockIdx.y, element = blockIdx.z * kBlockThreads + threadIdx.x, elements = dk * dv, slot = segment_slot[portion];
@@ -722,6 +745,8 @@ template <int DKP, bool VECTOR>
 __global__ void __launch_bounds__(kBlockThreads)
 linear_read_kernel(const float* __restrict__ q, const float* __restrict__ g, const float* __restrict__ states, float* __restrict__ out, const int* __restrict__ long_table, int long_portions, const int* __restrict__ segment_start,
                 const int* __restrict__ segment_length, int heads, int groups, int dk, int dv, int window) {
+    wait_for_previous_kernel();
+    allow_next_kernel();
     constexpr int P = DKP + 4;
     extern __shared__ __align__(16) float prepare_memory[];
     float* q_s = prepare_memory;
@@ -816,20 +841,23 @@ template <int DKP>
 int launch_recurrent_blocks(const float* q, const float* k, const float* g, const float* v, const float* beta, float* pack, float* vpack, float* state, float* out,
                             int most_blocks, int window_blocks, const int* long_table, int long_portions, const int* segment_start,
                             const int* segment_length, const int* segment_slot, int heads, int groups, int dk, int dv, int num_slots, int* status, cudaStream_t stream) {
-    const dim3 blocks(window_blocks, heads);
+    const dim3 blocks(window_blocks, heads), threads(kBlockThreads);
+    // Launched so that each may start while the one before still runs (it waits for it first): 1 to 2 us a launch.
+    cudaError_t error = cudaSuccess;
     if (beta != nullptr) {
         static OncePerDevice prepared, walked;
         auto prepare = recurrent_prepare_kernel<DKP>;
         auto walk = recurrent_walk_kernel<DKP>;
         if (allow_shared_memory(prepared, prepare, PrepareShared<DKP>::kBytes) != cudaSuccess) return static_cast<int>(cudaGetLastError());
         if (allow_shared_memory(walked, walk, WalkShared<DKP>::kBytes) != cudaSuccess) return static_cast<int>(cudaGetLastError());
-        for (int window = 0; window < most_blocks; window += window_blocks) {
-            prepare<<<blocks, kBlockThreads, PrepareShared<DKP>::kBytes, stream>>>(q, k, g, v, beta, pack, vpack, long_table, long_portions, segment_start, segment_length, heads,
-                                                                                   groups, dk, dv, window);
-            walk<<<dim3(long_portions, heads, (dv + kWalkCols - 1) / kWalkCols), kBlockThreads, WalkShared<DKP>::kBytes, stream>>>(
-                pack, vpack, state, out, long_table, segment_start, segment_length, segment_slot, heads, dk, dv, num_slots, status, window, window_blocks);
+        for (int window = 0; window < most_blocks && error == cudaSuccess; window += window_blocks) {
+            error = launch_overlapped(prepare, blocks, threads, PrepareShared<DKP>::kBytes, stream, q, k, g, v, beta, pack, vpack, long_table, long_portions, segment_start,
+                                      segment_length, heads, groups, dk, dv, window);
+            if (error == cudaSuccess)
+                error = launch_overlapped(walk, dim3(long_portions, heads, (dv + kWalkCols - 1) / kWalkCols), threads, WalkShared<DKP>::kBytes, stream, pack, vpack, state, out,
+                                          long_table, segment_start, segment_length, segment_slot, heads, dk, dv, num_slots, status, window, window_blocks);
         }
-        return static_cast<int>(cudaGetLastError());
+        return static_cast<int>(error != cudaSuccess ? error : cudaGetLastError());
     }
     static OncePerDevice prepared, read, read_any;
     auto prepare = linear_prepare_kernel<DKP>;
@@ -838,13 +866,17 @@ int launch_recurrent_blocks(const float* q, const float* k, const float* g, cons
     if (allow_shared_memory(prepared, prepare, prepare_bytes) != cudaSuccess) return static_cast<int>(cudaGetLastError());
     if (allow_shared_memory(dv % 4 == 0 ? read : read_any, read_out, read_bytes) != cudaSuccess) return static_cast<int>(cudaGetLastError());
     float* decays = pack + static_cast<size_t>(window_blocks) * heads * dk * dv;
-    for (int window = 0; window < most_blocks; window += window_blocks) {
-        prepare<<<blocks, kBlockThreads, prepare_bytes, stream>>>(q, k, g, v, pack, decays, out, long_table, long_portions, segment_start, segment_length, heads, groups, dk, dv, window);
-        linear_states_kernel<<<dim3(long_portions, heads, (dk * dv + kBlockThreads - 1) / kBlockThreads), kBlockThreads, 0, stream>>>(
-            pack, decays, state, long_table, segment_length, segment_slot, heads, dk, dv, num_slots, status, window, window_blocks);
-        read_out<<<blocks, kBlockThreads, read_bytes, stream>>>(q, g, pack, out, long_table, long_portions, segment_start, segment_length, heads, groups, dk, dv, window);
+    for (int window = 0; window < most_blocks && error == cudaSuccess; window += window_blocks) {
+        error = launch_overlapped(prepare, blocks, threads, prepare_bytes, stream, q, k, g, v, pack, decays, out, long_table, long_portions, segment_start, segment_length, heads,
+                                  groups, dk, dv, window);
+        if (error == cudaSuccess)
+            error = launch_overlapped(linear_states_kernel, dim3(long_portions, heads, (dk * dv + kBlockThreads - 1) / kBlockThreads), threads, 0, stream, pack, decays, state,
+                                      long_table, segment_length, segment_slot, heads, dk, dv, num_slots, status, window, window_blocks);
+        if (error == cudaSuccess)
+            error = launch_overlapped(read_out, blocks, threads, read_bytes, stream, q, g, pack, out, long_table, long_portions, segment_start, segment_length, heads, groups, dk, dv,
+                                      window);
     }
-    return static_cast<int>(cudaGetLastError());
+    return static_cast<int>(error != cudaSuccess ? error : cudaGetLastError());
 }
 
 }  // namespace lb
