@@ -2,7 +2,7 @@
 
 Every function checks what the kernel cannot check for itself (device, dtype, contiguity,
 size limits) and raises :class:`KernelError` with a clear message instead of launching with
-arguments the kernel does not support.  Matrix products of the 32-bit path go to the library
+arguments the kernel does not support.  Large matrix products of the 32-bit path go to the library
 (cuBLAS through ``torch.matmul``, with TF32 and reduced-precision reductions switched off), as
 the reference's go to XLA (``lalamo/weight_matrix.py:418-432``).
 """
@@ -2332,6 +2332,28 @@ def tcgen05_wait_probe(status: torch.Tensor, nanoseconds: int = 1_000_000) -> No
     _done(_lib().lb_tcgen05_wait_probe(status, nanoseconds, _stream()), "tcgen05_wait_probe")
 
 
+def float32_product_supported(tokens: int, rows: int, width: int) -> bool:
+    """Whether a product of the 32-bit path runs on the framework's own kernel: where the library's large tiles would leave most multiprocessors idle.  Measured, ours and the
+    library's: 5 and 12 tokens x 2048 x 1024 8 and 19 us, 32 x 9216 x 1024 24 and 25, 96 x 2048 x 2048 34 and 42, 64 x 4096 x 1024 19 and 24, 300 x 1024 x 1024 25 and 31, 400 x
+    1024 x 2048 55 and 57; beyond, 192 x 2048 x 1024 33 and 31, 96 x 3072 x 2048 61 and 43, 500 x 1024 x 2048 64 and 60.  (Of up to four tokens the library
+    adds up in another way, a tenth closer to 64 bits.)"""
+    if width % 4 or tokens < 5:
+        return False
+    tiles = -(-tokens // 64) * -(-rows // 64)
+    return (tokens <= 32 and rows <= 16384) or tiles <= 64 or (rows <= 1024 and tiles <= 112)
+
+
+def _product(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
+    """``x @ weight.T`` where none of the bfloat16 kernels takes it: on the kernel of the 32-bit path, else by the library."""
+    if (x.dtype == torch.float32 and x.dim() == 2 and float32_product_supported(x.shape[0], weight.shape[0], x.shape[1]) and x.stride(1) == 1 and x.stride(0) % 4 == 0
+            and x.stride(0) >= x.shape[1] and (x.data_ptr() | weight.data_ptr()) % 16 == 0
+            and not (torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad))):
+        out = torch.empty(x.shape[0], weight.shape[0], dtype=torch.float32, device=x.device)
+        _done(_lib().lb_gemm_float32(x, weight, out, x.shape[0], weight.shape[0], x.shape[1], x.stride(0), 0, _stream()), "gemm_float32")
+        return out
+    return torch.mm(x, weight.t())
+
+
 def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype | None = None, status: torch.Tensor | None = None) -> torch.Tensor:
     """``x @ weight.T`` with 32-bit accumulation; ``out_dtype`` float32 gives 32-bit results from
     bfloat16 operands (the LM head's logits).  Steps of up to 16 tokens go to the weight-streaming
@@ -2352,7 +2374,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype | None 
         return linear_tcgen05(x, weight, "store_float" if wants_float else "store", status=status)
     if wants_float:
         return torch.mm(x, weight.t(), out_dtype=out_dtype)
-    return torch.mm(x, weight.t())
+    return _product(x, weight)
 
 
 def linear_of_columns(x: torch.Tensor, first: int, weight: torch.Tensor, status: torch.Tensor | None = None) -> torch.Tensor:
@@ -2366,7 +2388,7 @@ def linear_of_columns(x: torch.Tensor, first: int, weight: torch.Tensor, status:
     columns = x[:, first : first + width]
     if columns.data_ptr() % 16 or x.shape[1] % 8 or x.dtype != torch.bfloat16 or not x.shape[0]:   # rows that do not start on 16 bytes, and the 32-bit path
         # (a copy also of a single row, whose columns count as contiguous where they lie)
-        return linear(columns.clone(memory_format=torch.contiguous_format), weight, status=status) if x.dtype == torch.bfloat16 else torch.mm(columns, weight.t())
+        return linear(columns.clone(memory_format=torch.contiguous_format), weight, status=status) if x.dtype == torch.bfloat16 else _product(columns, weight)
     if skinny_supported(columns, rows) and not (USE_TCGEN05 and rows >= TCGEN05_MIN_ROWS_FEW_TOKENS):
         out = torch.empty(x.shape[0], rows, dtype=x.dtype, device=x.device)
         _skinny(columns, weight, out, rows, "store", x_stride=x.shape[1])
@@ -2462,7 +2484,7 @@ def linear_accumulate(x: torch.Tensor, weight: torch.Tensor, residual: torch.Ten
     if USE_TCGEN05 and tcgen05_supported(x, weight.shape[0]):
         result = linear_tcgen05(x, weight, "residual_add", residual, status=status, defer_sum=DEFER_SLICE_SUMS)
         return result if isinstance(result, SlicedSum) else None
-    return torch.mm(x, weight.t())
+    return _product(x, weight)
 
 
 def gated_linear(x: torch.Tensor, up_gate: torch.Tensor, activation: str, status: torch.Tensor | None = None, limit: float = 0.0) -> torch.Tensor:
