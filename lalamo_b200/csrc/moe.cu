@@ -296,6 +296,8 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 moe_combine_wide_kernel(const float* __restrict__ expert_out, const float* __restrict__ weights, const int* __restrict__ chosen, int experts, T* __restrict__ out, int top,
                         int width) {
+    wait_for_previous_kernel();
+    allow_next_kernel();
     const int token = blockIdx.x;
     const size_t pair0 = static_cast<size_t>(token) * top;
     float weight[kCombineTop];
@@ -513,9 +515,9 @@ int lb_moe_combine(const float* expert_out, const float* weights, const int* cho
     if (tokens == 0) return 0;
     if (width % 4 == 0 && top <= lb::kCombineTop && reinterpret_cast<uintptr_t>(expert_out) % 16 == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0) {
         LB_DISPATCH_DTYPE(dtype, {
-            lb::moe_combine_wide_kernel<T><<<tokens, 256, 0, stream>>>(expert_out, weights, chosen, experts, static_cast<T*>(out), top, width);
+            return static_cast<int>(lb::launch_overlapped(lb::moe_combine_wide_kernel<T>, dim3(tokens), dim3(256), 0, stream, expert_out, weights, chosen, experts, static_cast<T*>(out), top,
+                                                          width));
         })
-        return LB_LAUNCH_RESULT();
     }
     LB_DISPATCH_DTYPE(dtype, {
         lb::moe_combine_kernel<T><<<tokens, 256, 0, stream>>>(expert_out, weights, chosen, experts, static_cast<T*>(out), top, width);

@@ -323,6 +323,51 @@ moe_gather_kernel(const uint4* __restrict__ x, const int* __restrict__ offsets, 
     for (int i = threadIdx.x; i < pieces; i += blockDim.x) destination[i] = source[i];
 }
 
+// Both at once for up to kMoeArrangePairs pairs: a block a pair, which counts the pairs before its own in the order of the experts (and, of one expert, of the
+// pairs), leaves its place and copies its row; one more block makes the offsets.  8 tokens of 4 experts: one launch of 4 us for two of 3 and 4.
+constexpr int kMoeArrangePairs = 1024;
+__global__ void __launch_bounds__(128)
+moe_arrange_kernel(const uint4* __restrict__ x, const int* __restrict__ chosen, int pairs, int experts, int top, int pieces, int* __restrict__ offsets, int* __restrict__ sorted,
+                   uint4* __restrict__ gathered) {
+    extern __shared__ int counters[];   // experts (the last block's), or four warps' counts
+    wait_for_previous_kernel();
+    allow_next_kernel();
+    const int pair = blockIdx.x, tid = threadIdx.x;
+    if (pair == pairs) {
+        for (int e = tid; e < experts; e += blockDim.x) counters[e] = 0;
+        __syncthreads();
+        for (int p = tid; p < pairs; p += blockDim.x) {
+            const int e = chosen[p];
+            if (e >= 0 && e < experts) atomicAdd(&counters[e], 1);
+        }
+        __syncthreads();
+        if (tid == 0) {
+            int total = 0;
+            for (int e = 0; e < experts; ++e) {
+                offsets[e] = total;
+                total += counters[e];
+            }
+            offsets[experts] = total;
+        }
+        return;
+    }
+    const int own = chosen[pair];
+    if (own < 0 || own >= experts) return;   // no expert: left out
+    int before = 0;
+    for (int p = tid; p < pairs; p += blockDim.x) {
+        const int e = chosen[p];
+        if (e >= 0 && (e < own || (e == own && p < pair))) ++before;
+    }
+    before = __reduce_add_sync(0xffffffffu, before);
+    if ((tid & 31) == 0) counters[tid >> 5] = before;
+    __syncthreads();
+    const int place = counters[0] + counters[1] + counters[2] + counters[3];
+    if (tid == 0) sorted[place] = pair;
+    const uint4* source = x + static_cast<size_t>(pair / top) * pieces;
+    uint4* destination = gathered + static_cast<size_t>(place) * pieces;
+    for (int i = tid; i < pieces; i += blockDim.x) destination[i] = source[i];
+}
+
 // A [rows, k] bfloat16 matrix seen through boxes of [box_rows, 64] with 128-byte swizzle; what lies outside reads as zero.
 static bool moe_map(CUtensorMap* map, const void* base, long long rows, int k, int box_rows) {
     EncodeTiled encode = encode_tiled();
@@ -375,11 +420,17 @@ int lb_moe_experts_grouped(const void* x, const void* gate, const void* up, cons
                            int* status) {
     if (pairs == 0) return 0;
     if (width % 8 != 0 || ff % 8 != 0 || experts < 1 || experts > lb::kMoeMaxExperts) return -2;
-    lb::moe_sort_kernel<<<1, 1024, 2 * experts * sizeof(int), stream>>>(chosen, pairs, experts, offsets, sorted);
-    cudaError_t error = cudaGetLastError();
-    if (error == cudaSuccess)
-        error = lb::launch_overlapped(lb::moe_gather_kernel, dim3(pairs), dim3(128), 0, stream, static_cast<const uint4*>(x), offsets, sorted, static_cast<uint4*>(gathered), experts,
-                                      top, width / 8);
+    cudaError_t error;
+    if (pairs <= lb::kMoeArrangePairs) {
+        error = lb::launch_overlapped(lb::moe_arrange_kernel, dim3(pairs + 1), dim3(128), (experts > 4 ? experts : 4) * sizeof(int), stream, static_cast<const uint4*>(x), chosen, pairs,
+                                      experts, top, width / 8, offsets, sorted, static_cast<uint4*>(gathered));
+    } else {
+        lb::moe_sort_kernel<<<1, 1024, 2 * experts * sizeof(int), stream>>>(chosen, pairs, experts, offsets, sorted);
+        error = cudaGetLastError();
+        if (error == cudaSuccess)
+            error = lb::launch_overlapped(lb::moe_gather_kernel, dim3(pairs), dim3(128), 0, stream, static_cast<const uint4*>(x), offsets, sorted, static_cast<uint4*>(gathered), experts,
+                                          top, width / 8);
+    }
     if (error != cudaSuccess) return static_cast<int>(error);
     lb::MoeTcParams p = {};
     p.offsets = offsets, p.sorted = sorted, p.experts = experts, p.activation = activation, p.limit = limit, p.status = status;

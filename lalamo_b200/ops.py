@@ -1695,6 +1695,7 @@ def moe_route(x: torch.Tensor, router: torch.Tensor, *, top: int, group_count: i
 # over both products, cold caches: of 2048 x 2048 experts 16 pairs 88 us streamed and 89 grouped, 24 pairs 130 and 94, 32 pairs 130 and 96; of 1024 x 1152 experts a layer of 20 pairs 66.5 and
 # 72.7, of 32 pairs 72.7 and 74.8, 48 pairs' products 75 and 52.
 MOE_STREAM_MAX_PAIRS = 32
+MOE_ARRANGE_PAIRS = 1024  # up to which the grouped kernels' pairs are sorted and gathered in one launch
 MOE_STREAM_MAX_ELEMENTS = 16 * 2048 * 2048
 
 
@@ -1747,7 +1748,7 @@ def moe_experts(x: torch.Tensor, gate: "torch.Tensor | None", up: torch.Tensor, 
                                           status)
         if code == -5:
             raise KernelError("moe_experts: the driver gave no tensor map (cuTensorMapEncodeTiled)")
-        _done(code, "moe_experts_grouped", 4)
+        _done(code, "moe_experts_grouped", 3 if pairs <= MOE_ARRANGE_PAIRS else 4)
     elif path == "stream":
         # few pairs: each streams its expert's rows, 16 bytes a lane, the rows shared out over many blocks
         if not wide_rows:
