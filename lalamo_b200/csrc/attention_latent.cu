@@ -113,6 +113,8 @@ __global__ void latent_prepare_kernel(const T* __restrict__ q, int q_stride, con
                                       const float* __restrict__ inv_freq, const int* __restrict__ positions, const int* __restrict__ token_segment,
                                       const int* __restrict__ block_table, LatentLayout layout, int tokens, int num_heads, int head_dim, int write_kv,
                                       int* status, float factor) {
+    wait_for_previous_kernel();
+    allow_next_kernel();
     extern __shared__ float shared[];
     const int half = layout.rope / 2, latent = layout.latent, rope = layout.rope;
     float* cosines = shared;            // half
@@ -568,6 +570,8 @@ latent_attention_mma_kernel(LatentMmaParams p) {
 // shared memory: a float per split.
 __global__ void latent_merge_kernel(const float* __restrict__ partial, __nv_bfloat16* __restrict__ out, int splits, int latent,
                                     const float* __restrict__ sink, int num_heads) {
+    wait_for_previous_kernel();
+    allow_next_kernel();
     extern __shared__ float split_weight[];
     const size_t row = blockIdx.x;
     const float* mine = partial + row * splits * (latent + 2);
@@ -601,7 +605,7 @@ __global__ void latent_merge_kernel(const float* __restrict__ partial, __nv_bflo
 
 
 void launch_latent_merge(const float* partial, __nv_bfloat16* out, int rows, int splits, int latent, const float* sink, int num_heads, cudaStream_t stream) {
-    latent_merge_kernel<<<rows, 128, splits * sizeof(float), stream>>>(partial, out, splits, latent, sink, num_heads);
+    launch_overlapped(latent_merge_kernel, dim3(rows), dim3(128), splits * sizeof(float), stream, partial, out, splits, latent, sink, num_heads);
 }
 
 // ------------------------------------------------------------------ one small product per head
@@ -629,6 +633,8 @@ struct HeadsProductParams {
 template <bool B_KN>
 __global__ void __launch_bounds__(128)
 heads_product_kernel(HeadsProductParams p) {
+    wait_for_previous_kernel();
+    allow_next_kernel();
     extern __shared__ __align__(16) unsigned char product_shared[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, head = blockIdx.y, token0 = blockIdx.x * 64;
     // grid.z shares out the blocks of 64 columns; a CTA takes blocks_per_cta neighbouring blocks, whose part of the head's matrix it loads at once
@@ -715,12 +721,12 @@ int lb_latent_prepare(const void* q, int q_stride, const void* q_latent, const v
     const size_t shared = (static_cast<size_t>(rope) + 33) * sizeof(float);
     if (shared > 48 * 1024) return -2;
     LB_DISPATCH_DTYPE(dtype, {
-        lb::latent_prepare_kernel<T><<<dim3(tokens, (q_latent != nullptr ? num_heads : 1) + (write_kv ? 1 : 0)), q_latent != nullptr ? 64 : 128, shared, stream>>>(
+        return static_cast<int>(lb::launch_overlapped(
+            lb::latent_prepare_kernel<T>, dim3(tokens, (q_latent != nullptr ? num_heads : 1) + (write_kv ? 1 : 0)), dim3(q_latent != nullptr ? 64 : 128), shared, stream,
             static_cast<const T*>(q), q_stride, static_cast<const T*>(q_latent), static_cast<const T*>(down), down_stride, static_cast<T*>(q_out),
             static_cast<T*>(pages), norm_weight, eps, scale_offset, inv_freq, positions, token_segment, block_table, layout, tokens, num_heads, head_dim,
-            write_kv, status, factor);
+            write_kv, status, factor));
     })
-    return LB_LAUNCH_RESULT();
 }
 
 // q_down and down: column slices of one product, `row_stride` elements a token; down null: no row is written.
@@ -846,9 +852,7 @@ int lb_heads_product(const void* a, long long a_token_stride, int a_head_stride,
     p.n = n;
     p.blocks_per_cta = blocks_per_cta;
     const dim3 grid(token_blocks, heads, (column_blocks + blocks_per_cta - 1) / blocks_per_cta);
-    if (b_is_kn) lb::heads_product_kernel<true><<<grid, 128, shared, stream>>>(p);
-    else lb::heads_product_kernel<false><<<grid, 128, shared, stream>>>(p);
-    return LB_LAUNCH_RESULT();
+    return static_cast<int>(lb::launch_overlapped(b_is_kn ? lb::heads_product_kernel<true> : lb::heads_product_kernel<false>, grid, dim3(128), shared, stream, p));
 }
 
 int lb_gate_heads(const void* values, const void* gate, int gate_stride, void* out, int tokens, int num_heads, int value_dim, int dtype,

@@ -115,6 +115,8 @@ latent_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    wait_for_previous_kernel();   // launched to start early: the queries and the newest rows are there from here on
+    allow_next_kernel();
     const uint32_t tmem_output = *tmem_slot, tmem_scores = tmem_output + 256;   // scores: two tiles of 128 columns
 
     if (warp == 9) {
@@ -445,7 +447,9 @@ int lb_latent_attention_tcgen05(const void* q, const void* pages, void* out, flo
     p.splits = splits;
     p.window = window;
     p.scale_log2 = scale * 1.4426950408889634f;
-    lb::latent_attention_tcgen05_kernel<<<dim3(num_items, splits), lb::kLtThreads, shared, stream>>>(map_q, map_q_rope, map_16_rows, map_16_rope, map_32_rows, map_32_rope, p);
+    const cudaError_t launched = lb::launch_overlapped(lb::latent_attention_tcgen05_kernel, dim3(num_items, splits), dim3(lb::kLtThreads), shared, stream, map_q, map_q_rope, map_16_rows,
+                                                       map_16_rope, map_32_rows, map_32_rope, p);
+    if (launched != cudaSuccess) return static_cast<int>(launched);
     if (splits > 1) lb::launch_latent_merge(partial, p.out, tokens * num_heads, splits, latent, sink, num_heads, stream);
     return LB_LAUNCH_RESULT();
 }

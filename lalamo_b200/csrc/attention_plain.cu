@@ -177,6 +177,8 @@ __global__ void qk_norm_rope_write_token_kernel(const T* __restrict__ qkv, T* __
                                                 const int* __restrict__ positions, const int* __restrict__ token_segment,
                                                 const int* __restrict__ block_table, PagedLayout layout, int num_heads,
                                                 int write_kv, const float* __restrict__ bias, int* status, RewriteExtras extra) {
+    wait_for_previous_kernel();
+    allow_next_kernel();
     extern __shared__ float rotation[];   // cos[half], sin[half]
     const int token = blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
@@ -274,6 +276,8 @@ __global__ void qk_norm_rope_write_vector_kernel(const __nv_bfloat16* __restrict
                                                  const int* __restrict__ positions, const int* __restrict__ token_segment,
                                                  const int* __restrict__ block_table, PagedLayout layout, int num_heads, int write_kv,
                                                  const float* __restrict__ bias, int* status, RewriteExtras extra) {
+    wait_for_previous_kernel();
+    allow_next_kernel();
     using T = __nv_bfloat16;
     extern __shared__ float rotation[];   // cos[half], sin[half]
     const int token = blockIdx.x;
@@ -382,6 +386,8 @@ __global__ void qk_norm_rope_write_run_kernel(const __nv_bfloat16* __restrict__ 
                                               const int* __restrict__ positions, const int* __restrict__ token_segment,
                                               const int* __restrict__ block_table, PagedLayout layout, int num_heads, int write_kv,
                                               int tokens, const float* __restrict__ bias, int* status, RewriteExtras extra) {
+    wait_for_previous_kernel();
+    allow_next_kernel();
     static_assert(RUN == 4 || RUN == 8, "a channel's rows leave as one 8- or 16-byte store");
     using T = __nv_bfloat16;
     extern __shared__ float rotation[];   // per token of the run: cos[half], sin[half]
@@ -536,6 +542,8 @@ __global__ void rewrite_pieces_kernel(const __nv_bfloat16* __restrict__ qkv, __n
                                       __nv_bfloat16* __restrict__ v_pages, const float* __restrict__ inv_freq, int rotary_dim, const int* __restrict__ positions,
                                       const int* __restrict__ token_segment, const int* __restrict__ block_table, PagedLayout layout, int num_heads, int write_kv,
                                       int tokens, int* status, RewriteExtras extra) {
+    wait_for_previous_kernel();
+    allow_next_kernel();
     using T = __nv_bfloat16;
     extern __shared__ float rotation[];   // per token of the run: cos[half], sin[half]
     const int first = blockIdx.x * RUN;
@@ -1047,14 +1055,12 @@ int lb_qk_norm_rope_write(const void* qkv, void* q_out, void* k_pages, void* v_p
         const size_t shared = static_cast<size_t>(rotary_dim > 0 ? rotary_dim : 2) * sizeof(float);
         if (tokens >= lb::kRunKernelMinTokens) {
             constexpr int kRun = 4;
-            lb::qk_norm_rope_write_run_kernel<kRun><<<(tokens + kRun - 1) / kRun, vector_threads, kRun * shared, stream>>>(
-                static_cast<const __nv_bfloat16*>(qkv), static_cast<__nv_bfloat16*>(q_out), static_cast<__nv_bfloat16*>(k_pages),
+            lb::launch_overlapped(lb::qk_norm_rope_write_run_kernel<kRun>, dim3((tokens + kRun - 1) / kRun), dim3(vector_threads), kRun * shared, stream, static_cast<const __nv_bfloat16*>(qkv), static_cast<__nv_bfloat16*>(q_out), static_cast<__nv_bfloat16*>(k_pages),
                 static_cast<__nv_bfloat16*>(v_pages), q_weight, k_weight, eps, scale_offset, inv_freq, rotary_dim, positions, token_segment, block_table,
                 layout, num_heads, write_kv, tokens, bias, status, extra);
             return LB_LAUNCH_RESULT();
         }
-        lb::qk_norm_rope_write_vector_kernel<<<tokens, vector_threads, shared, stream>>>(
-            static_cast<const __nv_bfloat16*>(qkv), static_cast<__nv_bfloat16*>(q_out), static_cast<__nv_bfloat16*>(k_pages),
+        lb::launch_overlapped(lb::qk_norm_rope_write_vector_kernel, dim3(tokens), dim3(vector_threads), shared, stream, static_cast<const __nv_bfloat16*>(qkv), static_cast<__nv_bfloat16*>(q_out), static_cast<__nv_bfloat16*>(k_pages),
             static_cast<__nv_bfloat16*>(v_pages), q_weight, k_weight, eps, scale_offset, inv_freq, rotary_dim, positions, token_segment, block_table,
             layout, num_heads, write_kv, bias, status, extra);
         return LB_LAUNCH_RESULT();
@@ -1066,12 +1072,10 @@ int lb_qk_norm_rope_write(const void* qkv, void* q_out, void* k_pages, void* v_p
         const int threads = pieces >= 256 ? 256 : (pieces + 31) / 32 * 32;
         const size_t shared = static_cast<size_t>(rotary_dim > 0 ? rotary_dim : 2) * sizeof(float);
         if (tokens >= lb::kRunKernelMinTokens)
-            lb::rewrite_pieces_kernel<4><<<(tokens + 3) / 4, threads, 4 * shared, stream>>>(
-                static_cast<const __nv_bfloat16*>(qkv), static_cast<__nv_bfloat16*>(q_out), static_cast<__nv_bfloat16*>(k_pages), static_cast<__nv_bfloat16*>(v_pages),
+            lb::launch_overlapped(lb::rewrite_pieces_kernel<4>, dim3((tokens + 3) / 4), dim3(threads), 4 * shared, stream, static_cast<const __nv_bfloat16*>(qkv), static_cast<__nv_bfloat16*>(q_out), static_cast<__nv_bfloat16*>(k_pages), static_cast<__nv_bfloat16*>(v_pages),
                 inv_freq, rotary_dim, positions, token_segment, block_table, layout, num_heads, write_kv, tokens, status, extra);
         else
-            lb::rewrite_pieces_kernel<1><<<tokens, threads, shared, stream>>>(
-                static_cast<const __nv_bfloat16*>(qkv), static_cast<__nv_bfloat16*>(q_out), static_cast<__nv_bfloat16*>(k_pages), static_cast<__nv_bfloat16*>(v_pages),
+            lb::launch_overlapped(lb::rewrite_pieces_kernel<1>, dim3(tokens), dim3(threads), shared, stream, static_cast<const __nv_bfloat16*>(qkv), static_cast<__nv_bfloat16*>(q_out), static_cast<__nv_bfloat16*>(k_pages), static_cast<__nv_bfloat16*>(v_pages),
                 inv_freq, rotary_dim, positions, token_segment, block_table, layout, num_heads, write_kv, tokens, status, extra);
         return LB_LAUNCH_RESULT();
     }
@@ -1079,8 +1083,7 @@ int lb_qk_norm_rope_write(const void* qkv, void* q_out, void* k_pages, void* v_p
         // Many tokens: one block per token, the rotation computed once for all of its heads.
         const size_t shared = static_cast<size_t>(rotary_dim > 0 ? rotary_dim : 2) * sizeof(float);
         LB_DISPATCH_DTYPE(dtype, {
-            lb::qk_norm_rope_write_token_kernel<T><<<dim3(tokens, (num_heads + num_groups + lb::kTokenKernelUnits - 1) / lb::kTokenKernelUnits), 128, shared, stream>>>(
-                static_cast<const T*>(qkv), static_cast<T*>(q_out), static_cast<T*>(k_pages), static_cast<T*>(v_pages), q_weight,
+            lb::launch_overlapped(lb::qk_norm_rope_write_token_kernel<T>, dim3(dim3(tokens, (num_heads + num_groups + lb::kTokenKernelUnits - 1) / lb::kTokenKernelUnits)), dim3(128), shared, stream, static_cast<const T*>(qkv), static_cast<T*>(q_out), static_cast<T*>(k_pages), static_cast<T*>(v_pages), q_weight,
                 k_weight, eps, scale_offset, inv_freq, rotary_dim, positions, token_segment, block_table, layout, num_heads,
                 write_kv, bias, status, extra);
         })

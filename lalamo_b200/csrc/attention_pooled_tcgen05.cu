@@ -189,6 +189,8 @@ pooled_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    wait_for_previous_kernel();   // launched to start early: the queries, the newest rows and blocks are there from here on
+    allow_next_kernel();
     const uint32_t tmem_output = *tmem_slot, tmem_scores = tmem_output + 64;   // two tiles of 64 columns
 
     if (warp == 9) {
@@ -544,7 +546,8 @@ int lb_pooled_attention_tcgen05(const void* q, const void* pages, const void* po
     const cudaError_t allowed = lb::allow_shared_memory(once, lb::pooled_attention_tcgen05_kernel, 120 * 1024);
     if (allowed != cudaSuccess) return static_cast<int>(allowed);
     const dim3 grid(static_cast<unsigned>(num_tiles) * groups * ((per_group + head_block - 1) / head_block), shares);
-    lb::pooled_attention_tcgen05_kernel<<<grid, lb::kPtThreads, shared, stream>>>(map_q, map_16, map_32, p);
+    const cudaError_t launched = lb::launch_overlapped(lb::pooled_attention_tcgen05_kernel, grid, dim3(lb::kPtThreads), shared, stream, map_q, map_16, map_32, p);
+    if (launched != cudaSuccess) return static_cast<int>(launched);
     if (shares > 1) lb::launch_pooled_finish(partial, shares, p.out, positions, total_rows, heads, 64, v_freq, v_interleaved, tiles, num_tiles, tile_tokens, stream);
     return LB_LAUNCH_RESULT();
 }

@@ -169,7 +169,8 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     // The out-projection that follows may ask for its weights meanwhile: it takes tensor memory of its own, so only now that this
-    // CTA has its share.
+    // CTA has its share (and launched early itself, it reads what the kernel before writes from here on).
+    wait_for_previous_kernel();
     allow_next_kernel();
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t tmem_scores = tmem_base, tmem_output = tmem_base + kTaKeys;
@@ -578,7 +579,8 @@ attention_tcgen05_halves_kernel(const __grid_constant__ CUtensorMap map_q, const
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     // The out-projection that follows may ask for its weights meanwhile: it takes tensor memory of its own, so only now that this
-    // CTA has its share.
+    // CTA has its share (and launched early itself, it reads what the kernel before writes from here on).
+    wait_for_previous_kernel();
     allow_next_kernel();
     const uint32_t tmem_output = *tmem_slot, tmem_scores = tmem_output + 128;   // two halves of 64 columns, two tiles of 64 columns
 
@@ -935,29 +937,31 @@ int lb_attention_prefill_tcgen05(const void* q, const void* k_pages, const void*
     if (value_dim == 128) {
         static lb::OncePerDevice configured;
         if (lb::allow_shared_memory(configured, lb::attention_tcgen05_kernel<128>, lb::TaShared<128>::kBytes) != cudaSuccess) return static_cast<int>(cudaGetLastError());
-        lb::attention_tcgen05_kernel<128><<<dim3(static_cast<unsigned>(num_tiles) * num_groups, 1, parts), lb::kTaThreads, lb::TaShared<128>::kBytes, stream>>>(map_q, map_k, map_v, p);
-        return static_cast<int>(cudaGetLastError());
+        return static_cast<int>(lb::launch_overlapped(lb::attention_tcgen05_kernel<128>, dim3(static_cast<unsigned>(num_tiles) * num_groups, 1, parts), dim3(lb::kTaThreads),
+                                                      lb::TaShared<128>::kBytes, stream, map_q, map_k, map_v, p));
     }
     static lb::OncePerDevice configured, configured_paired;
     if (lb::allow_shared_memory(configured, lb::attention_tcgen05_halves_kernel<false>, lb::kThBytes) != cudaSuccess ||
         lb::allow_shared_memory(configured_paired, lb::attention_tcgen05_halves_kernel<true>, lb::kThBytes) != cudaSuccess)
         return static_cast<int>(cudaGetLastError());
     if (split_tiles == 0) {
-        lb::attention_tcgen05_halves_kernel<false><<<dim3(static_cast<unsigned>(num_tiles) * num_groups, 1, parts), lb::kThThreads, lb::kThBytes, stream>>>(map_q, map_k, map_v, p);
-        return static_cast<int>(cudaGetLastError());
+        return static_cast<int>(lb::launch_overlapped(lb::attention_tcgen05_halves_kernel<false>, dim3(static_cast<unsigned>(num_tiles) * num_groups, 1, parts), dim3(lb::kThThreads), lb::kThBytes,
+                                                      stream, map_q, map_k, map_v, p));
     }
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3(2u * num_tiles * num_groups, 1, parts);
     config.blockDim = dim3(lb::kThThreads);
     config.dynamicSmemBytes = lb::kThBytes;
     config.stream = stream;
-    cudaLaunchAttribute attribute[1];
+    cudaLaunchAttribute attribute[2];
     attribute[0].id = cudaLaunchAttributeClusterDimension;
     attribute[0].val.clusterDim.x = 2;
     attribute[0].val.clusterDim.y = 1;
     attribute[0].val.clusterDim.z = 1;
+    attribute[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute[1].val.programmaticStreamSerializationAllowed = lb::overlap_launches() ? 1 : 0;
     config.attrs = attribute;
-    config.numAttrs = 1;
+    config.numAttrs = 2;
     const cudaError_t launched = cudaLaunchKernelEx(&config, lb::attention_tcgen05_halves_kernel<true>, map_q, map_k, map_v, p);
     if (launched != cudaSuccess) return static_cast<int>(launched);
     return static_cast<int>(cudaGetLastError());
