@@ -160,6 +160,9 @@ class Attention(Mixer):
                 raise ValueError(f"attention applies rotary position encodings, not {type(spec.position).__name__}")
             self.position = build_part(spec.position, {}, runtime)
         self.scale = spec.scale if spec.scale is not None else spec.head_dim**-0.5
+        # Whether a step whose tokens attend alone needs no more than the two products, the rewrite and the attention.
+        self.four_kernels = (runtime.dtype == torch.bfloat16 and self.maps == 1 and self.conv_weight is None and not spec.gated and not spec.has_bias and self.value_dim == spec.head_dim
+                             and not (spec.qk_norm is not None and spec.qk_norm_whole))
 
     @classmethod
     def tensor_decls(cls, spec: AttentionSpec) -> dict[str, TensorDecl]:
@@ -259,6 +262,17 @@ class Attention(Mixer):
         conv_view: SlotStateView | None = None
         if isinstance(cache, CompositeView):
             cache, conv_view = cache.views
+        planned = step.host_plans.get(self.step_plan_key()) if self.four_kernels and x.shape[0] <= ops.SKINNY_MAX_TOKENS else None
+        if planned is not None and planned["alone"].size == x.shape[0] == step.tokens:
+            position, temperature = self.position, spec.query_temperature
+            out = ops.attention_step(
+                x, self.qkv, self.out_proj, None if defer else residual, cache.k_pages, cache.v_pages, cache.block_table, step.positions, step.token_segment, self.q_norm, self.k_norm,
+                self.norm_eps, self.norm_offset, position.inv_freq if position is not None else None, position.rotary_dim if position is not None else 0,
+                position.magnitude if position is not None else 1.0, spec.num_heads, spec.num_groups, spec.head_dim, self.scale, spec.window, self.keep_first,
+                temperature.coefficient if temperature is not None else 0.0, temperature.every if temperature is not None else 0, cache.owns, step.max_context,
+                ALONE_LIMIT if cache.owns and EARLY_ATTENTION else None, self.runtime.status)
+            if out is not None:
+                return out if defer or residual is None else None
         projected = ops.linear(x, self.qkv, status=self.runtime.status)
         gate = None
         if spec.gated:

@@ -33,6 +33,10 @@ class GatedMLP(FeedForward):
     can_defer = True
 
     def forward(self, x: torch.Tensor, step: StepInputs | None = None, residual: torch.Tensor | None = None, defer: bool = False) -> "torch.Tensor | ops.SlicedSum | None":
+        if x.shape[0] <= ops.SKINNY_MAX_TOKENS:
+            out = ops.gated_mlp_step(x, self.up_gate, self.down, self.spec.activation, self.spec.limit, residual)
+            if out is not None:
+                return out if residual is None else None
         hidden = ops.gated_linear(x, self.up_gate, self.spec.activation, status=self.runtime.status, limit=self.spec.limit)
         if residual is not None:
             early = ops.gated_linear_starts_successor_early(x.shape[0], self.up_gate.shape[0], x.shape[1])
