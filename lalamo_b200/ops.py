@@ -2346,9 +2346,15 @@ def float32_product_supported(tokens: int, rows: int, width: int) -> bool:
 
 def _product(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     """``x @ weight.T`` where none of the bfloat16 kernels takes it: on the kernel of the 32-bit path, else by the library."""
-    if (x.dtype == torch.float32 and x.dim() == 2 and float32_product_supported(x.shape[0], weight.shape[0], x.shape[1]) and x.stride(1) == 1 and x.stride(0) % 4 == 0
-            and x.stride(0) >= x.shape[1] and (x.data_ptr() | weight.data_ptr()) % 16 == 0
-            and not (torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad))):
+def _watched(x: torch.Tensor, weight: torch.Tensor) -> bool:
+    """Whether somebody follows this product: autograd (backward or forward), a function transform such as ``vmap``, a trace, a dispatch mode.  A launch past
+    torch's operators would lose their tangents, batches or nodes."""
+    return ((torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad)) or torch.autograd.forward_ad._current_level >= 0
+            or torch._C._functorch.peek_interpreter_stack() is not None or torch._C._len_torch_dispatch_stack() > 0 or torch.jit.is_tracing())
+
+
+    if (x.dtype == torch.float32 and x.dim() == 2 and not _watched(x, weight) and float32_product_supported(x.shape[0], weight.shape[0], x.shape[1])
+            and x.stride(1) == 1 and x.stride(0) % 4 == 0 and x.stride(0) >= x.shape[1] and (x.data_ptr() | weight.data_ptr()) % 16 == 0):
         out = torch.empty(x.shape[0], weight.shape[0], dtype=torch.float32, device=x.device)
         _done(_lib().lb_gemm_float32(x, weight, out, x.shape[0], weight.shape[0], x.shape[1], x.stride(0), 0, _stream()), "gemm_float32")
         return out
