@@ -7,6 +7,8 @@ makes the invariants checkable: nothing is lost, held twice or freed twice.
 
 from __future__ import annotations
 
+from typing import Iterable
+
 __all__ = ["OutOfPages", "OutOfSlots", "PagePool", "SlotPool"]
 
 
@@ -77,9 +79,9 @@ class PagePool(_IdPool):
             raise OutOfPages(count, len(self._free), self.name)
         return [self._take() for _ in range(count)]
 
-    def release(self, pages: list[int]) -> None:
+    def release(self, pages: Iterable[int]) -> None:
         """Gives the pages back, the first of them to be handed out first again: pages that follow one another stay neighbours."""
-        for page in reversed(pages):
+        for page in reversed(list(pages)):
             self._give_back(page)
 
 

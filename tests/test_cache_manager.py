@@ -33,6 +33,16 @@ def test_page_pool_basics():
     pool.check()
 
 
+def test_pages_come_back_in_their_order_from_anything_that_lists_them():
+    pool = PagePool(5)
+    for listed in (list, tuple, iter, lambda pages: (page for page in pages)):
+        pages = pool.allocate(4)
+        pool.release(listed(pages))
+        assert pool.allocate(4) == pages
+        pool.release(pages)
+    pool.check()
+
+
 def test_slot_pool():
     slots = SlotPool(2)
     a, b = slots.allocate(), slots.allocate()
