@@ -23,7 +23,7 @@ constexpr int kPtRows = 128, kPtKeys = 64, kPtThreads = 320, kPtStages = 4;
 constexpr int kPtPanel = kPtKeys * 128;           // 64 rows of 64 channels
 constexpr int kPtStage = 2 * kPtPanel;            // keys, values
 constexpr float kPtMostX = 0.5f;                  // of a score over the cap, for the polynomial
-constexpr float kPtMostExponent = 60.0f;          // of 2^y in a weight's 1 / (1 + 2^y): two of them have a product, and 2^-60 is nothing beside the weights' rounding
+constexpr float kPtMostExponent = 60.0f;          // of 2^y in a weight's 1 / (1 + 2^y) up to which two weights share a reciprocal: their denominators then have a product
 
 struct PooledTcParams {
     const __nv_bfloat16* pooled_pages;
@@ -65,12 +65,6 @@ __device__ __forceinline__ float pt_reciprocal(float x) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-// the smaller one; not a number if either is not
-__device__ __forceinline__ float pt_least(float a, float b) {
-    float y;
-    asm("min.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
-    return y;
-}
 
 // The weights of a row's scores: 1 / (1 + 2^y), y = -(cap tanh(s scale / cap) + bias) log2 e.
 struct PooledWeights {
@@ -94,6 +88,8 @@ struct PooledWeights {
         wide_slope = 2.0f * cap * kLog2e;
         wide_offset = -(cap + bias) * kLog2e;
     }
+    // whether no y is beyond kPtMostExponent, without a cap, for scores of at most `top`
+    __device__ __forceinline__ bool near(float top) const { return fmaf(top, fabsf(slope), fabsf(offset)) <= kPtMostExponent; }
     // -log2 of what a weight's denominator adds to one, of two neighbours' scores; two 32-bit values an instruction where the form allows
     template <int FORM>   // 0: no cap, 1: the polynomial, 2: written out
     __device__ __forceinline__ uint64_t exponents(uint64_t s) const {
@@ -112,15 +108,19 @@ struct PooledWeights {
             return pack2(fmaf(pt_reciprocal(1.0f + pt_exp2(s0 * to_exponent)), wide_slope, wide_offset), fmaf(pt_reciprocal(1.0f + pt_exp2(s1 * to_exponent)), wide_slope, wide_offset));
         }
     }
-    // the two weights, rounded
-    template <int FORM>
+    // the two weights, rounded; NEAR: both exponents are within kPtMostExponent.  Beyond it each weight has a reciprocal of its own, down to the least
+    // normal number (2^-126), as in the kernels of single tokens
+    template <int FORM, bool NEAR>
     __device__ __forceinline__ uint32_t pair(float s0, float s1) const {
         float y0, y1, d0, d1, w0, w1;
         unpack2(exponents<FORM>(pack2(s0, s1)), y0, y1);
-        if constexpr (FORM != 1) y0 = pt_least(y0, kPtMostExponent), y1 = pt_least(y1, kPtMostExponent);
         unpack2(add2(pack2(pt_exp2(y0), pt_exp2(y1)), pack2(1.0f, 1.0f)), d0, d1);
-        const float r = pt_reciprocal(d0 * d1);
-        unpack2(mul2(pack2(d1, d0), pack2(r, r)), w0, w1);
+        if constexpr (NEAR) {
+            const float r = pt_reciprocal(d0 * d1);
+            unpack2(mul2(pack2(d1, d0), pack2(r, r)), w0, w1);
+        } else {
+            w0 = pt_reciprocal(d0), w1 = pt_reciprocal(d1);
+        }
         const __nv_bfloat162 weights = __floats2bfloat162_rn(w0, w1);
         return *reinterpret_cast<const uint32_t*>(&weights);
     }
@@ -369,21 +369,23 @@ pooled_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const
                 }
             }
             uint32_t packed[16];
-            auto weigh = [&](auto form) {
+            auto weigh = [&](auto form, auto near) {
 #pragma unroll
-                for (int i = 0; i < 16; ++i) packed[i] = weights.template pair<decltype(form)::value>(raw[2 * i], raw[2 * i + 1]);
+                for (int i = 0; i < 16; ++i) packed[i] = weights.template pair<decltype(form)::value, decltype(near)::value>(raw[2 * i], raw[2 * i + 1]);
             };
-            if (!(p.cap > 0.0f)) {
-                weigh(std::integral_constant<int, 0>{});
-            } else {
-                float top = 0.0f;
+            float top = 0.0f;
 #pragma unroll
-                for (int i = 0; i < 32; i += 2) asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(top) : "f"(top), "f"(raw[i]), "f"(raw[i + 1]));
-                // (by the row's own scores alone: what shares the warp changes no bit)
-                if (top <= weights.most) weigh(std::integral_constant<int, 1>{});
-                else weigh(std::integral_constant<int, 2>{});
-                __syncwarp();
+            for (int i = 0; i < 32; i += 2) asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(top) : "f"(top), "f"(raw[i]), "f"(raw[i + 1]));
+            // (by the row's own scores alone: what shares the warp changes no bit)
+            if (!(p.cap > 0.0f)) {
+                if (weights.near(top)) weigh(std::integral_constant<int, 0>{}, std::true_type{});
+                else weigh(std::integral_constant<int, 0>{}, std::false_type{});
+            } else if (top <= weights.most) {
+                weigh(std::integral_constant<int, 1>{}, std::true_type{});
+            } else {
+                weigh(std::integral_constant<int, 2>{}, std::false_type{});
             }
+            __syncwarp();
             if (!all_seen) {
 #pragma unroll
                 for (int i = 0; i < 16; ++i) packed[i] &= ((seen >> (2 * i)) & 1u ? 0x0000ffffu : 0u) | ((seen >> (2 * i + 1)) & 1u ? 0xffff0000u : 0u);

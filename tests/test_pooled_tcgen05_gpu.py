@@ -40,3 +40,35 @@ def test_a_token_without_numbers_reaches_no_earlier_one():
                              head_bias=None, window=150, pool=0, value_freq=None, status=status)
         out.append(found)
     assert int(status.item()) == 0 and torch.equal(out[0][:bad], out[1][:bad]) and bool(out[1][bad:].isnan().all())
+
+
+def _prompt(heads, tokens, seed, width=128):
+    """Queries, pages and what the kernels take beside them, for one prompt of ``tokens`` over one K/V head."""
+    generator = torch.Generator().manual_seed(seed)
+    ints = lambda x: torch.as_tensor(x, dtype=torch.int32).reshape(-1).cuda()  # noqa: E731
+    blocks = -(-tokens // 16)
+    q = torch.randn(tokens, heads * 64, generator=generator).bfloat16().cuda()
+    pages = torch.randn(blocks, 16, 1, width, generator=generator).bfloat16().cuda()
+    common = dict(positions=ints(range(tokens)), token_segment=ints([0] * tokens), block_table=torch.arange(blocks, dtype=torch.int32).view(1, blocks).cuda(), pool_table=None,
+                  num_heads=heads, num_groups=1, head_dim=64, value_dim=64, window=150, pool=0, status=torch.zeros(1, dtype=torch.int32, device="cuda"))
+    run = 16 * (8 // min(heads, 4))
+    tiles = [(i, min(run, tokens - i)) for i in range(0, tokens, run)]
+    return q, pages, dict(tiles=ints(tiles), num_tiles=len(tiles)), common
+
+
+# exponents that a pair of weights shares a reciprocal for, that it does not, and both within a head's scores
+@pytest.mark.parametrize("cap,scale", [(0.0, 0.125), (0.0, 1.0), (30.0, 0.125), (30.0, 1.0), (55.0, 1.0)])
+def test_closed_heads(cap, scale):
+    """Heads that a bias all but closes: weights down to 2 ** -115, as the 32-bit kernel has them."""
+    from lalamo_b200 import ops
+
+    tokens, heads = 200, 4
+    q, pages, tiles, common = _prompt(heads, tokens, 5)
+    common.update(scale=scale, softcap=cap, head_bias=torch.tensor([-2.0, -41.0, -45.0, -72.0 if scale < 1 else -47.0]).cuda(), value_freq=None)
+    found, plain = (torch.empty(tokens, heads * 64, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    ops.pooled_attention(q, pages, None, found, **tiles, **common)
+    ops.pooled_attention_plain(q, pages, None, plain, **common)
+    assert int(common["status"].item()) == 0
+    difference, size = ((x.double().view(tokens, heads, 64)).norm(dim=-1) for x in (found.double() - plain.double(), plain))
+    # the results' and the weights' roundings to bfloat16, of 2 ** -9 of a value each at most
+    assert float((difference / size).max()) < 2 * 2 ** -8
