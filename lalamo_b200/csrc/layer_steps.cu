@@ -25,6 +25,11 @@ static int skinny_product(const void* x, const void* w, void* out, int tokens, i
     return lb_gemm_skinny(x, w, out, tokens, k, n, epilogue, activation, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0, 0, 0, 1, nullptr, stream, limit, nullptr, k);
 }
 
+// What lb_gemm_skinny refuses, asked before a step's first launch: a step runs as a whole or not at all.
+static bool skinny_takes(const void* x, const void* w, int tokens, int k, int n) {
+    return tokens >= 1 && tokens <= 16 && k >= 32 && k % 32 == 0 && n >= 8 && n % 8 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0;
+}
+
 constexpr int kSkinnyIdentity = 2;   // the activation's code
 constexpr int kSkinnyGated = 3;      // the epilogue's
 
@@ -33,23 +38,30 @@ constexpr int kSkinnyGated = 3;      // the epilogue's
 extern "C" {
 
 // out [tokens, out_width] = (up * act(gate)) @ down.T for [up ; gate] = x @ up_gate.T; epilogue 0 stores bfloat16, 2 adds to a 32-bit `out`.
-// work: tokens * hidden bfloat16 values.  Returns 0, a CUDA error code or -2 for sizes or an alignment the products do not take.
+// work: tokens * hidden bfloat16 values.  Returns 0, a CUDA error code or -2, with nothing launched, for sizes or an alignment the products do not take.
 int lb_gated_mlp_step(const void* x, const void* up_gate, const void* down, void* out, void* work, long long work_bytes, int tokens, int width, int hidden, int out_width,
                       int activation, float limit, int epilogue, cudaStream_t stream) {
-    if (work_bytes < static_cast<long long>(tokens) * hidden * 2 || (epilogue != 0 && epilogue != 2)) return -2;
+    if (work_bytes < static_cast<long long>(tokens) * hidden * 2 || (epilogue != 0 && epilogue != 2) || !lb::skinny_takes(x, up_gate, tokens, width, hidden) ||
+        !lb::skinny_takes(work, down, tokens, hidden, out_width))
+        return -2;
     const int code = lb::skinny_product(x, up_gate, work, tokens, width, hidden, lb::kSkinnyGated, activation, limit, stream);
     return code != 0 ? code : lb::skinny_product(work, down, out, tokens, hidden, out_width, epilogue, lb::kSkinnyIdentity, 0.0f, stream);
 }
 
 // An attention layer whose tokens all attend alone: x @ qkv_weight.T, the rewrite of q, k and v, the split-key attention (with the merge of its
 // splits) and the out-projection.  epilogue as above; work: the product's rows, the queries, the heads' outputs (bfloat16, each from a multiple
-// of 256 bytes on), then the attention's scratch (tokens * heads * splits * (head_dim + 2) floats).
+// of 256 bytes on), then the attention's scratch (tokens * heads * splits * (head_dim + 2) floats).  Returns -2, with nothing launched, for
+// what one of the four would refuse.
 int lb_attention_step(const void* x, const void* qkv_weight, const void* out_weight, void* out, void* work, long long work_bytes, int tokens, int width, int qkv_width, int out_width,
                       int epilogue, void* k_pages, void* v_pages, const float* q_norm, const float* k_norm, float eps, float scale_offset, const float* inv_freq, int rotary_dim,
                       const int* positions, const int* token_segment, const int* block_table, int num_heads, int num_groups, int head_dim, int page_size, int num_pages,
                       int max_blocks, int write_kv, float turn_scale, float temperature, int temperature_every, float scale, int window, int keep_first, int splits,
                       int blocks_per_split, int fresh_keys, int* status, cudaStream_t stream) {
-    if (tokens < 1 || splits < 1 || (epilogue != 0 && epilogue != 2)) return -2;
+    if (num_groups < 1 || num_heads % num_groups != 0 || head_dim < 16 || head_dim > 128 || head_dim % 16 != 0 || page_size % 16 != 0 || rotary_dim < 0 || rotary_dim > head_dim ||
+        rotary_dim % 2 != 0 || temperature_every < 0 || splits < 1 || blocks_per_split < 1 || fresh_keys < -1 || keep_first < 0 || !(scale > 0.0f) ||
+        (epilogue != 0 && epilogue != 2) || qkv_width < num_heads * head_dim + (write_kv ? 2 * num_groups * head_dim : 0) ||
+        !lb::skinny_takes(x, qkv_weight, tokens, width, qkv_width) || !lb::skinny_takes(work, out_weight, tokens, num_heads * head_dim, out_width))
+        return -2;
     auto rounded = [](long long bytes) { return (bytes + 255) / 256 * 256; };
     const int heads_width = num_heads * head_dim;
     const long long queries_at = rounded(2LL * tokens * qkv_width), mixed_at = queries_at + rounded(2LL * tokens * heads_width), scratch_at = mixed_at + rounded(2LL * tokens * heads_width);

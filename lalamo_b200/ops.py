@@ -833,6 +833,8 @@ def qk_norm_rope_write(
             raise KernelError("qk_norm_rope_write: inv_freq must have rotary_dim / 2 elements, rotary_dim even and <= head_dim")
     _check(positions, "positions", torch.int32)
     _check(token_segment, "token_segment", torch.int32)
+    if positions.numel() < tokens or token_segment.numel() < tokens:
+        raise KernelError("qk_norm_rope_write: positions and token_segment must have an element per row of qkv")
     code = _lib().lb_qk_norm_rope_write(
         qkv, q_out, k_pages, v_pages, q_weight, k_weight, eps, scale_offset,
         inv_freq, rotary_dim, positions, token_segment, block_table, tokens, num_heads,
@@ -2570,7 +2572,7 @@ def attention_step(x: torch.Tensor, qkv_weight: torch.Tensor, out_weight: torch.
     was launched.  Eight tokens at a context of 4,096 through width 2048: 55.2 us with the four bindings, 37.5 here, 33 of them the kernels'."""
     bfloat16, float32, int32 = torch.bfloat16, torch.float32, torch.int32
     if not (_is_plain(x, bfloat16) and _is_plain(qkv_weight, bfloat16) and _is_plain(out_weight, bfloat16) and _is_plain(k_pages, bfloat16) and _is_plain(v_pages, bfloat16)
-            and _is_plain(block_table, int32) and _is_plain(positions, int32) and _is_plain(token_segment, int32)):
+            and _is_plain(block_table, int32) and _is_plain(positions, int32) and _is_plain(token_segment, int32) and _is_plain(status, int32)):
         return None
     if x.dim() != 2 or block_table.dim() != 2 or k_pages.dim() != 4 or head_dim not in DECODE_HEAD_DIMS or num_heads % num_groups:
         return None
@@ -2588,6 +2590,8 @@ def attention_step(x: torch.Tensor, qkv_weight: torch.Tensor, out_weight: torch.
         return None
     out = _step_output(x, out_rows, residual)
     if out is None:
+        return None
+    if positions.numel() < tokens or token_segment.numel() < tokens:
         return None
     keep_first = keep_first if window else 0
     splits, blocks_per_split = decode_attention_plan(tokens, num_heads, num_groups, max_context, window, head_dim, keep_first=keep_first)

@@ -82,3 +82,42 @@ def test_attention_step(lengths, contexts, heads, groups, hd, rotary, window, no
     out = step()
     assert (out is stream) == accumulate and torch.equal(out, expected)
     assert torch.equal(k_pages, keys) and torch.equal(v_pages, values) and status.item() == 0
+
+
+class _Step:
+    """An attention layer of two tokens, each of a request of its own."""
+
+    def __init__(self):
+        self.ints = lambda *values: torch.tensor(values, dtype=torch.int32, device="cuda")
+        self.x, self.qkv, self.out_weight = _values(2, 64, seed=1), _values(6 * 32, 64, seed=2), _values(64, 2 * 32, seed=3)
+        self.k_pages, self.v_pages = _values(2, 16, 2, 32, seed=4), _values(2, 2, 32, 16, seed=5)
+        self.table, self.status = self.ints(0, 1).view(2, 1), self.ints(0)
+
+    def run(self, scale=0.1, keep_first=0, every=0, window=None, out_weight=None, positions=None, segment=None):
+        return ops.attention_step(self.x, self.qkv, self.out_weight if out_weight is None else out_weight, None, self.k_pages, self.v_pages, self.table,
+                                  self.ints(3, 4) if positions is None else positions, self.ints(0, 1) if segment is None else segment, None, None, 1e-5, 0.0, None, 0, 1.0, 2, 2, 32, scale,
+                                  window, keep_first, 0.0, every, True, 16, 16, self.status)
+
+
+def test_a_refused_step_launches_nothing():
+    """What one of a step's kernels would refuse is refused before the first of them: no page, no row of the workspace is written."""
+    step = _Step()
+    keys, values = step.k_pages.clone(), step.v_pages.clone()
+    apart = _values(64 * 64 + 1, seed=3)[1:].view(64, 64)   # rows that start 2 bytes past a multiple of 16
+    for refused in (dict(scale=0.0), dict(scale=-1.0), dict(keep_first=-1, window=8), dict(every=-1), dict(out_weight=apart)):
+        assert step.run(**refused) is None
+        assert torch.equal(step.k_pages, keys) and torch.equal(step.v_pages, values), refused
+    assert step.run() is not None and not torch.equal(step.k_pages, keys) and step.status.item() == 0
+    up_gate, down, work = _values(64, 64, seed=6), _values(64 * 32 + 1, seed=7)[1:].view(64, 32), torch.full((2, 32), float("nan"), dtype=torch.bfloat16, device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    assert ops._lib().lb_gated_mlp_step(step.x, up_gate, down, torch.empty_like(step.x), work, 2 * 2 * 32, 2, 64, 32, 64, 1, 0.0, 0, stream) == -2
+    assert bool(work.isnan().all())
+
+
+def test_fewer_positions_than_tokens():
+    step = _Step()
+    assert step.run(positions=step.ints(3)) is None and step.run(segment=step.ints(0)) is None
+    for wrong in (dict(positions=step.ints(3), token_segment=step.ints(0, 1)), dict(positions=step.ints(3, 4), token_segment=step.ints(0))):
+        with pytest.raises(ops.KernelError):
+            ops.qk_norm_rope_write(ops.linear(step.x, step.qkv), step.x.new_empty(2, 64), step.k_pages, step.v_pages, q_weight=None, k_weight=None, eps=1e-5, scale_offset=0.0,
+                                   inv_freq=None, rotary_dim=0, block_table=step.table, num_heads=2, num_groups=2, head_dim=32, write_kv=True, status=step.status, **wrong)
