@@ -116,10 +116,12 @@ inline bool overlap_launches() {
     return overlap;
 }
 
+// The same where `early` says so, else the ordinary way.  What starts early settles where the kernel before leaves room first, several blocks to a
+// multiprocessor: worth it for blocks that are done at once or that fill the GPU whatever their places, not for some hundred blocks of long work, which
+// then share a few multiprocessors while the others idle.
 template <typename... Parameters, typename... Arguments>
-inline cudaError_t launch_overlapped(void (*kernel)(Parameters...), dim3 grid, dim3 block, size_t shared_bytes, cudaStream_t stream,
-                                     Arguments&&... arguments) {
-    const bool overlap = overlap_launches();
+inline cudaError_t launch_early_if(bool early, void (*kernel)(Parameters...), dim3 grid, dim3 block, size_t shared_bytes, cudaStream_t stream,
+                                   Arguments&&... arguments) {
     cudaLaunchConfig_t config = {};
     config.gridDim = grid;
     config.blockDim = block;
@@ -127,10 +129,16 @@ inline cudaError_t launch_overlapped(void (*kernel)(Parameters...), dim3 grid, d
     config.stream = stream;
     cudaLaunchAttribute attribute[1];
     attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attribute[0].val.programmaticStreamSerializationAllowed = overlap ? 1 : 0;
+    attribute[0].val.programmaticStreamSerializationAllowed = early && overlap_launches() ? 1 : 0;
     config.attrs = attribute;
     config.numAttrs = 1;
     return cudaLaunchKernelEx(&config, kernel, static_cast<Parameters>(arguments)...);
+}
+
+template <typename... Parameters, typename... Arguments>
+inline cudaError_t launch_overlapped(void (*kernel)(Parameters...), dim3 grid, dim3 block, size_t shared_bytes, cudaStream_t stream,
+                                     Arguments&&... arguments) {
+    return launch_early_if(true, kernel, grid, block, shared_bytes, stream, static_cast<Arguments&&>(arguments)...);
 }
 
 // Something a launcher must do once on every device before its first launch there (a kernel's
