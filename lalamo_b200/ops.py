@@ -1265,7 +1265,7 @@ def _recurrence(q: torch.Tensor, k: torch.Tensor, decay: torch.Tensor, v: torch.
     if num_direct > 0:
         code = lib.lb_gdr_scan(q, k, decay, v, beta, matrix_state, read_out, segment_start, segment_length,
                                segment_slot, num_direct, num_heads, num_groups, key_dim, value_dim, num_slots,
-                               status, _stream(), direct_list)
+                               status, _stream(), direct_list, 1 if segments == tokens else 0)
         _done(code, "gdr_scan")
     return read_out
 
