@@ -30,7 +30,8 @@ ALONE_LIMIT = 16
 TILE_TOKENS = ops.PREFILL_TILE
 EARLY_ATTENTION = os.environ.get("LALAMO_B200_EARLY_ATTENTION", "1") != "0"  # the split-key attention starts under the q/k/v rewrite
 SHARED_TILE_KEYS = 512  # where tiles are shared, a tile that sees at least this many keys is worked on by two CTAs
-LONG_TILE_KEYS = 3072  # a launch's tiles count as long if they see this many keys on average
+# How much better two CTAs a tile have to fill the multiprocessors, and the keys that the launch's tiles then see on average, for sharing to pay
+SHARED_TILE_GAINS = ((1.25, 4096), (1.15, 10240))
 
 
 def _slot_use(ctas: int, slots: int) -> float:
@@ -44,8 +45,10 @@ def shared_tile_keys(num_tiles: int, num_heads: int, num_groups: int, sms: int, 
     the keys, merged at the end); 0: never, the launch has one CTA per tile.  Two CTAs per tile pay where that
     fills the SMs better: with fewer CTAs than SMs; or, in steps that are never replayed (so that the answer may
     depend on the contexts), where tiles mostly see thousands of keys and their CTAs fill the resident slots
-    (three per SM) badly, as 512 CTAs fill 444.  Launching as clusters costs 12 to 25 % by itself, so whole
-    prompts from position 0, whose early tiles are short, stay unpaired."""
+    (two per SM) badly, as 384 CTAs fill 592.  Launching as clusters and merging costs 10 to 60 % of a launch whose tiles are short
+    and a few percent of one whose tiles see 15,000 keys.  Measured, one CTA a tile and two, 32 heads over 8: 1,280 tokens behind
+    3,072 100 and 96 us, behind 14,336 388 and 309, behind 1,024 45 and 57; 1,536 behind 4,096 135 and 128; 2,560 behind 4,096 212 and 220, behind 14,336 601
+    and 547; 2,048 and 3,072, which two CTAs a tile fill no better, behind 4,096 150 and 168, 238 and 274; 512 behind 0 11 and 12, behind 4,096 61 and 43."""
     per_group = num_heads // num_groups
     parts = -(-TILE_TOKENS // max(1, min(TILE_TOKENS, 128 // per_group)))
     ctas = num_tiles * num_groups * parts
@@ -53,7 +56,8 @@ def shared_tile_keys(num_tiles: int, num_heads: int, num_groups: int, sms: int, 
         return SHARED_TILE_KEYS
     if tokens > REPLAY_MAX_TOKENS and contexts:
         keys = sum(length * (context + length / 2) for length, context in zip(lengths, contexts))
-        if keys / max(1, sum(lengths)) >= LONG_TILE_KEYS and _slot_use(2 * ctas, 3 * sms) > _slot_use(ctas, 3 * sms) + 0.1:
+        gain = _slot_use(2 * ctas, 2 * sms) / _slot_use(ctas, 2 * sms)
+        if any(gain >= least and keys >= least_keys * sum(lengths) for least, least_keys in SHARED_TILE_GAINS):
             return SHARED_TILE_KEYS
     return 0
 

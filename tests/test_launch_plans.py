@@ -75,11 +75,17 @@ def test_when_prefill_attention_tiles_are_shared_by_two_ctas():
     # 512 tokens of one request, 32 heads over 8: 16 tiles x 8 = 128 CTAs
     assert shared_tile_keys(16, 32, 8, sms, 512, (512,), (0,)) == SHARED_TILE_KEYS
     assert shared_tile_keys(16, 32, 8, sms, 512, (512,), (16000,)) == SHARED_TILE_KEYS
-    # 1,024 tokens: 256 CTAs on 444 slots; twice as many would need a second, nearly empty round
+    # 1,024 tokens: 256 CTAs on 296 slots, two CTAs a multiprocessor; twice as many fill two rounds no better
     assert shared_tile_keys(32, 32, 8, sms, 1024, (1024,), (15000,)) == 0
-    # 2,048 tokens: 512 CTAs need two rounds; paired, 1,024 need 2.3: only where the tiles are long
+    # 2,048 tokens: 512 CTAs fill two rounds as well as 1,024 fill four
     assert shared_tile_keys(64, 32, 8, sms, 2048, (2048,), (0,)) == 0
-    assert shared_tile_keys(64, 32, 8, sms, 2048, (2048,), (14336,)) == SHARED_TILE_KEYS
+    assert shared_tile_keys(64, 32, 8, sms, 2048, (2048,), (14336,)) == 0
+    # 1,536 tokens: 384 CTAs fill 0.65 of two rounds, 768 0.86 of three: where the tiles see 4,096 keys on average
+    assert shared_tile_keys(48, 32, 8, sms, 1536, (1536,), (2048,)) == 0
+    assert shared_tile_keys(48, 32, 8, sms, 1536, (1536,), (4096,)) == SHARED_TILE_KEYS
+    # 2,560 tokens: 0.72 and 0.86 of the slots: where the tiles see 10,240
+    assert shared_tile_keys(80, 32, 8, sms, 2560, (2560,), (4096,)) == 0
+    assert shared_tile_keys(80, 32, 8, sms, 2560, (2560,), (14336,)) == SHARED_TILE_KEYS
     # a whole long prompt in one step: thousands of CTAs fill the slots either way
     assert shared_tile_keys(512, 32, 8, sms, 16384, (16384,), (0,)) == 0
     # replayable steps get the same answer whatever the contexts
