@@ -171,13 +171,14 @@ class LatentAttention(Mixer):
         if ops.latent_attention_supported(runtime.dtype, latent, rope, cache.k_pages.shape[1]):
             lists, host_lists = step.plan_of(self)
             num_items = host_lists["items"].size // 2
-            double = False
-            if self.tcgen05:
+            longest = int(host_lists["items"][1::2].max()) if num_items else 0
+            double, tcgen05 = False, self.tcgen05 and not ops.latent_attention_few_rows(num_items, longest, heads, step.max_context)
+            if tcgen05:
                 splits = ops.latent_attention_tcgen05_splits(num_items, tokens, heads, spec.window, step.max_context)
             else:
-                double = num_items > 0 and int(host_lists["items"][1::2].max()) > ops.latent_attention_tiling(heads)[1]
+                double = longest > ops.latent_attention_tiling(heads)[1]
                 splits = ops.latent_attention_splits(num_items, heads, latent, spec.window, step.max_context, double=double)
-            ops.latent_attention(queries, cache.k_pages, summed, items=lists["items"], num_items=num_items, splits=splits, double=double, tcgen05=self.tcgen05, **common)
+            ops.latent_attention(queries, cache.k_pages, summed, items=lists["items"], num_items=num_items, splits=splits, double=double, tcgen05=tcgen05, **common)
         else:
             ops.latent_attention_plain(queries, cache.k_pages, summed, **common)
         mixed = runtime.empty(tokens, heads * spec.value_dim)
