@@ -2343,18 +2343,23 @@ def tcgen05_wait_probe(status: torch.Tensor, nanoseconds: int = 1_000_000) -> No
 
 
 def float32_product_supported(tokens: int, rows: int, width: int) -> bool:
-    """Whether a product of the 32-bit path runs on the framework's own kernel: where the library's large tiles would leave most multiprocessors idle.  Measured, ours and the
-    library's: 5 and 12 tokens x 2048 x 1024 8 and 19 us, 32 x 9216 x 1024 24 and 25, 96 x 2048 x 2048 34 and 42, 64 x 4096 x 1024 19 and 24, 300 x 1024 x 1024 25 and 31, 400 x
-    1024 x 2048 55 and 57; beyond, 192 x 2048 x 1024 33 and 31, 96 x 3072 x 2048 61 and 43, 500 x 1024 x 2048 64 and 60.  (Of up to four tokens the library
-    adds up in another way, a tenth closer to 64 bits.)"""
+    """Whether a product of the 32-bit path runs on the framework's own kernel: where the library's large tiles would leave most multiprocessors idle, and K is long enough
+    to be shared out.  Measured, our time over the library's, tokens x rows x width: 8 x 2048 x 1024 0.48, 8 x 64 x 512 1.0, 8 x 64 x 384 1.4, 8 x 64 x 8192 1.6, 8 x 3072 x 128 0.9, 8 x
+    9216 x 1024 0.9, 8 x 16384 x 256 1.05; 32 x 4608 x 1024 0.84, 32 x 4608 x 192 1.06, 32 x 6144 x 512 1.04, 32 x 9216 x 1024 1.04, 32 x 16384 x 2048 0.94, 32 x 9216 x 4608 0.76;
+    64 x 4096 x 1024 0.87, 64 x 4096 x 384 1.1, 64 x 4608 x 1024 1.17, 384 x 1024 x 1024 0.87, 400 x 1024 x 1024 1.15, 1000 x 8 x 2048 1.07.  (Of up to four tokens the
+    library adds up in another way, a tenth closer to 64 bits.)"""
     if width % 4 or tokens < 5:
         return False
+    if tokens <= 16:
+        return (width >= 512 or rows >= 3072) and (rows >= 512 or width <= 4096) and rows <= (16384 if width >= 1024 else 12288)
+    if tokens <= 32:
+        if rows <= 4608:
+            return width <= 128 or width >= 256
+        return rows <= 16384 and width >= (1024 if rows <= 6144 else 2048 if rows >= 12288 else 4096)
     tiles = -(-tokens // 64) * -(-rows // 64)
-    return (tokens <= 32 and rows <= 16384) or tiles <= 64 or (rows <= 1024 and tiles <= 112)
+    return width >= 512 and (tiles <= 64 or (rows <= 1024 and tiles <= 96)) and (rows >= 64 or tokens <= 768)
 
 
-def _product(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
-    """``x @ weight.T`` where none of the bfloat16 kernels takes it: on the kernel of the 32-bit path, else by the library."""
 def _watched(x: torch.Tensor, weight: torch.Tensor) -> bool:
     """Whether somebody follows this product: autograd (backward or forward), a function transform such as ``vmap``, a trace, a dispatch mode.  A launch past
     torch's operators would lose their tangents, batches or nodes."""

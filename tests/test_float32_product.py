@@ -1,4 +1,5 @@
-"""Products of the 32-bit path that autograd, a transform or a trace follows stay torch's operator: the framework's kernel would lose what they follow."""
+"""Which products of the 32-bit path the framework's kernel takes: not those that autograd, a transform or a trace follows (it would lose what they follow), and
+not the sizes that the library does sooner."""
 
 import pytest
 import torch
@@ -14,10 +15,10 @@ class _NoLaunch:
 @pytest.fixture(autouse=True)
 def no_launch(monkeypatch):
     monkeypatch.setattr(ops, "_lib", lambda: _NoLaunch())
-    assert ops.float32_product_supported(8, 16, 32)
+    assert ops.float32_product_supported(8, 16, 512)
 
 
-X, W = torch.randn(8, 32, generator=torch.Generator().manual_seed(1)), torch.randn(16, 32, generator=torch.Generator().manual_seed(2))
+X, W = torch.randn(8, 512, generator=torch.Generator().manual_seed(1)), torch.randn(16, 512, generator=torch.Generator().manual_seed(2))
 
 
 def test_forward_mode():
@@ -31,12 +32,12 @@ def test_forward_mode():
 def test_backward():
     weight = W.clone().requires_grad_()
     ops._product(X, weight).sum().backward()
-    assert torch.allclose(weight.grad, X.sum(0).expand(16, 32))
+    assert torch.allclose(weight.grad, X.sum(0).expand(16, 512))
 
 
 def test_vmap():
     rows = torch.stack([X, -X, 3 * X])
-    assert torch.allclose(torch.func.vmap(lambda x: ops._product(x, W))(rows), rows @ W.T, atol=1e-5)
+    assert torch.allclose(torch.func.vmap(lambda x: ops._product(x, W))(rows), rows @ W.T, atol=1e-4)
 
 
 def test_traces():
@@ -45,3 +46,15 @@ def test_traces():
     traced = make_fx(lambda x: ops._product(x, W))(X)
     assert torch.equal(traced(2 * X), (2 * X) @ W.T)
     assert torch.equal(torch.jit.trace(lambda x: ops._product(x, W), X, check_trace=False)(2 * X), (2 * X) @ W.T)
+
+
+@pytest.mark.parametrize("taken,left", [((8, 64, 512), (8, 64, 384)), ((8, 3072, 128), (8, 2048, 256)), ((8, 64, 4096), (8, 64, 8192)), ((16, 16384, 1024), (16, 16384, 256)),
+                                        ((17, 4608, 64), (17, 4608, 192)), ((32, 6144, 1024), (32, 6144, 512)), ((32, 16384, 2048), (32, 9216, 2048)), ((32, 9216, 4608), (32, 16448, 4608)),
+                                        ((64, 4096, 512), (64, 4096, 384)), ((64, 4096, 1024), (64, 4608, 1024)), ((384, 1024, 1024), (400, 1024, 1024)), ((700, 8, 2048), (1000, 8, 2048)),
+                                        ((5, 2048, 1024), (4, 2048, 1024)), ((8, 2048, 1024), (8, 2048, 1022))])
+def test_sizes(taken, left):
+    def takes(size):
+        tokens, rows, width = size
+        return ops.float32_product_supported(tokens, rows, width)
+
+    assert takes(taken) and not takes(left)
