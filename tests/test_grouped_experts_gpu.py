@@ -8,7 +8,9 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("gated,weigh", [(True, False), (True, True), (False, False)])
-@pytest.mark.parametrize("counts,width,ff", [((0, 1, 31, 33, 0, 127), 72, 40), ((129, 128, 0, 257), 256, 264), ((5, 0, 3), 1032, 136), ((700, 9), 64, 520)])
+@pytest.mark.parametrize("counts,width,ff", [((0, 1, 31, 33, 0, 127), 72, 40), ((129, 128, 0, 257), 256, 264), ((5, 0, 3), 1032, 136), ((700, 9), 64, 520),
+                                             # as many pairs as one launch sorts and gathers, two more, and several thousand: two launches
+                                             ((0, 511, 1, 0, 380, 128, 0), 72, 40), ((300, 0, 722, 0), 64, 72), ((0, 1900, 1, 257, 0, 1843, 0), 40, 64)])
 def test_ragged_experts(counts, width, ff, gated, weigh):
     from lalamo_b200 import ops
 
