@@ -2367,6 +2367,8 @@ def _watched(x: torch.Tensor, weight: torch.Tensor) -> bool:
             or torch._C._functorch.peek_interpreter_stack() is not None or torch._C._len_torch_dispatch_stack() > 0 or torch.jit.is_tracing())
 
 
+def _product(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
+    """``x @ weight.T`` where none of the bfloat16 kernels takes it: on the kernel of the 32-bit path, else by the library."""
     if (x.dtype == torch.float32 and x.dim() == 2 and not _watched(x, weight) and float32_product_supported(x.shape[0], weight.shape[0], x.shape[1])
             and x.stride(1) == 1 and x.stride(0) % 4 == 0 and x.stride(0) >= x.shape[1] and (x.data_ptr() | weight.data_ptr()) % 16 == 0):
         out = torch.empty(x.shape[0], weight.shape[0], dtype=torch.float32, device=x.device)
@@ -2589,6 +2591,8 @@ def attention_step(x: torch.Tensor, qkv_weight: torch.Tensor, out_weight: torch.
     if x.dim() != 2 or block_table.dim() != 2 or k_pages.dim() != 4 or head_dim not in DECODE_HEAD_DIMS or num_heads % num_groups:
         return None
     tokens, width = x.shape
+    if positions.numel() < tokens or token_segment.numel() < tokens:
+        return None
     num_pages, page_size, groups, channels = k_pages.shape
     heads_width, (rows, row_width), (out_rows, out_row_width) = num_heads * head_dim, qkv_weight.shape, out_weight.shape
     if (groups != num_groups or channels != head_dim or page_size % 16 or v_pages.shape != (num_pages, num_groups, head_dim, page_size) or row_width != width
@@ -2602,8 +2606,6 @@ def attention_step(x: torch.Tensor, qkv_weight: torch.Tensor, out_weight: torch.
         return None
     out = _step_output(x, out_rows, residual)
     if out is None:
-        return None
-    if positions.numel() < tokens or token_segment.numel() < tokens:
         return None
     keep_first = keep_first if window else 0
     splits, blocks_per_split = decode_attention_plan(tokens, num_heads, num_groups, max_context, window, head_dim, keep_first=keep_first)
