@@ -72,3 +72,58 @@ def test_closed_heads(cap, scale):
     difference, size = ((x.double().view(tokens, heads, 64)).norm(dim=-1) for x in (found.double() - plain.double(), plain))
     # the results' and the weights' roundings to bfloat16, of 2 ** -9 of a value each at most
     assert float((difference / size).max()) < 2 * 2 ** -8
+
+
+@pytest.mark.parametrize("interleaved", [False, True])
+@pytest.mark.parametrize("shares", [1, 3])
+@pytest.mark.parametrize("heads", [1, 2, 3, 6])
+def test_sums_turned_back(heads, shares, interleaved):
+    """Both pairings of the channels that the sums are turned back by, in the epilogue and in the kernel that adds up shares, against the 32-bit sums turned back in 64 bits."""
+    from lalamo_b200 import ops
+
+    tokens = 131
+    q, pages, tiles, common = _prompt(heads, tokens, heads)
+    freq = (200.0 ** (-torch.arange(32, dtype=torch.float64) / 32)).float().cuda()
+    common.update(scale=0.125, softcap=30.0, head_bias=torch.linspace(-2, 1, heads).cuda())
+    found, sums = torch.empty(tokens, heads * 64, dtype=torch.bfloat16, device="cuda"), torch.empty(tokens, heads * 64, device="cuda")
+    ops.pooled_attention(q, pages, None, found, value_freq=freq, interleaved=interleaved, shares=shares, **tiles, **common)
+    ops.pooled_attention_plain(q.float(), pages.float(), None, sums, value_freq=None, **common)
+    sums = sums.double().view(tokens, heads, 64)
+    first, second = (sums[..., 0::2], sums[..., 1::2]) if interleaved else (sums[..., :32], sums[..., 32:])
+    angle = torch.arange(tokens, device="cuda", dtype=torch.float64)[:, None, None] * freq.double()
+    turned = first * angle.cos() + second * angle.sin(), second * angle.cos() - first * angle.sin()
+    want = torch.stack(turned, dim=-1).flatten(2) if interleaved else torch.cat(turned, dim=-1)
+    assert int(common["status"].item()) == 0
+    # the result's and the weights' roundings to bfloat16, of 2 ** -9 of a value each at most
+    assert float(((found.double().view_as(want) - want).norm(dim=-1) / want.norm(dim=-1)).max()) < 2 * 2 ** -8
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("pool", [1, 8, 63, 64, 65, 72, 100, 129])
+def test_means_of_long_blocks(pool, dtype):
+    """Blocks of as many positions as a block of threads looks up at once, and of more; begun and ended within pages, several completed by one step."""
+    from lalamo_b200 import ops
+
+    generator = torch.Generator().manual_seed(pool)
+    groups, page, contexts, lengths = 2, 16, [0, pool // 2, 3 * pool - 1], [2 * pool + 5, pool, 1]
+    blocks = -(-max(c + n for c, n in zip(contexts, lengths)) // page)
+    ints = lambda x: torch.as_tensor(x, dtype=torch.int32).cuda()  # noqa: E731
+    table = torch.randperm(len(lengths) * blocks, generator=generator).view(len(lengths), blocks)
+    pages = torch.randn(len(lengths) * blocks, page, groups, 24, generator=generator).to(dtype)
+    columns = max(c + n for c, n in zip(contexts, lengths)) // pool + 1
+    means = torch.full((len(lengths) * columns, 1, groups, 24), float("nan"), dtype=dtype, device="cuda")   # a block a page
+    pool_table = torch.arange(means.shape[0]).view(len(lengths), columns)
+    status = ints([0])
+    ops.pooled_means(pages.cuda(), means, segment_length=ints(lengths), segment_context=ints(contexts), block_table=ints(table), pool_table=ints(pool_table), segments=len(lengths),
+                     max_length=max(lengths), num_groups=groups, head_dim=16, value_dim=8, pool=pool, status=status)
+    assert int(status.item()) == 0
+    written = torch.zeros(means.shape[0], dtype=torch.bool)
+    for i, (n, c) in enumerate(zip(lengths, contexts)):
+        rows = pages[table[i]].reshape(blocks * page, groups, 24).double()
+        for block in range(c // pool, (c + n) // pool):
+            written[pool_table[i, block]] = True
+            want = rows[block * pool : (block + 1) * pool].mean(0)
+            # `pool` additions in 32-bit of values of size one, and the rounding of the mean: half of the last of bfloat16's eight bits
+            bound = pool * 2.0 ** -24 * 4 + (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -24) * want.abs().max()
+            assert float((means[pool_table[i, block], 0].double().cpu() - want).abs().max()) <= bound
+    assert written.sum() >= 3 and bool(means[~written.cuda()].isnan().all())
