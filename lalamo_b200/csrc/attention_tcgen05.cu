@@ -50,18 +50,17 @@ struct TaParams {
     int* status;
 };
 
-// VD: channels of a value head.
-template <int VD>
+constexpr int kTaValues = 128;     // channels of a value head in the kernel with a thread a row
+
 struct TaShared {
     static constexpr int kQBytes = kTaRows * kTaChannels * 2;          // 16 KB
     static constexpr int kPBytes = kTaRows * kTaKeys * 2;              // 16 KB
     static constexpr int kKeyBytes = kTaKeys * kTaChannels * 2;        // 8 KB: four boxes of 16 rows
-    static constexpr int kValueBox = VD * 32;                          // VD channels x 16 keys
+    static constexpr int kValueBox = kTaValues * 32;                   // kTaValues channels x 16 keys
     static constexpr int kValueBytes = 4 * kValueBox;
     static constexpr int kStageBytes = kKeyBytes + kValueBytes;
     static constexpr int kBytes = kQBytes + kPBytes + 2 * kStageBytes + 1024 /* alignment */ + 256 /* barriers */;
-    static constexpr int kColumns = kTaKeys + VD <= 128 ? 128 : 256;   // of tensor memory: scores, output
-    static constexpr int kCtasPerSm = VD == 64 ? 3 : 2;
+    static constexpr int kColumns = 256;   // of tensor memory: scores, output
 };
 
 __device__ __forceinline__ void tma_load_3d(void* destination, const CUtensorMap* map, int x, int y, int z, uint64_t* barrier) {
@@ -97,11 +96,10 @@ __device__ __forceinline__ float exp2_hardware(float x) {
 }
 
 // grid (tile records x K/V heads, 1, parts of a record), 192 threads: the records with most keys, of all heads, start first.
-template <int VD>
-__global__ void __launch_bounds__(kTaThreads, TaShared<VD>::kCtasPerSm)   // several CTAs per SM: one's softmax runs under the others' products
+__global__ void __launch_bounds__(kTaThreads, 2)   // two CTAs per SM: one's softmax runs under the other's products
 attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                          const TaParams p) {
-    using Shared = TaShared<VD>;
+    using Shared = TaShared;
     extern __shared__ unsigned char raw_shared[];
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(raw_shared) + 1023) & ~static_cast<uintptr_t>(1023));
     unsigned char* q_tile = base;
@@ -227,9 +225,9 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         }
         if (__any_sync(0xffffffffu, bad) && lane == 0) report_error(p.status, kBadPage);
     } else if (warp == 1 && lane == 0) {
-        // Product issuer.  It waits parked: three CTAs' issuers polling on one scheduler took the ALU
-        // slots of the softmax warps there, and every tile waits for its slowest softmax warp.
-        constexpr uint32_t idesc_scores = instruction_descriptor<kTaKeys>(), idesc_output = instruction_descriptor<VD>();   // N = 64 keys; VD channels
+        // Product issuer.  It waits parked: CTAs' issuers polling on one scheduler take the ALU slots
+        // of the softmax warps there, and every tile waits for its slowest softmax warp.
+        constexpr uint32_t idesc_scores = instruction_descriptor<kTaKeys>(), idesc_output = instruction_descriptor<kTaValues>();   // N = 64 keys; 128 channels
         bool ok = barrier_wait(q_full, 0);
         if (!ok) atomicExch(&failed, 1);
         const uint64_t desc_q = tile_descriptor(q_tile), desc_p = tile_descriptor(p_tile);
@@ -286,8 +284,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         float reference = -INFINITY, row_sum = 0.0f;
         bool ok = true;
         // The warp's lanes leave the loop together or not at all: what follows a wait is warp-wide.
-        // One lane waits, parked in hardware: with three CTAs on an SM a warp waits for nearly half of
-        // the time, and polling warps took the ALU slots that the other CTAs' softmax needed.
+        // They wait parked in hardware: polling warps would take the ALU slots that the other CTA's softmax needs.
         auto wait_together = [](uint64_t* barrier, uint32_t parity) {
             // every lane waits on the same barrier (one instruction per warp, as for one lane; no exchange after it)
             return __all_sync(0xffffffffu, barrier_wait_parked(barrier, parity));
@@ -303,7 +300,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             // Only tiles that reach past some token's own position, or before some token's window, need masks.
             const bool needs_mask = key0 + kTaKeys - 1 > first_position || (p.window > 0 && key0 < last_position - p.window + 1);
             // The row is read twice, 32 scores at a time (once for its maximum, once for its terms): a
-            // thread then needs half the registers, and three CTAs fit an SM.  Both passes exist with and
+            // thread then needs half the registers.  Both passes exist with and
             // without the mask, chosen by one branch per tile: with the test inside the loops the mask's
             // comparisons ran for every score of every tile, and the ALU pipe was the kernel's limit.
             float tops[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
@@ -347,7 +344,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 if (__any_sync(0xffffffffu, rescale != 1.0f)) {
 #pragma unroll
-                    for (int half = 0; half < VD / 32; ++half) {
+                    for (int half = 0; half < kTaValues / 32; ++half) {
                         uint32_t held[32];
                         tmem_load_32(tmem_output + lane_field + 32 * half, held);
 #pragma unroll
@@ -419,14 +416,14 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             if (needs_mask) {
                 // Keys outside [first visible, last position] of the tile hold whatever was left in the page,
                 // or were not loaded at all: clear their values, since a zero probability does not silence
-                // a non-finite value in the product.  VD channels x 64 keys, 128 / VD threads per channel.
+                // a non-finite value in the product.  128 channels x 64 keys, a thread per channel.
                 if (!wait_together(&v_full[s], (tile >> 1) & 1)) {
                     ok = false;
                     break;
                 }
                 unsigned char* values = stages + s * Shared::kStageBytes + Shared::kKeyBytes;
-                constexpr int kKeysHere = kTaKeys * VD / kTaRows;
-                const int channel = row % VD, key_part = row / VD;
+                constexpr int kKeysHere = kTaKeys * kTaValues / kTaRows;
+                const int channel = row % kTaValues, key_part = row / kTaValues;
                 for (int i = 0; i < kKeysHere; ++i) {
                     const int local_key = kKeysHere * key_part + i, key = key0 + local_key;
                     if ((key < first_visible && key >= p.keep_first) || key > last_position) {
@@ -446,9 +443,9 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         if (!ok) atomicExch(&failed, 1);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const float inverse = row_sum > 0.0f ? 1.0f / row_sum : 0.0f;
-        const size_t out_row = (static_cast<size_t>(first_token + token_local) * p.num_heads + group * heads_per_group + head_local) * VD;
+        const size_t out_row = (static_cast<size_t>(first_token + token_local) * p.num_heads + group * heads_per_group + head_local) * kTaValues;
 #pragma unroll
-        for (int half = 0; half < VD / 32; ++half) {
+        for (int half = 0; half < kTaValues / 32; ++half) {
             uint32_t held[32];
             tmem_load_32(tmem_output + lane_field + 32 * half, held);
             if (valid_row && ok) {
@@ -936,9 +933,9 @@ int lb_attention_prefill_tcgen05(const void* q, const void* k_pages, const void*
     const unsigned parts = static_cast<unsigned>((lb::kTaTileTokens + p.tokens_per_cta - 1) / p.tokens_per_cta);
     if (value_dim == 128) {
         static lb::OncePerDevice configured;
-        if (lb::allow_shared_memory(configured, lb::attention_tcgen05_kernel<128>, lb::TaShared<128>::kBytes) != cudaSuccess) return static_cast<int>(cudaGetLastError());
-        return static_cast<int>(lb::launch_overlapped(lb::attention_tcgen05_kernel<128>, dim3(static_cast<unsigned>(num_tiles) * num_groups, 1, parts), dim3(lb::kTaThreads),
-                                                      lb::TaShared<128>::kBytes, stream, map_q, map_k, map_v, p));
+        if (lb::allow_shared_memory(configured, lb::attention_tcgen05_kernel, lb::TaShared::kBytes) != cudaSuccess) return static_cast<int>(cudaGetLastError());
+        return static_cast<int>(lb::launch_overlapped(lb::attention_tcgen05_kernel, dim3(static_cast<unsigned>(num_tiles) * num_groups, 1, parts), dim3(lb::kTaThreads),
+                                                      lb::TaShared::kBytes, stream, map_q, map_k, map_v, p));
     }
     static lb::OncePerDevice configured, configured_paired;
     if (lb::allow_shared_memory(configured, lb::attention_tcgen05_halves_kernel<false>, lb::kThBytes) != cudaSuccess ||

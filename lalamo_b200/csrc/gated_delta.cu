@@ -490,7 +490,7 @@ gdr_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, const 
 
 // grid (tokens, slices of the heads), a warp per head: out[t, h, :] = T(o / sqrt(mean(o^2) + eps) * w * sigmoid(gate[t, h, :]));
 // without gates (ag null) the last factor is left out.  FOURS: rows that come in fours, on addresses that do, of at most 128 channels: a lane has
-// four neighbours, and a row and its gates are on their way together (2,048 tokens of 8 heads of 128: see below 12 us without).
+// four neighbours, and a row and its gates are on their way together (2,048 tokens of 8 heads of 128 5.9 us, 11.0 a channel at a time).
 template <typename T, bool FOURS>
 __global__ void gdr_output_kernel(const float* __restrict__ o, const T* __restrict__ ag, int ag_width, int gate_offset,
                                   const float* __restrict__ norm_weight, T* __restrict__ out, int heads, int dv, float eps, int gate_silu) {

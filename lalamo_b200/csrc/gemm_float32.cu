@@ -153,7 +153,7 @@ extern "C" {
 // out [m, n] = x [m, k] w [n, k]^T in float32; rows of x x_stride elements apart.  k and x_stride multiples of 4, x and w 16-byte aligned: -2 otherwise.
 // slices: CTAs of a cluster that share out k (1, 2, 4 or 8), 0: chosen by the sizes.  Measured, ours and cuBLAS: 8 x 2048 x 1024 8 and 19 us, 20 x 2048 x 2048 15 and 37,
 // 64 x 1024 x 4608 37 and 70, 300 x 1024 x 1024 24 and 31, 300 x 2048 x 1024 42 and 47; one row 7 and 5, 256 x 16384 x 2048 383 and 311 (its larger tiles
-// do 78 % of the multiply-adds' rate, these 54 %).  Errors against 64 bits 2.1e-7 and 5.7e-7 (1,024 columns).
+// do 78 % of the multiply-adds' rate, these 54 %).  Errors against 64 bits 2.1e-7 and 5.7e-7 (1,024 columns).  Which sizes come here: ops.float32_product_supported.
 int lb_gemm_float32(const float* x, const float* w, float* out, int m, int n, int k, int x_stride, int slices, cudaStream_t stream) {
     if (m == 0 || n == 0) return 0;
     if (m < 1 || n < 1 || k < 4 || k % 4 != 0 || x_stride < k || x_stride % 4 != 0 || (slices != 0 && slices != 1 && slices != 2 && slices != 4 && slices != 8) ||

@@ -324,7 +324,9 @@ moe_gather_kernel(const uint4* __restrict__ x, const int* __restrict__ offsets, 
 }
 
 // Both at once for up to kMoeArrangePairs pairs: a block a pair, which counts the pairs before its own in the order of the experts (and, of one expert, of the
-// pairs), leaves its place and copies its row; one more block makes the offsets.  8 tokens of 4 experts: one launch of 4 us for two of 3 and 4.
+// pairs), leaves its place and copies its row; one more block makes the offsets.  8 tokens of 4 experts: one launch of 4 us for two of 3 and 4.  Every block reads all
+// pairs, work that grows with their square.  Both products with two launches and with one, 16 experts of 1024 x 1152 and 64 of 1024 x 512: 32 pairs 34.3 and 32.8 us, 30.6 and
+// 27.9; 512 43.6 and 43.0, 54.4 and 52.6; 1,024 45.5 and 45.3, 57.5 and 55.8; 2,048 61.9 and 62.5, 62.4 and 62.1; 4,096 82.9 and 90.3, 73.0 and 79.4.
 constexpr int kMoeArrangePairs = 1024;
 __global__ void __launch_bounds__(128)
 moe_arrange_kernel(const uint4* __restrict__ x, const int* __restrict__ chosen, int pairs, int experts, int top, int pieces, int* __restrict__ offsets, int* __restrict__ sorted,
