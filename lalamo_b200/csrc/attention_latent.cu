@@ -633,6 +633,7 @@ struct HeadsProductParams {
 template <bool B_KN>
 __global__ void __launch_bounds__(128)
 heads_product_kernel(HeadsProductParams p) {
+    wait_for_previous_kernel();
     allow_next_kernel();
     extern __shared__ __align__(16) unsigned char product_shared[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, head = blockIdx.y, token0 = blockIdx.x * 64;
@@ -851,10 +852,7 @@ int lb_heads_product(const void* a, long long a_token_stride, int a_head_stride,
     p.n = n;
     p.blocks_per_cta = blocks_per_cta;
     const dim3 grid(token_blocks, heads, (column_blocks + blocks_per_cta - 1) / blocks_per_cta);
-    // (no early start, see launch_early_if: layers of 600 tokens 64.4 us with one and 59.6 without, of 256 that decode 53.7 and 50.6, of 8 the same)
-    auto kernel = b_is_kn ? lb::heads_product_kernel<true> : lb::heads_product_kernel<false>;
-    kernel<<<grid, 128, shared, stream>>>(p);
-    return LB_LAUNCH_RESULT();
+    return static_cast<int>(lb::launch_overlapped(b_is_kn ? lb::heads_product_kernel<true> : lb::heads_product_kernel<false>, grid, dim3(128), shared, stream, p));
 }
 
 int lb_gate_heads(const void* values, const void* gate, int gate_stride, void* out, int tokens, int num_heads, int value_dim, int dtype,
