@@ -177,6 +177,7 @@ __global__ void qk_norm_rope_write_token_kernel(const T* __restrict__ qkv, T* __
                                                 const int* __restrict__ positions, const int* __restrict__ token_segment,
                                                 const int* __restrict__ block_table, PagedLayout layout, int num_heads,
                                                 int write_kv, const float* __restrict__ bias, int* status, RewriteExtras extra) {
+    wait_for_previous_kernel();
     allow_next_kernel();
     extern __shared__ float rotation[];   // cos[half], sin[half]
     const int token = blockIdx.x;
@@ -385,6 +386,7 @@ __global__ void qk_norm_rope_write_run_kernel(const __nv_bfloat16* __restrict__ 
                                               const int* __restrict__ positions, const int* __restrict__ token_segment,
                                               const int* __restrict__ block_table, PagedLayout layout, int num_heads, int write_kv,
                                               int tokens, const float* __restrict__ bias, int* status, RewriteExtras extra) {
+    wait_for_previous_kernel();
     allow_next_kernel();
     static_assert(RUN == 4 || RUN == 8, "a channel's rows leave as one 8- or 16-byte store");
     using T = __nv_bfloat16;
@@ -1022,8 +1024,8 @@ int lb_qk_norm_rope_write(const void* qkv, void* q_out, void* k_pages, void* v_p
                           const int* positions, const int* token_segment, const int* block_table, int tokens,
                           int num_heads, int num_groups, int head_dim, int page_size, int num_pages, int max_blocks,
                           int write_kv, int dtype, int* status, cudaStream_t stream, int value_dim, const float* bias, float* row_inv,
-                          float turn_scale, int row_stride, int value_groups, float temperature, int temperature_every) {
-    // value_groups (0: num_groups): value heads, a divisor of the key heads; temperature, temperature_every: see RewriteExtras; write_kv 0:
+                          float turn_scale, int row_stride, int value_groups, float temperature, int temperature_every, int requests) {
+    // requests: whose tokens these are (rows of the block table); value_groups (0: num_groups): value heads, a divisor of the key heads; temperature, temperature_every: see RewriteExtras; write_kv 0:
     // qkv needs no more columns than the queries'.
     // row_inv: scratch [tokens][2] for a norm over the whole q and the whole k projection (null: the norm is per head);
     // turn_scale: a factor on sines and cosines; row_stride: elements between qkv's rows (0: the q, k and v columns).
@@ -1044,9 +1046,9 @@ int lb_qk_norm_rope_write(const void* qkv, void* q_out, void* k_pages, void* v_p
         })
     }
     lb::PagedLayout layout{page_size, num_pages, max_blocks, num_groups, head_dim, value_dim, value_groups};
-    // A block a token starts early (see launch_early_if) while every block finds a multiprocessor of its own; runs of tokens and the 32-bit path's larger blocks never do.
-    // Layers of 16 heads over 8 behind 1,000, early and not: 100 tokens 35.6 and 38.0 us, 128 36.2 and 39.0, 144 37.5 and 36.9, 200 40.9 and 36.4, 1,024 58.0 and 55.1; 16
-    // prompts of 64 tokens 40.4 and 33.9.
+    // A block a token starts early (see launch_early_if) while every block finds a multiprocessor of its own, runs of tokens where they are one request's: layers of 16 heads
+    // over 8, early and not, 100 tokens behind 1,000 38.0 and 42.4 us, 144 39.1 and 39.5, 200 42.7 and 39.3, 300 46.7 and 42.5; 2,048 69.6 and 70.6, 1,024 46.6 and 45.4, but two
+    // requests' 500 tokens each 49.9 and 44.4, five of 300 52.8 and 46.6 (their last tiles, which see the most keys, then share multiprocessors).
     const bool early = tokens <= lb::multiprocessor_count();
     const bool plain_layout = value_dim == head_dim && value_groups == num_groups && temperature_every == 0;   // what the 16-byte kernels below take
     const bool power_of_two_head = head_dim == 16 || head_dim == 32 || head_dim == 64 || head_dim == 128;
@@ -1058,9 +1060,9 @@ int lb_qk_norm_rope_write(const void* qkv, void* q_out, void* k_pages, void* v_p
         const auto q16 = static_cast<__nv_bfloat16*>(q_out), k16 = static_cast<__nv_bfloat16*>(k_pages), v16 = static_cast<__nv_bfloat16*>(v_pages);
         if (tokens >= lb::kRunKernelMinTokens) {
             constexpr int kRun = 4;
-            lb::qk_norm_rope_write_run_kernel<kRun><<<(tokens + kRun - 1) / kRun, vector_threads, kRun * shared, stream>>>(
-                static_cast<const __nv_bfloat16*>(qkv), q16, k16, v16, q_weight, k_weight, eps, scale_offset, inv_freq, rotary_dim, positions, token_segment, block_table, layout,
-                num_heads, write_kv, tokens, bias, status, extra);
+            lb::launch_early_if(requests == 1, lb::qk_norm_rope_write_run_kernel<kRun>, dim3((tokens + kRun - 1) / kRun), dim3(vector_threads), kRun * shared, stream,
+                                static_cast<const __nv_bfloat16*>(qkv), q16, k16, v16, q_weight, k_weight, eps, scale_offset, inv_freq, rotary_dim, positions, token_segment,
+                                block_table, layout, num_heads, write_kv, tokens, bias, status, extra);
             return LB_LAUNCH_RESULT();
         }
         lb::launch_early_if(early, lb::qk_norm_rope_write_vector_kernel, dim3(tokens), dim3(vector_threads), shared, stream, static_cast<const __nv_bfloat16*>(qkv), q16, k16, v16,
@@ -1075,8 +1077,8 @@ int lb_qk_norm_rope_write(const void* qkv, void* q_out, void* k_pages, void* v_p
         const size_t shared = static_cast<size_t>(rotary_dim > 0 ? rotary_dim : 2) * sizeof(float);
         const auto q16 = static_cast<__nv_bfloat16*>(q_out), k16 = static_cast<__nv_bfloat16*>(k_pages), v16 = static_cast<__nv_bfloat16*>(v_pages);
         if (tokens >= lb::kRunKernelMinTokens)
-            lb::rewrite_pieces_kernel<4><<<(tokens + 3) / 4, threads, 4 * shared, stream>>>(
-                static_cast<const __nv_bfloat16*>(qkv), q16, k16, v16, inv_freq, rotary_dim, positions, token_segment, block_table, layout, num_heads, write_kv, tokens, status, extra);
+            lb::launch_early_if(requests == 1, lb::rewrite_pieces_kernel<4>, dim3((tokens + 3) / 4), dim3(threads), 4 * shared, stream, static_cast<const __nv_bfloat16*>(qkv), q16, k16,
+                                v16, inv_freq, rotary_dim, positions, token_segment, block_table, layout, num_heads, write_kv, tokens, status, extra);
         else
             lb::launch_early_if(early, lb::rewrite_pieces_kernel<1>, dim3(tokens), dim3(threads), shared, stream, static_cast<const __nv_bfloat16*>(qkv), q16, k16, v16, inv_freq,
                                 rotary_dim, positions, token_segment, block_table, layout, num_heads, write_kv, tokens, status, extra);
@@ -1086,9 +1088,9 @@ int lb_qk_norm_rope_write(const void* qkv, void* q_out, void* k_pages, void* v_p
         // Many tokens: one block per token, the rotation computed once for all of its heads.
         const size_t shared = static_cast<size_t>(rotary_dim > 0 ? rotary_dim : 2) * sizeof(float);
         LB_DISPATCH_DTYPE(dtype, {
-            lb::qk_norm_rope_write_token_kernel<T><<<dim3(tokens, (num_heads + num_groups + lb::kTokenKernelUnits - 1) / lb::kTokenKernelUnits), 128, shared, stream>>>(
-                static_cast<const T*>(qkv), static_cast<T*>(q_out), static_cast<T*>(k_pages), static_cast<T*>(v_pages), q_weight, k_weight, eps, scale_offset, inv_freq, rotary_dim,
-                positions, token_segment, block_table, layout, num_heads, write_kv, bias, status, extra);
+            lb::launch_overlapped(lb::qk_norm_rope_write_token_kernel<T>, dim3(tokens, (num_heads + num_groups + lb::kTokenKernelUnits - 1) / lb::kTokenKernelUnits), dim3(128), shared,
+                                  stream, static_cast<const T*>(qkv), static_cast<T*>(q_out), static_cast<T*>(k_pages), static_cast<T*>(v_pages), q_weight, k_weight, eps, scale_offset,
+                                  inv_freq, rotary_dim, positions, token_segment, block_table, layout, num_heads, write_kv, bias, status, extra);
         })
         return LB_LAUNCH_RESULT();
     }

@@ -588,16 +588,16 @@ int lb_gdr_conv_state(const void* proj, int proj_width, void* conv_state, const 
 
 // segment_list (may be null): the portions to run, `segments` of them.
 // beta null: the plain linear recurrence (no delta rule).
-// single_tokens: every portion of the step is one token, and the scan starts early (see launch_early_if).  Longer ones: five portions of 100 tokens or less, 128
-// key channels, a layer of the delta rule 116 us with an early start and 96 without, of linear attention 98 and 79; three of 250 176 and 150, 155 and 130.
+// few_tokens: the scan's work is short and it starts early (see launch_early_if).  Layers of linear attention with 128 key channels, with an early start and without: 64 single
+// tokens 94 and 95.5 us, 64 portions of two 102 and 103, one of 17 30.6 and 32.2, of 48 44.2 and 44.1; five of 20 51 and 48, of 100 105 and 85, one of 130 103 and 70.
 int lb_gdr_scan(const float* q, const float* k, const float* g, const float* v, const float* beta, float* state, float* out,
                 const int* segment_start, const int* segment_length, const int* segment_slot, int segments, int heads, int groups, int dk, int dv,
-                int num_slots, int* status, cudaStream_t stream, const int* segment_list, int single_tokens) {
+                int num_slots, int* status, cudaStream_t stream, const int* segment_list, int few_tokens) {
     if (segments == 0) return 0;
     if (dk < 1 || dk > 256 || dv < 1 || heads % groups != 0) return -2;
     const dim3 grid(segments, heads, (dv + lb::kScanCols - 1) / lb::kScanCols);
     auto launch = dk <= 32 ? lb::launch_scan<32, 4> : dk <= 64 ? lb::launch_scan<64, 8> : dk <= 128 ? lb::launch_scan<128, 16> : lb::launch_scan<256, 32>;
-    return launch(grid, stream, q, k, g, v, beta, state, out, segment_start, segment_length, segment_slot, heads, groups, dk, dv, num_slots, status, segment_list, single_tokens != 0);
+    return launch(grid, stream, q, k, g, v, beta, state, out, segment_start, segment_length, segment_slot, heads, groups, dk, dv, num_slots, status, segment_list, few_tokens != 0);
 }
 
 int lb_gdr_output(const float* o, const void* ag, int ag_width, int gate_offset, const float* norm_weight, void* out, int tokens, int heads, int dv,

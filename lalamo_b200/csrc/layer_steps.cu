@@ -12,7 +12,7 @@ int lb_gemm_skinny(const void* x, const void* w, void* out, int tokens, int k, i
 int lb_qk_norm_rope_write(const void* qkv, void* q_out, void* k_pages, void* v_pages, const float* q_weight, const float* k_weight, float eps, float scale_offset,
                           const float* inv_freq, int rotary_dim, const int* positions, const int* token_segment, const int* block_table, int tokens, int num_heads,
                           int num_groups, int head_dim, int page_size, int num_pages, int max_blocks, int write_kv, int dtype, int* status, cudaStream_t stream,
-                          int value_dim, const float* bias, float* row_inv, float turn_scale, int row_stride, int value_groups, float temperature, int temperature_every);
+                          int value_dim, const float* bias, float* row_inv, float turn_scale, int row_stride, int value_groups, float temperature, int temperature_every, int requests);
 int lb_attention_decode(const void* q, const void* k_pages, const void* v_pages, void* out, float* scratch, const int* positions, const int* token_segment,
                         const int* block_table, const int* token_list, int tokens, int num_heads, int num_groups, int head_dim, int page_size, int num_pages, int max_blocks,
                         float scale, int window, int splits, int blocks_per_split, int fresh_keys, int* status, cudaStream_t stream, int keep_first, int value_dim,
@@ -72,7 +72,7 @@ int lb_attention_step(const void* x, const void* qkv_weight, const void* out_wei
     if (code != 0) return code;
     code = lb_qk_norm_rope_write(work, queries, k_pages, v_pages, q_norm, k_norm, eps, scale_offset, inv_freq, rotary_dim, positions, token_segment, block_table, tokens, num_heads,
                                  num_groups, head_dim, page_size, num_pages, max_blocks, write_kv, lb::kBFloat16, status, stream, head_dim, nullptr, nullptr, turn_scale, qkv_width,
-                                 num_groups, temperature, temperature_every);
+                                 num_groups, temperature, temperature_every, tokens);
     if (code != 0) return code;
     code = lb_attention_decode(queries, k_pages, v_pages, mixed, reinterpret_cast<float*>(memory + scratch_at), positions, token_segment, block_table, nullptr, tokens, num_heads,
                                num_groups, head_dim, page_size, num_pages, max_blocks, scale, window, splits, blocks_per_split, fresh_keys, status, stream, keep_first, head_dim,

@@ -235,6 +235,8 @@ __global__ void __launch_bounds__(kBlockThreads, DKP <= 128 ? 3 : 1)
 recurrent_prepare_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ g, const float* __restrict__ v,
                          const float* __restrict__ beta, float* __restrict__ pack, float* __restrict__ vpack, const int* __restrict__ long_table, int long_portions, const int* __restrict__ segment_start,
                 const int* __restrict__ segment_length, int heads, int groups, int dk, int dv, int window) {
+    wait_for_previous_kernel();
+    allow_next_kernel();
     using Pack = BlockPack<DKP>;
     using Shared = PrepareShared<DKP>;
     constexpr int P = Shared::kPitch, VP = Shared::kValuePitch, TP = kTrianglePitch;
@@ -431,7 +433,8 @@ __global__ void __launch_bounds__(kBlockThreads, DKP <= 64 ? 2 : 1)
 recurrent_walk_kernel(const float* __restrict__ pack, const float* __restrict__ vpack, float* __restrict__ state, float* __restrict__ out,
                       const int* __restrict__ long_table, const int* __restrict__ segment_start, const int* __restrict__ segment_length,
                       const int* __restrict__ segment_slot, int heads, int dk, int dv, int num_slots, int* status, int window, int window_blocks) {
-    allow_next_kernel();   // the output's, whose blocks are short
+    wait_for_previous_kernel();
+    allow_next_kernel();
     using Pack = BlockPack<DKP>;
     using Shared = WalkShared<DKP>;
     constexpr int kStages = Shared::kStages;
@@ -594,6 +597,8 @@ linear_prepare_kernel(const float* __restrict__ q, const float* __restrict__ k, 
                       float* __restrict__ decays, float* __restrict__ out, const int* __restrict__ long_table, int long_portions, const int* __restrict__ segment_start,
                 const int* __restrict__ segment_length, int heads,
                       int groups, int dk, int dv, int window) {
+    wait_for_previous_kernel();
+    allow_next_kernel();
     constexpr int P = DKP + 4, VP = 132;
     extern __shared__ __align__(16) float prepare_memory[];
     float* k_s = prepare_memory;   // keys; then as between_halves wants them
@@ -695,6 +700,8 @@ __global__ void __launch_bounds__(kBlockThreads)
 linear_states_kernel(float* __restrict__ sums, const float* __restrict__ decays, float* __restrict__ state, const int* __restrict__ long_table,
                      const int* __restrict__ segment_length, const int* __restrict__ segment_slot, int heads, int dk, int dv, int num_slots, int* status,
                      int window, int window_blocks) {
+    wait_for_previous_kernel();
+    allow_next_kernel();
     const int portion = long_table[3 * blockIdx.x], offset = blocks_before(long_table, segment_length, blockIdx.x) - window;   // of its blocks' numbers
     const int first = max(0, -offset), blocks = min((segment_length[portion] + kBlockTokens - 1) / kBlockTokens, window_blocks - offset) - first;
     const int head = blockIdx.y, element = blockIdx.z * kBlockThreads + threadIdx.x, elements = dk * dv, slot = segment_slot[portion];
@@ -738,7 +745,8 @@ template <int DKP, bool VECTOR>
 __global__ void __launch_bounds__(kBlockThreads)
 linear_read_kernel(const float* __restrict__ q, const float* __restrict__ g, const float* __restrict__ states, float* __restrict__ out, const int* __restrict__ long_table, int long_portions, const int* __restrict__ segment_start,
                 const int* __restrict__ segment_length, int heads, int groups, int dk, int dv, int window) {
-    allow_next_kernel();   // the output's, whose blocks are short
+    wait_for_previous_kernel();
+    allow_next_kernel();
     constexpr int P = DKP + 4;
     extern __shared__ __align__(16) float prepare_memory[];
     float* q_s = prepare_memory;
@@ -833,23 +841,28 @@ template <int DKP>
 int launch_recurrent_blocks(const float* q, const float* k, const float* g, const float* v, const float* beta, float* pack, float* vpack, float* state, float* out,
                             int most_blocks, int window_blocks, const int* long_table, int long_portions, const int* segment_start,
                             const int* segment_length, const int* segment_slot, int heads, int groups, int dk, int dv, int num_slots, int* status, cudaStream_t stream) {
-    const dim3 blocks(window_blocks, heads);
-    // Launched the ordinary way: started early, their blocks share the multiprocessors that the kernel before leaves first.  Measured early and so, whole layers:
-    // the delta rule over 4,096 tokens of 64 key channels 339 and 262 us, over 700 96 and 81; linear attention, 128 key channels, over 300 86 and 68, over 700
-    // 105 and 87, over 2,048 160 and 160.
+    const dim3 blocks(window_blocks, heads), threads(kBlockThreads);
+    // Which of them start early (see launch_early_if), as measured with launches in a stream and in a recorded graph.  The walk, except where two CTAs share a multiprocessor and
+    // there are no more CTAs than multiprocessors: the delta rule over 4,096 tokens of 64 key channels 343 us with an early start and 271 without, 128 channels 369 and
+    // 371.  Linear attention's first and last kernel with more blocks than two to a multiprocessor (1,500 tokens of 128 key channels 133 and 137 us; 1,000 116 and 105,
+    // 300 90 and 75), the last with 64 key channels also where it has few (500 tokens 58.7 and 60.4; 850 74.7 and 72.3, the first without in all four).
+    const int sms = multiprocessor_count(), grid = window_blocks * heads;
+    cudaError_t error = cudaSuccess;
     if (beta != nullptr) {
         static OncePerDevice prepared, walked;
         auto prepare = recurrent_prepare_kernel<DKP>;
         auto walk = recurrent_walk_kernel<DKP>;
         if (allow_shared_memory(prepared, prepare, PrepareShared<DKP>::kBytes) != cudaSuccess) return static_cast<int>(cudaGetLastError());
         if (allow_shared_memory(walked, walk, WalkShared<DKP>::kBytes) != cudaSuccess) return static_cast<int>(cudaGetLastError());
-        for (int window = 0; window < most_blocks; window += window_blocks) {
-            prepare<<<blocks, kBlockThreads, PrepareShared<DKP>::kBytes, stream>>>(q, k, g, v, beta, pack, vpack, long_table, long_portions, segment_start, segment_length, heads,
-                                                                                   groups, dk, dv, window);
-            walk<<<dim3(long_portions, heads, (dv + kWalkCols - 1) / kWalkCols), kBlockThreads, WalkShared<DKP>::kBytes, stream>>>(
-                pack, vpack, state, out, long_table, segment_start, segment_length, segment_slot, heads, dk, dv, num_slots, status, window, window_blocks);
+        const bool walk_early = DKP > 64 || long_portions * heads * ((dv + kWalkCols - 1) / kWalkCols) > sms;
+        for (int window = 0; window < most_blocks && error == cudaSuccess; window += window_blocks) {
+            error = launch_overlapped(prepare, blocks, threads, PrepareShared<DKP>::kBytes, stream, q, k, g, v, beta, pack, vpack, long_table, long_portions, segment_start,
+                                      segment_length, heads, groups, dk, dv, window);
+            if (error == cudaSuccess)
+                error = launch_early_if(walk_early, walk, dim3(long_portions, heads, (dv + kWalkCols - 1) / kWalkCols), threads, WalkShared<DKP>::kBytes, stream, pack, vpack, state,
+                                        out, long_table, segment_start, segment_length, segment_slot, heads, dk, dv, num_slots, status, window, window_blocks);
         }
-        return static_cast<int>(cudaGetLastError());
+        return static_cast<int>(error != cudaSuccess ? error : cudaGetLastError());
     }
     static OncePerDevice prepared, read, read_any;
     auto prepare = linear_prepare_kernel<DKP>;
@@ -858,13 +871,18 @@ int launch_recurrent_blocks(const float* q, const float* k, const float* g, cons
     if (allow_shared_memory(prepared, prepare, prepare_bytes) != cudaSuccess) return static_cast<int>(cudaGetLastError());
     if (allow_shared_memory(dv % 4 == 0 ? read : read_any, read_out, read_bytes) != cudaSuccess) return static_cast<int>(cudaGetLastError());
     float* decays = pack + static_cast<size_t>(window_blocks) * heads * dk * dv;
-    for (int window = 0; window < most_blocks; window += window_blocks) {
-        prepare<<<blocks, kBlockThreads, prepare_bytes, stream>>>(q, k, g, v, pack, decays, out, long_table, long_portions, segment_start, segment_length, heads, groups, dk, dv, window);
-        linear_states_kernel<<<dim3(long_portions, heads, (dk * dv + kBlockThreads - 1) / kBlockThreads), kBlockThreads, 0, stream>>>(
-            pack, decays, state, long_table, segment_length, segment_slot, heads, dk, dv, num_slots, status, window, window_blocks);
-        read_out<<<blocks, kBlockThreads, read_bytes, stream>>>(q, g, pack, out, long_table, long_portions, segment_start, segment_length, heads, groups, dk, dv, window);
+    const bool prepare_early = grid > 2 * sms, read_early = grid > 2 * sms || (DKP <= 64 && 3 * grid <= 4 * sms);
+    for (int window = 0; window < most_blocks && error == cudaSuccess; window += window_blocks) {
+        error = launch_early_if(prepare_early, prepare, blocks, threads, prepare_bytes, stream, q, k, g, v, pack, decays, out, long_table, long_portions, segment_start, segment_length,
+                                heads, groups, dk, dv, window);
+        if (error == cudaSuccess)
+            error = launch_overlapped(linear_states_kernel, dim3(long_portions, heads, (dk * dv + kBlockThreads - 1) / kBlockThreads), threads, 0, stream, pack, decays, state,
+                                      long_table, segment_length, segment_slot, heads, dk, dv, num_slots, status, window, window_blocks);
+        if (error == cudaSuccess)
+            error = launch_early_if(read_early, read_out, blocks, threads, read_bytes, stream, q, g, pack, out, long_table, long_portions, segment_start, segment_length, heads, groups,
+                                    dk, dv, window);
     }
-    return static_cast<int>(cudaGetLastError());
+    return static_cast<int>(error != cudaSuccess ? error : cudaGetLastError());
 }
 
 }  // namespace lb

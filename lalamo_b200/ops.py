@@ -840,7 +840,7 @@ def qk_norm_rope_write(
         inv_freq, rotary_dim, positions, token_segment, block_table, tokens, num_heads,
         num_groups, head_dim, page_size, num_pages, max_blocks, 1 if write_kv else 0,
         dtype_code(qkv.dtype), status, _stream(), value_dim, bias, row_inv, turn_scale, qkv.stride(0),
-        value_groups or 0, temperature, temperature_every)
+        value_groups or 0, temperature, temperature_every, block_table.shape[0])
     _done(code, "qk_norm_rope_write", 2 if whole_norm and tokens > 64 else 1)   # few tokens: the statistic is computed in the rewrite itself
 
 
@@ -1265,7 +1265,7 @@ def _recurrence(q: torch.Tensor, k: torch.Tensor, decay: torch.Tensor, v: torch.
     if num_direct > 0:
         code = lib.lb_gdr_scan(q, k, decay, v, beta, matrix_state, read_out, segment_start, segment_length,
                                segment_slot, num_direct, num_heads, num_groups, key_dim, value_dim, num_slots,
-                               status, _stream(), direct_list, 1 if segments == tokens else 0)
+                               status, _stream(), direct_list, 1 if tokens <= max(64, 2 * segments) else 0)
         _done(code, "gdr_scan")
     return read_out
 
