@@ -2369,7 +2369,8 @@ def _watched(x: torch.Tensor, weight: torch.Tensor) -> bool:
 
 def _product(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     """``x @ weight.T`` where none of the bfloat16 kernels takes it: on the kernel of the 32-bit path, else by the library."""
-    if (x.dtype == torch.float32 and x.dim() == 2 and not _watched(x, weight) and float32_product_supported(x.shape[0], weight.shape[0], x.shape[1])
+    if (x.dtype == torch.float32 and x.dim() == 2 and x.is_cuda and not _watched(x, weight) and float32_product_supported(x.shape[0], weight.shape[0], x.shape[1])
+            and x.get_device() == weight.get_device() == torch.cuda.current_device()   # (torch's operator finds the device by itself, and refuses two)
             and x.stride(1) == 1 and x.stride(0) % 4 == 0 and x.stride(0) >= x.shape[1] and (x.data_ptr() | weight.data_ptr()) % 16 == 0):
         out = torch.empty(x.shape[0], weight.shape[0], dtype=torch.float32, device=x.device)
         _done(_lib().lb_gemm_float32(x, weight, out, x.shape[0], weight.shape[0], x.shape[1], x.stride(0), 0, _stream()), "gemm_float32")

@@ -15,10 +15,38 @@ class _NoLaunch:
 @pytest.fixture(autouse=True)
 def no_launch(monkeypatch):
     monkeypatch.setattr(ops, "_lib", lambda: _NoLaunch())
+    monkeypatch.setattr(ops, "_stream", lambda: 0)
     assert ops.float32_product_supported(8, 16, 512)
 
 
 X, W = torch.randn(8, 512, generator=torch.Generator().manual_seed(1)), torch.randn(16, 512, generator=torch.Generator().manual_seed(2))
+
+
+class _OnCuda(torch.Tensor):
+    """A tensor that says that it lies on a device of a certain number."""
+
+    is_cuda = True
+    device_number = 0
+
+    def get_device(self):
+        return self.device_number
+
+    @classmethod
+    def __torch_function__(cls, function, types, arguments=(), keywords=None):
+        with torch._C.DisableTorchFunctionSubclass():
+            return function(*arguments, **(keywords or {}))
+
+
+@pytest.mark.parametrize("x_device,weight_device", [(0, 1), (1, 1)])
+def test_devices(x_device, weight_device, monkeypatch):
+    """The kernel runs on the current device; torch's operator on the tensors' own, if it is one."""
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    x, weight = X.as_subclass(_OnCuda), W.as_subclass(_OnCuda)
+    x.device_number, weight.device_number = x_device, weight_device
+    assert torch.equal(ops._product(x, weight), X @ W.T)
+    x.device_number = weight.device_number = 0
+    with pytest.raises(AssertionError, match="launched"):
+        ops._product(x, weight)
 
 
 def test_forward_mode():
