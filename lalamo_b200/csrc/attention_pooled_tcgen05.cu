@@ -7,7 +7,8 @@
 //   warps 0-7  two threads a row, 32 scores each: there is no denominator, so that nothing is exchanged and nothing rescaled
 //   warp 8     allocates tensor memory; one lane issues O += P V of a tile, then S = Q K^T of the tile after next
 //   warp 9     asks for the boxes of the positions, and copies the pooled blocks
-// What bounds it: the transcendental unit.  Two CTAs share a multiprocessor, so that every warp finds scores to weigh.  Written out a weight takes four
+// What bounds it: the weighing warps' dependent instructions, with the transcendental unit as the busiest pipe (45 % of the time on average, issue slots 54 %).  Two
+// CTAs share a multiprocessor, so that every warp finds scores to weigh.  Written out a weight takes four
 // of its operations, tanh(x) = 1 - 2 / (1 + 2^(2 x log2 e)) and 1 / (1 + 2^-y); here a polynomial stands for the tanh where all of a thread's scores
 // are within half of the cap (else it is written out), and two weights share a reciprocal: three operations for two weights.  Measured, 16 heads over 4, a
 // window of 1,024 and blocks of 8: a prompt of 3,000 48 us (mma.sync 118 and 14 to add up two shares; 65 with the tiles of one head after the other's, which
