@@ -1571,11 +1571,11 @@ def latent_attention_tcgen05_supported(dtype: torch.dtype, latent: int, rope: in
             and 384 * 2 * (latent + rope) + 3328 <= 226 * 1024)
 
 
-def latent_attention_few_rows(num_items: int, longest: int, num_heads: int, max_context: int, sms: int | None = None) -> bool:
-    """Whether a step's items, each of at most ``longest`` tokens, see so few cached rows that the ``mma.sync`` kernel is the faster one: more items than multiprocessors,
+def latent_attention_few_rows(num_items: int, max_context: int, sms: int | None = None) -> bool:
+    """Whether a step's items see so few cached rows that the ``mma.sync`` kernel is the faster one, if its runs are long enough for them: more items than multiprocessors,
     of which that kernel runs several at a time on each.  Measured, it and the kernel on the fifth-generation tensor cores, 16 heads over 256 + 32 channels:
     200 tokens that decode behind 16 11 and 18 us, behind 64 14 and 17, behind 96 20 and 17; 512 behind 64 26 and 33, behind 96 39 and 33; 148 behind 16 11 and 10."""
-    return num_items > (sms or sm_count()) and max_context <= 64 and longest <= latent_attention_tiling(num_heads)[1]
+    return max_context <= 64 and num_items > (sms or sm_count())
 
 
 def latent_attention_tcgen05_splits(num_items: int, tokens: int, num_heads: int, window: int | None, max_context: int, sms: int | None = None) -> int:

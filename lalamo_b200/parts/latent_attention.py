@@ -171,12 +171,13 @@ class LatentAttention(Mixer):
         if ops.latent_attention_supported(runtime.dtype, latent, rope, cache.k_pages.shape[1]):
             lists, host_lists = step.plan_of(self)
             num_items = host_lists["items"].size // 2
-            longest = int(host_lists["items"][1::2].max()) if num_items else 0
-            double, tcgen05 = False, self.tcgen05 and not ops.latent_attention_few_rows(num_items, longest, heads, step.max_context)
+            run = ops.latent_attention_tiling(heads)[1]
+            longest = lambda: int(host_lists["items"][1::2].max()) if num_items else 0  # noqa: E731
+            double, tcgen05 = False, self.tcgen05 and not (ops.latent_attention_few_rows(num_items, step.max_context) and longest() <= run)
             if tcgen05:
                 splits = ops.latent_attention_tcgen05_splits(num_items, tokens, heads, spec.window, step.max_context)
             else:
-                double = longest > ops.latent_attention_tiling(heads)[1]
+                double = longest() > run
                 splits = ops.latent_attention_splits(num_items, heads, latent, spec.window, step.max_context, double=double)
             ops.latent_attention(queries, cache.k_pages, summed, items=lists["items"], num_items=num_items, splits=splits, double=double, tcgen05=tcgen05, **common)
         else:

@@ -50,3 +50,38 @@ def test_sizes_not_taken():
     assert not supported(torch.bfloat16, 256, 64, 16, 16, 0.1) and not supported(torch.bfloat16, 144, 32, 16, 16, 0.1) and not supported(torch.bfloat16, 256, 12, 16, 16, 0.1)
     assert not supported(torch.float32, 256, 32, 16, 16, 0.1) and not supported(torch.bfloat16, 256, 32, 8, 16, 0.1) and not supported(torch.bfloat16, 256, 32, 16, 65, 0.1)
     assert not supported(torch.bfloat16, 256, 32, 16, 16, 0.0) and not supported(torch.bfloat16, 256, 32, 16, 16, -0.1)
+
+
+@pytest.mark.parametrize("counts,few", [([1] * 200, True), ([4] * 150, True), ([1] * 140 + [5] * 20, False), ([1] * 100, False)])
+def test_which_kernel_a_layer_takes(counts, few, monkeypatch):
+    """More items than multiprocessors behind next to nothing go to the mma.sync kernel where its runs are long enough; both give the same layer."""
+    from lalamo_b200 import ops
+    from lalamo_b200.cache import CacheManager
+    from lalamo_b200.config import plan
+    from lalamo_b200.engine import StepEntry
+    from lalamo_b200.engine.executor import BatchBuilder
+    from lalamo_b200.parts import Runtime, build_part
+
+    heads, dim, rope, rank, width = 16, 64, 32, 256, 64
+    spec = plan.LatentAttentionSpec(model_dim=width, num_heads=heads, head_dim=dim, rope_dim=rope, value_dim=dim, latent_dim=rank, latent_norm=plan.RMSNormSpec(dim=rank, eps=1e-6, exact=True),
+                                    position=plan.RopeSpec(rotary_dim=rope, theta=10000.0), window=2048)
+    generator = torch.Generator().manual_seed(4)
+    matrix = lambda *shape: (torch.randn(*shape, generator=generator) * shape[1] ** -0.5).bfloat16().cuda()  # noqa: E731
+    tensors = {"q_proj": matrix(heads * (dim + rope), width), "down_proj": matrix(rank + rope, width), "latent_norm": torch.ones(rank).cuda(), "key_up_proj": matrix(heads * dim, rank),
+               "value_up_proj": matrix(heads * dim, rank), "out_proj": matrix(width, heads * dim)}
+    runtime = Runtime(device=torch.device("cuda:0"), dtype=torch.bfloat16)
+    part = build_part(spec, tensors, runtime)
+    cache = CacheManager([part.cache_need()], [None], runtime, page_size=16, num_pages=len(counts), num_slots=len(counts))
+    for i in range(len(counts)):
+        cache.admit(i)
+    built = BatchBuilder(cache, runtime.device, 100, planners=[part]).build([StepEntry(i, [0] * n) for i, n in enumerate(counts)])
+    view = cache.views(built.block_tables, built.inputs.segment_slot)[0]
+    x = torch.randn(sum(counts), width, generator=generator).bfloat16().cuda()
+    taken, real = [], ops.latent_attention
+    monkeypatch.setattr(ops, "latent_attention", lambda *arguments, **keywords: (taken.append(keywords["tcgen05"]), real(*arguments, **keywords)))
+    out = part.forward(x, built.inputs, view)
+    monkeypatch.setattr(ops, "latent_attention_few_rows", lambda *arguments: not few)
+    other = part.forward(x, built.inputs, view)
+    assert taken == ([False, True] if few else [True, max(counts) > 4]) and int(runtime.status.item()) == 0
+    # the weights' and the sums' roundings to bfloat16, of 2 ** -8 of a value each at most, and the layer's rounding
+    assert float((out.float() - other.float()).norm() / other.float().norm()) < 3 * 2 ** -8
